@@ -21,6 +21,7 @@
 #include "bm_triples.cuh"
 #include "bm_quads.cuh"
 #include "bm_select.cuh"
+#include "bm_commit.cuh"
 #include "bm_combine_tma.cuh"
 #include "bm_hub.cuh"
 #include "bm_hub_ws.cuh"
@@ -174,8 +175,8 @@ static void free_ctx(bm_ctx* c) {
     if (c->diagS) cudaFree(c->diagS);
     for (void* b : {(void*)c->hubs, (void*)c->is_hub, (void*)c->hubA, (void*)c->hubB, (void*)c->hub_err})
         if (b) cudaFree(b);
-    if (c->cinfo) cudaFree(c->cinfo);
-    if (c->cgrid) cudaFree(c->cgrid);
+    if (c->csets) cudaFree(c->csets);
+    if (c->cset) cudaFree(c->cset);
     for (void* b : {(void*)c->pS, (void*)c->pinvS, (void*)c->moved, (void*)c->minfo, (void*)c->mwork})
         if (b) cudaFree(b);
     if (c->ev_hub) cudaEventDestroy(c->ev_hub);
@@ -791,6 +792,56 @@ static bm_status ensure_adj(bm_ctx* ctx) {
     return BM_OK;
 }
 
+template <bool W16, int K>
+bm_status launch_set_commit(bm_ctx* ctx, const unsigned long long* keys, const int4* sets, int lim, int max_verify,
+                            int ctas, int stall) {
+    const int n = ctx->n;
+    constexpr size_t kCtl = 4;   // ints of the control words, rounded up to 16 bytes
+    static_assert(sizeof(SetCtl) <= kCtl * sizeof(int), "control words");
+    if (!ctx->cset) {
+        const size_t ints = kCtl + kSetBufInts + (size_t)n;
+        CK(dalloc(ctx, &ctx->cset, ints * sizeof(int)));
+        CK(cudaMemsetAsync(ctx->cset, 0, ints * sizeof(int), ctx->st));
+    } else {
+        CK(cudaMemsetAsync(ctx->cset, 0, kCtl * sizeof(int), ctx->st));
+    }
+    SetArgs a;
+    a.keys = keys; a.sets = sets; a.lim = lim; a.max_verify = max_verify; a.st = ctx->cstats;
+    a.ctl = reinterpret_cast<SetCtl*>(ctx->cset);
+    a.buf = ctx->cset + kCtl;
+    a.newp = a.buf + kSetBufInts;
+    a.stall = stall;
+    // a quarter of the list entries a step scans on average per CTA's thread:
+    // windows of hub pairs scan several times the average, and the grid
+    // barrier of 148 CTAs costs about 1 us more than that of 8 (n = 1,000 /
+    // E = 2e4: 16, 64 and 148 CTAs 113, 107 and 109 us; n = 18,524 / E = 5e6:
+    // 1,188, 682 and 627 us)
+    int grid = ctas;
+    if (grid <= 0) {
+        const double per_step = 2.0 * (double)ctx->e1 / n * K * kSetW;
+        grid = (int)std::min<double>(ctx->num_sms, std::max(8.0, per_step / 256));
+    }
+    grid = std::min(grid, ctx->num_sms);
+    const size_t smem = SetSmem<K>::bytes(n);
+    CK(cudaFuncSetAttribute(k_commit_sets<W16, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DevView<W16> g = view<W16>(ctx);
+    void* args[] = {&g, &a};
+    CK(cudaLaunchCooperativeKernel((const void*)k_commit_sets<W16, K>, dim3(grid), dim3(kSetThreads), args, smem,
+                                   ctx->st));
+    return BM_OK;
+}
+
+template bm_status launch_set_commit<true, 2>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
+template bm_status launch_set_commit<false, 2>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
+
+const int* set_commit_err(bm_ctx* ctx) { return &reinterpret_cast<SetCtl*>(ctx->cset)->err; }
+
+bm_status set_commit_reset(bm_ctx* ctx) {
+    CK(cudaMemsetAsync(ctx->cset, 0, (4 + kSetBufInts) * sizeof(int), ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));
+    return BM_OK;
+}
+
 template <bool W16>
 static bm_status stage_commit(bm_ctx* ctx, const bm_sweep_opts* o) {
     const int n = ctx->n;
@@ -802,32 +853,15 @@ static bm_status stage_commit(bm_ctx* ctx, const bm_sweep_opts* o) {
     const int max_scan = o ? o->max_candidates : 0;
     const int max_verify = o ? o->max_verify : -1;
     const int lim = (max_scan > 0 && max_scan < n) ? max_scan : n;
-    {   // G1 lists and offsets into L2 for the commit's scattered list reads
-        const size_t es = W16 ? 4 : 8;
-        k_prefetch_l2<<<ctx->num_sms * 4, 256, 0, ctx->st>>>((const char*)ctx->ent1o, (size_t)ctx->e1 * es);
-        k_prefetch_l2<<<ctx->num_sms * 4, 256, 0, ctx->st>>>((const char*)ctx->ent1i, (size_t)ctx->e1 * es);
-        k_prefetch_l2<<<ctx->num_sms, 256, 0, ctx->st>>>((const char*)ctx->off1o, (size_t)(n + 2) * sizeof(int));
-        k_prefetch_l2<<<ctx->num_sms, 256, 0, ctx->st>>>((const char*)ctx->off1i, (size_t)(n + 2) * sizeof(int));
-        CK(cudaGetLastError());
-    }
-    if (!ctx->cinfo) CK(dalloc(ctx, &ctx->cinfo, (size_t)n * 2 * sizeof(int4)));
-    k_cand_info<W16><<<(lim + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, lim, ctx->cinfo);
-    CK(cudaGetLastError());
     const size_t smem = commit_group_smem(n);
     if (smem + 4096 > ctx->smem_optin) {
         set_err(ctx, "set commit needs %zu bytes of shared memory for n=%d (limit %zu): n too large for a sweep",
                 smem, n, ctx->smem_optin);
         return BM_E_INPUT;
     }
-    int ctas = o && o->commit_ctas > 0 ? o->commit_ctas : kCommitDefaultCtas;
-    ctas = std::min(std::min(ctas, kCommitMaxCtas), ctx->num_sms);
-    if (!ctx->cgrid) {
-        CK(dalloc(ctx, &ctx->cgrid, commit_grid_ints() * sizeof(int)));
-        CK(cudaMemset(ctx->cgrid, 0, commit_grid_ints() * sizeof(int)));
-    }
-    CK(launch_commit_group<W16>(view<W16>(ctx), ctx->ckeys_sorted, lim, max_verify, ctx->cstats, ctx->cinfo, ctas,
-                                ctx->cgrid, smem, ctx->st, ctas > 1 ? take_stall(BM_STALL_COMMIT) : 0));
-    return BM_OK;
+    const int ctas = o && o->commit_ctas > 0 ? std::min(o->commit_ctas, kCommitMaxCtas) : 0;
+    return launch_set_commit<W16, 2>(ctx, ctx->ckeys_sorted, nullptr, lim, max_verify, ctas,
+                                     ctas != 1 ? take_stall(BM_STALL_COMMIT) : 0);
 }
 
 extern "C" bm_status bm_all_deltas(bm_ctx* ctx, int32_t* out) {
@@ -890,8 +924,7 @@ extern "C" bm_status bm_sweep(bm_ctx* ctx, const bm_sweep_opts* opts, bm_sweep_s
     CK(cudaMemcpyAsync(small, ctx->small, 3 * sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(&terms, ctx->work_sum, sizeof terms, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(&herr, ctx->hub_err, sizeof herr, cudaMemcpyDeviceToHost, ctx->st));
-    if (ctx->cgrid)
-        CK(cudaMemcpyAsync(&cerr, ctx->cgrid, sizeof cerr, cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&cerr, set_commit_err(ctx), sizeof cerr, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     if (herr || cerr) {
         // the matching may be partly committed and S is not trusted: the
@@ -899,9 +932,10 @@ extern "C" bm_status bm_sweep(bm_ctx* ctx, const bm_sweep_opts* opts, bm_sweep_s
         set_err(ctx, "bm_sweep: %s wait timed out",
                 (herr & (1 << kCmbErrBit)) ? "pair combine tile" : herr ? "tensor-core hub GEMM"
                                                                         : "set commit cluster barrier");
-        if (herr) CK(cudaMemset(ctx->hub_err, 0, sizeof(int)));
         ctx->mapped = false;
         ctx->S_exact = false;
+        if (herr) CK(cudaMemset(ctx->hub_err, 0, sizeof(int)));
+        if (cerr && (s = set_commit_reset(ctx))) return s;
         return BM_E_TIMEOUT;
     }
     ctx->score = before + cs.total_delta;

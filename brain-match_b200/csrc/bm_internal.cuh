@@ -47,8 +47,8 @@ struct bm_ctx {
     int* small = nullptr;          // [0]=row counter [1]=ncand [2]=best delta
     unsigned long long* score_acc = nullptr;
     CommitStats* cstats = nullptr;
-    int4* cinfo = nullptr;  // list extents of the sorted candidates (2 per candidate)
-    int* cgrid = nullptr;   // set commit across CTAs: partial sums [2][32][8][3], barrier [2], error [1]
+    int* cset = nullptr;    // set commit: control words, step results, images of moved vertices
+    int4* csets = nullptr;  // vertices and permutations of the sorted 3- and 4-set candidates
     // S kept exact across commits: the matching it is exact for, and the moved-vertex update
     bool S_exact = false;
     int *pS = nullptr, *pinvS = nullptr;  // n+1 entries each
@@ -142,3 +142,13 @@ template <bool W16> bm_status stage_profit(bm_ctx* ctx);
 // stage_profit.  *mode: 0 rebuilt, 1 updated, 2 already exact.
 template <bool W16> bm_status stage_refresh(bm_ctx* ctx, int* mode);
 bm_status stage_combine(bm_ctx* ctx, int* all_out);
+// Enqueues the set commit of the first lim sorted candidate keys (K = 2: pairs
+// in the keys; K = 3, 4: the sets in `sets`) on ctx's stream; statistics go to
+// ctx->cstats.  ctas <= 0: as many CTAs as the window's lists need.
+template <bool W16, int K>
+bm_status launch_set_commit(bm_ctx* ctx, const unsigned long long* keys, const int4* sets, int lim, int max_verify,
+                            int ctas, int stall);
+// Error word of the last set commit (device), and the clean-up after a wait of
+// it ran out.
+const int* set_commit_err(bm_ctx* ctx);
+bm_status set_commit_reset(bm_ctx* ctx);

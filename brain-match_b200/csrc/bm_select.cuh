@@ -6,9 +6,10 @@
 //   vertex of the tile, its best partner inside the tile to a partial array
 //   P[tile column][vertex]; k_best_reduce folds the partials into rowbest.
 //   No atomics; every (tile, vertex) slot is written exactly once.
-// k_commit_group: the sequential set commit (candidates sorted by delta desc,
-//   skip a pair whose vertex already moved, re-evaluate it on the current
-//   matching, commit iff > 0), several pairs per step.
+// commit_group: the sequential set commit of a batched instance by one CTA
+//   (candidates sorted by delta desc, skip a pair whose vertex already moved,
+//   re-evaluate it on the current matching, commit iff > 0), several pairs per
+//   step.  bm_commit.cuh has the set commit of a single instance.
 #pragma once
 #include <climits>
 #include "bm_kernels.cuh"
@@ -157,9 +158,7 @@ static __global__ void k_best_reduce(const unsigned long long* __restrict__ part
 // at its vertices and their G1 neighbours, so every decision equals the
 // one-at-a-time rule's, re-verification budget included, and no pair is
 // scanned twice.
-constexpr int kCG = 16;                // pairs per step of the cluster commit (16-bit vertex marks)
-constexpr int kCGWide = 32;            // ... when 32-bit marks fit in shared memory
-constexpr int kCGBatch = 8;            // pairs per step of a one-CTA commit (batched instances)
+constexpr int kCGBatch = 8;            // pairs per step (batched instances)
 
 // 16-bit atomic OR in shared memory through the aligned 32-bit word.
 __device__ __forceinline__ void atomicOr_u16(uint16_t* p, uint16_t v) {
@@ -168,83 +167,12 @@ __device__ __forceinline__ void atomicOr_u16(uint16_t* p, uint16_t v) {
     atomicOr(w, (unsigned)v << ((addr & 2) ? 16 : 0));
 }
 
-// Several CTAs on one set commit, as one thread-block cluster: every CTA keeps
-// the same shared state and makes the same gather and the same ordered
-// decisions; only the step's list scan is divided.  Each CTA publishes its
-// per-pair partial sums in its own shared memory (two buffers, by step
-// parity), arrives on every CTA's step mbarrier, waits on its own (bounded),
-// and reads the others' partials through distributed shared memory.
-struct CommitGrid {
-    int nct;          // CTAs of the cluster (1: a single CTA, no exchange)
-    int* err;         // bit 1 set when a cluster wait runs out
-    int stall = 0;    // test hook (bm_test_stall): no CTA arrives in the first exchange
-};
-
-__device__ __forceinline__ uint32_t cluster_map(uint32_t local_addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
-    return r;
-}
-
-// Arrive on the step mbarrier of every CTA of the cluster, then wait (bounded)
-// for this CTA's to complete the phase; false on timeout.  Thread 0 of each
-// CTA does the arrivals and the wait; the CTA syncs around it.
-//
-// A CTA whose wait runs out stays resident for one more full wait window
-// before it reports the timeout (and the caller leaves): a peer whose own wait
-// completed just then still reads this CTA's partial sums and arrives on its
-// mbarrier at the next step, and both must reach a CTA that has not exited.
-// That peer then times out at the next step in turn, so every CTA stops
-// within two steps.  `stall` (the test hook) skips this CTA's arrivals and
-// shortens both windows: when every CTA stalls, every wait runs out at the
-// same step and no CTA touches another's shared memory afterwards.
-__device__ __forceinline__ bool cluster_step_sync(uint32_t bar, uint32_t phase, int nct, int* err, bool stall = false) {
-    __shared__ int s_cok;
-    __syncthreads();
-    if (!stall && threadIdx.x < (unsigned)nct) {  // thread r arrives on CTA r's mbarrier
-        const uint32_t rb = cluster_map(bar, threadIdx.x);
-        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(rb) : "memory");
-    }
-    if (threadIdx.x == 0) {
-        const int limit = stall ? (1 << 12) : (1 << 22);
-        int ok = 0;
-        for (int it = 0; it < limit; it++) {
-            uint32_t done;
-            asm volatile(
-                "{\n\t.reg .pred p;\n\t"
-                "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-                "selp.u32 %0, 1, 0, p;\n\t}"
-                : "=r"(done) : "r"(bar), "r"(phase) : "memory");
-            if (done) { ok = 1; break; }
-        }
-        if (!ok) {
-            // the linger window: as many polls again, whatever they return
-            // (a poll suspends while the phase is open and returns at once
-            // after it completes, so this lasts at least milliseconds)
-            for (int it = 0; it < limit; it++)
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%0], %1;\n\t}"
-                    :: "r"(bar), "r"(phase) : "memory");
-            atomicOr(err, 2);
-        }
-        s_cok = ok;
-    }
-    __syncthreads();
-    return s_cok != 0;
-}
-
 // The set commit of one instance; all 1024 threads of the block call it.
 // smem: commit_group_smem(n) bytes of dynamic shared memory.
-// Per-vertex step marks: bit i = the vertex belongs to pair i of the step.
-template <int CG> struct MarkOf { typedef uint16_t T; };
-template <> struct MarkOf<32> { typedef uint32_t T; };
-
-template <bool W16, int CG = kCG>
+template <bool W16, int CG>
 __device__ __forceinline__ void commit_group(const DevView<W16>& g, const unsigned long long* __restrict__ keys,
                                              int lim, int max_verify, CommitStats* __restrict__ st,
-                                             unsigned char* smem, const int4* __restrict__ cinfo = nullptr,
-                                             CommitGrid grid = CommitGrid{1, nullptr}) {
+                                             unsigned char* smem) {
     typedef Ent<W16> EN;
     // shared: used[n] flags, then the matching and the pre-move images as
     // 16-bit ids (n <= 65535, so the "unmatched" value n fits)
@@ -252,8 +180,7 @@ __device__ __forceinline__ void commit_group(const DevView<W16>& g, const unsign
     unsigned char* used = smem;
     uint16_t* p16 = reinterpret_cast<uint16_t*>(smem + ((n + 15) & ~15));
     uint16_t* q16 = p16 + ((n + 8) & ~7);
-    typedef typename MarkOf<CG>::T MarkT;
-    MarkT* mark = reinterpret_cast<MarkT*>(q16 + ((n + 8) & ~7));  // bit i set: vertex belongs to pair i of the step
+    uint16_t* mark = q16 + ((n + 8) & ~7);  // bit i set: vertex belongs to pair i of the step
     __shared__ int s_lo[CG], s_hi[CG], s_d0[CG];
     __shared__ int s_corr[CG], s_cnt[CG], s_pre[CG + 1];
     __shared__ unsigned s_imask[CG];   // earlier pairs of the step G1-adjacent to this one
@@ -264,38 +191,12 @@ __device__ __forceinline__ void commit_group(const DevView<W16>& g, const unsign
     __shared__ int s_segoff[4 * CG];      // first entry of segment 4j + k in ent1o (k even) or ent1i (k odd)
     __shared__ int s_n, s_k, s_scanned;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int nct = grid.nct;
-    int ct = 0;
-    if (nct > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(ct));
-    int gstep = 0;      // steps taken, the same in every CTA
-    bool aborted = false;
-    __shared__ __align__(8) unsigned long long s_cbar;   // the step mbarrier (nct arrivals per phase)
-    constexpr int kPart = (3 + CG + 3) & ~3;            // a pair's partials, padded to whole 16-byte words
-    __shared__ __align__(16) int s_cpart[2][CG][kPart];  // this CTA's partial sums, by step parity
     __shared__ int s_cc[CG][CG];   // s_cc[j][i]: change of pair j's delta if earlier pair i commits
-    const uint32_t cbar = (uint32_t)__cvta_generic_to_shared(&s_cbar);
-    if (nct > 1) {
-        if (tid == 0) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(cbar), "r"(nct) : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-        // every CTA's mbarrier is initialised before anyone arrives on it
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    }
     for (int i = tid; i < n; i += blockDim.x) { used[i] = 0; p16[i] = (uint16_t)g.p[i]; mark[i] = 0; }
     for (int i = tid; i < CG * CG; i += blockDim.x) (&s_cc[0][0])[i] = 0;
     if (tid == 0) { s_n = 0; s_k = 0; s_scanned = 0; p16[n] = (uint16_t)n; }
     long long total = 0, entries = 0;
     int verified = 0, committed = 0, steps = 0;
-    // warp 0: the next kPF candidates (keys and list extents), prefetched into
-    // shared memory at the end of each step; a step scans ~180 candidates early
-    // in a descent, so a 32-wide window left one L2 round trip per further 32
-    constexpr int kPF = 256;
-    int pf_base = -1;                  // warp 0: first candidate of the prefetched window
-    bool pf_waited = false;
-    __shared__ unsigned long long s_pfkey[kPF];
-    __shared__ int4 s_pfinf[kPF][2];
     __syncthreads();
     for (;;) {
         // ---- warp 0: the next live candidates, then the
@@ -304,20 +205,7 @@ __device__ __forceinline__ void commit_group(const DevView<W16>& g, const unsign
             int cnt = s_n, k = s_k, scanned = s_scanned;
             while (cnt < CG && k < lim) {
                 const int idx = k + lane;
-                unsigned long long key;
-                int4 i0 = make_int4(0, 0, 0, 0), i1 = make_int4(0, 0, 0, 0);
-                const int off = k - pf_base;
-                if (cinfo && pf_base >= 0 && off >= 0 && off + 32 <= kPF) {   // inside the prefetched window
-                    if (!pf_waited) {   // every lane's copies have landed (lanes read each other's slots)
-                        asm volatile("cp.async.wait_group 0;" ::: "memory");
-                        __syncwarp();
-                        pf_waited = true;
-                    }
-                    key = s_pfkey[off + lane]; i0 = s_pfinf[off + lane][0]; i1 = s_pfinf[off + lane][1];
-                } else {
-                    key = idx < lim ? keys[idx] : ~0ull;
-                    if (cinfo && idx < lim) { i0 = cinfo[2 * idx]; i1 = cinfo[2 * idx + 1]; }
-                }
+                const unsigned long long key = idx < lim ? keys[idx] : ~0ull;
                 const bool valid = key != ~0ull;
                 const int lo = valid ? (int)((key >> 16) & 0xffffu) : 0;
                 const int hi = valid ? (int)(key & 0xffffu) : 0;
@@ -337,12 +225,11 @@ __device__ __forceinline__ void commit_group(const DevView<W16>& g, const unsign
                     const int q = cnt + before;
                     s_lo[q] = lo; s_hi[q] = hi;
                     s_d0[q] = (int)(0x7fffffffu - (unsigned)(key >> 32));
-                    if (!cinfo) {  // list extents straight from the offsets
-                        i0.x = g.off1o[lo]; i0.y = g.off1o[lo + 1] - i0.x;
-                        i0.z = g.off1i[lo]; i0.w = g.off1i[lo + 1] - i0.z;
-                        i1.x = g.off1o[hi]; i1.y = g.off1o[hi + 1] - i1.x;
-                        i1.z = g.off1i[hi]; i1.w = g.off1i[hi + 1] - i1.z;
-                    }
+                    int4 i0, i1;   // list extents
+                    i0.x = g.off1o[lo]; i0.y = g.off1o[lo + 1] - i0.x;
+                    i0.z = g.off1i[lo]; i0.w = g.off1i[lo + 1] - i0.z;
+                    i1.x = g.off1o[hi]; i1.y = g.off1o[hi + 1] - i1.x;
+                    i1.z = g.off1i[hi]; i1.w = g.off1i[hi + 1] - i1.z;
                     s_inf[q][0] = i0.x; s_inf[q][1] = i0.y; s_inf[q][2] = i0.z; s_inf[q][3] = i0.w;
                     s_inf[q][4] = i1.x; s_inf[q][5] = i1.y; s_inf[q][6] = i1.z; s_inf[q][7] = i1.w;
                 }
@@ -351,44 +238,14 @@ __device__ __forceinline__ void commit_group(const DevView<W16>& g, const unsign
                 scanned += consumed;
                 if (consumed == nvalid && nvalid < 32) { k = lim; break; }
             }
-            // prefetch the next window (its keys and list extents); it is used as
-            // is, since only the used flags change and those are read at use
-            if (cinfo) {  // asynchronous copies straight into shared memory, lane l the slots l, l + 32, ...
-                if (!pf_waited && pf_base >= 0) {   // copies of a window never read must land first
-                    asm volatile("cp.async.wait_group 0;" ::: "memory");
-                }
-                __syncwarp();   // every lane is done reading the previous window
-                pf_base = k;
-                pf_waited = false;
-                for (int h = 0; h < kPF / 32; h++) {
-                    const int slot = 32 * h + lane, idx = k + slot;
-                    if (idx < lim) {
-                        const uint32_t dk = (uint32_t)__cvta_generic_to_shared(&s_pfkey[slot]);
-                        const uint32_t di = (uint32_t)__cvta_generic_to_shared(&s_pfinf[slot][0]);
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(dk), "l"(keys + idx) : "memory");
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(di), "l"(cinfo + 2 * idx) : "memory");
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(di + 16), "l"(cinfo + 2 * idx + 1) : "memory");
-                    } else {
-                        s_pfkey[slot] = ~0ull;
-                        s_pfinf[slot][0] = make_int4(0, 0, 0, 0);
-                        s_pfinf[slot][1] = make_int4(0, 0, 0, 0);
-                    }
-                }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-            }
             __syncwarp();
             int len = 0;
             if (lane < cnt) {
                 const int a = s_lo[lane], b = s_hi[lane];
                 len = s_inf[lane][1] + s_inf[lane][3] + s_inf[lane][5] + s_inf[lane][7];
                 s_corr[lane] = 0; s_cnt[lane] = 0; s_imask[lane] = 0;
-                if (sizeof(MarkT) == 2) {
-                    atomicOr_u16(reinterpret_cast<uint16_t*>(&mark[a]), (uint16_t)(1u << lane));
-                    atomicOr_u16(reinterpret_cast<uint16_t*>(&mark[b]), (uint16_t)(1u << lane));
-                } else {
-                    atomicOr(reinterpret_cast<unsigned*>(&mark[a]), 1u << lane);
-                    atomicOr(reinterpret_cast<unsigned*>(&mark[b]), 1u << lane);
-                }
+                atomicOr_u16(&mark[a], (uint16_t)(1u << lane));
+                atomicOr_u16(&mark[b], (uint16_t)(1u << lane));
             }
             __syncwarp();
             if (lane < cnt) {  // earlier pairs of the step that share a vertex: read off the marks
@@ -439,11 +296,9 @@ __device__ __forceinline__ void commit_group(const DevView<W16>& g, const unsign
         //      thread resolves kMLP entries and issues their loads together ----
         {
             constexpr int kMLP = 4;
-            const int all = s_pre[cnt];
-            // this CTA's slice of the step's entries
-            const int first = (int)((long long)all * ct / nct), tot = (int)((long long)all * (ct + 1) / nct);
+            const int tot = s_pre[cnt];
             const int nseg = 4 * cnt;
-            for (int base = first; base < tot; base += kMLP * blockDim.x) {
+            for (int base = 0; base < tot; base += kMLP * blockDim.x) {
                 int jj[kMLP], kind[kMLP];
                 typename EN::T en[kMLP];
                 // this thread's kMLP consecutive entries: one segment search, then
@@ -520,45 +375,6 @@ __device__ __forceinline__ void commit_group(const DevView<W16>& g, const unsign
         }
         const int my_lo = tid < cnt ? s_lo[tid] : 0, my_hi = tid < cnt ? s_hi[tid] : 0;
         __syncthreads();
-        if (nct > 1) {  // exchange the per-pair partial sums of the CTAs' slices
-            const int buf = gstep & 1;
-            if (tid < cnt) {
-                s_cpart[buf][tid][0] = s_corr[tid]; s_cpart[buf][tid][1] = s_cnt[tid];
-                s_cpart[buf][tid][2] = (int)s_imask[tid];
-            }
-            if (tid < cnt * CG) {
-                const int j = tid / CG, i = tid - j * CG;
-                s_cpart[buf][j][3 + i] = s_cc[j][i];
-            }
-            __syncthreads();
-            if (tid < cnt) { s_corr[tid] = 0; s_cnt[tid] = 0; s_imask[tid] = 0; }
-            if (tid < cnt * CG) (&s_cc[0][0])[tid] = 0;
-            if (!cluster_step_sync(cbar, (uint32_t)buf, nct, grid.err, grid.stall && gstep == 0)) {
-                aborted = true;
-                break;
-            }
-            constexpr int kW = kPart / 4;   // 16-byte words per pair
-            for (int t = tid; t < nct * cnt * kW; t += blockDim.x) {
-                // (c, j, w): word w of CTA c's partials of pair j (integer sums: any order)
-                const int c = t / (cnt * kW), r = t - c * (cnt * kW);
-                const int j = r / kW, w = r - j * kW;
-                const uint32_t q = cluster_map((uint32_t)__cvta_generic_to_shared(&s_cpart[buf][j][4 * w]), (uint32_t)c);
-                int v[4];
-                asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(q) : "memory");
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int k = 4 * w + u;
-                    if (!v[u] || k >= 3 + CG) continue;
-                    if (k == 0) atomicAdd(&s_corr[j], v[u]);
-                    else if (k == 1) atomicOr(&s_cnt[j], v[u]);
-                    else if (k == 2) atomicOr(&s_imask[j], (unsigned)v[u]);
-                    else atomicAdd(&s_cc[j][k - 3], v[u]);
-                }
-            }
-            __syncthreads();
-        }
-        gstep++;
         // ---- clear the step's marks; decide in order in warp 0: lane j holds pair
         //      j's fields, every lane replays the same bitmask logic over the
         //      shuffled fields, then the lanes apply their own outcomes ----
@@ -598,18 +414,14 @@ __device__ __forceinline__ void commit_group(const DevView<W16>& g, const unsign
                 const int fa = p16[a], fb = p16[b];
                 q16[a] = (uint16_t)fa; q16[b] = (uint16_t)fb;
                 p16[a] = (uint16_t)fb; p16[b] = (uint16_t)fa;
-                if (ct == 0) {
-                    if (fb < n) g.pinv[fb] = a;
-                    if (fa < n) g.pinv[fa] = b;
-                }
+                if (fb < n) g.pinv[fb] = a;
+                if (fa < n) g.pinv[fa] = b;
                 used[a] = 1; used[b] = 1;
             }
             if (lane == 0) s_n = 0;
         }
         __syncthreads();
     }
-    if (nct > 1 && !aborted) cluster_step_sync(cbar, (uint32_t)(gstep & 1), nct, grid.err);
-    if (ct != 0) return;
     for (int i = tid; i < n; i += blockDim.x) g.p[i] = p16[i];
     if (tid == 0) {
         st->total_delta = total;
@@ -622,100 +434,10 @@ __device__ __forceinline__ void commit_group(const DevView<W16>& g, const unsign
     }
 }
 
-// Pulls [p, p + bytes) into L2 (one prefetch per 128-byte line).  The set
-// commit reads G1 list entries of scattered vertices from a single CTA; the
-// profit matrix traffic before it has evicted those lists, so without this
-// every first touch of a list goes to HBM.
-static __global__ void k_prefetch_l2(const char* __restrict__ p, size_t bytes) {
-    const size_t lines = (bytes + 127) / 128;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < lines; i += (size_t)gridDim.x * blockDim.x)
-        asm volatile("prefetch.global.L2 [%0];" :: "l"(p + i * 128));
-}
-
-// List extents of each sorted candidate for the set commit, two int4 per
-// candidate: (out-offset, out-length, in-offset, in-length) of its lower and of
-// its higher vertex; zeros for the "no candidate" key ~0.
-template <bool W16>
-__global__ void k_cand_info(DevView<W16> g, const unsigned long long* __restrict__ keys, int lim,
-                            int4* __restrict__ info) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= lim) return;
-    const unsigned long long key = keys[i];
-    int4 x = make_int4(0, 0, 0, 0), y = x;
-    if (key != ~0ull) {
-        const int lo = (int)((key >> 16) & 0xffffu), hi = (int)(key & 0xffffu);
-        x.x = g.off1o[lo]; x.y = g.off1o[lo + 1] - x.x; x.z = g.off1i[lo]; x.w = g.off1i[lo + 1] - x.z;
-        y.x = g.off1o[hi]; y.y = g.off1o[hi + 1] - y.x; y.z = g.off1i[hi]; y.w = g.off1i[hi + 1] - y.z;
-    }
-    info[2 * i] = x;
-    info[2 * i + 1] = y;
-}
-
-constexpr int kCommitMaxCtas = 8;      // a portable cluster
-constexpr int kCommitDefaultCtas = 8;
-// The set commit's error word (one int; bit 1: a cluster wait ran out).
-__host__ __device__ inline size_t commit_grid_ints() { return 4; }
-
-// Launches the set commit on `ctas` CTAs forming one thread-block cluster (a
-// plain launch for one); `buf` holds commit_grid_ints() ints: the error word,
-// reset here.  Returns the launch status.
-template <bool W16>
-__host__ inline cudaError_t launch_commit_group(const DevView<W16>& g, const unsigned long long* keys, int lim,
-                                               int max_verify, CommitStats* st, const int4* cinfo, int ctas,
-                                               int* buf, size_t smem, cudaStream_t stream, int stall = 0);
-
 // Shared memory bytes of commit_group for n vertices (used flags, matching,
-// pre-move images, step marks of mark_bytes each).
-__host__ __device__ inline size_t commit_group_smem(int n, int mark_bytes = 2) {
-    return (size_t)((n + 15) & ~15) + (4 + mark_bytes) * (size_t)((n + 8) & ~7);
-}
-
-template <bool W16, int CG = kCG>
-__global__ void __launch_bounds__(1024)
-k_commit_group(DevView<W16> g, const unsigned long long* __restrict__ keys, int lim, int max_verify,
-               CommitStats* __restrict__ st, const int4* __restrict__ cinfo, CommitGrid grid) {
-    extern __shared__ unsigned char smem[];
-    commit_group<W16, CG>(g, keys, lim, max_verify, st, smem, cinfo, grid);
-}
-
-template <bool W16>
-__host__ inline cudaError_t launch_commit_group(const DevView<W16>& g, const unsigned long long* keys, int lim,
-                                               int max_verify, CommitStats* st, const int4* cinfo, int ctas,
-                                               int* buf, size_t smem, cudaStream_t stream, int stall) {
-    cudaError_t e = cudaFuncSetAttribute(k_commit_group<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    CommitGrid grid{1, buf, stall};
-    if (ctas <= 1) {
-        k_commit_group<W16><<<1, 1024, smem, stream>>>(g, keys, lim, max_verify, st, cinfo, grid);
-        return cudaGetLastError();
-    }
-    // a cluster decides 32 pairs per step when 32-bit marks fit (n up to about
-    // 23,000), else 16
-    bool wide = false;
-    const size_t wsmem = commit_group_smem(g.n, 4);
-    if (cudaFuncSetAttribute(k_commit_group<W16, kCGWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsmem) ==
-        cudaSuccess) {
-        int per_sm = 0;
-        wide = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_commit_group<W16, kCGWide>, 1024, wsmem) ==
-                   cudaSuccess && per_sm >= 1;
-    }
-    cudaGetLastError();   // a refused attribute is not an error of this launch
-    grid.nct = ctas;
-    if ((e = cudaMemsetAsync(grid.err, 0, sizeof(int), stream)) != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(1024);
-    cfg.dynamicSmemBytes = wide ? wsmem : smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ctas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (wide) return cudaLaunchKernelEx(&cfg, k_commit_group<W16, kCGWide>, g, keys, lim, max_verify, st, cinfo, grid);
-    return cudaLaunchKernelEx(&cfg, k_commit_group<W16>, g, keys, lim, max_verify, st, cinfo, grid);
+// pre-move images, step marks).
+__host__ __device__ inline size_t commit_group_smem(int n) {
+    return (size_t)((n + 15) & ~15) + 6 * (size_t)((n + 8) & ~7);
 }
 
 }  // namespace bm
