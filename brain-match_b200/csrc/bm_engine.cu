@@ -833,6 +833,10 @@ bm_status launch_set_commit(bm_ctx* ctx, const unsigned long long* keys, const i
 
 template bm_status launch_set_commit<true, 2>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
 template bm_status launch_set_commit<false, 2>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
+template bm_status launch_set_commit<true, 3>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
+template bm_status launch_set_commit<false, 3>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
+template bm_status launch_set_commit<true, 4>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
+template bm_status launch_set_commit<false, 4>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
 
 const int* set_commit_err(bm_ctx* ctx) { return &reinterpret_cast<SetCtl*>(ctx->cset)->err; }
 
@@ -1190,6 +1194,16 @@ extern "C" bm_status bm_triple_deltas(bm_ctx* ctx, int64_t k, const int32_t* a, 
     return BM_OK;
 }
 
+// A wait of the round's set commit ran out: the matching may be partly
+// committed, and the caller sets one again before the next call.
+static bm_status set_commit_timeout(bm_ctx* ctx, const char* fn) {
+    set_err(ctx, "%s: set commit wait timed out", fn);
+    ctx->mapped = false;
+    ctx->S_exact = false;
+    const bm_status s = set_commit_reset(ctx);
+    return s ? s : BM_E_TIMEOUT;
+}
+
 template <bool W16>
 static bm_status triple_round_impl(bm_ctx* ctx, const bm_triple_opts* o, bm_triple_stats* stats) {
     const int n = ctx->n;
@@ -1214,19 +1228,22 @@ static bm_status triple_round_impl(bm_ctx* ctx, const bm_triple_opts* o, bm_trip
     CK(cudaEventRecord(ctx->ev[2], ctx->st));
     size_t tb = ctx->cub_bytes;
     CK(cub::DeviceRadixSort::SortKeys(ctx->cub_tmp, tb, ctx->ckeys, ctx->ckeys_sorted, n, 0, 64, ctx->st));
-    const size_t smem = 2 * (size_t)n;
-    CK(cudaFuncSetAttribute(k_triple_commit<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_triple_commit<W16><<<1, 1024, smem, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, n, o->max_candidates,
-                                                      o->max_verify, o->seed, ctx->cstats);
+    if (!ctx->csets) CK(dalloc(ctx, &ctx->csets, (size_t)n * sizeof(int4)));
+    k_triple_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets,
+                                                           ctx->tcount + 1);
     CK(cudaGetLastError());
+    const int lim = o->max_candidates > 0 ? std::min(o->max_candidates, n) : n;
+    if ((s = launch_set_commit<W16, 3>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0, 0))) return s;
     CK(cudaEventRecord(ctx->ev[3], ctx->st));
     CommitStats cs;
-    unsigned long long cnt[2];
-    std::vector<unsigned long long> keys(n);
+    unsigned long long cnt[2], top = 0;
+    int cerr = 0;
     CK(cudaMemcpyAsync(&cs, ctx->cstats, sizeof cs, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(cnt, ctx->tcount, sizeof cnt, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(keys.data(), ctx->ckeys_sorted, n * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&top, ctx->ckeys_sorted, sizeof top, cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&cerr, set_commit_err(ctx), sizeof cerr, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
+    if (cerr) return set_commit_timeout(ctx, "bm_triple_round");
     ctx->score = before + cs.total_delta;
     if (stats) {
         memset(stats, 0, sizeof *stats);
@@ -1234,10 +1251,8 @@ static bm_status triple_round_impl(bm_ctx* ctx, const bm_triple_opts* o, bm_trip
         stats->score_after = ctx->score;
         stats->triples = (long long)cnt[0];
         stats->rotations = 2 * (long long)cnt[0];
-        int nc = 0;
-        while (nc < n && keys[nc] != ~0ull) nc++;
-        stats->candidates = nc;
-        stats->best_delta = nc ? (int)(0x7fffffffu - (unsigned)(keys[0] >> 32)) : 0;
+        stats->candidates = (int32_t)cnt[1];
+        stats->best_delta = cnt[1] ? (int)(0x7fffffffu - (unsigned)(top >> 32)) : 0;
         stats->scanned = cs.scanned;
         stats->verified = cs.verified;
         stats->committed = cs.committed;
@@ -1315,19 +1330,22 @@ static bm_status quad_round_impl(bm_ctx* ctx, const bm_quad_opts* o, bm_quad_sta
     CK(cudaEventRecord(ctx->ev[2], ctx->st));
     size_t tb = ctx->cub_bytes;
     CK(cub::DeviceRadixSort::SortKeys(ctx->cub_tmp, tb, ctx->ckeys, ctx->ckeys_sorted, n, 0, 64, ctx->st));
-    const size_t smem = 2 * (size_t)n;
-    CK(cudaFuncSetAttribute(k_quad_commit<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_quad_commit<W16><<<1, 1024, smem, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, n, o->max_candidates,
-                                                    o->max_verify, o->seed, ctx->cstats);
+    if (!ctx->csets) CK(dalloc(ctx, &ctx->csets, (size_t)n * sizeof(int4)));
+    k_quad_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets,
+                                                           ctx->tcount + 1);
     CK(cudaGetLastError());
+    const int lim = o->max_candidates > 0 ? std::min(o->max_candidates, n) : n;
+    if ((s = launch_set_commit<W16, 4>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0, 0))) return s;
     CK(cudaEventRecord(ctx->ev[3], ctx->st));
     CommitStats cs;
-    unsigned long long cnt[2];
-    std::vector<unsigned long long> keys(n);
+    unsigned long long cnt[2], top = 0;
+    int cerr = 0;
     CK(cudaMemcpyAsync(&cs, ctx->cstats, sizeof cs, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(cnt, ctx->tcount, sizeof cnt, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(keys.data(), ctx->ckeys_sorted, n * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&top, ctx->ckeys_sorted, sizeof top, cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(&cerr, set_commit_err(ctx), sizeof cerr, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
+    if (cerr) return set_commit_timeout(ctx, "bm_quad_round");
     ctx->score = before + cs.total_delta;
     if (stats) {
         memset(stats, 0, sizeof *stats);
@@ -1335,10 +1353,8 @@ static bm_status quad_round_impl(bm_ctx* ctx, const bm_quad_opts* o, bm_quad_sta
         stats->score_after = ctx->score;
         stats->quads = (long long)cnt[0];
         stats->permutations = 23 * (long long)cnt[0];
-        int nc = 0;
-        while (nc < n && keys[nc] != ~0ull) nc++;
-        stats->candidates = nc;
-        stats->best_delta = nc ? (int)(0x7fffffffu - (unsigned)(keys[0] >> 32)) : 0;
+        stats->candidates = (int32_t)cnt[1];
+        stats->best_delta = cnt[1] ? (int)(0x7fffffffu - (unsigned)(top >> 32)) : 0;
         stats->scanned = cs.scanned;
         stats->verified = cs.verified;
         stats->committed = cs.committed;

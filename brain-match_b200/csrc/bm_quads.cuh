@@ -252,80 +252,21 @@ k_quad_eval(DevView<W16> g, const unsigned* __restrict__ adj, int words, int par
     }
 }
 
-// Sequential commit of the sorted 4-set candidates (one CTA), the rule of the
-// 3-cycle round: skip a set with a vertex already moved, re-evaluate exactly
-// a set with a moved G1 neighbour, commit iff the delta is > 0.
+// The sets of the sorted 4-set candidates for the set commit (SetArgs::sets),
+// and the number of candidates (*count, zero before).
 template <bool W16>
-__global__ void __launch_bounds__(1024)
-k_quad_commit(DevView<W16> g, const unsigned long long* __restrict__ keys, int nkeys, int max_scan,
-              int max_verify, unsigned long long seed, CommitStats* __restrict__ st) {
-    typedef Ent<W16> EN;
-    extern __shared__ unsigned char flags[];
-    unsigned char* used = flags;
-    unsigned char* taint = flags + g.n;
-    __shared__ int red[32];
-    __shared__ int s_delta;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    for (int i = tid; i < 2 * g.n; i += blockDim.x) flags[i] = 0;
-    long long total = 0;
-    int scanned = 0, verified = 0, committed = 0;
-    __syncthreads();
-    const int lim = (max_scan > 0 && max_scan < nkeys) ? max_scan : nkeys;
-    for (int k = 0; k < lim; k++) {
-        const unsigned long long key = keys[k];
-        if (key == ~0ull) break;
-        const int a = (int)((key >> 16) & 0xffffu), j = (int)((key >> 5) & 0x7ffu), q = (int)(key & 31u);
-        const int d0 = (int)(0x7fffffffu - (unsigned)(key >> 32));
-        int b = 0, c = 0, d = 0;
-        sample_quad<W16>(g, seed, a, j, b, c, d);
-        scanned++;
-        if (used[a] | used[b] | used[c] | used[d]) continue;
-        const int M[4] = {a, b, c, d};
-        int dd = d0;
-        if (taint[a] | taint[b] | taint[c] | taint[d]) {
-            if (max_verify >= 0 && verified >= max_verify) continue;
-            verified++;
-            int part = quad_delta_walk_part<W16>(g, M, q, tid, blockDim.x);
-            for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-            if (lane == 0) red[wid] = part;
-            __syncthreads();
-            if (wid == 0) {
-                int v = lane < (int)(blockDim.x >> 5) ? red[lane] : 0;
-                for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                if (lane == 0) s_delta = v;
-            }
-            __syncthreads();
-            dd = s_delta;
-            __syncthreads();
-        }
-        if (dd <= 0) continue;
-        if (tid == 0) {
-            int f[4];
-            for (int i = 0; i < 4; i++) f[i] = g.p[M[i]];
-            for (int i = 0; i < 4; i++) {
-                const int nf = f[kQuadPerm[q][i]];
-                g.p[M[i]] = nf;
-                if (nf < g.n) g.pinv[nf] = M[i];
-                used[M[i]] = 1;
-            }
-        }
-        total += dd;
-        committed++;
-        for (int i = 0; i < 4; i++) {
-            const int x = M[i];
-            const int o0 = g.off1o[x], o1 = g.off1o[x + 1] - o0;
-            const int i0 = g.off1i[x], i1 = g.off1i[x + 1] - i0;
-            for (int r = tid; r < o1 + i1; r += blockDim.x)
-                taint[r < o1 ? EN::id(g.ent1o[o0 + r]) : EN::id(g.ent1i[i0 + r - o1])] = 1;
-        }
-        __syncthreads();
-    }
-    if (tid == 0) {
-        st->total_delta = total;
-        st->scanned = scanned;
-        st->verified = verified;
-        st->committed = committed;
-    }
+__global__ void k_quad_sets(DevView<W16> g, const unsigned long long* __restrict__ keys, unsigned long long seed,
+                            int4* __restrict__ sets, unsigned long long* __restrict__ count) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned long long key = i < g.n ? keys[i] : ~0ull;
+    const unsigned valid = __ballot_sync(0xffffffffu, key != ~0ull);
+    if ((threadIdx.x & 31) == 0 && valid) atomicAdd(count, (unsigned long long)__popc(valid));
+    if (key == ~0ull) return;
+    const int a = (int)((key >> 16) & 0xffffu), j = (int)((key >> 5) & 0x7ffu), q = (int)(key & 31u);
+    int b = 0, c = 0, d = 0;
+    sample_quad<W16>(g, seed, a, j, b, c, d);
+    const unsigned char* sg = kQuadPerm[q];
+    sets[i] = make_int4(a | b << 16, c | d << 16, sg[0] | sg[1] << 8 | sg[2] << 16 | sg[3] << 24, 0);
 }
 
 }  // namespace bm

@@ -228,79 +228,21 @@ k_triple_eval(DevView<W16> g, const unsigned* __restrict__ adj, int words, int p
     }
 }
 
-// Sequential commit of sorted 3-cycle candidates (one CTA); same rule as
-// k_commit: skip if a vertex was moved, re-verify if a vertex is tainted.
+// The sets of the sorted 3-cycle candidates for the set commit (SetArgs::sets),
+// and the number of candidates (*count, zero before).
 template <bool W16>
-__global__ void __launch_bounds__(1024)
-k_triple_commit(DevView<W16> g, const unsigned long long* __restrict__ keys, int nkeys, int max_scan,
-                int max_verify, unsigned long long seed, CommitStats* __restrict__ st) {
-    typedef Ent<W16> EN;
-    extern __shared__ unsigned char flags[];
-    unsigned char* used = flags;
-    unsigned char* taint = flags + g.n;
-    __shared__ int red[32];
-    __shared__ int s_delta;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    for (int i = tid; i < 2 * g.n; i += blockDim.x) flags[i] = 0;
-    long long total = 0;
-    int scanned = 0, verified = 0, committed = 0;
-    __syncthreads();
-    const int lim = (max_scan > 0 && max_scan < nkeys) ? max_scan : nkeys;
-    for (int k = 0; k < lim; k++) {
-        const unsigned long long key = keys[k];
-        if (key == ~0ull) break;
-        const int a = (int)((key >> 16) & 0xffffu), j = (int)((key >> 1) & 0x7fffu), rot = (int)(key & 1u);
-        const int d0 = (int)(0x7fffffffu - (unsigned)(key >> 32));
-        int b = 0, c = 0;
-        sample_triple<W16>(g, seed, a, j, b, c);
-        scanned++;
-        if (used[a] | used[b] | used[c]) continue;
-        int d = d0;
-        if (taint[a] | taint[b] | taint[c]) {
-            if (max_verify >= 0 && verified >= max_verify) continue;
-            verified++;
-            int part = triple_delta_walk_part<W16>(g, a, b, c, rot, tid, blockDim.x);
-            for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-            if (lane == 0) red[wid] = part;
-            __syncthreads();
-            if (wid == 0) {
-                int v = lane < (int)(blockDim.x >> 5) ? red[lane] : 0;
-                for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                if (lane == 0) s_delta = v;
-            }
-            __syncthreads();
-            d = s_delta;
-            __syncthreads();
-        }
-        if (d <= 0) continue;
-        if (tid == 0) {
-            const int fa = g.p[a], fb = g.p[b], fc = g.p[c];
-            int na, nb, nc;
-            if (rot == 0) { na = fb; nb = fc; nc = fa; } else { na = fc; nb = fa; nc = fb; }
-            g.p[a] = na; g.p[b] = nb; g.p[c] = nc;
-            if (na < g.n) g.pinv[na] = a;
-            if (nb < g.n) g.pinv[nb] = b;
-            if (nc < g.n) g.pinv[nc] = c;
-            used[a] = used[b] = used[c] = 1;
-        }
-        total += d;
-        committed++;
-        const int M[3] = {a, b, c};
-        for (int i = 0; i < 3; i++) {
-            const int x = M[i];
-            const int o0 = g.off1o[x], o1 = g.off1o[x + 1] - o0;
-            const int i0 = g.off1i[x], i1 = g.off1i[x + 1] - i0;
-            for (int q = tid; q < o1 + i1; q += blockDim.x)
-                taint[q < o1 ? EN::id(g.ent1o[o0 + q]) : EN::id(g.ent1i[i0 + q - o1])] = 1;
-        }
-        __syncthreads();
-    }
-    if (tid == 0) {
-        st->total_delta = total;
-        st->scanned = scanned;
-        st->verified = verified;
-        st->committed = committed;
-    }
+__global__ void k_triple_sets(DevView<W16> g, const unsigned long long* __restrict__ keys, unsigned long long seed,
+                              int4* __restrict__ sets, unsigned long long* __restrict__ count) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned long long key = i < g.n ? keys[i] : ~0ull;
+    const unsigned valid = __ballot_sync(0xffffffffu, key != ~0ull);
+    if ((threadIdx.x & 31) == 0 && valid) atomicAdd(count, (unsigned long long)__popc(valid));
+    if (key == ~0ull) return;
+    const int a = (int)((key >> 16) & 0xffffu), j = (int)((key >> 1) & 0x7fffu);
+    int b = 0, c = 0;
+    sample_triple<W16>(g, seed, a, j, b, c);
+    // images come from (b, c, a) in rotation 0, from (c, a, b) in rotation 1
+    sets[i] = make_int4(a | b << 16, c, (key & 1u) ? 0x010002 : 0x000201, 0);
 }
 
 // ---------------------------------------------------------------------------
