@@ -16,11 +16,9 @@
 //   * y moved in an earlier step: the change above goes into corr[j];
 //   * y is in earlier sets i of the window: pair (j, i) is marked adjacent and
 //     the change that set i's move would make goes into cc[j][i].
-// CTA 0 then replays the sequential rule on corr and cc alone, 32 sets at a
-// time: sets whose earlier neighbours in the block are all decided are decided
-// together, and the block's commits are added to the later sets at once.  The
-// decisions, the re-verification budget included, are those of the
-// one-at-a-time rule.
+// CTA 0 then replays the sequential rule on corr and cc alone (set_decide) and
+// publishes the committed sets.  The decisions, the re-verification budget
+// included, are those of the one-at-a-time rule.
 //
 // What bounds it: the serial chain per step, at n = 18,524 / E = 5e6 about
 // 20 us -- select and tables 2.3, list scan 6.3 (three dependent gathers),

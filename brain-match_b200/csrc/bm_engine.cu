@@ -19,6 +19,7 @@
 #include "bm.h"
 #include "bm_internal.cuh"
 #include "bm_triples.cuh"
+#include "bm_first.cuh"
 #include "bm_quads.cuh"
 #include "bm_select.cuh"
 #include "bm_commit.cuh"
@@ -166,7 +167,7 @@ static void free_ctx(bm_ctx* c) {
                     c->ent2o, c->ent2i, c->ent1oP, c->ent1iP, c->ent2oP, c->ent2iP, c->W2, c->p,
                     c->pinv, c->S, c->rowbest, c->ckeys, c->ckeys_sorted, c->wkeys, c->wkeys_sorted,
                     c->wvals, c->order, c->cub_tmp, c->small, c->score_acc, c->cstats, c->scratch_pairs,
-                    c->adj, c->rowd, c->first, c->fi_acc, c->tcount};
+                    c->adj, c->first, c->fi_acc, c->tcount};
     for (void* b : bufs) if (b) cudaFree(b);
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);
     for (auto& e : c->uev) if (e) cudaEventDestroy(e);
@@ -1106,47 +1107,84 @@ extern "C" bm_status bm_hillclimb(bm_ctx* ctx, int32_t max_sweeps, const bm_swee
 
 // ---------------------------------------------------------------------------
 // Reference-order first improvement (src/graph-alignment-optimized.c:515-577).
-__global__ void k_first_reset(int* first, int n) { first[0] = n; }
-__global__ void k_first_publish(int* first, int n) { first[1] = first[0]; first[0] = n; }
+// Whether k_first_rows runs: its row, contributions and matchings fit a CTA's
+// shared memory, a 16-CTA cluster of them can be placed, and a row's terms
+// (which one CTA sums) are few enough to beat the grid's pairs.
+template <bool W16>
+static bool first_rows_fit(bm_ctx* ctx, cudaLaunchConfig_t* cfg) {
+    const size_t smem = first_rows_smem(ctx->n);
+    const double terms = 4.0 * (double)ctx->e1 / ctx->n * (double)ctx->e2 / ctx->n;
+    if (smem + 1024 > ctx->smem_optin || terms > kRowsTerms) return false;
+    cfg->dynamicSmemBytes = smem;
+    int clusters = 0;
+    const bool ok =
+        cudaFuncSetAttribute(k_first_rows<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+        cudaFuncSetAttribute(k_first_rows<W16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, k_first_rows<W16>, cfg) == cudaSuccess && clusters > 0;
+    cudaGetLastError();   // a refused attribute is not an error of the launches
+    return ok;
+}
 
 template <bool W16>
 static bm_status first_improvement_impl(bm_ctx* ctx, int max_passes, long long* commits, int* passes) {
+    if (max_passes == 0) return BM_OK;
     const int n = ctx->n;
-    if (!ctx->rowd) CK(dalloc(ctx, &ctx->rowd, n * sizeof(int)));
-    if (!ctx->first) CK(dalloc(ctx, &ctx->first, 2 * sizeof(int)));
-    if (!ctx->fi_acc) CK(dalloc(ctx, &ctx->fi_acc, 2 * sizeof(long long)));
-    CK(cudaMemsetAsync(ctx->fi_acc, 0, 2 * sizeof(long long), ctx->st));
-    k_first_reset<<<1, 1, 0, ctx->st>>>(ctx->first, n);
     DevView<W16> g = view<W16>(ctx);
-    long long total = 0;
-    int pass = 0;
-    const int blocks = std::min((n + 7) / 8, ctx->num_sms * 16);
-    for (; pass < max_passes; pass++) {
-        long long in_pass = 0;
-        for (int m1 = 0; m1 < n; m1++) {
-            int start = 0;
-            while (start < n) {
-                k_row_first<W16><<<blocks, 256, 0, ctx->st>>>(g, m1, start, ctx->rowd, ctx->first);
-                k_apply_first<<<1, 1, 0, ctx->st>>>(ctx->p, ctx->pinv, n, m1, ctx->first, ctx->rowd, ctx->fi_acc);
-                k_first_publish<<<1, 1, 0, ctx->st>>>(ctx->first, n);
-                CK(cudaGetLastError());
-                int m2 = n;
-                CK(cudaMemcpyAsync(&m2, ctx->first + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
-                CK(cudaStreamSynchronize(ctx->st));
-                if (m2 >= n) break;
-                in_pass++;
-                start = m2 + 1;
-            }
-        }
-        total += in_pass;
-        if (in_pass == 0) { pass++; break; }
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(kRowsCluster);
+    cfg.blockDim = dim3(kRowsThreads);
+    cfg.stream = ctx->st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kRowsCluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const bool rows = first_rows_fit<W16>(ctx, &cfg);
+    int grid = 0;
+    const size_t smem = (size_t)n * sizeof(unsigned short);
+    if (!rows) {
+        CK(cudaFuncSetAttribute(k_first<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        int per_sm = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_first<W16>, kFirstThreads, smem));
+        if (per_sm < 1) { set_err(ctx, "first-improvement kernel does not fit (n=%d)", n); return BM_E_INPUT; }
+        // short lists are bound by the step's latency, which more CTAs lengthen
+        // (n = 600: one CTA per SM 24.6, two 28.5 ms); long ones by the loads in flight
+        grid = ctx->num_sms * (4.0 * (double)ctx->e1 / n >= kFirstLongLists ? per_sm : 1);
     }
-    long long acc[2] = {0, 0};
-    CK(cudaMemcpyAsync(acc, ctx->fi_acc, sizeof acc, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    ctx->score += acc[0];
-    *commits = total;
-    *passes = pass;
+    // behind the state: the contributions of k_first_rows or the slots of k_first
+    const size_t slot_bytes = 2 * (size_t)grid * sizeof(unsigned long long);
+    static_assert(sizeof(FirstState) % sizeof(unsigned long long) == 0, "the slots follow the state");
+    if (!ctx->first)   // the path depends on the context alone
+        CK(dalloc(ctx, (char**)&ctx->first, sizeof(FirstState) + (rows ? (size_t)n * sizeof(int) : slot_bytes)));
+    CK(cudaMemsetAsync(ctx->first, 0, sizeof(FirstState), ctx->st));
+    FirstState* st = static_cast<FirstState*>(ctx->first);
+    unsigned long long* slots = reinterpret_cast<unsigned long long*>(st + 1);
+    int* contrib = reinterpret_cast<int*>(st + 1);
+    if (rows) {
+        k_contrib_int<W16><<<(n + 7) / 8, 256, 0, ctx->st>>>(g, contrib);
+        CK(cudaGetLastError());
+    }
+    FirstState h;
+    do {
+        if (rows) {
+            CK(cudaLaunchKernelEx(&cfg, k_first_rows<W16>, g, st, contrib, max_passes));
+        } else {
+            CK(cudaMemsetAsync(slots, 0, slot_bytes, ctx->st));   // a launch starts again at tag 1
+            void* args[] = {&g, &st, &slots, &max_passes};
+            CK(cudaLaunchCooperativeKernel((const void*)k_first<W16>, dim3(grid), dim3(kFirstThreads), args, smem, ctx->st));
+        }
+        CK(cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, ctx->st));
+        CK(cudaStreamSynchronize(ctx->st));
+        if (h.err) {
+            set_err(ctx, "bm_first_improvement: exchange wait timed out");
+            ctx->mapped = false;
+            return BM_E_TIMEOUT;
+        }
+    } while (!h.done);
+    ctx->score += h.delta;
+    *commits = h.commits;
+    *passes = h.passes;
     return BM_OK;
 }
 
@@ -1394,8 +1432,7 @@ __global__ void k_pair_deltas_static(DevView<W16> g, const int* __restrict__ m1,
     long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
     for (; w < k; w += nw) {
-        int d = swap_delta_part<W16>(g, m1[w] - 1, m2[w] - 1, lane, 32);
-        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        const int d = swap_delta_warp<W16>(g, [&](int v) { return g.p[v]; }, m1[w] - 1, m2[w] - 1, lane);
         if (lane == 0) out[w] = d;
     }
 }

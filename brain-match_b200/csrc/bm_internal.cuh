@@ -60,9 +60,8 @@ struct bm_ctx {
     long long scratch_cap = 0;
     unsigned* adj = nullptr;       // G1 adjacency bitmap (3-cycles)
     int adj_words = 0;
-    int* rowd = nullptr;           // reference-order row deltas
-    int* first = nullptr;          // [0] = first improving partner, [1] = copy for the host
-    long long* fi_acc = nullptr;   // [0] = delta sum, [1] = commits
+    void* first = nullptr;         // first improvement: scan state, then the exchange slots
+    long long* fi_acc = nullptr;   // best-swap descent: [0] = delta sum, [1] = commits
     unsigned long long* tcount = nullptr;
     long long dev_bytes = 0;
     cudaEvent_t ev[6] = {};

@@ -459,6 +459,66 @@ __device__ __forceinline__ int swap_delta_part(const DevView<W16>& g, int a, int
     return d;
 }
 
+// The same delta by `parts` warps, img(v) the matching: the sum of part 0 ..
+// parts - 1, each returned to every lane of its warp.
+// Lanes load the list extents in one round, then take four entries each per
+// round: their entries, images and W2 terms are in flight together, so a pair
+// of 128 list entries costs three dependent loads instead of twelve.
+template <bool W16, typename Img>
+__device__ __forceinline__ int swap_delta_warp(const DevView<W16>& g, Img img, int a, int b, int lane, int part = 0,
+                                               int parts = 1) {
+    typedef Ent<W16> EN;
+    constexpr int U = 4;
+    const int pa = img(a), pb = img(b);
+    int ext = 0;   // lanes 0..7: out- and in-list of a, of b; lanes 8..11: their self-loops
+    {
+        const int v = (lane >> 1 & 1) ? b : a;
+        const int* off = lane < 4 ? g.off1o : lane < 8 ? g.off1i : g.offs;
+        if (lane < 12) ext = off[v + (lane & 1)];
+    }
+    const int oa = __shfl_sync(0xffffffffu, ext, 0), ob = __shfl_sync(0xffffffffu, ext, 2);
+    const int ia = __shfl_sync(0xffffffffu, ext, 4), ib = __shfl_sync(0xffffffffu, ext, 6);
+    const int e0 = __shfl_sync(0xffffffffu, ext, 1) - oa;          // ends of: out a,
+    const int e1 = e0 + __shfl_sync(0xffffffffu, ext, 3) - ob;     // out b,
+    const int e2 = e1 + __shfl_sync(0xffffffffu, ext, 5) - ia;     // in a,
+    const int e3 = e2 + __shfl_sync(0xffffffffu, ext, 7) - ib;     // in b
+    int d = 0;
+    for (int k0 = 32 * U * part; k0 < e3; k0 += 32 * U * parts) {
+        typename EN::T e[U];
+        int lo[U], ln[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int k = k0 + 32 * u + lane;
+            if (k < e3) e[u] = k < e1 ? g.ent1o[k < e0 ? oa + k : ob + (k - e0)] : g.ent1i[k < e2 ? ia + (k - e1) : ib + (k - e2)];
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int k = k0 + 32 * u + lane;
+            lo[u] = ln[u] = 0;
+            if (k >= e3) continue;
+            const bool out = k < e1, isa = out ? k < e0 : k < e2;
+            const int v = EN::id(e[u]);
+            const int po = isa ? pa : pb, pn = isa ? pb : pa;       // this end's image, and the one it takes
+            const bool other = v == (isa ? b : a);
+            if (other && !out) continue;                            // counted from its source's out-list
+            const int q = img(v), qn = other ? po : q;
+            lo[u] = out ? g.w2(po, q) : g.w2t(q, po);
+            ln[u] = out ? g.w2(pn, qn) : g.w2t(q, pn);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (k0 + 32 * u + lane < e3) d += imin(EN::w(e[u]), ln[u]) - imin(EN::w(e[u]), lo[u]);
+    }
+    const int sa = __shfl_sync(0xffffffffu, ext, 8), ta = __shfl_sync(0xffffffffu, ext, 9);
+    const int sb = __shfl_sync(0xffffffffu, ext, 10), tb = __shfl_sync(0xffffffffu, ext, 11);
+    if (part == 0 && (ta > sa || tb > sb)) {   // G1 self-loops
+        const int da = g.w2d(pa), db = g.w2d(pb);
+        for (int q = sa + lane; q < ta; q += 32) d += imin(g.selfw[q], db) - imin(g.selfw[q], da);
+        for (int q = sb + lane; q < tb; q += 32) d += imin(g.selfw[q], da) - imin(g.selfw[q], db);
+    }
+    return __reduce_add_sync(0xffffffffu, d);
+}
+
 // One warp per requested pair.
 template <bool W16>
 __global__ void k_pair_deltas(DevView<W16> g, const int* __restrict__ pa, const int* __restrict__ pb,
@@ -467,8 +527,7 @@ __global__ void k_pair_deltas(DevView<W16> g, const int* __restrict__ pa, const 
     long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
     for (; w < k; w += nw) {
-        int d = swap_delta_part<W16>(g, pa[w], pb[w], lane, 32);
-        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        const int d = swap_delta_warp<W16>(g, [&](int v) { return g.p[v]; }, pa[w], pb[w], lane);
         if (lane == 0) out[w] = d;
     }
 }

@@ -1,5 +1,4 @@
-// bm_triples.cuh -- 3-cycle moves and the reference-order (first-improvement)
-// row scan.
+// bm_triples.cuh -- 3-cycle moves.
 //
 // A 3-cycle on G1 vertices (a,b,c) moves their images around: rotation 0 is
 // permutation 3 of calculateThreeNodeSwapKernel, (f1,f2,f3) <- (f2,f3,f1);
@@ -243,39 +242,6 @@ __global__ void k_triple_sets(DevView<W16> g, const unsigned long long* __restri
     sample_triple<W16>(g, seed, a, j, b, c);
     // images come from (b, c, a) in rotation 0, from (c, a, b) in rotation 1
     sets[i] = make_int4(a | b << 16, c, (key & 1u) ? 0x010002 : 0x000201, 0);
-}
-
-// ---------------------------------------------------------------------------
-// Reference-order row scan: deltas of (m1, m2) for every m2 >= start, m2 != m1,
-// on the current matching, and the smallest m2 whose delta is > 0.
-template <bool W16>
-__global__ void k_row_first(DevView<W16> g, int m1, int start, int* __restrict__ row_d,
-                            int* __restrict__ first) {
-    const int lane = threadIdx.x & 31;
-    int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int m2 = start + w; m2 < g.n; m2 += nw) {
-        if (m2 == m1) continue;
-        int d = swap_delta_part<W16>(g, m1, m2, lane, 32);
-        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-        if (lane == 0) {
-            row_d[m2] = d;
-            if (d > 0) atomicMin(first, m2);
-        }
-    }
-}
-
-// Applies the swap (m1, *first) when *first < n and records its delta.
-static __global__ void k_apply_first(int* p, int* pinv, int n, int m1, const int* __restrict__ first,
-                              const int* __restrict__ row_d, long long* __restrict__ acc) {
-    const int m2 = *first;
-    if (m2 >= n) return;
-    const int f1 = p[m1], f2 = p[m2];
-    p[m1] = f2; p[m2] = f1;
-    if (f2 < n) pinv[f2] = m1;
-    if (f1 < n) pinv[f1] = m2;
-    acc[0] += row_d[m2];
-    acc[1] += 1;
 }
 
 }  // namespace bm
