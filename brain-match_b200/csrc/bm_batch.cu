@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kBThreads, 1) k_b_sweep(BSweepArgs<W16> a) {
                 const DevView<W16> g = a.views[i];
                 if (a.rpt[i] == 1) {   // profit row `local` of instance i by the whole group
                     // (the long-list queue of the group's first half: halves of other groups use theirs)
-                    profit_row_on<W16, 256>(g, local, acc, s_long[2 * grp], &s_nlong[2 * grp], nullptr, 0, nullptr,
+                    profit_row_on<W16, 256>(g, local, acc, s_long[2 * grp], &s_nlong[2 * grp], nullptr, 0,
                                             nullptr, nullptr, [grp] { b_group_sync(grp); });
                     __threadfence();     // every thread's part of the row is visible before it counts
                     b_group_sync(grp);
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(kBThreads, 1) k_b_sweep(BSweepArgs<W16> a) {
                     const int hb = 2 * grp + half;   // the half's barrier: 5 + hb, 128 threads
                     if (r < I.n)
                         profit_row_on<W16, 128>(g, r, acc + half * ((I.n + 1 + 3) & ~3), s_long[hb], &s_nlong[hb],
-                                                nullptr, 0, nullptr, nullptr, nullptr, [hb] {
+                                                nullptr, 0, nullptr, nullptr, [hb] {
                                                     asm volatile("bar.sync %0, 128;" :: "r"(5 + hb) : "memory");
                                                 });
                     __threadfence();

@@ -165,8 +165,8 @@ static void free_ctx(bm_ctx* c) {
     if (c->W2D) cudaFree(c->W2D);
     void* bufs[] = {c->off1o, c->off1i, c->off2o, c->off2i, c->offs, c->selfw, c->ent1o, c->ent1i,
                     c->ent2o, c->ent2i, c->ent1oP, c->ent1iP, c->ent2oP, c->ent2iP, c->W2, c->p,
-                    c->pinv, c->S, c->rowbest, c->ckeys, c->ckeys_sorted, c->wkeys, c->wkeys_sorted,
-                    c->wvals, c->order, c->cub_tmp, c->small, c->score_acc, c->cstats, c->scratch_pairs,
+                    c->pinv, c->S, c->rowbest, c->ckeys, c->ckeys_sorted, 
+                    c->order, c->cub_tmp, c->small, c->score_acc, c->cstats, c->scratch_pairs,
                     c->adj, c->first, c->fi_acc, c->tcount};
     for (void* b : bufs) if (b) cudaFree(b);
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);
@@ -329,6 +329,7 @@ extern "C" bm_status bm_create(bm_ctx** out, int32_t n, int64_t e1, const int32_
         CK(cudaEventCreate(&ctx->ev_hub));
         CK(dalloc(ctx, &ctx->hub_err, sizeof(int)));
         CK(cudaMemset(ctx->hub_err, 0, sizeof(int)));
+        std::vector<int> hub_list;
         if (!(flags & BM_FLAG_NO_HUB_GEMM)) {
             // hubs: G1 vertices of out-degree >= max(64, n/9), at most kHubMaxHubs,
             // topped up by the next-largest out-degrees to a multiple of 16 so the
@@ -350,6 +351,7 @@ extern "C" bm_status bm_create(bm_ctx** out, int32_t n, int64_t e1, const int32_
                     std::vector<unsigned char> flag(n, 0);
                     std::vector<int> hv(byd.begin(), byd.begin() + nh);
                     for (int v : hv) flag[v] = 1;
+                    hub_list = hv;
                     ctx->nh = nh;
                     ctx->hubK = nh * kHubT;
                     ctx->Mpad = (n + 2 * kGemmM - 1) / (2 * kGemmM) * (2 * kGemmM);  // whole 256-row tiles
@@ -366,18 +368,36 @@ extern "C" bm_status bm_create(bm_ctx** out, int32_t n, int64_t e1, const int32_
         CK(dalloc(ctx, &ctx->rowbest, n * sizeof(unsigned long long)));
         CK(dalloc(ctx, &ctx->ckeys, n * sizeof(unsigned long long)));
         CK(dalloc(ctx, &ctx->ckeys_sorted, n * sizeof(unsigned long long)));
-        CK(dalloc(ctx, &ctx->wkeys, n * sizeof(unsigned long long)));
-        CK(dalloc(ctx, &ctx->wkeys_sorted, n * sizeof(unsigned long long)));
-        CK(dalloc(ctx, &ctx->wvals, n * sizeof(int)));
-        CK(dalloc(ctx, &ctx->order, n * sizeof(int)));
+        {   // profit rows, heaviest first: the terms of a row, half on a random
+            // matching and half on one that matches degrees
+            const double mean = (double)ctx->e2 / n;
+            std::vector<char> hub(n, 0);
+            for (int v : hub_list) hub[v] = 1;
+            std::vector<std::pair<float, int>> w(n);
+            for (int a = 0; a < n; a++) {
+                double t = 0;
+                for (int i = g1o.off[a]; i < g1o.off[a + 1]; i++) {
+                    const int v = g1o.id[i];
+                    t += mean + (g1i.off[v + 1] - g1i.off[v]);
+                }
+                for (int i = g1i.off[a]; i < g1i.off[a + 1]; i++) {
+                    const int u = g1i.id[i];
+                    if (!hub[u]) t += mean + (g1o.off[u + 1] - g1o.off[u]);
+                }
+                w[a] = {(float)-t, a};
+            }
+            std::sort(w.begin(), w.end());
+            std::vector<int> order(n);
+            for (int a = 0; a < n; a++) order[a] = w[a].second;
+            CK(dalloc(ctx, &ctx->order, n * sizeof(int)));
+            CK(cudaMemcpy(ctx->order, order.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+        }
         CK(dalloc(ctx, &ctx->small, 16 * sizeof(int)));
         CK(dalloc(ctx, &ctx->score_acc, sizeof(unsigned long long)));
         CK(dalloc(ctx, &ctx->cstats, sizeof(CommitStats)));
-        size_t b1 = 0, b2 = 0;
+        size_t b1 = 0;
         CK(cub::DeviceRadixSort::SortKeys(nullptr, b1, ctx->ckeys, ctx->ckeys_sorted, n));
-        CK(cub::DeviceRadixSort::SortPairsDescending(nullptr, b2, ctx->wkeys, ctx->wkeys_sorted,
-                                                     ctx->wvals, ctx->order, n));
-        ctx->cub_bytes = std::max(b1, b2);
+        ctx->cub_bytes = b1;
         CK(dalloc(ctx, &ctx->cub_tmp, ctx->cub_bytes));
         CK(cudaDeviceSynchronize());
         return BM_OK;
@@ -406,9 +426,9 @@ extern "C" bm_status bm_get_info(const bm_ctx* ctx, bm_info* info) {
 // ---------------------------------------------------------------------------
 static bm_status compute_score(bm_ctx* ctx, long long* out) {
     CK(cudaMemsetAsync(ctx->score_acc, 0, sizeof(unsigned long long), ctx->st));
-    const int blocks = ctx->num_sms * 4;
-    if (ctx->w16) k_score<true><<<blocks, 256, 0, ctx->st>>>(view<true>(ctx), ctx->score_acc);
-    else k_score<false><<<blocks, 256, 0, ctx->st>>>(view<false>(ctx), ctx->score_acc);
+    const int blocks = (int)std::min<long long>(ctx->num_sms * 8LL, ctx->e1 / (8 * kScoreRun) + 1);
+    if (ctx->w16) k_score<true><<<blocks, 256, 0, ctx->st>>>(view<true>(ctx), (int)ctx->e1, ctx->score_acc);
+    else k_score<false><<<blocks, 256, 0, ctx->st>>>(view<false>(ctx), (int)ctx->e1, ctx->score_acc);
     CK(cudaGetLastError());
     unsigned long long v = 0;
     CK(cudaMemcpyAsync(&v, ctx->score_acc, sizeof v, cudaMemcpyDeviceToHost, ctx->st));
@@ -435,7 +455,6 @@ extern "C" bm_status bm_set_mapping(bm_ctx* ctx, const int32_t* map) {
     CK(cudaMemcpyAsync(ctx->p, p.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(ctx->pinv, pinv.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
     ctx->mapped = true;
-    ctx->work_valid = false;   // row scheduling keys are estimated afresh for a new matching
     return compute_score(ctx, &ctx->score);
 }
 
@@ -529,25 +548,19 @@ bm_status stage_profit(bm_ctx* ctx) {
     DevView<W16> g = view<W16>(ctx);
     const int n = ctx->n;
     ctx->S_exact = false;
-    const int rb = ctx->num_sms * 8;
-    k_relabel<W16><<<rb, 256, 0, ctx->st>>>((const E*)ctx->ent1o, (E*)ctx->ent1oP, ctx->e1, ctx->p);
-    k_relabel<W16><<<rb, 256, 0, ctx->st>>>((const E*)ctx->ent1i, (E*)ctx->ent1iP, ctx->e1, ctx->p);
-    k_relabel<W16><<<rb, 256, 0, ctx->st>>>((const E*)ctx->ent2o, (E*)ctx->ent2oP, ctx->e2, ctx->pinv);
-    k_relabel<W16><<<rb, 256, 0, ctx->st>>>((const E*)ctx->ent2i, (E*)ctx->ent2iP, ctx->e2, ctx->pinv);
-    if (ctx->nh && ctx->e2H)
-        k_relabel<W16><<<rb, 256, 0, ctx->st>>>((const E*)ctx->ent2oH, (E*)ctx->ent2oHP, ctx->e2H, ctx->pinv);
+    RelabelLists<W16> rl = {};
+    auto list = [&](int l, const void* in, void* out, const int* map, long long len) {
+        rl.in[l] = (const E*)in; rl.out[l] = (E*)out; rl.map[l] = map; rl.len[l] = len;
+    };
+    list(0, ctx->ent1o, ctx->ent1oP, ctx->p, ctx->e1);
+    list(1, ctx->ent1i, ctx->ent1iP, ctx->p, ctx->e1);
+    list(2, ctx->ent2o, ctx->ent2oP, ctx->pinv, ctx->e2);
+    list(3, ctx->ent2i, ctx->ent2iP, ctx->pinv, ctx->e2);
+    list(4, ctx->ent2oH, ctx->ent2oHP, ctx->pinv, ctx->nh ? ctx->e2H : 0);
+    rl.row_counter = ctx->small;
+    rl.work_total = ctx->work_sum;
+    k_relabel<W16><<<ctx->num_sms * 8, 256, 0, ctx->st>>>(rl);
     CK(cudaGetLastError());
-    // heaviest rows first: each rebuild records its rows' work for the next
-    // one; after a new matching the estimate is computed afresh
-    if (!ctx->work_valid) {
-        k_row_work<W16><<<(n + 7) / 8, 256, 0, ctx->st>>>(g, ctx->is_hub, ctx->wkeys, ctx->wvals, nullptr);
-        CK(cudaGetLastError());
-    }
-    CK(cudaMemsetAsync(ctx->work_sum, 0, sizeof(unsigned long long), ctx->st));
-    size_t tb = ctx->cub_bytes;
-    CK(cub::DeviceRadixSort::SortPairsDescending(ctx->cub_tmp, tb, ctx->wkeys, ctx->wkeys_sorted,
-                                                 ctx->wvals, ctx->order, n, 0, 32, ctx->st));
-    CK(cudaMemsetAsync(ctx->small, 0, sizeof(int), ctx->st));
     CK(cudaEventRecord(ctx->ev_hub, ctx->st));
     if (ctx->nh) {
         // hub in-edge terms up to the threshold: one exact u8 GEMM on the tensor cores into S
@@ -585,10 +598,8 @@ bm_status stage_profit(bm_ctx* ctx) {
     if (per_sm < 1) { set_err(ctx, "profit kernel does not fit (n=%d)", n); return BM_E_INPUT; }
     CK(cudaEventRecord(ctx->ev[4], ctx->st));
     k_profit<W16><<<ctx->num_sms * per_sm, 512, smem, ctx->st>>>(g, ctx->order, ctx->small,
-                                                                ctx->nh ? ctx->is_hub : nullptr, kHubT,
-                                                                ctx->wkeys, ctx->work_sum);
+                                                                ctx->nh ? ctx->is_hub : nullptr, kHubT, ctx->work_sum);
     CK(cudaGetLastError());
-    ctx->work_valid = true;
     CK(record_exact_mapping(ctx));
     CK(cudaEventRecord(ctx->ev[5], ctx->st));
     return BM_OK;
@@ -774,7 +785,7 @@ bm_status stage_combine(bm_ctx* ctx, int* all_out) {
         k_combine64<<<grid, 256, 0, ctx->st>>>(ctx->S, n, ctx->part, all_out);
     }
     CK(cudaGetLastError());
-    k_best_reduce<<<(n + 255) / 256, 256, 0, ctx->st>>>(ctx->part, n, t, ctx->rowbest);
+    k_best_reduce<<<(n + 31) / 32, 256, 0, ctx->st>>>(ctx->part, n, t, ctx->rowbest, ctx->small + 1);
     CK(cudaGetLastError());
     return BM_OK;
 }
@@ -793,23 +804,37 @@ static bm_status ensure_adj(bm_ctx* ctx) {
     return BM_OK;
 }
 
+// The set commit's control words, step results (zero between launches) and images.
+static cudaError_t ensure_set(bm_ctx* ctx) {
+    if (ctx->cset) return cudaSuccess;
+    const size_t bytes = (kSetCtlInts + kSetBufInts + (size_t)ctx->n) * sizeof(int);
+    const cudaError_t e = dalloc(ctx, &ctx->cset, bytes);
+    return e != cudaSuccess ? e : cudaMemsetAsync(ctx->cset, 0, bytes, ctx->st);
+}
+
+// ctx->ckeys[0, *count) sorted into ctx->ckeys_sorted, ~0 behind (with n >
+// kRankMax, ckeys holds ~0 behind its keys).
+static cudaError_t sort_keys(bm_ctx* ctx, const int* count) {
+    const int n = ctx->n;
+    if (n <= kRankMax) {
+        k_rank_sort<<<(n + 31) / 32, 256, 0, ctx->st>>>(ctx->ckeys, count, n, ctx->ckeys_sorted);
+        return cudaGetLastError();
+    }
+    size_t tb = ctx->cub_bytes;
+    return cub::DeviceRadixSort::SortKeys(ctx->cub_tmp, tb, ctx->ckeys, ctx->ckeys_sorted, n, 0, 64, ctx->st);
+}
+
 template <bool W16, int K>
 bm_status launch_set_commit(bm_ctx* ctx, const unsigned long long* keys, const int4* sets, int lim, int max_verify,
-                            int ctas, int stall) {
+                            int ctas, int stall, bool ctl_clear) {
     const int n = ctx->n;
-    constexpr size_t kCtl = 4;   // ints of the control words, rounded up to 16 bytes
-    static_assert(sizeof(SetCtl) <= kCtl * sizeof(int), "control words");
-    if (!ctx->cset) {
-        const size_t ints = kCtl + kSetBufInts + (size_t)n;
-        CK(dalloc(ctx, &ctx->cset, ints * sizeof(int)));
-        CK(cudaMemsetAsync(ctx->cset, 0, ints * sizeof(int), ctx->st));
-    } else {
-        CK(cudaMemsetAsync(ctx->cset, 0, kCtl * sizeof(int), ctx->st));
-    }
+    static_assert(sizeof(SetCtl) <= kSetCtlInts * sizeof(int), "control words");
+    CK(ensure_set(ctx));
+    if (!ctl_clear) CK(cudaMemsetAsync(ctx->cset, 0, kSetCtlInts * sizeof(int), ctx->st));
     SetArgs a;
     a.keys = keys; a.sets = sets; a.lim = lim; a.max_verify = max_verify; a.st = ctx->cstats;
     a.ctl = reinterpret_cast<SetCtl*>(ctx->cset);
-    a.buf = ctx->cset + kCtl;
+    a.buf = ctx->cset + kSetCtlInts;
     a.newp = a.buf + kSetBufInts;
     a.stall = stall;
     // a quarter of the list entries a step scans on average per CTA's thread:
@@ -832,17 +857,17 @@ bm_status launch_set_commit(bm_ctx* ctx, const unsigned long long* keys, const i
     return BM_OK;
 }
 
-template bm_status launch_set_commit<true, 2>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
-template bm_status launch_set_commit<false, 2>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
-template bm_status launch_set_commit<true, 3>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
-template bm_status launch_set_commit<false, 3>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
-template bm_status launch_set_commit<true, 4>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
-template bm_status launch_set_commit<false, 4>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int);
+template bm_status launch_set_commit<true, 2>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int, bool);
+template bm_status launch_set_commit<false, 2>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int, bool);
+template bm_status launch_set_commit<true, 3>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int, bool);
+template bm_status launch_set_commit<false, 3>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int, bool);
+template bm_status launch_set_commit<true, 4>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int, bool);
+template bm_status launch_set_commit<false, 4>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int, bool);
 
 const int* set_commit_err(bm_ctx* ctx) { return &reinterpret_cast<SetCtl*>(ctx->cset)->err; }
 
 bm_status set_commit_reset(bm_ctx* ctx) {
-    CK(cudaMemsetAsync(ctx->cset, 0, (4 + kSetBufInts) * sizeof(int), ctx->st));
+    CK(cudaMemsetAsync(ctx->cset, 0, (kSetCtlInts + kSetBufInts) * sizeof(int), ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return BM_OK;
 }
@@ -850,11 +875,12 @@ bm_status set_commit_reset(bm_ctx* ctx) {
 template <bool W16>
 static bm_status stage_commit(bm_ctx* ctx, const bm_sweep_opts* o) {
     const int n = ctx->n;
-    CK(cudaMemsetAsync(ctx->small + 1, 0, 2 * sizeof(int), ctx->st));
-    k_candidates<<<(n + 255) / 256, 256, 0, ctx->st>>>(ctx->rowbest, n, ctx->ckeys, ctx->small + 1, ctx->small + 2);
+    CK(ensure_set(ctx));
+    if (n > kRankMax) CK(cudaMemsetAsync(ctx->ckeys, 0xff, n * sizeof(unsigned long long), ctx->st));
+    k_candidates<<<(n + 255) / 256, 256, 0, ctx->st>>>(ctx->rowbest, n, ctx->ckeys, ctx->small + 1, ctx->small + 2,
+                                                       ctx->cset);
     CK(cudaGetLastError());
-    size_t tb = ctx->cub_bytes;
-    CK(cub::DeviceRadixSort::SortKeys(ctx->cub_tmp, tb, ctx->ckeys, ctx->ckeys_sorted, n, 0, 64, ctx->st));
+    CK(sort_keys(ctx, ctx->small + 1));
     const int max_scan = o ? o->max_candidates : 0;
     const int max_verify = o ? o->max_verify : -1;
     const int lim = (max_scan > 0 && max_scan < n) ? max_scan : n;
@@ -866,7 +892,7 @@ static bm_status stage_commit(bm_ctx* ctx, const bm_sweep_opts* o) {
     }
     const int ctas = o && o->commit_ctas > 0 ? std::min(o->commit_ctas, kCommitMaxCtas) : 0;
     return launch_set_commit<W16, 2>(ctx, ctx->ckeys_sorted, nullptr, lim, max_verify, ctas,
-                                     ctas != 1 ? take_stall(BM_STALL_COMMIT) : 0);
+                                     ctas != 1 ? take_stall(BM_STALL_COMMIT) : 0, true);
 }
 
 extern "C" bm_status bm_all_deltas(bm_ctx* ctx, int32_t* out) {
@@ -1259,19 +1285,18 @@ static bm_status triple_round_impl(bm_ctx* ctx, const bm_triple_opts* o, bm_trip
     if (s) return s;
     CK(cudaEventRecord(ctx->ev[1], ctx->st));
     CK(cudaMemsetAsync(ctx->tcount, 0, 2 * sizeof(unsigned long long), ctx->st));
+    if (n > kRankMax) CK(cudaMemsetAsync(ctx->ckeys, 0xff, n * sizeof(unsigned long long), ctx->st));
     const int blocks = std::min(n, ctx->num_sms * 8);
     k_triple_eval<W16><<<blocks, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->adj, ctx->adj_words, partners,
                                                     o->seed, ctx->ckeys, ctx->tcount);
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev[2], ctx->st));
-    size_t tb = ctx->cub_bytes;
-    CK(cub::DeviceRadixSort::SortKeys(ctx->cub_tmp, tb, ctx->ckeys, ctx->ckeys_sorted, n, 0, 64, ctx->st));
+    CK(sort_keys(ctx, reinterpret_cast<int*>(ctx->tcount + 1)));
     if (!ctx->csets) CK(dalloc(ctx, &ctx->csets, (size_t)n * sizeof(int4)));
-    k_triple_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets,
-                                                           ctx->tcount + 1);
+    k_triple_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets);
     CK(cudaGetLastError());
     const int lim = o->max_candidates > 0 ? std::min(o->max_candidates, n) : n;
-    if ((s = launch_set_commit<W16, 3>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0, 0))) return s;
+    if ((s = launch_set_commit<W16, 3>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0, 0, false))) return s;
     CK(cudaEventRecord(ctx->ev[3], ctx->st));
     CommitStats cs;
     unsigned long long cnt[2], top = 0;
@@ -1361,19 +1386,18 @@ static bm_status quad_round_impl(bm_ctx* ctx, const bm_quad_opts* o, bm_quad_sta
     if (s) return s;
     CK(cudaEventRecord(ctx->ev[1], ctx->st));
     CK(cudaMemsetAsync(ctx->tcount, 0, 2 * sizeof(unsigned long long), ctx->st));
+    if (n > kRankMax) CK(cudaMemsetAsync(ctx->ckeys, 0xff, n * sizeof(unsigned long long), ctx->st));
     const int blocks = std::min(n, ctx->num_sms * 8);
     k_quad_eval<W16><<<blocks, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->adj, ctx->adj_words, partners, o->seed,
                                                   ctx->ckeys, ctx->tcount);
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev[2], ctx->st));
-    size_t tb = ctx->cub_bytes;
-    CK(cub::DeviceRadixSort::SortKeys(ctx->cub_tmp, tb, ctx->ckeys, ctx->ckeys_sorted, n, 0, 64, ctx->st));
+    CK(sort_keys(ctx, reinterpret_cast<int*>(ctx->tcount + 1)));
     if (!ctx->csets) CK(dalloc(ctx, &ctx->csets, (size_t)n * sizeof(int4)));
-    k_quad_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets,
-                                                           ctx->tcount + 1);
+    k_quad_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets);
     CK(cudaGetLastError());
     const int lim = o->max_candidates > 0 ? std::min(o->max_candidates, n) : n;
-    if ((s = launch_set_commit<W16, 4>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0, 0))) return s;
+    if ((s = launch_set_commit<W16, 4>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0, 0, false))) return s;
     CK(cudaEventRecord(ctx->ev[3], ctx->st));
     CommitStats cs;
     unsigned long long cnt[2], top = 0;

@@ -40,8 +40,7 @@ struct bm_ctx {
     int* S = nullptr;
     unsigned long long* rowbest = nullptr;
     unsigned long long *ckeys = nullptr, *ckeys_sorted = nullptr;
-    unsigned long long *wkeys = nullptr, *wkeys_sorted = nullptr;
-    int *wvals = nullptr, *order = nullptr;
+    int* order = nullptr;          // profit rows, heaviest first
     void* cub_tmp = nullptr;
     size_t cub_bytes = 0;
     int* small = nullptr;          // [0]=row counter [1]=ncand [2]=best delta
@@ -67,7 +66,6 @@ struct bm_ctx {
     cudaEvent_t ev[6] = {};
     cudaEvent_t uev[8] = {};       // bm_timer_* slots
     unsigned long long* work_sum = nullptr;   // min terms of the last rebuild
-    bool work_valid = false;                  // wkeys hold the last rebuild's row work (scheduling keys)
     unsigned long long* part = nullptr;   // per-tile best partners (combine)
     // TMA-fed combine (n % 4 == 0): tensor map over S, S's diagonal, grid size
     alignas(64) CUtensorMap tmS;
@@ -143,10 +141,11 @@ template <bool W16> bm_status stage_refresh(bm_ctx* ctx, int* mode);
 bm_status stage_combine(bm_ctx* ctx, int* all_out);
 // Enqueues the set commit of the first lim sorted candidate keys (K = 2: pairs
 // in the keys; K = 3, 4: the sets in `sets`) on ctx's stream; statistics go to
-// ctx->cstats.  ctas <= 0: as many CTAs as the window's lists need.
+// ctx->cstats.  ctas <= 0: as many CTAs as the window's lists need; ctl_clear:
+// an earlier kernel cleared the control words (ctx->cset).
 template <bool W16, int K>
 bm_status launch_set_commit(bm_ctx* ctx, const unsigned long long* keys, const int4* sets, int lim, int max_verify,
-                            int ctas, int stall);
+                            int ctas, int stall, bool ctl_clear = false);
 // Error word of the last set commit (device), and the clean-up after a wait of
 // it ran out.
 const int* set_commit_err(bm_ctx* ctx);

@@ -80,48 +80,40 @@ template <bool W16> struct DevView {
 __device__ __forceinline__ int imin(int a, int b) { return a < b ? a : b; }
 
 // ---------------------------------------------------------------------------
-// Relabel list ids through a map (p for G1 lists, pinv for G2 lists).
+// Relabel list ids through a map (p for G1 lists, pinv for G2 lists), all lists
+// in one launch: 16 bytes per thread, the lists end to end.  Five launches of
+// 4-byte entries took 48 us at E = 5e6, this one 26 (160 MB).  Thread 0 also
+// clears the rebuild's counters.
+constexpr int kRelabelLists = 5;
+template <bool W16> struct RelabelLists {
+    const typename Ent<W16>::T* in[kRelabelLists];
+    typename Ent<W16>::T* out[kRelabelLists];
+    const int* map[kRelabelLists];
+    long long len[kRelabelLists];
+    int* row_counter;
+    unsigned long long* work_total;
+};
 template <bool W16>
-__global__ void k_relabel(const typename Ent<W16>::T* __restrict__ in,
-                          typename Ent<W16>::T* __restrict__ out, long long m,
-                          const int* __restrict__ map) {
+__global__ void __launch_bounds__(256) k_relabel(const __grid_constant__ RelabelLists<W16> a) {
     typedef Ent<W16> EN;
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    long long stride = (long long)gridDim.x * blockDim.x;
-    for (; i < m; i += stride) {
-        typename EN::T e = in[i];
-        out[i] = EN::make(__ldg(&map[EN::id(e)]), EN::w(e));
-    }
-}
-
-// Work estimate of a profit row: number of min terms it scatters.
-template <bool W16>
-__global__ void k_row_work(DevView<W16> g, const unsigned char* __restrict__ is_hub,
-                           unsigned long long* __restrict__ key, int* __restrict__ val,
-                           unsigned long long* __restrict__ total) {
-    typedef Ent<W16> EN;
-    const int lane = threadIdx.x & 31;
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int a = warp; a < g.n; a += nwarps) {
-        long long w = 0;
-        for (int i = g.off1o[a] + lane; i < g.off1o[a + 1]; i += 32) {
-            int f = EN::id(g.ent1oP[i]);
-            w += g.off2i[f + 1] - g.off2i[f];
+    typedef typename EN::T E;
+    constexpr int V = 16 / sizeof(E);   // entries per 16 bytes
+    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    if (tid == 0) { *a.row_counter = 0; *a.work_total = 0; }
+#pragma unroll
+    for (int l = 0; l < kRelabelLists; l++) {
+        const E* in = a.in[l];
+        E* out = a.out[l];
+        const int* map = a.map[l];
+        const long long m = a.len[l], mv = m / V;
+        for (long long i = tid; i < mv; i += step) {
+            union { uint4 q; E e[V]; } x;
+            x.q = reinterpret_cast<const uint4*>(in)[i];
+#pragma unroll
+            for (int u = 0; u < V; u++) x.e[u] = EN::make(__ldg(&map[EN::id(x.e[u])]), EN::w(x.e[u]));
+            reinterpret_cast<uint4*>(out)[i] = x.q;
         }
-        for (int i = g.off1i[a] + lane; i < g.off1i[a + 1]; i += 32) {
-            if (is_hub && is_hub[EN::id(g.ent1i[i])]) continue;  // tensor-core term
-            int f = EN::id(g.ent1iP[i]);
-            w += g.off2o[f + 1] - g.off2o[f];
-        }
-        for (int o = 16; o; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-        if (lane == 0) {
-            if (total) atomicAdd(total, (unsigned long long)w);   // min terms the row scatters
-            w += (g.off1o[a + 1] - g.off1o[a]) + (g.off1i[a + 1] - g.off1i[a]);
-            if (g.offs[a + 1] > g.offs[a]) w += g.n;
-            key[a] = (unsigned long long)min(w, 0xffffffffLL);   // 32-bit sort keys
-            val[a] = a;
-        }
+        for (long long i = mv * V + tid; i < m; i += step) out[i] = EN::make(__ldg(&map[EN::id(in[i])]), EN::w(in[i]));
     }
 }
 
@@ -179,13 +171,11 @@ __device__ __forceinline__ void scatter_residual(int* acc, const typename Ent<W1
 // whole block (NT = 0), or the NT threads (a power of two) of the block's
 // NT-aligned group; `sync` is a barrier over exactly those threads.  It ends
 // with a barrier.  acc holds n+1 ints of shared memory.
-// With `work`, the row also records its scheduling key for the next rebuild
-// (its scattered min terms + its edges + n if it has self-loops, the
-// estimate k_row_work makes) in work[a], and adds its terms to *work_total.
+// With `work_total`, the row adds its scattered min terms to it.
 template <bool W16, int NT, typename Sync>
 __device__ __forceinline__ void profit_row_on(const DevView<W16>& g, int a, int* acc, int2* s_long, int* s_nlong,
                                               const unsigned char* __restrict__ is_hub, int hub_thr, int* s_terms,
-                                              unsigned long long* work, unsigned long long* work_total, Sync sync) {
+                                              unsigned long long* work_total, Sync sync) {
     static_assert(NT == 0 || (NT & (NT - 1)) == 0, "group size is a power of two");
     typedef Ent<W16> EN;
     typedef typename EN::T E;
@@ -195,7 +185,7 @@ __device__ __forceinline__ void profit_row_on(const DevView<W16>& g, int a, int*
     const int lane = tid & 31, wid = tid >> 5, nw = nthr >> 5;
     if (tid == 0) {
         *s_nlong = 0;
-        if (work) *s_terms = 0;
+        if (work_total) *s_terms = 0;
     }
     // the row's scattered terms start from zero; with hubs, the tensor-core
     // hub terms already in S are added when the row is written back
@@ -231,7 +221,7 @@ __device__ __forceinline__ void profit_row_on(const DevView<W16>& g, int a, int*
                 b1 = off[f + 1];
             }
         }
-        if (work) {   // the chunk's scattered terms
+        if (work_total) {   // the chunk's scattered terms
             int c = kind ? b1 - b0 : 0;
             for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
             if (lane == 0 && c) atomicAdd(s_terms, c);
@@ -300,12 +290,7 @@ __device__ __forceinline__ void profit_row_on(const DevView<W16>& g, int a, int*
         }
     }
     sync();
-    if (work && tid == 0) {
-        const long long terms = *s_terms;
-        atomicAdd(work_total, (unsigned long long)terms);
-        long long w = terms + tot + (g.offs[a + 1] > g.offs[a] ? n : 0);
-        work[a] = (unsigned long long)min(w, 0xffffffffLL);
-    }
+    if (work_total && tid == 0) atomicAdd(work_total, (unsigned long long)*s_terms);
     int* row = g.S + (size_t)a * (size_t)n;
     if ((n & 3) == 0) {
         int4* r4 = reinterpret_cast<int4*>(row);
@@ -342,17 +327,15 @@ __device__ __forceinline__ void profit_row_on(const DevView<W16>& g, int a, int*
 template <bool W16>
 __device__ __forceinline__ void profit_row(const DevView<W16>& g, int a, int* acc, int2* s_long, int* s_nlong,
                                            const unsigned char* __restrict__ is_hub, int hub_thr,
-                                           int* s_terms = nullptr, unsigned long long* work = nullptr,
-                                           unsigned long long* work_total = nullptr) {
-    profit_row_on<W16, 0>(g, a, acc, s_long, s_nlong, is_hub, hub_thr, s_terms, work, work_total,
+                                           int* s_terms = nullptr, unsigned long long* work_total = nullptr) {
+    profit_row_on<W16, 0>(g, a, acc, s_long, s_nlong, is_hub, hub_thr, s_terms, work_total,
                           [] { __syncthreads(); });
 }
 
 template <bool W16>
 __global__ void __launch_bounds__(512, 3)
 k_profit(DevView<W16> g, const int* __restrict__ order, int* __restrict__ counter,
-         const unsigned char* __restrict__ is_hub, int hub_thr, unsigned long long* __restrict__ work,
-         unsigned long long* __restrict__ work_total) {
+         const unsigned char* __restrict__ is_hub, int hub_thr, unsigned long long* __restrict__ work_total) {
     extern __shared__ int acc[];
     __shared__ int s_row, s_nlong, s_terms;
     __shared__ int2 s_long[kLongQueue];  // (G2 vertex, w1 | kind << 31)
@@ -361,7 +344,7 @@ k_profit(DevView<W16> g, const int* __restrict__ order, int* __restrict__ counte
         __syncthreads();
         const int r = s_row;
         if (r >= g.n) break;
-        profit_row<W16>(g, order[r], acc, s_long, &s_nlong, is_hub, hub_thr, &s_terms, work, work_total);
+        profit_row<W16>(g, order[r], acc, s_long, &s_nlong, is_hub, hub_thr, &s_terms, work_total);
     }
 }
 
@@ -375,22 +358,36 @@ __device__ __forceinline__ unsigned long long kmax(unsigned long long x, unsigne
     return x > y ? x : y;
 }
 
+// Appends the warp's keys (lanes with `has`) to keys[*count ...], in any order.
+// All lanes call it.
+__device__ __forceinline__ void append_key(bool has, unsigned long long key, unsigned long long* __restrict__ keys,
+                                           int* __restrict__ count) {
+    const int lane = threadIdx.x & 31;
+    const unsigned m = __ballot_sync(0xffffffffu, has);
+    if (!m) return;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(count, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (has) keys[at + __popc(m & ((1u << lane) - 1u))] = key;
+}
+
 // Candidate keys: one per row whose best partner improves, deduplicated when
 // two rows pick each other.  Sort key: (0x7fffffff - delta) << 32 | lo << 16 | hi
-// -> ascending order = delta desc, lo asc, hi asc.  Rows without a candidate
-// get ~0.
+// -> ascending order = delta desc, lo asc, hi asc.  ctl: kSetCtlInts words of
+// the set commit that follows, cleared here.
+constexpr int kSetCtlInts = 4;
 static __global__ void k_candidates(const unsigned long long* __restrict__ rowbest, int n,
                              unsigned long long* __restrict__ keys, int* __restrict__ ncand,
-                             int* __restrict__ best_delta) {
+                             int* __restrict__ best_delta, int* __restrict__ ctl) {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= n) return;
-    const unsigned long long k = rowbest[a];
+    if (a < kSetCtlInts) ctl[a] = 0;
+    const unsigned long long k = a < n ? rowbest[a] : 0ull;
     unsigned long long out = ~0ull;
+    int d = 0;
     if (k) {
-        const int d = (int)((unsigned)(k >> 32) - 0x80000000u);
+        d = max((int)((unsigned)(k >> 32) - 0x80000000u), 0);
         const int b = (int)(~(unsigned)(k & 0xffffffffu));
         if (d > 0) {
-            atomicMax(best_delta, d);
             const unsigned long long kb = rowbest[b];
             const int bb = (int)(~(unsigned)(kb & 0xffffffffu));
             const bool mutual = (kb != 0) && (bb == a);
@@ -398,11 +395,49 @@ static __global__ void k_candidates(const unsigned long long* __restrict__ rowbe
                 const int lo = a < b ? a : b, hi = a < b ? b : a;
                 out = ((unsigned long long)(0x7fffffffu - (unsigned)d) << 32) |
                       ((unsigned long long)lo << 16) | (unsigned long long)hi;
-                atomicAdd(ncand, 1);
             }
         }
     }
-    keys[a] = out;
+    d = __reduce_max_sync(0xffffffffu, d);
+    if ((threadIdx.x & 31) == 0 && d > 0) atomicMax(best_delta, d);
+    append_key(out != ~0ull, out, keys, ncand);
+}
+
+// Sorts the distinct keys[0, *count) into sorted[0, *count) and fills
+// sorted[*count, n) with ~0: each key's place is the number of smaller keys, a
+// warp counting for kRankKeys keys at once.  Quadratic, but one launch that
+// reads the keys from L1 (980, 5,200 and 17,000 keys: 6, 17 and 57 us) where a
+// radix sort of 64-bit keys takes ten launches over all n (12 us for a single
+// tile, 65 to 80 us from a few thousand keys); beyond kRankMax keys the radix
+// sort wins.
+constexpr int kRankKeys = 4, kRankMax = 20480;
+static __global__ void __launch_bounds__(256) k_rank_sort(const unsigned long long* __restrict__ keys,
+                                                          const int* __restrict__ count, int n,
+                                                          unsigned long long* __restrict__ sorted) {
+    constexpr int per = 8 * kRankKeys;   // keys of a block
+    const int m = *count;
+    const int lane = threadIdx.x & 31;
+    {
+        const int i = blockIdx.x * per + threadIdx.x;
+        if (threadIdx.x < per && i >= m && i < n) sorted[i] = ~0ull;
+    }
+    const int i0 = blockIdx.x * per + (threadIdx.x >> 5) * kRankKeys;
+    if (i0 >= m) return;
+    unsigned long long k[kRankKeys];
+    int at[kRankKeys];
+#pragma unroll
+    for (int u = 0; u < kRankKeys; u++) { k[u] = keys[min(i0 + u, m - 1)]; at[u] = 0; }
+#pragma unroll 8
+    for (int j = lane; j < m; j += 32) {
+        const unsigned long long x = __ldg(&keys[j]);
+#pragma unroll
+        for (int u = 0; u < kRankKeys; u++) at[u] += x < k[u];
+    }
+#pragma unroll
+    for (int u = 0; u < kRankKeys; u++) {
+        at[u] = __reduce_add_sync(0xffffffffu, at[u]);
+        if (lane == u && i0 + u < m) sorted[at[u]] = k[u];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -532,23 +567,42 @@ __global__ void k_pair_deltas(DevView<W16> g, const int* __restrict__ pa, const 
     }
 }
 
-// Alignment score (src/graph-alignment-optimized.c:292-307): one warp per row.
+// Row of CSR entry i: the last row r with off[r] <= i, r in [0, n).
+__device__ __forceinline__ int row_of(const int* __restrict__ off, int n, int i) {
+    int lo = 0, hi = n;   // off[lo] <= i < off[hi]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (off[mid] <= i) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// Alignment score (src/graph-alignment-optimized.c:292-307).  A warp takes
+// kScoreRun consecutive G1 entries, whatever their rows: with a warp per row
+// the power-law rows' longest held the launch (54 us at n = 8,192 / E = 1e6).
+constexpr int kScoreRun = 128;
 template <bool W16>
-__global__ void k_score(DevView<W16> g, unsigned long long* __restrict__ out) {
+__global__ void k_score(DevView<W16> g, int m, unsigned long long* __restrict__ out) {
     typedef Ent<W16> EN;
     const int lane = threadIdx.x & 31;
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     long long s = 0;
-    for (int a = warp; a < g.n; a += nwarps) {
-        const int pa = g.p[a];
-        for (int i = g.off1o[a] + lane; i < g.off1o[a + 1]; i += 32) {
+    for (long long r0 = (long long)warp * kScoreRun; r0 < m; r0 += (long long)nwarps * kScoreRun) {
+        int a = row_of(g.off1o, g.n, (int)r0), end = g.off1o[a + 1];
+        const int r1 = (int)min((long long)m, r0 + kScoreRun);
+#pragma unroll
+        for (int u = 0; u < kScoreRun / 32; u++) {
+            const int i = (int)r0 + 32 * u + lane;
+            if (i >= r1) continue;
+            while (i >= end) end = g.off1o[++a + 1];
             const typename EN::T e = g.ent1o[i];
-            s += imin(EN::w(e), g.w2(pa, g.p[EN::id(e)]));
+            s += imin(EN::w(e), g.w2(g.p[a], g.p[EN::id(e)]));
         }
-        if (lane == 0)
-            for (int q = g.offs[a]; q < g.offs[a + 1]; q++) s += imin(g.selfw[q], g.w2(pa, pa));
     }
+    const int loops = g.offs[g.n];   // G1 self-loops
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < loops; i += gridDim.x * blockDim.x)
+        s += imin(g.selfw[i], g.w2d(g.p[row_of(g.offs, g.n, i)]));
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0 && s) atomicAdd(out, (unsigned long long)s);
 }

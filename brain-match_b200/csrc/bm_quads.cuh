@@ -216,7 +216,7 @@ __device__ void quad_best(const DevView<W16>& g, const unsigned* __restrict__ ad
 template <bool W16>
 __global__ void __launch_bounds__(256)
 k_quad_eval(DevView<W16> g, const unsigned* __restrict__ adj, int words, int partners, unsigned long long seed,
-            unsigned long long* __restrict__ keys, unsigned long long* __restrict__ counters /* [0] valid sets */) {
+            unsigned long long* __restrict__ keys, unsigned long long* __restrict__ counters /* [0] = valid sets, [1] = candidates */) {
     __shared__ unsigned long long best[8];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (int a = blockIdx.x; a < g.n; a += gridDim.x) {
@@ -246,21 +246,18 @@ k_quad_eval(DevView<W16> g, const unsigned* __restrict__ adj, int words, int par
         if (tid == 0) {
             unsigned long long m = best[0];
             for (int i = 1; i < (int)(blockDim.x >> 5); i++) m = best[i] < m ? best[i] : m;
-            keys[a] = m;
+            if (m != ~0ull) keys[atomicAdd(reinterpret_cast<int*>(counters + 1), 1)] = m;
         }
         __syncthreads();
     }
 }
 
-// The sets of the sorted 4-set candidates for the set commit (SetArgs::sets),
-// and the number of candidates (*count, zero before).
+// The sets of the sorted 4-set candidates for the set commit (SetArgs::sets).
 template <bool W16>
 __global__ void k_quad_sets(DevView<W16> g, const unsigned long long* __restrict__ keys, unsigned long long seed,
-                            int4* __restrict__ sets, unsigned long long* __restrict__ count) {
+                            int4* __restrict__ sets) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned long long key = i < g.n ? keys[i] : ~0ull;
-    const unsigned valid = __ballot_sync(0xffffffffu, key != ~0ull);
-    if ((threadIdx.x & 31) == 0 && valid) atomicAdd(count, (unsigned long long)__popc(valid));
     if (key == ~0ull) return;
     const int a = (int)((key >> 16) & 0xffffu), j = (int)((key >> 5) & 0x7ffu), q = (int)(key & 31u);
     int b = 0, c = 0, d = 0;

@@ -123,14 +123,28 @@ k_combine64(const int* __restrict__ S, int n, unsigned long long* __restrict__ p
     combine_tile<kTile>(S, n, ti, tj, part, all_out);
 }
 
-// rowbest[x] = max over tile columns t of part[t][x]
-static __global__ void k_best_reduce(const unsigned long long* __restrict__ part, int n, int tiles,
-                              unsigned long long* __restrict__ rowbest) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= n) return;
+// rowbest[x] = max over tile columns t of part[t][x]; 32 vertices per block,
+// its 8 warps sharing the tile columns (a thread per vertex walking them all
+// took 16 us at n = 8,192).  Also clears the candidate count and best delta.
+static __global__ void __launch_bounds__(256) k_best_reduce(const unsigned long long* __restrict__ part, int n, int tiles,
+                                                            unsigned long long* __restrict__ rowbest,
+                                                            int* __restrict__ counters) {
+    __shared__ unsigned long long s_k[8][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int x = blockIdx.x * 32 + lane;
+    if (blockIdx.x == 0 && threadIdx.x < 2) counters[threadIdx.x] = 0;
     unsigned long long k = 0;
-    for (int t = 0; t < tiles; t++) k = kmax(k, part[(size_t)t * n + x]);
-    rowbest[x] = k;
+    if (x < n) {
+#pragma unroll 4
+        for (int t = wid; t < tiles; t += 8) k = kmax(k, part[(size_t)t * n + x]);
+    }
+    s_k[wid][lane] = k;
+    __syncthreads();
+    if (wid == 0 && x < n) {
+#pragma unroll
+        for (int w = 1; w < 8; w++) k = kmax(k, s_k[w][lane]);
+        rowbest[x] = k;
+    }
 }
 
 // ---------------------------------------------------------------------------

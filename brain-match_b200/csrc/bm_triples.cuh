@@ -187,12 +187,13 @@ __global__ void k_adj_bits(DevView<W16> g, unsigned* __restrict__ bits, int word
 // Sample `partners` triples per vertex, evaluate both rotations from S and
 // keep, per vertex a, the best improving (delta, slot, rotation) as a sort key
 //   (0x7fffffff - delta) << 32 | a << 16 | slot << 1 | rot     (~0 if none)
-// so ascending order is delta desc, a asc, slot asc, rotation asc.
+// so ascending order is delta desc, a asc, slot asc, rotation asc; the keys are
+// appended in any order.
 template <bool W16>
 __global__ void __launch_bounds__(256)
 k_triple_eval(DevView<W16> g, const unsigned* __restrict__ adj, int words, int partners,
               unsigned long long seed, unsigned long long* __restrict__ keys,
-              unsigned long long* __restrict__ counters /* [0]=valid triples */) {
+              unsigned long long* __restrict__ counters /* [0] = valid triples, [1] = candidates */) {
     __shared__ unsigned long long best[8];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (int a = blockIdx.x; a < g.n; a += gridDim.x) {
@@ -221,21 +222,18 @@ k_triple_eval(DevView<W16> g, const unsigned* __restrict__ adj, int words, int p
         if (tid == 0) {
             unsigned long long m = best[0];
             for (int i = 1; i < (int)(blockDim.x >> 5); i++) m = best[i] < m ? best[i] : m;
-            keys[a] = m;
+            if (m != ~0ull) keys[atomicAdd(reinterpret_cast<int*>(counters + 1), 1)] = m;
         }
         __syncthreads();
     }
 }
 
-// The sets of the sorted 3-cycle candidates for the set commit (SetArgs::sets),
-// and the number of candidates (*count, zero before).
+// The sets of the sorted 3-cycle candidates for the set commit (SetArgs::sets).
 template <bool W16>
 __global__ void k_triple_sets(DevView<W16> g, const unsigned long long* __restrict__ keys, unsigned long long seed,
-                              int4* __restrict__ sets, unsigned long long* __restrict__ count) {
+                              int4* __restrict__ sets) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned long long key = i < g.n ? keys[i] : ~0ull;
-    const unsigned valid = __ballot_sync(0xffffffffu, key != ~0ull);
-    if ((threadIdx.x & 31) == 0 && valid) atomicAdd(count, (unsigned long long)__popc(valid));
     if (key == ~0ull) return;
     const int a = (int)((key >> 16) & 0xffffu), j = (int)((key >> 1) & 0x7fffu);
     int b = 0, c = 0;

@@ -73,3 +73,18 @@ def test_rounds_match_oracle(shape, n, flags, max_candidates, max_verify):
                 assert {k: st[k] for k in COUNTS} == {k: ost[k] for k in COUNTS}
                 np.testing.assert_array_equal(E.get_mapping(), m)
         assert E.score() == O.score(m)
+
+
+@pytest.mark.parametrize("n", [2, 31, 33, 20480, 20481])
+def test_candidate_sort_at_its_edges(n):
+    """Below, at and above the largest size the counting sort takes, and fewer
+    rows than one of its blocks; sparse pairs keep the oracle quick."""
+    g = bm.generate(bm.gen_params(n=n, e=max(1, n // 2), seed=n, wmax=60))
+    O = oracle.Oracle.from_pair(g)
+    m = g["map0"].copy()
+    with bm.Engine.from_pair(g) as E:
+        E.set_mapping(m)
+        st, ost = E.sweep(), O.sweep(m)
+        assert {k: st[k] for k in COUNTS} == {k: ost[k] for k in COUNTS}
+        np.testing.assert_array_equal(E.get_mapping(), m)
+        assert E.score() == O.score(m)
