@@ -817,7 +817,7 @@ static cudaError_t ensure_set(bm_ctx* ctx) {
 static cudaError_t sort_keys(bm_ctx* ctx, const int* count) {
     const int n = ctx->n;
     if (n <= kRankMax) {
-        k_rank_sort<<<(n + 31) / 32, 256, 0, ctx->st>>>(ctx->ckeys, count, n, ctx->ckeys_sorted);
+        k_rank_sort<false><<<(n + 31) / 32, 256, 0, ctx->st>>>(ctx->ckeys, count, n, ctx->ckeys_sorted);
         return cudaGetLastError();
     }
     size_t tb = ctx->cub_bytes;
@@ -1188,7 +1188,9 @@ static bm_status first_improvement_impl(bm_ctx* ctx, int max_passes, long long* 
     unsigned long long* slots = reinterpret_cast<unsigned long long*>(st + 1);
     int* contrib = reinterpret_cast<int*>(st + 1);
     if (rows) {
-        k_contrib_int<W16><<<(n + 7) / 8, 256, 0, ctx->st>>>(g, contrib);
+        CK(cudaMemsetAsync(contrib, 0, (size_t)n * sizeof(int), ctx->st));
+        k_contrib<W16><<<(int)std::min<long long>(ctx->num_sms * 8LL, ctx->e1 / (8 * kScoreRun) + 1), 256, 0, ctx->st>>>(
+            g, (int)ctx->e1, contrib);
         CK(cudaGetLastError());
     }
     FirstState h;

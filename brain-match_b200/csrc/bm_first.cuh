@@ -174,25 +174,6 @@ __global__ void __launch_bounds__(kFirstThreads) k_first(DevView<W16> g, FirstSt
     }
 }
 
-// Current contribution of every vertex: what its G1 edges and self-loops earn.
-template <bool W16>
-__global__ void k_contrib_int(DevView<W16> g, int* __restrict__ C) {
-    typedef Ent<W16> EN;
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; a < g.n; a += nw) {
-        const int pa = g.p[a];
-        int s = 0;
-        for (int i = g.off1o[a] + lane; i < g.off1o[a + 1]; i += 32)
-            s += imin(EN::w(g.ent1o[i]), g.w2(pa, g.p[EN::id(g.ent1o[i])]));
-        for (int i = g.off1i[a] + lane; i < g.off1i[a + 1]; i += 32)
-            s += imin(EN::w(g.ent1i[i]), g.w2t(g.p[EN::id(g.ent1i[i])], pa));
-        for (int q = g.offs[a] + lane; q < g.offs[a + 1]; q += 32) s += imin(g.selfw[q], g.w2d(pa));
-        s = __reduce_add_sync(0xffffffffu, s);
-        if (lane == 0) C[a] = s;
-    }
-}
-
 // Shared memory of k_first_rows: acc (n + 1), C (n), matching and its inverse.
 __host__ __device__ inline size_t first_rows_smem(int n) {
     return (2 * (size_t)n + 1) * sizeof(int) + 2 * ((size_t)n + 1) * sizeof(unsigned short);

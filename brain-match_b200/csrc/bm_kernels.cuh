@@ -403,15 +403,16 @@ static __global__ void k_candidates(const unsigned long long* __restrict__ rowbe
     append_key(out != ~0ull, out, keys, ncand);
 }
 
-// Sorts the distinct keys[0, *count) into sorted[0, *count) and fills
-// sorted[*count, n) with ~0: each key's place is the number of smaller keys, a
-// warp counting for kRankKeys keys at once.  Quadratic, but one launch that
+// Sorts keys[0, *count) (distinct, or with DUP any) into sorted[0, *count) and
+// fills sorted[*count, n) with ~0: each key's place is the number of smaller
+// keys (equal ones by index), a warp counting for kRankKeys keys at once.  Quadratic, but one launch that
 // reads the keys from L1 (980, 5,200 and 17,000 keys: 6, 17 and 57 us) where a
 // radix sort of 64-bit keys takes ten launches over all n (12 us for a single
 // tile, 65 to 80 us from a few thousand keys); beyond kRankMax keys the radix
 // sort wins.
 constexpr int kRankKeys = 4, kRankMax = 20480;
-static __global__ void __launch_bounds__(256) k_rank_sort(const unsigned long long* __restrict__ keys,
+template <bool DUP>
+__global__ void __launch_bounds__(256) k_rank_sort(const unsigned long long* __restrict__ keys,
                                                           const int* __restrict__ count, int n,
                                                           unsigned long long* __restrict__ sorted) {
     constexpr int per = 8 * kRankKeys;   // keys of a block
@@ -431,7 +432,7 @@ static __global__ void __launch_bounds__(256) k_rank_sort(const unsigned long lo
     for (int j = lane; j < m; j += 32) {
         const unsigned long long x = __ldg(&keys[j]);
 #pragma unroll
-        for (int u = 0; u < kRankKeys; u++) at[u] += x < k[u];
+        for (int u = 0; u < kRankKeys; u++) at[u] += x < k[u] || (DUP && x == k[u] && j < i0 + u);
     }
 #pragma unroll
     for (int u = 0; u < kRankKeys; u++) {
@@ -441,61 +442,10 @@ static __global__ void __launch_bounds__(256) k_rank_sort(const unsigned long lo
 }
 
 // ---------------------------------------------------------------------------
-// Exact swap delta of (a,b) on the current matching, one element of the four
-// edge lists per thread of the group, as calculate_swap_delta computes it
+// Exact swap delta of (a,b) by `parts` warps, img(v) the matching: the sum of
+// part 0 .. parts - 1, each returned to every lane of its warp.  The four edge
+// lists of a and b as calculate_swap_delta walks them
 // (src/graph-alignment-optimized.c:321-408), plus the exact self-loop terms.
-template <bool W16>
-__device__ __forceinline__ int swap_delta_part(const DevView<W16>& g, int a, int b, int t, int nt) {
-    typedef Ent<W16> EN;
-    const int pa = g.p[a], pb = g.p[b];
-    int d = 0;
-    const int la0 = g.off1o[a], la = g.off1o[a + 1] - la0;
-    const int ia0 = g.off1i[a], ia = g.off1i[a + 1] - ia0;
-    const int lb0 = g.off1o[b], lb = g.off1o[b + 1] - lb0;
-    const int ib0 = g.off1i[b], ib = g.off1i[b + 1] - ib0;
-    const int tot = la + ia + lb + ib;
-    for (int k = t; k < tot; k += nt) {
-        int q = k;
-        if (q < la) {  // out-edge a->v
-            const typename EN::T e = g.ent1o[la0 + q];
-            const int v = EN::id(e), w = EN::w(e);
-            if (v == b) d += imin(w, g.w2(pb, pa)) - imin(w, g.w2(pa, pb));
-            else { const int pv = g.p[v]; d += imin(w, g.w2(pb, pv)) - imin(w, g.w2(pa, pv)); }
-            continue;
-        }
-        q -= la;
-        if (q < ia) {  // in-edge u->a
-            const typename EN::T e = g.ent1i[ia0 + q];
-            const int u = EN::id(e), w = EN::w(e);
-            if (u != b) { const int pu = g.p[u]; d += imin(w, g.w2(pu, pb)) - imin(w, g.w2(pu, pa)); }
-            continue;  // the edge b->a is counted once, from b's out-list
-        }
-        q -= ia;
-        if (q < lb) {  // out-edge b->v
-            const typename EN::T e = g.ent1o[lb0 + q];
-            const int v = EN::id(e), w = EN::w(e);
-            if (v == a) d += imin(w, g.w2(pa, pb)) - imin(w, g.w2(pb, pa));
-            else { const int pv = g.p[v]; d += imin(w, g.w2(pa, pv)) - imin(w, g.w2(pb, pv)); }
-            continue;
-        }
-        q -= lb;
-        {  // in-edge u->b
-            const typename EN::T e = g.ent1i[ib0 + q];
-            const int u = EN::id(e), w = EN::w(e);
-            if (u != a) { const int pu = g.p[u]; d += imin(w, g.w2(pu, pa)) - imin(w, g.w2(pu, pb)); }
-        }
-    }
-    if (t == 0) {
-        for (int q = g.offs[a]; q < g.offs[a + 1]; q++)
-            d += imin(g.selfw[q], g.w2(pb, pb)) - imin(g.selfw[q], g.w2(pa, pa));
-        for (int q = g.offs[b]; q < g.offs[b + 1]; q++)
-            d += imin(g.selfw[q], g.w2(pa, pa)) - imin(g.selfw[q], g.w2(pb, pb));
-    }
-    return d;
-}
-
-// The same delta by `parts` warps, img(v) the matching: the sum of part 0 ..
-// parts - 1, each returned to every lane of its warp.
 // Lanes load the list extents in one round, then take four entries each per
 // round: their entries, images and W2 terms are in flight together, so a pair
 // of 128 list entries costs three dependent loads instead of twelve.
@@ -605,6 +555,35 @@ __global__ void k_score(DevView<W16> g, int m, unsigned long long* __restrict__ 
         s += imin(g.selfw[i], g.w2d(g.p[row_of(g.offs, g.n, i)]));
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0 && s) atomicAdd(out, (unsigned long long)s);
+}
+
+// C[a] += what vertex a's G1 edges and self-loops earn now; one pass over the
+// G1 entries, dealt as in k_score (C zero before).  Most terms of an early
+// matching are zero and add nothing.
+template <bool W16>
+__global__ void k_contrib(DevView<W16> g, int m, int* __restrict__ C) {
+    typedef Ent<W16> EN;
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (long long r0 = (long long)warp * kScoreRun; r0 < m; r0 += (long long)nwarps * kScoreRun) {
+        int a = row_of(g.off1o, g.n, (int)r0), end = g.off1o[a + 1];
+        const int r1 = (int)min((long long)m, r0 + kScoreRun);
+#pragma unroll
+        for (int u = 0; u < kScoreRun / 32; u++) {
+            const int i = (int)r0 + 32 * u + lane;
+            if (i >= r1) continue;
+            while (i >= end) end = g.off1o[++a + 1];
+            const typename EN::T e = g.ent1o[i];
+            const int v = EN::id(e), t = imin(EN::w(e), g.w2(g.p[a], g.p[v]));
+            if (t) { atomicAdd(&C[a], t); atomicAdd(&C[v], t); }
+        }
+    }
+    const int loops = g.offs[g.n];   // G1 self-loops
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < loops; i += gridDim.x * blockDim.x) {
+        const int a = row_of(g.offs, g.n, i), t = imin(g.selfw[i], g.w2d(g.p[a]));
+        if (t) atomicAdd(&C[a], t);
+    }
 }
 
 // ---------------------------------------------------------------------------

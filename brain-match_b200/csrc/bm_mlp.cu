@@ -33,6 +33,8 @@
 namespace {
 
 constexpr int kFeat = 32;
+// evaluated pairs up to which their keys are sorted by counting (about half improve)
+constexpr int kLearnedRankMax = 2 * kRankMax;
 // exhaustive sweeps of the learned paths keep the profit matrix exact across
 // commits (updated from the moved vertices where that is cheaper): same moves
 const bm_sweep_opts kIncremental = {0, -1, 0, 1, {0, 0, 0, 0}};
@@ -41,30 +43,6 @@ constexpr int oW1 = 0, oB1 = oW1 + kMlpHid * kMlpIn, oW2 = oB1 + kMlpHid, oB2 = 
               oW3 = oB2 + kMlpHid, oB3 = oW3 + kMlpHid, kParams = oB3 + 1;
 
 // ---- features ----
-template <bool W16>
-__global__ void k_contrib(DevView<W16> g, float* __restrict__ contrib) {
-    typedef Ent<W16> EN;
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; a < g.n; a += nw) {
-        const int pa = g.p[a];
-        long long s = 0;
-        for (int i = g.off1o[a] + lane; i < g.off1o[a + 1]; i += 32) {
-            const typename EN::T e = g.ent1o[i];
-            s += imin(EN::w(e), g.w2(pa, g.p[EN::id(e)]));
-        }
-        for (int i = g.off1i[a] + lane; i < g.off1i[a + 1]; i += 32) {
-            const typename EN::T e = g.ent1i[i];
-            s += imin(EN::w(e), g.w2(g.p[EN::id(e)], pa));
-        }
-        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) {
-            for (int q = g.offs[a]; q < g.offs[a + 1]; q++) s += imin(g.selfw[q], g.w2(pa, pa));
-            contrib[a] = (float)s;
-        }
-    }
-}
-
 // Structural features of one graph (G1 lists if g2 == 0, else G2's): a warp
 // per vertex.
 template <bool W16>
@@ -113,58 +91,69 @@ __global__ void k_static_features(DevView<W16> g, int g2, float* __restrict__ F)
 }
 
 // Dynamic features 9, 10: current contribution (G2 side: of pinv(f)).
-__global__ void k_dyn_features(const float* __restrict__ contrib, const int* __restrict__ pinv, int n,
+__global__ void k_dyn_features(const int* __restrict__ contrib, const int* __restrict__ pinv, int n,
                                float* __restrict__ F1, float* __restrict__ F2) {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= n) return;
-    const float c = contrib[a];
+    const float c = (float)contrib[a];
     const float tot1 = expm1f(F1[(size_t)a * kFeat + 2]) + expm1f(F1[(size_t)a * kFeat + 3]);
     F1[(size_t)a * kFeat + 9] = log1pf(c);
     F1[(size_t)a * kFeat + 10] = c / (tot1 + 1.f);
     const int b = pinv[a];  // a read as a G2 vertex
-    const float c2 = b < n ? contrib[b] : 0.f;
+    const float c2 = b < n ? (float)contrib[b] : 0.f;
     const float tot2 = expm1f(F2[(size_t)a * kFeat + 2]) + expm1f(F2[(size_t)a * kFeat + 3]);
     F2[(size_t)a * kFeat + 9] = log1pf(c2);
     F2[(size_t)a * kFeat + 10] = c2 / (tot2 + 1.f);
 }
 
-// Column statistics of the features (block c: F1 column c for c < 32, F2
-// column c - 32): mean and 1/std (population), 0 for a constant column.
-__global__ void k_col_stats(const float* __restrict__ F1, const float* __restrict__ F2, int n,
-                            float* __restrict__ mean, float* __restrict__ scale) {
-    const int c = blockIdx.x;
-    const float* F = c < kFeat ? F1 : F2;
-    const int col = c & (kFeat - 1);
+// Column sums of the features and of their squares, in double: slot t of 256
+// sums rows t, t + 256, ...; block (w, g) folds slots 32 w .. 32 w + 31 of graph
+// g into part[g][w][column] (sums, then squares 8 * 32 further).  A warp reads
+// whole rows (a block per column read 4 bytes of each 128-byte row, 21 us at
+// n = 8,192; now 8).
+__global__ void __launch_bounds__(1024) k_col_sums(const float* __restrict__ F1, const float* __restrict__ F2, int n,
+                                                   double* __restrict__ part) {
+    __shared__ double ts[32][33], tq[32][33];
+    const float* F = blockIdx.y ? F2 : F1;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     double s = 0, q = 0;
-    for (int a = threadIdx.x; a < n; a += blockDim.x) {
-        const double v = F[(size_t)a * kFeat + col];
+#pragma unroll 4
+    for (int a = blockIdx.x * 32 + wid; a < n; a += 256) {
+        const double v = F[(size_t)a * kFeat + lane];
         s += v;
         q += v * v;
     }
-    __shared__ double rs[32], rq[32];
-    for (int o = 16; o; o >>= 1) { s += __shfl_xor_sync(0xffffffffu, s, o); q += __shfl_xor_sync(0xffffffffu, q, o); }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) { rs[wid] = s; rq[wid] = q; }
+    ts[wid][lane] = s;   // [slot][column]
+    tq[wid][lane] = q;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        s = 0; q = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) { s += rs[w]; q += rq[w]; }
-        const double mu = s / n, var = q / n - mu * mu;
-        const double sd = var > 0 ? sqrt(var) : 0.0;
-        mean[c] = (float)mu;
-        scale[c] = sd > 1e-6 ? (float)(1.0 / sd) : 0.f;
+    s = ts[lane][wid];   // lane = slot, warp = column
+    q = tq[lane][wid];
+    for (int o = 16; o; o >>= 1) { s += __shfl_xor_sync(0xffffffffu, s, o); q += __shfl_xor_sync(0xffffffffu, q, o); }
+    if (lane == 0) {
+        double* p = part + (size_t)blockIdx.y * 2 * 8 * kFeat + blockIdx.x * kFeat + wid;
+        p[0] = s;
+        p[8 * kFeat] = q;
     }
 }
 
-// F = (F - mean) * scale, column-wise (z-scores).
-__global__ void k_normalise(float* __restrict__ F1, float* __restrict__ F2, int n, const float* __restrict__ mean,
-                            const float* __restrict__ scale) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long half = (long long)n * kFeat;
-    if (i >= 2 * half) return;
-    const int c = (int)(i % kFeat) + (i < half ? 0 : kFeat);
-    float* F = i < half ? F1 + i : F2 + (i - half);
-    *F = (*F - mean[c]) * scale[c];
+// F = (F - mean) * scale, column-wise (z-scores): mean and 1/std (population),
+// 0 for a constant column, from the partial sums.  64 rows per block.
+__global__ void __launch_bounds__(256) k_normalise(float* __restrict__ F1, float* __restrict__ F2, int n,
+                                                   const double* __restrict__ part) {
+    __shared__ float mean[kFeat], scale[kFeat];
+    if (threadIdx.x < kFeat) {
+        const double* p = part + (size_t)blockIdx.y * 2 * 8 * kFeat + threadIdx.x;
+        double s = 0, q = 0;
+        for (int w = 0; w < 8; w++) { s += p[w * kFeat]; q += p[(8 + w) * kFeat]; }
+        const double mu = s / n, var = q / n - mu * mu;
+        const double sd = var > 0 ? sqrt(var) : 0.0;
+        mean[threadIdx.x] = (float)mu;
+        scale[threadIdx.x] = sd > 1e-6 ? (float)(1.0 / sd) : 0.f;
+    }
+    __syncthreads();
+    float* F = (blockIdx.y ? F2 : F1) + (size_t)blockIdx.x * 64 * kFeat;
+    const int m = min(64, n - (int)blockIdx.x * 64) * kFeat;
+    for (int i = threadIdx.x; i < m; i += 256) F[i] = (F[i] - mean[i & (kFeat - 1)]) * scale[i & (kFeat - 1)];
 }
 
 // Training batch: rows i < k take sample j = ((off + i) * mul + add) mod count,
@@ -274,22 +263,22 @@ __global__ void k_samples(DevView<W16> g, const unsigned long long* __restrict__
     }
 }
 
-// Exact deltas of many selected pairs, one 256-thread block per pair (a hub
-// pair's lists spread over eight warps instead of one).
+// Exact deltas of many selected pairs, four warps per pair (a hub pair's lists
+// would hold a single warp).
+constexpr int kPairWarps = 4;
 template <bool W16>
-__global__ void __launch_bounds__(256) k_pair_deltas_block(DevView<W16> g, const int* __restrict__ pa,
-                                                           const int* __restrict__ pb, long long k,
-                                                           int* __restrict__ out) {
-    __shared__ int part[8];
+__global__ void __launch_bounds__(32 * kPairWarps) k_pair_deltas_block(DevView<W16> g, const int* __restrict__ pa,
+                                                                      const int* __restrict__ pb, long long k,
+                                                                      int* __restrict__ out) {
+    __shared__ int part[kPairWarps];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (long long i = blockIdx.x; i < k; i += gridDim.x) {
-        int d = swap_delta_part<W16>(g, pa[i], pb[i], threadIdx.x, 256);
-        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        const int d = swap_delta_warp<W16>(g, [&](int v) { return g.p[v]; }, pa[i], pb[i], lane, wid, kPairWarps);
         if (lane == 0) part[wid] = d;
         __syncthreads();
         if (threadIdx.x == 0) {
             int t = 0;
-            for (int w = 0; w < 8; w++) t += part[w];
+            for (int w = 0; w < kPairWarps; w++) t += part[w];
             out[i] = t;
         }
         __syncthreads();
@@ -342,17 +331,17 @@ __global__ void k_gather_pairs(const int* __restrict__ idx, int k, const int* __
     qa[i] = pa[idx[i]]; qb[i] = pb[idx[i]];
 }
 
-// Candidate keys of exactly evaluated pairs (delta > 0), ~0 otherwise.
+// Candidate keys of exactly evaluated pairs with delta > 0, appended in any order
+// (a pair drawn twice appears twice).
 __global__ void k_learned_keys(const int* __restrict__ qa, const int* __restrict__ qb, const int* __restrict__ d,
-                               int k, unsigned long long* __restrict__ keys) {
+                               int k, unsigned long long* __restrict__ keys, int* __restrict__ count) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= k) return;
     unsigned long long out = ~0ull;
-    if (d[i] > 0) {
+    if (i < k && d[i] > 0) {
         const int lo = min(qa[i], qb[i]), hi = max(qa[i], qb[i]);
         out = ((unsigned long long)(0x7fffffffu - (unsigned)d[i]) << 32) | ((unsigned long long)lo << 16) | hi;
     }
-    keys[i] = out;
+    append_key(out != ~0ull, out, keys, count);
 }
 
 // Grow-only device buffer.
@@ -629,7 +618,7 @@ template <bool W16>
 static bm_status features(bm_ctx* ctx, bm_mlp* M) {
     const int n = ctx->n;
     const size_t fbytes = (size_t)n * kFeat * sizeof(float);
-    MK(M->contrib.need((size_t)n * sizeof(float)));
+    MK(M->contrib.need((size_t)n * sizeof(int)));
     MK(M->F1.need(fbytes));
     MK(M->F2.need(fbytes));
     DevView<W16> g = view<W16>(ctx);
@@ -644,15 +633,15 @@ static bm_status features(bm_ctx* ctx, bm_mlp* M) {
     }
     MK(cudaMemcpyAsync(M->F1.p, M->S1.p, fbytes, cudaMemcpyDeviceToDevice, M->cs));
     MK(cudaMemcpyAsync(M->F2.p, M->S2.p, fbytes, cudaMemcpyDeviceToDevice, M->cs));
-    k_contrib<W16><<<blocks, 256, 0, M->cs>>>(g, M->contrib.as<float>());
-    k_dyn_features<<<(n + 255) / 256, 256, 0, M->cs>>>(M->contrib.as<float>(), ctx->pinv, n, M->F1.as<float>(),
+    MK(cudaMemsetAsync(M->contrib.p, 0, (size_t)n * sizeof(int), M->cs));
+    k_contrib<W16><<<(int)std::min<long long>(ctx->num_sms * 8LL, ctx->e1 / (8 * kScoreRun) + 1), 256, 0, M->cs>>>(
+        g, (int)ctx->e1, M->contrib.as<int>());
+    k_dyn_features<<<(n + 255) / 256, 256, 0, M->cs>>>(M->contrib.as<int>(), ctx->pinv, n, M->F1.as<float>(),
                                                        M->F2.as<float>());
-    MK(M->fstat.need(4 * kFeat * sizeof(float)));
-    float* mean = M->fstat.as<float>();
-    k_col_stats<<<2 * kFeat, 256, 0, M->cs>>>(M->F1.as<float>(), M->F2.as<float>(), n, mean, mean + 2 * kFeat);
-    const long long tot = 2LL * n * kFeat;
-    k_normalise<<<(unsigned)((tot + 255) / 256), 256, 0, M->cs>>>(M->F1.as<float>(), M->F2.as<float>(), n, mean,
-                                                                   mean + 2 * kFeat);
+    MK(M->fstat.need(2 * 8 * 2 * kFeat * sizeof(double)));
+    double* part = M->fstat.as<double>();
+    k_col_sums<<<dim3(8, 2), 1024, 0, M->cs>>>(M->F1.as<float>(), M->F2.as<float>(), n, part);
+    k_normalise<<<dim3((n + 63) / 64, 2), 256, 0, M->cs>>>(M->F1.as<float>(), M->F2.as<float>(), n, part);
     MK(cudaGetLastError());
     return BM_OK;
 }
@@ -666,7 +655,7 @@ static bm_status rank_pairs_dev(bm_ctx* ctx, bm_mlp* M, const int* pa, const int
     if (!uv_current) {
         MK(M->U.need((size_t)n * kMlpHid * sizeof(float)));
         MK(M->V.need((size_t)n * kMlpHid * sizeof(float)));
-        k_uv<<<(n + 7) / 8, 256, 0, M->cs>>>(M->F1.as<float>(), M->F2.as<float>(), ctx->p, n, M->W1b, M->P + oB1,
+        k_uv<<<(n + kUvRows - 1) / kUvRows, 256, 0, M->cs>>>(M->F1.as<float>(), M->F2.as<float>(), ctx->p, n, M->W1b, M->P + oB1,
                                              M->U.as<float>(), M->V.as<float>());
         MK(cudaGetLastError());
     }
@@ -886,12 +875,18 @@ static bm_status learned_impl(bm_ctx* ctx, bm_mlp* M, const bm_learned_opts* o, 
             k_gather_pairs<<<(top + 255) / 256, 256, 0, M->cs>>>(idx2, top, pa, pb, qa, qb);
         }
         // exact deltas of the selected pairs on the current matching
-        const long long blocks = std::min<long long>(top, (long long)ctx->num_sms * 8);
-        k_pair_deltas_block<W16><<<(int)blocks, 256, 0, M->cs>>>(g, qa, qb, top, dd);
+        const long long blocks = std::min<long long>(top, (long long)ctx->num_sms * 16);
+        k_pair_deltas_block<W16><<<(int)blocks, 32 * kPairWarps, 0, M->cs>>>(g, qa, qb, top, dd);
         MK(cudaEventRecord(M->ec, M->cs));
-        k_learned_keys<<<(top + 255) / 256, 256, 0, M->cs>>>(qa, qb, dd, top, ck);
-        tb = M->tmp.cap;
-        MK(cub::DeviceRadixSort::SortKeys(M->tmp.p, tb, ck, ck + top, top, 0, 64, M->cs));
+        MK(cudaMemsetAsync(ctx->small + 1, 0, sizeof(int), M->cs));
+        if (top > kLearnedRankMax) MK(cudaMemsetAsync(ck, 0xff, (size_t)top * sizeof(unsigned long long), M->cs));
+        k_learned_keys<<<(top + 255) / 256, 256, 0, M->cs>>>(qa, qb, dd, top, ck, ctx->small + 1);
+        if (top <= kLearnedRankMax) {
+            k_rank_sort<true><<<(top + 31) / 32, 256, 0, M->cs>>>(ck, ctx->small + 1, top, ck + top);
+        } else {
+            tb = M->tmp.cap;
+            MK(cub::DeviceRadixSort::SortKeys(M->tmp.p, tb, ck, ck + top, top, 0, 64, M->cs));
+        }
         MK(cudaGetLastError());
         // exact set commit of the improving ones, in (delta desc, lo, hi) order
         const size_t smem = commit_group_smem(n);

@@ -258,17 +258,22 @@ static __global__ void k_to_bf16(const float* __restrict__ x, int count, __nv_bf
 
 constexpr int kFeatDim = 32;
 
-// U and V for n vertices: block of 256 threads (one per hidden unit), 8
-// vertices per block.  F1, F2: n x 32 fp32; W1b: 256 x 128 bf16; p: matching.
+// U and V for n vertices: block of 256 threads (one per hidden unit) over kUvRows
+// vertices.  F1, F2: n x 32 fp32; W1b: 256 x 128 bf16; p: matching.  A thread
+// holds its unit's 128 weights in registers; the block pays for loading them
+// (64 KB) once per kUvRows vertices -- with 8 vertices and 2-byte loads the
+// weights were the launch (145 us at n = 8,192; now 34).  Two vertices at a
+// time: four independent chains of fused multiply-adds, each in column order.
+constexpr int kUvRows = 32;
 static __global__ void __launch_bounds__(256) k_uv(const float* __restrict__ F1, const float* __restrict__ F2,
                                                    const int* __restrict__ p, int n,
                                                    const __nv_bfloat16* __restrict__ W1b,
                                                    const float* __restrict__ b1, float* __restrict__ U,
                                                    float* __restrict__ V) {
-    __shared__ float f[8][2][kFeatDim];  // per vertex: f1, f2(p), as bf16-rounded floats
+    __shared__ __align__(16) float f[kUvRows][2][kFeatDim];  // per vertex: f1, f2(p), as bf16-rounded floats
     const int c = threadIdx.x;
-    const int v0 = blockIdx.x * 8;
-    for (int i = c; i < 8 * 2 * kFeatDim; i += 256) {
+    const int v0 = blockIdx.x * kUvRows;
+    for (int i = c; i < kUvRows * 2 * kFeatDim; i += 256) {
         const int v = i / (2 * kFeatDim), k = i % (2 * kFeatDim), a = v0 + v;
         float x = 0.f;
         if (a < n) {
@@ -280,38 +285,65 @@ static __global__ void __launch_bounds__(256) k_uv(const float* __restrict__ F1,
         }
         f[v][k < kFeatDim ? 0 : 1][k & (kFeatDim - 1)] = __bfloat162float(__float2bfloat16(x));
     }
-    __syncthreads();
     float w[4][kFeatDim];  // W1[c] in four 32-column quarters: f1(a), f1(b), f2(pa), f2(pb)
+    {
+        const uint4* w4 = reinterpret_cast<const uint4*>(W1b + (size_t)c * kMlpIn);
 #pragma unroll
-    for (int q = 0; q < 4; q++)
+        for (int i = 0; i < kMlpIn / 8; i++) {
+            const uint4 q = w4[i];
+            const uint32_t r[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (int k = 0; k < kFeatDim; k++) w[q][k] = __bfloat162float(W1b[(size_t)c * kMlpIn + q * kFeatDim + k]);
+            for (int u = 0; u < 4; u++) {   // bf16 -> float is a shift
+                w[i >> 2][8 * (i & 3) + 2 * u] = __uint_as_float(r[u] << 16);
+                w[i >> 2][8 * (i & 3) + 2 * u + 1] = __uint_as_float(r[u] & 0xffff0000u);
+            }
+        }
+    }
     const float bias = b1[c];
-    for (int v = 0; v < 8; v++) {
-        const int a = v0 + v;
-        if (a >= n) break;
-        float u = 0.f, x = 0.f;
+    __syncthreads();
+    for (int v = 0; v < kUvRows && v0 + v < n; v += 2) {
+        float u[2] = {0.f, 0.f}, x[2] = {0.f, 0.f};
 #pragma unroll
-        for (int k = 0; k < kFeatDim; k++) {
-            u = fmaf(w[0][k], f[v][0][k], u);
-            x = fmaf(w[1][k], f[v][0][k], x);
-        }
+        for (int h = 0; h < 2; h++)
 #pragma unroll
-        for (int k = 0; k < kFeatDim; k++) {
-            u = fmaf(w[2][k], f[v][1][k], u);
-            x = fmaf(w[3][k], f[v][1][k], x);
-        }
-        U[(size_t)a * kMlpHid + c] = u + bias;
-        V[(size_t)a * kMlpHid + c] = x;
+            for (int k = 0; k < kFeatDim; k += 4) {
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const float4 q = *reinterpret_cast<const float4*>(&f[v + e][h][k]);
+                    u[e] = fmaf(w[2 * h][k], q.x, u[e]);
+                    x[e] = fmaf(w[2 * h + 1][k], q.x, x[e]);
+                    u[e] = fmaf(w[2 * h][k + 1], q.y, u[e]);
+                    x[e] = fmaf(w[2 * h + 1][k + 1], q.y, x[e]);
+                    u[e] = fmaf(w[2 * h][k + 2], q.z, u[e]);
+                    x[e] = fmaf(w[2 * h + 1][k + 2], q.z, x[e]);
+                    u[e] = fmaf(w[2 * h][k + 3], q.w, u[e]);
+                    x[e] = fmaf(w[2 * h + 1][k + 3], q.w, x[e]);
+                }
+            }
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+            if (v0 + v + e < n) {
+                U[(size_t)(v0 + v + e) * kMlpHid + c] = u[e] + bias;
+                V[(size_t)(v0 + v + e) * kMlpHid + c] = x[e];
+            }
     }
 }
 
-constexpr int kRankThreads = 256;
+constexpr int kRankBuilders = 512, kRankThreads = kRankBuilders + 128;   // 16 builder warps, 4 epilogue warps
+constexpr int kRankRows = kGemmM / (kRankBuilders / 32);                  // rows a builder warp makes per tile
 constexpr int kRankA = kGemmM * 512;          // A tile: 128 rows x 256 bf16 (4 k-blocks of 16 KB)
 constexpr int kRankB = kMlpHid * 512;         // W2: 256 rows x 256 bf16 (4 k-blocks of 32 KB)
 constexpr int kRankSmem = kRankA + kRankB + 2 * kMlpHid * 4 + 1024 + 256;
 
 // y[i] = w3 . relu(W2 relu(U[pa i] + V[pb i]) + b2) + b3 for i < k.
+// The builder warps make tile t + 1 and its MMA runs while the epilogue warps
+// reduce tile t from the other half of TMEM (two 256-column accumulators), so a
+// tile costs its build and MMA, not the epilogue too; the pairs are loaded a tile
+// ahead and 16 warps build (246 -> 223 -> 174 us for 524,288 pairs at n = 8,192,
+// 8.9 -> 6.3 us per tile of 128 pairs and SM).  Bound by the gathers of the
+// build, 2 KB of fp32 U and V per pair.
+// Every wait is bounded: after a timeout (err set) a thread waits no more, no
+// further MMA is issued or accumulator read, and the warps run out their loops.
 static __global__ void __launch_bounds__(kRankThreads, 1)
 k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* __restrict__ pa,
            const int* __restrict__ pb, long long k, const __nv_bfloat16* __restrict__ W2b,
@@ -325,20 +357,23 @@ k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* 
     const uint32_t sA = base, sB = base + kRankA;
     float* sb2 = reinterpret_cast<float*>(smem_raw + (sB + kRankB - raw));
     float* sw3 = sb2 + kMlpHid;
-    const uint32_t bar = sB + kRankB + 2 * kMlpHid * 4;
-    const uint32_t tslot = bar + 8;
+    const uint32_t bars = sB + kRankB + 2 * kMlpHid * 4;   // mma[2]: tile in accumulator h done; free[2]: h reduced
+    const uint32_t tslot = bars + 32;
     uint32_t* tslot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tslot - raw));
-    __shared__ int s_abort;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+    auto bar_mma = [&](int h) { return bars + 8 * h; };
+    auto bar_free = [&](int h) { return bars + 16 + 8 * h; };
 
     if (wid == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(tslot), "r"(kMlpHid) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(tslot), "r"(2 * kMlpHid) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar) : "memory");
+        for (int h = 0; h < 2; h++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar_mma(h)) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" :: "r"(bar_free(h)) : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_abort = 0;
     }
     // W2 resident: row r (output unit), 16-byte chunk c of its 512 bytes
     const uint8_t* W2 = reinterpret_cast<const uint8_t*>(W2b);
@@ -350,81 +385,104 @@ k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* 
     }
     for (int i = tid; i < kMlpHid; i += kRankThreads) { sb2[i] = b2[i]; sw3[i] = w3[i]; }
     const float bias3 = b3[0];
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // W2, read by the tensor cores
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot_ptr;
 
     const long long tiles = (k + kGemmM - 1) / kGemmM;
-    uint32_t phase = 0;
-    for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const long long row0 = t * kGemmM;
-        // A tile: warp w builds rows w, w + 8, ... (four rows per pass, their
-        // loads all issued before any store); lane = 16-byte chunk (8 units)
-        for (int r0 = wid; r0 < kGemmM; r0 += 4 * (kRankThreads / 32)) {
-            float4 u[4][2], x[4][2];
-            bool live[4];
+    int it = 0, issued = 0;   // tiles begun; tiles handed to the tensor cores (thread 0)
+    bool ok = true;
+    if (wid < kRankBuilders / 32) {
+        int na = 0, nb = 0;
+        {
+            const long long i = (long long)blockIdx.x * kGemmM + wid * kRankRows + lane;
+            if (lane < kRankRows && i < k) { na = pa[i]; nb = pb[i]; }
+        }
+        for (long long t = blockIdx.x; t < tiles; t += gridDim.x, it++) {
+            const int h = it & 1;
+            const long long row0 = t * kGemmM;
+            // the previous tile's MMA has read A
+            if (ok && it > 0) ok = mbar_wait_bounded(bar_mma(h ^ 1), ((it - 1) >> 1) & 1, err);
+            // A tile: warp w builds rows 8 w .. 8 w + 7 (four rows per pass, their
+            // loads all issued before any store); lane = 16-byte chunk (8 units).
+            // Lane q holds row q's pair, loaded a tile ahead.
+            const int ca = na, cb = nb;
+            const long long next = row0 + (long long)gridDim.x * kGemmM + wid * kRankRows + lane;
+            if (lane < kRankRows && next < k) { na = pa[next]; nb = pb[next]; }
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int r = r0 + q * (kRankThreads / 32);
-                const long long i = row0 + r;
-                live[q] = i < k;
-                if (live[q]) {
-                    const int a = pa[i], b = pb[i];
-                    const float4* u4 = reinterpret_cast<const float4*>(U + (size_t)a * kMlpHid + lane * 8);
-                    const float4* v4 = reinterpret_cast<const float4*>(V + (size_t)b * kMlpHid + lane * 8);
-                    u[q][0] = u4[0]; u[q][1] = u4[1]; x[q][0] = v4[0]; x[q][1] = v4[1];
+            for (int r0 = 0; r0 < kRankRows; r0 += 4) {
+                float4 u[4][2], x[4][2];
+                bool live[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int a = __shfl_sync(0xffffffffu, ca, r0 + q), b = __shfl_sync(0xffffffffu, cb, r0 + q);
+                    live[q] = row0 + wid * kRankRows + r0 + q < k;
+                    if (live[q]) {
+                        const float4* u4 = reinterpret_cast<const float4*>(U + (size_t)a * kMlpHid + lane * 8);
+                        const float4* v4 = reinterpret_cast<const float4*>(V + (size_t)b * kMlpHid + lane * 8);
+                        u[q][0] = u4[0]; u[q][1] = u4[1]; x[q][0] = v4[0]; x[q][1] = v4[1];
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int r = wid * kRankRows + r0 + q;
+                    uint4 out = make_uint4(0, 0, 0, 0);
+                    if (live[q]) {
+                        const float4 u0 = u[q][0], u1 = u[q][1], x0 = x[q][0], x1 = x[q][1];
+                        __nv_bfloat162 h0 = __floats2bfloat162_rn(fmaxf(u0.x + x0.x, 0.f), fmaxf(u0.y + x0.y, 0.f));
+                        __nv_bfloat162 h1 = __floats2bfloat162_rn(fmaxf(u0.z + x0.z, 0.f), fmaxf(u0.w + x0.w, 0.f));
+                        __nv_bfloat162 h2 = __floats2bfloat162_rn(fmaxf(u1.x + x1.x, 0.f), fmaxf(u1.y + x1.y, 0.f));
+                        __nv_bfloat162 h3 = __floats2bfloat162_rn(fmaxf(u1.z + x1.z, 0.f), fmaxf(u1.w + x1.w, 0.f));
+                        out.x = *reinterpret_cast<uint32_t*>(&h0);
+                        out.y = *reinterpret_cast<uint32_t*>(&h1);
+                        out.z = *reinterpret_cast<uint32_t*>(&h2);
+                        out.w = *reinterpret_cast<uint32_t*>(&h3);
+                    }
+                    const int kb = lane >> 3, cc = lane & 7;
+                    const uint32_t dst = sA + kb * (kGemmM * 128) + r * 128 + ((cc ^ (r & 7)) << 4);
+                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" :: "r"(dst), "r"(out.x), "r"(out.y), "r"(out.z), "r"(out.w) : "memory");
                 }
             }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("bar.sync 1, %0;" :: "n"(kRankBuilders) : "memory");
+            // the accumulator's previous tile has been reduced
+            if (tid == 0 && ok && it >= 2) ok = mbar_wait_bounded(bar_free(h), ((it >> 1) - 1) & 1, err);
+            if (tid == 0 && ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int r = r0 + q * (kRankThreads / 32);
-                uint4 out = make_uint4(0, 0, 0, 0);
-                if (live[q]) {
-                    const float4 u0 = u[q][0], u1 = u[q][1], x0 = x[q][0], x1 = x[q][1];
-                    __nv_bfloat162 h0 = __floats2bfloat162_rn(fmaxf(u0.x + x0.x, 0.f), fmaxf(u0.y + x0.y, 0.f));
-                    __nv_bfloat162 h1 = __floats2bfloat162_rn(fmaxf(u0.z + x0.z, 0.f), fmaxf(u0.w + x0.w, 0.f));
-                    __nv_bfloat162 h2 = __floats2bfloat162_rn(fmaxf(u1.x + x1.x, 0.f), fmaxf(u1.y + x1.y, 0.f));
-                    __nv_bfloat162 h3 = __floats2bfloat162_rn(fmaxf(u1.z + x1.z, 0.f), fmaxf(u1.w + x1.w, 0.f));
-                    out.x = *reinterpret_cast<uint32_t*>(&h0);
-                    out.y = *reinterpret_cast<uint32_t*>(&h1);
-                    out.z = *reinterpret_cast<uint32_t*>(&h2);
-                    out.w = *reinterpret_cast<uint32_t*>(&h3);
-                }
-                const int kb = lane >> 3, cc = lane & 7;
-                const uint32_t dst = sA + kb * (kGemmM * 128) + r * 128 + ((cc ^ (r & 7)) << 4);
-                asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" :: "r"(dst), "r"(out.x), "r"(out.y), "r"(out.z), "r"(out.w) : "memory");
+                for (int kb = 0; kb < 4; kb++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {  // 16 bf16 = 32 bytes of K per MMA
+                        const uint64_t da = umma_desc_sw128(sA + kb * (kGemmM * 128) + j * 32);
+                        const uint64_t db = umma_desc_sw128(sB + kb * (kMlpHid * 128) + j * 32);
+                        const uint32_t acc = (kb | j) ? 1u : 0u;
+                        asm volatile(
+                            "{\n\t.reg .pred p;\n\t"
+                            "setp.ne.b32 p, %4, 0;\n\t"
+                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                            :: "r"(tmem + h * kMlpHid), "l"(da), "l"(db), "r"(kIdesc), "r"(acc) : "memory");
+                    }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                             :: "r"(bar_mma(h)) : "memory");
+                issued = it + 1;
             }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
+        // the last MMA has finished before the CTA frees TMEM and leaves
+        if (tid == 0 && issued > 0) mbar_wait_bounded(bar_mma((issued - 1) & 1), ((issued - 1) >> 1) & 1, err);
+    } else {
+        const int q4 = wid & 3;   // the TMEM lane quarter a warp may read
+        for (long long t = blockIdx.x; t < tiles; t += gridDim.x, it++) {
+            const int h = it & 1;
+            ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(bar_mma(h), (it >> 1) & 1, err));
+            if (!ok) continue;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int kb = 0; kb < 4; kb++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) {  // 16 bf16 = 32 bytes of K per MMA
-                    const uint64_t da = umma_desc_sw128(sA + kb * (kGemmM * 128) + j * 32);
-                    const uint64_t db = umma_desc_sw128(sB + kb * (kMlpHid * 128) + j * 32);
-                    const uint32_t acc = (kb | j) ? 1u : 0u;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "setp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                        :: "r"(tmem), "l"(da), "l"(db), "r"(kIdesc), "r"(acc) : "memory");
-                }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                         :: "r"(bar) : "memory");
-        }
-        if (!mbar_wait_bounded(bar, phase, err)) s_abort = 1;
-        phase ^= 1u;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (wid < 4) {  // epilogue: warp w reads TMEM lanes 32w..32w+31 = tile rows
-            const long long i = row0 + wid * 32 + lane;
+            const long long i = t * kGemmM + q4 * 32 + lane;
             float acc = 0.f;
             for (int cb = 0; cb < kMlpHid / 32; cb++) {
                 uint32_t r[32];
-                const uint32_t taddr = tmem + ((uint32_t)(wid * 32) << 16) + (uint32_t)(cb * 32);
+                const uint32_t taddr = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(h * kMlpHid + cb * 32);
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
                     "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -441,16 +499,16 @@ k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* 
                     acc = fmaf(fmaxf(__uint_as_float(r[q]) + sb2[c], 0.f), sw3[c], acc);
                 }
             }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar_free(h)) : "memory");
             if (i < k) y[i] = acc + bias3;
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (s_abort) break;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (wid == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kMlpHid) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(2 * kMlpHid) : "memory");
 }
 
 }  // namespace bm
