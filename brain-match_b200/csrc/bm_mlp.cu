@@ -161,12 +161,12 @@ __global__ void __launch_bounds__(256) k_normalise(float* __restrict__ F1, float
 // sweep-major, `per` to a sweep, and sweep s has its own features
 // (F1s + s*n*32, F2s + s*n*32) and matching (ps + s*n).  X row i gets
 // [F1 a, F1 b, F2 p(a), F2 p(b)] in bf16 (zero rows from k to kpad), t[i]
-// the target.
+// the target, XT the transpose of X.
 __global__ void k_batch_inputs(const int* __restrict__ pa, const int* __restrict__ pb, const float* __restrict__ tall,
                                long long count, long long per, long long off, long long mul, long long add, int k,
                                int kpad, const float* __restrict__ F1s, const float* __restrict__ F2s,
                                const int* __restrict__ ps, int n, __nv_bfloat16* __restrict__ X,
-                               float* __restrict__ t) {
+                               __nv_bfloat16* __restrict__ XT, float* __restrict__ t) {
     const int i = blockIdx.x, c = threadIdx.x;  // 128 threads
     if (i >= kpad) return;
     float v = 0.f;
@@ -187,6 +187,7 @@ __global__ void k_batch_inputs(const int* __restrict__ pa, const int* __restrict
         if (c == 0) t[i] = tall[j];
     }
     X[(size_t)i * kMlpIn + c] = __float2bfloat16(v);
+    XT[(size_t)c * kpad + i] = __float2bfloat16(v);
 }
 
 // acc += loss * k (the batch's share of an epoch's mean loss).
@@ -371,9 +372,10 @@ struct bm_mlp {
     float *P = nullptr, *G = nullptr;
     __nv_bfloat16 *W1b = nullptr, *W2b = nullptr, *W2Tb = nullptr;
     int cap = 0;  // batch capacity (multiple of 128)
-    __nv_bfloat16 *X = nullptr, *H1b = nullptr, *H2b = nullptr, *dH2b = nullptr, *dH1b = nullptr;
-    __nv_bfloat16 *T1 = nullptr, *T2 = nullptr;  // transposes, 256 x cap
-    float *H1f = nullptr, *H2f = nullptr, *dH1f = nullptr, *y = nullptr, *t = nullptr, *loss = nullptr;
+    __nv_bfloat16 *X = nullptr, *H1b = nullptr, *dH2b = nullptr;
+    __nv_bfloat16 *XT = nullptr, *H1T = nullptr, *dH2T = nullptr, *dH1T = nullptr;  // transposes, ld = padded rows
+    float *H1f = nullptr, *H2f = nullptr, *y = nullptr, *t = nullptr;
+    float* loss = nullptr;  // behind the gradients
     int* err_d = nullptr;
     // engine-side workspace: features, pool, ranking, exact evaluation
     DBuf contrib, F1, F2, fstat, pa, pb, ys, key, key2, idx, idx2, qa, qb, dd, ckeys, tmp, tall, xin;
@@ -401,8 +403,8 @@ extern "C" const char* bm_mlp_last_error(const bm_mlp* M) { return M ? M->err : 
 
 static void mlp_free(bm_mlp* M) {
     if (!M) return;
-    void* b[] = {M->P, M->G, M->W1b, M->W2b, M->W2Tb, M->X, M->H1b, M->H2b, M->dH2b, M->dH1b, M->T1, M->T2,
-                 M->H1f, M->H2f, M->dH1f, M->y, M->t, M->loss, M->err_d};
+    void* b[] = {M->P, M->G, M->W1b, M->W2b, M->W2Tb, M->X, M->XT, M->H1b, M->H1T, M->dH2b, M->dH2T, M->dH1T,
+                 M->H1f, M->H2f, M->y, M->t, M->err_d};
     for (void* p : b) if (p) cudaFree(p);
     DBuf* w[] = {&M->contrib, &M->F1, &M->F2, &M->fstat, &M->pa, &M->pb, &M->ys, &M->key, &M->key2, &M->idx,
                  &M->idx2, &M->qa, &M->qb, &M->dd, &M->ckeys, &M->tmp, &M->tall, &M->xin,
@@ -414,10 +416,9 @@ static void mlp_free(bm_mlp* M) {
 }
 extern "C" void bm_mlp_destroy(bm_mlp* M) { mlp_free(M); }
 
-static bm_status mlp_refresh_bf16(bm_mlp* M) {
-    k_to_bf16<<<(kMlpHid * kMlpIn + 255) / 256, 256, 0, M->cs>>>(M->P + oW1, kMlpHid * kMlpIn, M->W1b);
-    k_to_bf16<<<(kMlpHid * kMlpHid + 255) / 256, 256, 0, M->cs>>>(M->P + oW2, kMlpHid * kMlpHid, M->W2b);
-    k_transpose_bf16<<<dim3(kMlpHid / 32, kMlpHid / 32), dim3(32, 8), 0, M->cs>>>(M->W2b, kMlpHid, kMlpHid, M->W2Tb);
+// params -= lr * grads (unless grads == nullptr) and the bf16 copies of the weights.
+static bm_status mlp_update(bm_mlp* M, const float* grads, float lr) {
+    k_sgd<<<(kParams + 255) / 256, 256, 0, M->cs>>>(M->P, grads, kParams, lr, oW1, oW2, M->W1b, M->W2b, M->W2Tb);
     MK(cudaGetLastError());
     return BM_OK;
 }
@@ -425,22 +426,15 @@ static bm_status mlp_refresh_bf16(bm_mlp* M) {
 static bm_status mlp_reserve(bm_mlp* M, int rows) {
     const int need = (rows + 127) / 128 * 128;
     if (need <= M->cap) return BM_OK;
-    void** bufs[] = {(void**)&M->X, (void**)&M->H1b, (void**)&M->H2b, (void**)&M->dH2b, (void**)&M->dH1b,
-                     (void**)&M->T1, (void**)&M->T2, (void**)&M->H1f, (void**)&M->H2f, (void**)&M->dH1f,
-                     (void**)&M->y, (void**)&M->t};
+    void** bufs[] = {(void**)&M->X, (void**)&M->XT, (void**)&M->H1b, (void**)&M->H1T, (void**)&M->dH2b,
+                     (void**)&M->dH2T, (void**)&M->dH1T, (void**)&M->H1f, (void**)&M->H2f, (void**)&M->y, (void**)&M->t};
     for (void** b : bufs) if (*b) { cudaFree(*b); *b = nullptr; }
     M->cap = 0;
     const size_t c = (size_t)need;
-    MK(cudaMalloc(&M->X, c * kMlpIn * sizeof(__nv_bfloat16)));
-    MK(cudaMalloc(&M->H1b, c * kMlpHid * sizeof(__nv_bfloat16)));
-    MK(cudaMalloc(&M->H2b, c * kMlpHid * sizeof(__nv_bfloat16)));
-    MK(cudaMalloc(&M->dH2b, c * kMlpHid * sizeof(__nv_bfloat16)));
-    MK(cudaMalloc(&M->dH1b, c * kMlpHid * sizeof(__nv_bfloat16)));
-    MK(cudaMalloc(&M->T1, c * kMlpHid * sizeof(__nv_bfloat16)));
-    MK(cudaMalloc(&M->T2, c * kMlpHid * sizeof(__nv_bfloat16)));
-    MK(cudaMalloc(&M->H1f, c * kMlpHid * sizeof(float)));
-    MK(cudaMalloc(&M->H2f, c * kMlpHid * sizeof(float)));
-    MK(cudaMalloc(&M->dH1f, c * kMlpHid * sizeof(float)));
+    for (__nv_bfloat16** q : {&M->X, &M->XT}) MK(cudaMalloc(q, c * kMlpIn * sizeof(__nv_bfloat16)));
+    for (__nv_bfloat16** q : {&M->H1b, &M->H1T, &M->dH2b, &M->dH2T, &M->dH1T})
+        MK(cudaMalloc(q, c * kMlpHid * sizeof(__nv_bfloat16)));
+    for (float** q : {&M->H1f, &M->H2f}) MK(cudaMalloc(q, c * kMlpHid * sizeof(float)));
     MK(cudaMalloc(&M->y, c * sizeof(float)));
     MK(cudaMalloc(&M->t, c * sizeof(float)));
     M->cap = need;
@@ -458,11 +452,11 @@ extern "C" bm_status bm_mlp_create(bm_mlp** out, uint64_t seed) {
         M->cs = M->st;
         for (cudaEvent_t* e : {&M->e0, &M->e1, &M->ea, &M->eb, &M->ec}) MK(cudaEventCreate(e));
         MK(cudaMalloc(&M->P, kParams * sizeof(float)));
-        MK(cudaMalloc(&M->G, kParams * sizeof(float)));
+        MK(cudaMalloc(&M->G, (kParams + 1) * sizeof(float)));
+        M->loss = M->G + kParams;
         MK(cudaMalloc(&M->W1b, kMlpHid * kMlpIn * sizeof(__nv_bfloat16)));
         MK(cudaMalloc(&M->W2b, kMlpHid * kMlpHid * sizeof(__nv_bfloat16)));
         MK(cudaMalloc(&M->W2Tb, kMlpHid * kMlpHid * sizeof(__nv_bfloat16)));
-        MK(cudaMalloc(&M->loss, sizeof(float)));
         MK(cudaMalloc(&M->err_d, sizeof(int)));
         MK(cudaMemset(M->err_d, 0, sizeof(int)));
         // He-uniform initialisation from a seeded generator; zero biases
@@ -477,7 +471,7 @@ extern "C" bm_status bm_mlp_create(bm_mlp** out, uint64_t seed) {
         fill(oW2, kMlpHid * kMlpHid, kMlpHid);
         fill(oW3, kMlpHid, kMlpHid);
         MK(cudaMemcpy(M->P, h.data(), kParams * sizeof(float), cudaMemcpyHostToDevice));
-        bm_status s = mlp_refresh_bf16(M);
+        bm_status s = mlp_update(M, nullptr, 0.f);
         if (s) return s;
         MK(cudaStreamSynchronize(M->cs));
         return BM_OK;
@@ -498,54 +492,57 @@ extern "C" bm_status bm_mlp_get_params(bm_mlp* M, float* params) {
 extern "C" bm_status bm_mlp_set_params(bm_mlp* M, const float* params) {
     if (!M || !params) return BM_E_INPUT;
     MK(cudaMemcpyAsync(M->P, params, kParams * sizeof(float), cudaMemcpyHostToDevice, M->cs));
-    bm_status s = mlp_refresh_bf16(M);
+    bm_status s = mlp_update(M, nullptr, 0.f);
     if (s) return s;
     MK(cudaStreamSynchronize(M->cs));
     return BM_OK;
 }
 
+// A (m x k) times B (n x k) transposed; `splits` shares of K (their results must
+// be added: o.add).
 template <int BN>
-static bm_status gemm(bm_mlp* M, const __nv_bfloat16* A, const __nv_bfloat16* B, int m, int n, int k, float* C,
-                      const float* bias, int relu, __nv_bfloat16* Cb) {
+static bm_status gemm(bm_mlp* M, const __nv_bfloat16* A, const __nv_bfloat16* B, int m, int n, int k, const GemmOut& o,
+                      int splits = 1) {
     MK(cudaFuncSetAttribute(k_gemm_bf16<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_bf16_smem<BN>()));
-    k_gemm_bf16<BN><<<dim3(n / BN, m / kGemmM), kGemmThreads, gemm_bf16_smem<BN>(), M->cs>>>(
-        A, B, m, n, k, C, bias, relu, Cb, M->err_d, take_stall(BM_STALL_MLP_GEMM));
+    k_gemm_bf16<BN><<<dim3(n / BN, m / kGemmM, splits), kGemmThreads, gemm_bf16_smem<BN>(), M->cs>>>(
+        A, B, m, n, k, o, M->err_d, take_stall(BM_STALL_MLP_GEMM));
     MK(cudaGetLastError());
     return BM_OK;
 }
 
-// Forward of rows [0, kpad) of M->X through both wide layers.
-static bm_status mlp_forward_dev(bm_mlp* M, int kpad) {
+// Forward of rows [0, kpad) of M->X through both wide layers; for a backward
+// pass also bf16 H1 transposed.
+static bm_status mlp_forward_dev(bm_mlp* M, int kpad, bool backward) {
     bm_status s;
-    if ((s = gemm<256>(M, M->X, M->W1b, kpad, kMlpHid, kMlpIn, M->H1f, M->P + oB1, 1, M->H1b))) return s;
-    if ((s = gemm<256>(M, M->H1b, M->W2b, kpad, kMlpHid, kMlpHid, M->H2f, M->P + oB2, 1, M->H2b))) return s;
+    GemmOut o1, o2;
+    o1.bias = M->P + oB1; o1.relu = 1; o1.Cb = M->H1b;
+    if (backward) { o1.C = M->H1f; o1.CbT = M->H1T; }
+    if ((s = gemm<64>(M, M->X, M->W1b, kpad, kMlpHid, kMlpIn, o1))) return s;
+    o2.bias = M->P + oB2; o2.relu = 1; o2.C = M->H2f;
+    if ((s = gemm<64>(M, M->H1b, M->W2b, kpad, kMlpHid, kMlpHid, o2))) return s;
     return BM_OK;
 }
 
-// One forward + backward on rows [0,k) of X with targets t; gradients into M->G.
+// One forward + backward on rows [0,k) of X (XT its transpose) with targets t;
+// gradients into M->G.
 static bm_status mlp_fwd_bwd_dev(bm_mlp* M, int k) {
     const int kpad = (k + 127) / 128 * 128;
-    bm_status s = mlp_forward_dev(M, kpad);
+    bm_status s = mlp_forward_dev(M, kpad, true);
     if (s) return s;
-    MK(cudaMemsetAsync(M->G, 0, kParams * sizeof(float), M->cs));
-    MK(cudaMemsetAsync(M->loss, 0, sizeof(float), M->cs));
-    k_head<<<(kpad * 32 + 255) / 256, 256, 0, M->cs>>>(M->H2f, k, kpad, M->P + oW3, M->P + oB3, M->y, M->t, M->loss,
-                                                       M->dH2b, M->G + oW3, M->G + oB3);
+    MK(cudaMemsetAsync(M->G, 0, (kParams + 1) * sizeof(float), M->cs));   // gradients and loss
+    k_head<<<kpad / 32, kMlpHid, 0, M->cs>>>(M->H2f, k, kpad, M->P + oW3, M->P + oB3, M->y, M->t, M->loss, M->dH2b,
+                                             M->dH2T, M->G + oW3, M->G + oB3, M->G + oB2);
     MK(cudaGetLastError());
-    // dW2 = dH2^T H1 ; db2 = colsum dH2
-    k_transpose_bf16<<<dim3(kMlpHid / 32, kpad / 32), dim3(32, 8), 0, M->cs>>>(M->dH2b, kpad, kMlpHid, M->T1);
-    k_transpose_bf16<<<dim3(kMlpHid / 32, kpad / 32), dim3(32, 8), 0, M->cs>>>(M->H1b, kpad, kMlpHid, M->T2);
-    MK(cudaGetLastError());
-    if ((s = gemm<256>(M, M->T1, M->T2, kMlpHid, kMlpHid, kpad, M->G + oW2, nullptr, 0, nullptr))) return s;
-    k_colsum_bf16<<<dim3(1, 64), kMlpHid, 0, M->cs>>>(M->dH2b, kpad, kMlpHid, M->G + oB2);
-    // dH1 = dH2 W2, masked by ReLU'(H1); db1
-    if ((s = gemm<256>(M, M->dH2b, M->W2Tb, kpad, kMlpHid, kMlpHid, M->dH1f, nullptr, 0, nullptr))) return s;
-    k_relu_bwd<<<dim3(1, 64), kMlpHid, 0, M->cs>>>(M->dH1f, M->H1f, kpad, kMlpHid, M->dH1b, M->G + oB1);
-    // dW1 = dH1^T X
-    k_transpose_bf16<<<dim3(kMlpHid / 32, kpad / 32), dim3(32, 8), 0, M->cs>>>(M->dH1b, kpad, kMlpHid, M->T1);
-    k_transpose_bf16<<<dim3(kMlpIn / 32, kpad / 32), dim3(32, 8), 0, M->cs>>>(M->X, kpad, kMlpIn, M->T2);
-    MK(cudaGetLastError());
-    if ((s = gemm<128>(M, M->T1, M->T2, kMlpHid, kMlpIn, kpad, M->G + oW1, nullptr, 0, nullptr))) return s;
+    // dH1 = dH2 W2, masked by ReLU'(H1), only its bf16 transpose is read; db1
+    GemmOut oh, o2, o1;
+    oh.mask = M->H1f; oh.CbT = M->dH1T; oh.colsum = M->G + oB1;
+    if ((s = gemm<64>(M, M->dH2b, M->W2Tb, kpad, kMlpHid, kMlpHid, oh))) return s;
+    // dW2 = dH2^T H1, dW1 = dH1^T X, over shares of 512 rows
+    const int splits = std::max(1, kpad / 512);
+    o2.add = M->G + oW2;
+    if ((s = gemm<64>(M, M->dH2T, M->H1T, kMlpHid, kMlpHid, kpad, o2, splits))) return s;
+    o1.add = M->G + oW1;
+    if ((s = gemm<64>(M, M->dH1T, M->XT, kMlpHid, kMlpIn, kpad, o1, splits))) return s;
     return BM_OK;
 }
 
@@ -562,13 +559,13 @@ static bm_status check_err(bm_mlp* M) {
     return BM_OK;
 }
 
-// Host rows x (k x 128 fp32) into M->X as bf16, padded with zero rows.
-static bm_status upload_rows(bm_mlp* M, int64_t k, const float* x, int kpad) {
+// Host rows x (k x 128 fp32) into M->X as bf16, padded with zero rows, and
+// transposed into M->XT for a backward pass.
+static bm_status upload_rows(bm_mlp* M, int64_t k, const float* x, int kpad, bool backward) {
     MK(M->xin.need((size_t)kpad * kMlpIn * sizeof(float)));
     float* xf = M->xin.as<float>();
-    MK(cudaMemsetAsync(xf, 0, (size_t)kpad * kMlpIn * sizeof(float), M->cs));
     MK(cudaMemcpyAsync(xf, x, (size_t)k * kMlpIn * sizeof(float), cudaMemcpyHostToDevice, M->cs));
-    k_to_bf16<<<(kpad * kMlpIn + 255) / 256, 256, 0, M->cs>>>(xf, kpad * kMlpIn, M->X);
+    k_rows_bf16<<<kpad / 32, kMlpIn, 0, M->cs>>>(xf, (int)k, kpad, M->X, backward ? M->XT : nullptr);
     MK(cudaGetLastError());
     return BM_OK;
 }
@@ -580,10 +577,10 @@ extern "C" bm_status bm_mlp_forward(bm_mlp* M, int64_t k, const float* x, float*
     bm_status s = mlp_reserve(M, (int)k);
     if (s) return s;
     const int kpad = ((int)k + 127) / 128 * 128;
-    if ((s = upload_rows(M, k, x, kpad))) return s;
-    if ((s = mlp_forward_dev(M, kpad))) return s;
-    k_head<<<(kpad * 32 + 255) / 256, 256, 0, M->cs>>>(M->H2f, (int)k, kpad, M->P + oW3, M->P + oB3, M->y, nullptr,
-                                                       nullptr, nullptr, nullptr, nullptr);
+    if ((s = upload_rows(M, k, x, kpad, false))) return s;
+    if ((s = mlp_forward_dev(M, kpad, false))) return s;
+    k_head<<<kpad / 32, kMlpHid, 0, M->cs>>>(M->H2f, (int)k, kpad, M->P + oW3, M->P + oB3, M->y, nullptr, nullptr, nullptr,
+                                             nullptr, nullptr, nullptr, nullptr);
     MK(cudaGetLastError());
     MK(cudaMemcpyAsync(out, M->y, (size_t)k * sizeof(float), cudaMemcpyDeviceToHost, M->cs));
     return check_err(M);
@@ -596,14 +593,13 @@ extern "C" bm_status bm_mlp_train_step(bm_mlp* M, int64_t k, const float* x, con
     bm_status s = mlp_reserve(M, (int)k);
     if (s) return s;
     const int kpad = ((int)k + 127) / 128 * 128;
-    if ((s = upload_rows(M, k, x, kpad))) return s;
+    if ((s = upload_rows(M, k, x, kpad, true))) return s;
     MK(cudaMemcpyAsync(M->t, target, (size_t)k * sizeof(float), cudaMemcpyHostToDevice, M->cs));
     if ((s = mlp_fwd_bwd_dev(M, (int)k))) return s;
     if (grads) MK(cudaMemcpyAsync(grads, M->G, kParams * sizeof(float), cudaMemcpyDeviceToHost, M->cs));
     if (loss) MK(cudaMemcpyAsync(loss, M->loss, sizeof(float), cudaMemcpyDeviceToHost, M->cs));
     if (lr != 0.f) {
-        k_sgd<<<(kParams + 255) / 256, 256, 0, M->cs>>>(M->P, M->G, kParams, lr, nullptr);
-        if ((s = mlp_refresh_bf16(M))) return s;
+        if ((s = mlp_update(M, M->G, lr))) return s;
     }
     return check_err(M);
 }
@@ -778,12 +774,11 @@ static bm_status train_from_impl(bm_mlp* M, bm_ctx* ctx, int sweeps, int extra, 
             const int kpad = (k + 127) / 128 * 128;
             k_batch_inputs<<<kpad, kMlpIn, 0, M->cs>>>(pa, pb, tall, count, per, off, mul, add, k, kpad,
                                                        M->F1s.as<float>(), M->F2s.as<float>(), M->ps.as<int>(),
-                                                       n, M->X, M->t);
+                                                       n, M->X, M->XT, M->t);
             if ((s = mlp_fwd_bwd_dev(M, k))) return s;
             if (ep == 0) k_loss_acc<<<1, 32, 0, M->cs>>>(M->loss, k, eacc);
             if (ep == epochs - 1) k_loss_acc<<<1, 32, 0, M->cs>>>(M->loss, k, eacc + 1);
-            k_sgd<<<(kParams + 255) / 256, 256, 0, M->cs>>>(M->P, M->G, kParams, lr, nullptr);
-            if ((s = mlp_refresh_bf16(M))) return s;
+            if ((s = mlp_update(M, M->G, lr))) return s;
             samples += k;
             steps++;
         }

@@ -16,26 +16,46 @@ namespace bm {
 
 constexpr int kMlpIn = 128, kMlpHid = 256;
 
-// C[M x N] (+ bias[col]) (ReLU) = A[M x K] * B[N x K]^T; M % 128 == 0,
-// N % BN == 0, K % 64 == 0.  Optional bf16 copy of the result.
+// What the GEMM's epilogue does with C[M x N] = A[M x K] * B[N x K]^T.
+struct GemmOut {
+    const float* bias = nullptr;      // + bias[col]
+    int relu = 0;                     // max(., 0)
+    const float* mask = nullptr;      // M x N: 0 where mask <= 0
+    float* C = nullptr;               // M x N fp32
+    float* add = nullptr;             // M x N fp32, added atomically (split K)
+    float* colsum = nullptr;          // N: += column sums
+    __nv_bfloat16* Cb = nullptr;      // M x N bf16
+    __nv_bfloat16* CbT = nullptr;     // N x M bf16, transposed
+};
+
+// M % 128 == 0, N % BN == 0, K % 64 == 0; grid (N / BN, M / 128, splits of K).
+// The network's GEMMs are small (1,024 x 256 x 256 for a training batch), so a
+// launch is bound by its latency and by how many SMs it uses: 64 columns per
+// CTA (32 CTAs per batch instead of 8 with whole rows), the four K-chunks of a
+// layer all in flight, and the passes that followed the GEMMs -- ReLU' and
+// bias gradient, transposes for the weight gradients -- done in the epilogue
+// from registers (a GEMM 21 -> 10 us; ReLU' 17 us and six transposes of 3.4 us
+// gone; a step of 1,024 rows 178 -> 74 us of kernels).
+constexpr int kMlpStages = 4;
 template <int BN>
 static __global__ void __launch_bounds__(kGemmThreads, 1)
 k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, int M, int N, int K,
-            float* __restrict__ C, const float* __restrict__ bias, int relu, __nv_bfloat16* __restrict__ Cb,
-            int* __restrict__ err, int stall) {
+            GemmOut o, int* __restrict__ err, int stall) {
     constexpr int kStage = (kGemmM + BN) * kGemmKC;                   // bytes per stage
     constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) |  // f32 accum, bf16 x bf16
                                 ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kGemmM >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
-    const uint32_t bars = base + kGemmStages * kStage;
-    const uint32_t tslot = bars + 8 * kGemmStages;
+    const uint32_t bars = base + kMlpStages * kStage;
+    const uint32_t tslot = bars + 8 * kMlpStages;
     uint32_t* tslot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tslot - raw));
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int b0 = blockIdx.x * BN, a0 = blockIdx.y * kGemmM;
     const int KB = K * 2;                        // bytes per row
-    const int KC = KB / kGemmKC;                 // 128-byte chunks
+    const int all = KB / kGemmKC;                // 128-byte chunks; this split's are [k0, k0 + KC)
+    const int k0 = (int)((long long)all * blockIdx.z / gridDim.z);
+    const int KC = (int)((long long)all * (blockIdx.z + 1) / gridDim.z) - k0;
     const uint8_t* Ab = reinterpret_cast<const uint8_t*>(A);
     const uint8_t* Bb = reinterpret_cast<const uint8_t*>(B);
 
@@ -44,7 +64,7 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (int s = 0; s < kGemmStages; s++)
+        for (int s = 0; s < kMlpStages; s++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bars + 8 * s) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -56,7 +76,7 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
 
     auto load = [&](int st, int kc) {
         const uint32_t sA = base + st * kStage, sB = sA + kGemmM * kGemmKC;
-        const size_t koff = (size_t)kc * kGemmKC;
+        const size_t koff = (size_t)(k0 + kc) * kGemmKC;
         for (int i = tid; i < kGemmM * 8; i += kGemmThreads) {
             const int r = i >> 3, c = i & 7;
             cp_async16(sA + r * 128 + ((c ^ (r & 7)) << 4), Ab + (size_t)(a0 + r) * KB + koff + c * 16);
@@ -66,26 +86,26 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
             cp_async16(sB + r * 128 + ((c ^ (r & 7)) << 4), Bb + (size_t)(b0 + r) * KB + koff + c * 16);
         }
     };
-    for (int s = 0; s < kGemmStages - 1; s++) {
+    for (int s = 0; s < kMlpStages - 1; s++) {
         if (s < KC) load(s, s);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     for (int kc = 0; kc < KC; kc++) {
-        const int nxt = kc + kGemmStages - 1;
+        const int nxt = kc + kMlpStages - 1;
         if (nxt < KC) {
             if (kc >= 1) {
                 const int prev = kc - 1;
-                ok = ok && mbar_wait_bounded(bars + 8 * (prev % kGemmStages), (prev / kGemmStages) & 1, err);
+                ok = ok && mbar_wait_bounded(bars + 8 * (prev % kMlpStages), (prev / kMlpStages) & 1, err);
             }
-            load(nxt % kGemmStages, nxt);
+            load(nxt % kMlpStages, nxt);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group %0;" :: "n"(kGemmStages - 1) : "memory");
+        asm volatile("cp.async.wait_group %0;" :: "n"(kMlpStages - 1) : "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (tid == 0 && ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int st = kc % kGemmStages;
+            const int st = kc % kMlpStages;
             const uint32_t sa = base + st * kStage, sb = sa + kGemmM * kGemmKC;
 #pragma unroll
             for (int j = 0; j < kGemmKC / 32; j++) {  // 16 bf16 = 32 bytes of K per MMA
@@ -104,10 +124,10 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (KC > 0) {
         const int last = KC - 1;
-        ok = ok && mbar_wait_bounded(bars + 8 * (last % kGemmStages), (last / kGemmStages) & 1, err);
+        ok = ok && mbar_wait_bounded(bars + 8 * (last % kMlpStages), (last / kMlpStages) & 1, err);
         // test hook (bm_test_stall): the barrier's next phase never completes
-        if (stall && blockIdx.x == 0 && blockIdx.y == 0)
-            ok = ok && mbar_wait_bounded(bars + 8 * (last % kGemmStages), ((last / kGemmStages) + 1) & 1, err,
+        if (stall && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
+            ok = ok && mbar_wait_bounded(bars + 8 * (last % kMlpStages), ((last / kMlpStages) + 1) & 1, err,
                                          kStallPolls);
     }
     __syncthreads();
@@ -126,26 +146,56 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
               "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
             : "r"(taddr));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (ok && row < M) {
-            const int c0 = b0 + cb * 32;
-            float v[32];
+        if (!__all_sync(0xffffffffu, ok)) continue;
+        const int c0 = b0 + cb * 32;
+        float v[32];
 #pragma unroll
-            for (int q = 0; q < 32; q++) {
-                float x = __uint_as_float(r[q]);
-                if (bias) x += bias[c0 + q];
-                if (relu) x = fmaxf(x, 0.f);
-                v[q] = x;
-            }
-            if (C) {
-                float4* d4 = reinterpret_cast<float4*>(C + (size_t)row * N + c0);
+        for (int q = 0; q < 32; q++) {
+            float x = __uint_as_float(r[q]);
+            if (o.bias) x += o.bias[c0 + q];
+            if (o.relu) x = fmaxf(x, 0.f);
+            v[q] = x;
+        }
+        if (o.mask) {
+            const float4* m4 = reinterpret_cast<const float4*>(o.mask + (size_t)row * N + c0);
 #pragma unroll
-                for (int q = 0; q < 8; q++) d4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            for (int q = 0; q < 8; q++) {
+                const float4 m = m4[q];
+                if (!(m.x > 0.f)) v[4 * q] = 0.f;
+                if (!(m.y > 0.f)) v[4 * q + 1] = 0.f;
+                if (!(m.z > 0.f)) v[4 * q + 2] = 0.f;
+                if (!(m.w > 0.f)) v[4 * q + 3] = 0.f;
             }
-            if (Cb) {
-                __nv_bfloat162* d2 = reinterpret_cast<__nv_bfloat162*>(Cb + (size_t)row * N + c0);
+        }
+        if (o.C) {
+            float4* d4 = reinterpret_cast<float4*>(o.C + (size_t)row * N + c0);
 #pragma unroll
-                for (int q = 0; q < 16; q++) d2[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+            for (int q = 0; q < 8; q++) d4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        }
+        if (o.add) {
+#pragma unroll
+            for (int q = 0; q < 32; q++) atomicAdd(o.add + (size_t)row * N + c0 + q, v[q]);
+        }
+        if (o.Cb) {
+            __nv_bfloat162* d2 = reinterpret_cast<__nv_bfloat162*>(o.Cb + (size_t)row * N + c0);
+#pragma unroll
+            for (int q = 0; q < 16; q++) d2[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+        }
+        if (o.CbT) {   // a warp's 32 rows are consecutive: 64 bytes per column
+#pragma unroll
+            for (int q = 0; q < 32; q++) o.CbT[(size_t)(c0 + q) * M + row] = __float2bfloat16(v[q]);
+        }
+        if (o.colsum) {   // halving: lane q ends with column q
+#pragma unroll
+            for (int w = 16; w; w >>= 1) {
+                const bool up = lane & w;
+#pragma unroll
+                for (int q = 0; q < w; q++) {
+                    const float give = up ? v[q] : v[q + w], keep = up ? v[q + w] : v[q];
+                    v[q] = keep + __shfl_xor_sync(0xffffffffu, give, w);
+                }
             }
+            atomicAdd(o.colsum + c0 + lane, v[0]);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -155,92 +205,109 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
 }
 
 template <int BN>
-constexpr int gemm_bf16_smem() { return kGemmStages * (kGemmM + BN) * kGemmKC + 1024 + 256; }
+constexpr int gemm_bf16_smem() { return kMlpStages * (kGemmM + BN) * kGemmKC + 1024 + 256; }
 
-// out[c][r] = in[r][c] for an R x C bf16 matrix.
-static __global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ in, int R, int C,
-                                        __nv_bfloat16* __restrict__ out) {
-    __shared__ __nv_bfloat16 t[32][33];
-    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int r = r0 + y, c = c0 + threadIdx.x;
-        t[y][threadIdx.x] = (r < R && c < C) ? in[(size_t)r * C + c] : __float2bfloat16(0.f);
+// out[i] = bf16(x[i]) for a rows x kMlpIn matrix (zero rows from k on), and its
+// transpose (ld = rows) if outT is given.  32 rows per block of 128 threads.
+static __global__ void __launch_bounds__(kMlpIn) k_rows_bf16(const float* __restrict__ x, int k, int rows,
+                                                             __nv_bfloat16* __restrict__ out,
+                                                             __nv_bfloat16* __restrict__ outT) {
+    const int c = threadIdx.x, r0 = blockIdx.x * 32;
+    __align__(16) __nv_bfloat16 col[32];
+#pragma unroll
+    for (int r = 0; r < 32; r++) {
+        col[r] = __float2bfloat16(r0 + r < k ? x[(size_t)(r0 + r) * kMlpIn + c] : 0.f);
+        out[(size_t)(r0 + r) * kMlpIn + c] = col[r];
     }
-    __syncthreads();
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int c = c0 + y, r = r0 + threadIdx.x;
-        if (c < C && r < R) out[(size_t)c * R + r] = t[threadIdx.x][y];
+    if (outT) {
+        uint4* dst = reinterpret_cast<uint4*>(outT + (size_t)c * rows + r0);
+#pragma unroll
+        for (int q = 0; q < 4; q++) dst[q] = reinterpret_cast<const uint4*>(col)[q];
     }
 }
 
 // Head and loss: y = H2 . w3 + b3 (rows < Bv valid), dy = 2 (y - t) / Bv,
-// dH2 = dy w3 masked by ReLU'(H2) (bf16), dw3 += H2^T dy, db3 += sum dy.
-// One warp per row.
-static __global__ void k_head(const float* __restrict__ H2, int Bv, int Bpad, const float* __restrict__ w3,
-                              const float* __restrict__ b3, float* __restrict__ y, const float* __restrict__ target,
-                              float* __restrict__ loss, __nv_bfloat16* __restrict__ dH2, float* __restrict__ dw3,
-                              float* __restrict__ db3) {
-    const int lane = threadIdx.x & 31;
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (row >= Bpad) return;
-    const float* h = H2 + (size_t)row * kMlpHid;
-    float s = 0.f;
-    for (int c = lane; c < kMlpHid; c += 32) s += h[c] * w3[c];
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const float out = s + b3[0];
-    if (lane == 0 && y && row < Bv) y[row] = out;
+// dH2 = dy w3 masked by ReLU'(H2) (bf16, and its transpose), dw3 += H2^T dy,
+// db3 += sum dy, db2 += column sums of dH2.  32 rows per block: warps take four
+// rows' dot products each, then a thread per column walks the rows, so the
+// column gradients cost an atomic per block and column (one per row and column
+// before, 11 us, and a pass of its own for db2, 10 us).
+static __global__ void __launch_bounds__(kMlpHid) k_head(const float* __restrict__ H2, int Bv, int Bpad,
+                                                         const float* __restrict__ w3, const float* __restrict__ b3,
+                                                         float* __restrict__ y, const float* __restrict__ target,
+                                                         float* __restrict__ loss, __nv_bfloat16* __restrict__ dH2,
+                                                         __nv_bfloat16* __restrict__ dH2T, float* __restrict__ dw3,
+                                                         float* __restrict__ db3, float* __restrict__ db2) {
+    __shared__ float s_dy[32], s_loss[32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, r0 = blockIdx.x * 32;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int r = 4 * wid + q, row = r0 + r;
+        const float* h = H2 + (size_t)row * kMlpHid;
+        float s = 0.f;
+#pragma unroll
+        for (int c = lane; c < kMlpHid; c += 32) s += h[c] * w3[c];
+        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) {
+            const float out = s + b3[0];
+            if (y && row < Bv) y[row] = out;
+            float dy = 0.f, l = 0.f;
+            if (target && row < Bv) {
+                const float d = out - target[row];
+                dy = 2.f * d / (float)Bv;
+                l = d * d / (float)Bv;
+            }
+            s_dy[r] = dy;
+            s_loss[r] = l;
+        }
+    }
     if (!target) return;
-    const float dy = row < Bv ? 2.f * (out - target[row]) / (float)Bv : 0.f;
-    if (lane == 0 && row < Bv) {
-        atomicAdd(loss, (out - target[row]) * (out - target[row]) / (float)Bv);
-        atomicAdd(db3, dy);
+    __syncthreads();
+    if (wid == 0) {
+        float l = s_loss[lane], d = s_dy[lane];
+        for (int o = 16; o; o >>= 1) { l += __shfl_xor_sync(0xffffffffu, l, o); d += __shfl_xor_sync(0xffffffffu, d, o); }
+        if (lane == 0) { atomicAdd(loss, l); atomicAdd(db3, d); }
     }
-    for (int c = lane; c < kMlpHid; c += 32) {
-        const float hv = h[c];
-        dH2[(size_t)row * kMlpHid + c] = __float2bfloat16(hv > 0.f ? dy * w3[c] : 0.f);
-        if (dy != 0.f) atomicAdd(&dw3[c], hv * dy);
+    const int c = tid;
+    const float w = w3[c];
+    float g3 = 0.f, g2 = 0.f;
+    __align__(16) __nv_bfloat16 col[32];
+#pragma unroll
+    for (int r = 0; r < 32; r++) {
+        const float hv = H2[(size_t)(r0 + r) * kMlpHid + c], dy = s_dy[r];
+        col[r] = __float2bfloat16(hv > 0.f ? dy * w : 0.f);
+        dH2[(size_t)(r0 + r) * kMlpHid + c] = col[r];
+        g3 += hv * dy;
+        g2 += __bfloat162float(col[r]);
     }
+    uint4* dst = reinterpret_cast<uint4*>(dH2T + (size_t)c * Bpad + r0);
+#pragma unroll
+    for (int q = 0; q < 4; q++) dst[q] = reinterpret_cast<const uint4*>(col)[q];
+    atomicAdd(&dw3[c], g3);
+    atomicAdd(&db2[c], g2);
 }
 
-// dH1 (fp32 from the GEMM) masked by ReLU'(H1), to bf16; db (column sums of
-// the masked gradient) accumulated.
-static __global__ void k_relu_bwd(const float* __restrict__ dH, const float* __restrict__ H, int rows, int cols,
-                                  __nv_bfloat16* __restrict__ out, float* __restrict__ db) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float acc = 0.f;
-    for (int r = blockIdx.y; r < rows; r += gridDim.y) {
-        const float g = H[(size_t)r * cols + c] > 0.f ? dH[(size_t)r * cols + c] : 0.f;
-        out[(size_t)r * cols + c] = __float2bfloat16(g);
-        acc += g;
-    }
-    if (db) atomicAdd(&db[c], acc);
-}
-
-// Column sums of a bf16 gradient (bias gradient of the second hidden layer).
-static __global__ void k_colsum_bf16(const __nv_bfloat16* __restrict__ G, int rows, int cols, float* __restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float acc = 0.f;
-    for (int r = blockIdx.y; r < rows; r += gridDim.y) acc += __bfloat162float(G[(size_t)r * cols + c]);
-    atomicAdd(&out[c], acc);
-}
-
-// SGD on fp32 master weights, refreshing the bf16 copy: w -= lr * g, the
-// product and the difference each rounded to nearest (no fused multiply-add),
-// so the update is reproducible on any IEEE host.
-static __global__ void k_sgd(float* __restrict__ w, const float* __restrict__ g, int count, float lr,
-                             __nv_bfloat16* __restrict__ wb) {
+// SGD on the fp32 master weights, refreshing the bf16 copies the GEMMs read
+// (W1, W2 and W2's transpose): w -= lr * g, the product and the difference each
+// rounded to nearest (no fused multiply-add), so the update is reproducible on
+// any IEEE host.  With g == nullptr only the copies are refreshed.
+static __global__ void k_sgd(float* __restrict__ w, const float* __restrict__ g, int count, float lr, int oW1, int oW2,
+                             __nv_bfloat16* __restrict__ W1b, __nv_bfloat16* __restrict__ W2b,
+                             __nv_bfloat16* __restrict__ W2Tb) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    const float v = __fsub_rn(w[i], __fmul_rn(lr, g[i]));
-    w[i] = v;
-    if (wb) wb[i] = __float2bfloat16(v);
-}
-
-static __global__ void k_to_bf16(const float* __restrict__ x, int count, __nv_bfloat16* __restrict__ y) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count) y[i] = __float2bfloat16(x[i]);
+    float v = w[i];
+    if (g) {
+        v = __fsub_rn(v, __fmul_rn(lr, g[i]));
+        w[i] = v;
+    }
+    const int j1 = i - oW1, j2 = i - oW2;
+    if (j1 >= 0 && j1 < kMlpHid * kMlpIn) W1b[j1] = __float2bfloat16(v);
+    if (j2 >= 0 && j2 < kMlpHid * kMlpHid) {
+        const __nv_bfloat16 b = __float2bfloat16(v);
+        W2b[j2] = b;
+        W2Tb[(j2 % kMlpHid) * kMlpHid + j2 / kMlpHid] = b;
+    }
 }
 
 // ---------------------------------------------------------------------------
