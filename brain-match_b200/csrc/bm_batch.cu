@@ -113,7 +113,7 @@ template <bool W16>
 __global__ void __launch_bounds__(512)
 k_b_profit(const DevView<W16>* __restrict__ views, const int* __restrict__ row_base, int nb, int total,
            const int* __restrict__ order, int* __restrict__ counter) {
-    extern __shared__ int acc[];
+    extern __shared__ __align__(16) int acc[];
     __shared__ int s_item, s_nlong;
     __shared__ int2 s_long[kLongQueue];
     for (;;) {
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kBThreads, 1) k_b_sweep(BSweepArgs<W16> a) {
                     const int half = gtid >> 7, r = 2 * local + half;
                     const int hb = 2 * grp + half;   // the half's barrier: 5 + hb, 128 threads
                     if (r < I.n)
-                        profit_row_on<W16, 128>(g, r, acc + half * ((I.n + 1 + 3) & ~3), s_long[hb], &s_nlong[hb],
+                        profit_row_on<W16, 128>(g, r, acc + half * (row_smem(I.n) / sizeof(int)), s_long[hb], &s_nlong[hb],
                                                 nullptr, 0, nullptr, nullptr, [hb] {
                                                     asm volatile("bar.sync %0, 128;" :: "r"(5 + hb) : "memory");
                                                 });
@@ -761,8 +761,7 @@ extern "C" bm_status bm_batch_scores(bm_batch* B, int64_t* scores) {
 // tile stage, whichever is larger.
 template <int T>
 static size_t persistent_group_bytes(int max_n) {
-    const size_t row = (size_t)((max_n + 1 + 3) & ~3) * sizeof(int);
-    return (std::max(row, sizeof(CombineSmem<T>)) + 15) & ~(size_t)15;
+    return (std::max(row_smem(max_n), sizeof(CombineSmem<T>)) + 15) & ~(size_t)15;
 }
 
 template <int T>
@@ -855,7 +854,7 @@ static bm_status enqueue_eval(bm_batch* B) {
     BK(cub::DeviceRadixSort::SortPairsDescending(B->cub_tmp, tb, B->wkeys, B->wkeys_sorted, B->wvals, B->order,
                                                  B->total, 0, 64, B->st));
     BK(cudaMemsetAsync(B->counter, 0, sizeof(int), B->st));
-    const size_t smem = (size_t)(B->max_n + 1) * sizeof(int);
+    const size_t smem = row_smem(B->max_n);
     BK(cudaFuncSetAttribute(k_b_profit<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0, sms = B->ctx[0]->num_sms;
     BK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_b_profit<W16>, B->profit_threads, smem));

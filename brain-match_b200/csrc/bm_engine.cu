@@ -538,7 +538,7 @@ static cudaError_t record_exact_mapping(bm_ctx* ctx) {
 
 bm_status ensure_S(bm_ctx* ctx) {
     if (ctx->S) return BM_OK;
-    CK(dalloc(ctx, &ctx->S, (size_t)ctx->n * ctx->n * sizeof(int)));
+    CK(dalloc(ctx, &ctx->S, (size_t)ctx->n * s_pitch(ctx->n) * sizeof(int)));
     return BM_OK;
 }
 
@@ -591,7 +591,7 @@ bm_status stage_profit(bm_ctx* ctx) {
         }
         CK(cudaGetLastError());
     }
-    const size_t smem = (size_t)(n + 1) * sizeof(int);
+    const size_t smem = row_smem(n);
     CK(cudaFuncSetAttribute(k_profit<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_profit<W16>, 512, smem));
@@ -698,9 +698,9 @@ bm_status stage_refresh(bm_ctx* ctx, int* mode) {
 template bm_status stage_refresh<true>(bm_ctx*, int*);
 template bm_status stage_refresh<false>(bm_ctx*, int*);
 
-// The tensor map of S for the TMA-fed combine: rows of n int32, 64x64 boxes,
-// zero fill outside the matrix.  Needs the row stride (4n bytes) to be a
-// multiple of 16; returns false (the caller keeps k_combine64) otherwise.
+// The tensor map of S for the TMA-fed combine: rows of n int32, boxes of 64 rows
+// x 32 columns, zero fill outside the matrix.  Returns false for a matrix
+// smaller than a tile (the caller keeps k_combine64).
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     static std::once_flag once;
@@ -744,15 +744,15 @@ static bool hub_ws_setup(bm_ctx* ctx) {
 
 static bool combine_tma_setup(bm_ctx* ctx) {
     const int n = ctx->n;
-    if ((n & 3) != 0 || n < kCmbT) return false;
+    if (n < kCmbT) return false;
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
     if (!encode) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)n, (cuuint64_t)n};
-    const cuuint64_t strides[1] = {(cuuint64_t)n * sizeof(int)};
-    const cuuint32_t box[2] = {kCmbT, kCmbT};
+    const cuuint64_t strides[1] = {(cuuint64_t)s_pitch(n) * sizeof(int)};
+    const cuuint32_t box[2] = {kCmbBox, kCmbT};
     const cuuint32_t estr[2] = {1, 1};
     if (encode(&ctx->tmS, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, ctx->S, dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
     if (cudaFuncSetAttribute(k_combine_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, kCmbSmem) != cudaSuccess)
@@ -922,7 +922,7 @@ extern "C" bm_status bm_profit_row(bm_ctx* ctx, int32_t a, int32_t* out) {
     if (s) return s;
     s = ctx->w16 ? stage_profit<true>(ctx) : stage_profit<false>(ctx);
     if (s) return s;
-    CK(cudaMemcpyAsync(out, ctx->S + (size_t)(a - 1) * ctx->n, ctx->n * sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
+    CK(cudaMemcpyAsync(out, ctx->S + (size_t)(a - 1) * s_pitch(ctx->n), ctx->n * sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return BM_OK;
 }

@@ -188,17 +188,12 @@ k_hub_gemm(const uint8_t* __restrict__ A, const uint8_t* __restrict__ B, int K, 
             : "r"(taddr));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (ok && a < n) {
-            int* row = S + (size_t)a * n;
             const int c0 = b0 + cb * 32;
-            if ((n & 3) == 0 && c0 + 32 <= n) {
-                int4* d4 = reinterpret_cast<int4*>(row + c0);
+            int4* d4 = reinterpret_cast<int4*>(S + (size_t)a * s_pitch(n) + c0);
 #pragma unroll
-                for (int q = 0; q < 8; q++)
+            for (int q = 0; q < 8; q++)
+                if (c0 + 4 * q < n)
                     d4[q] = make_int4((int)r[4 * q], (int)r[4 * q + 1], (int)r[4 * q + 2], (int)r[4 * q + 3]);
-            } else {
-                for (int q = 0; q < 32; q++)
-                    if (c0 + q < n) row[c0 + q] = (int)r[q];
-            }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

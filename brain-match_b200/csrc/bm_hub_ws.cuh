@@ -207,18 +207,13 @@ k_hub_gemm_ws(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ C
                 for (int u = 0; u < 32; u++) blk[lane * kWsEpiStride + u] = (int)r[u];
                 __syncwarp();
                 const int c0 = b0 + cb * 32, cl = 4 * (lane & 7);
-                const bool full = (n & 3) == 0 && c0 + 32 <= n;
 #pragma unroll
                 for (int jr = 0; jr < 8; jr++) {
                     const int rl = 4 * jr + (lane >> 3), ar = a - lane + rl;   // ar: that row's vertex
                     const int* src = blk + rl * kWsEpiStride + cl;
-                    if (ar < n) {
-                        int* dst = S + (size_t)ar * n + c0 + cl;
-                        if (full) *reinterpret_cast<int4*>(dst) = make_int4(src[0], src[1], src[2], src[3]);
-                        else
-                            for (int u = 0; u < 4; u++)
-                                if (c0 + cl + u < n) dst[u] = src[u];
-                    }
+                    if (ar < n && c0 + cl < n)
+                        *reinterpret_cast<int4*>(S + (size_t)ar * s_pitch(n) + c0 + cl) =
+                            make_int4(src[0], src[1], src[2], src[3]);
                 }
                 __syncwarp();
             }

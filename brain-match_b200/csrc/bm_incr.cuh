@@ -116,7 +116,6 @@ __global__ void k_corner(DevView<W16> g, const int* __restrict__ pm, const int* 
     typedef Ent<W16> EN;
     if (dcount) count = min(count, *dcount);
     if ((int)blockIdx.x >= count) return;
-    const int n = g.n;
     const int m = moved[blockIdx.x];
     const int so = g.off1o[m], lo = g.off1o[m + 1] - so;
     const int si = g.off1i[m], li = g.off1i[m + 1] - si;
@@ -133,7 +132,7 @@ __global__ void k_corner(DevView<W16> g, const int* __restrict__ pm, const int* 
     }
     const int pa = pm[a], pb = pm[b];
     const int c = corner_term(x, g.w2(pa, pb), g.w2t(pb, pa), g.w2d(pa), g.w2d(pb));
-    if (c) atomicAdd(&g.S[(size_t)a * n + b], sign * c);
+    if (c) atomicAdd(&g.S[g.at(a, b)], sign * c);
 }
 
 // Step 2: for every row, new S[a][b] = old S[a][pinvS[p b]] for b in moved
@@ -152,7 +151,7 @@ __global__ void k_perm_cols(int* __restrict__ S, int n, const int* __restrict__ 
     }
     __syncthreads();
     for (int a = blockIdx.x; a < n; a += gridDim.x) {
-        int* row = S + (size_t)a * n;
+        int* row = S + (size_t)a * s_pitch(n);
         for (int j = threadIdx.x; j < count; j += blockDim.x) buf[j] = src[j] < 0 ? 0 : row[src[j]];
         __syncthreads();
         for (int j = threadIdx.x; j < count; j += blockDim.x) row[dst[j]] = buf[j];
@@ -194,7 +193,7 @@ __global__ void __launch_bounds__(256) k_terms(DevView<W16> g, const int* __rest
             row = EN::id(e); w1 = EN::w(e);
             off = g.off2o; list = g.ent2o;
         }
-        int* srow = g.S + (size_t)row * n;
+        int* srow = g.S + g.at(row, 0);
         for (int k = off[fo] + lane; k < off[fo + 1]; k += 32) {
             const E e = list[k];
             const int col = g.pinv[EN::id(e)];
@@ -254,7 +253,7 @@ __global__ void __launch_bounds__(kIncrRowThreads) k_terms_rows(DevView<W16> g, 
             atomicAdd(&rowbuf[g.pinv[EN::id(e)]], imin(w1, EN::w(e)));
         }
         __syncthreads();
-        int* srow = g.S + (size_t)row * n;
+        int* srow = g.S + g.at(row, 0);
         for (int c = threadIdx.x; c < n; c += blockDim.x) {
             const int v = rowbuf[c];
             if (v) { atomicAdd(&srow[c], v); rowbuf[c] = 0; }
@@ -287,7 +286,7 @@ __global__ void k_perm_cols_small(int* __restrict__ S, int n, const int* __restr
         }
     }
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-        int* row = S + (size_t)a * n;
+        int* row = S + (size_t)a * s_pitch(n);
 #pragma unroll
         for (int j = 0; j < kSmallMoved; j++)
             if (j < count) val[j] = src[j] < 0 ? 0 : row[src[j]];
@@ -360,8 +359,8 @@ __global__ void k_delta_rows(const int* __restrict__ S, int n, int a0, int rows,
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
         const int a = a0 + (int)(i / n), b = (int)(i % n);
-        out[i] = a == b ? 0
-                        : S[(size_t)a * n + b] + S[(size_t)b * n + a] - S[(size_t)a * n + a] - S[(size_t)b * n + b];
+        const size_t ld = s_pitch(n);
+        out[i] = a == b ? 0 : S[a * ld + b] + S[b * ld + a] - S[a * ld + a] - S[b * ld + b];
     }
 }
 

@@ -67,7 +67,7 @@ struct bm_ctx {
     cudaEvent_t uev[8] = {};       // bm_timer_* slots
     unsigned long long* work_sum = nullptr;   // min terms of the last rebuild
     unsigned long long* part = nullptr;   // per-tile best partners (combine)
-    // TMA-fed combine (n % 4 == 0): tensor map over S, S's diagonal, grid size
+    // TMA-fed combine (n >= 64): tensor map over S, S's diagonal, grid size
     alignas(64) CUtensorMap tmS;
     // persistent warp-specialised hub GEMM: tensor maps of its operands
     alignas(64) CUtensorMap tmHubA;

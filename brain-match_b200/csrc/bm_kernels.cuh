@@ -48,6 +48,13 @@ template <bool W16> struct Dense;
 template <> struct Dense<true> { typedef uint16_t T; };
 template <> struct Dense<false> { typedef int32_t T; };
 
+// Row pitch of the profit matrix S: rows start on 16-byte boundaries at every n,
+// so that S is read and written in 16-byte pieces and by TMA.  Columns n .. pitch
+// - 1 hold no meaning.
+__host__ __device__ __forceinline__ int s_pitch(int n) { return (n + 3) & ~3; }
+// Shared memory of a profit row's accumulator: n + 1 ints in whole 16-byte words.
+__host__ __device__ __forceinline__ size_t row_smem(int n) { return (size_t)((n + 4) & ~3) * sizeof(int); }
+
 // Device view of a context.
 template <bool W16> struct DevView {
     typedef typename Ent<W16>::T E;
@@ -65,7 +72,7 @@ template <bool W16> struct DevView {
     const D* W2T;                       // its transpose (columns of W2 read as rows)
     const int* W2D;                     // its diagonal W2[f][f], f = 0..n
     int* p; int* pinv;                  // n+1 entries, [n] = n
-    int* S;                             // n*n profit matrix
+    int* S;                             // profit matrix, n rows of s_pitch(n)
     __device__ __forceinline__ int w2(int f, int g) const {
         return (int)W2[(size_t)f * (size_t)(n + 1) + (size_t)g];
     }
@@ -73,6 +80,8 @@ template <bool W16> struct DevView {
     __device__ __forceinline__ int w2t(int f, int g) const {
         return (int)W2T[(size_t)g * (size_t)(n + 1) + (size_t)f];
     }
+    // S[a][b]
+    __device__ __forceinline__ size_t at(int a, int b) const { return (size_t)a * s_pitch(n) + b; }
     // same value as w2(f, f)
     __device__ __forceinline__ int w2d(int f) const { return W2D[f]; }
 };
@@ -170,7 +179,8 @@ __device__ __forceinline__ void scatter_residual(int* acc, const typename Ent<W1
 // One profit row of S by a group of threads that all call it together: the
 // whole block (NT = 0), or the NT threads (a power of two) of the block's
 // NT-aligned group; `sync` is a barrier over exactly those threads.  It ends
-// with a barrier.  acc holds n+1 ints of shared memory.
+// with a barrier.  acc holds row_smem(n) bytes of
+// shared memory on a 16-byte boundary.
 // With `work_total`, the row adds its scattered min terms to it.
 template <bool W16, int NT, typename Sync>
 __device__ __forceinline__ void profit_row_on(const DevView<W16>& g, int a, int* acc, int2* s_long, int* s_nlong,
@@ -189,12 +199,9 @@ __device__ __forceinline__ void profit_row_on(const DevView<W16>& g, int a, int*
     }
     // the row's scattered terms start from zero; with hubs, the tensor-core
     // hub terms already in S are added when the row is written back
-    if ((n & 3) == 0) {
+    {
         int4* a4 = reinterpret_cast<int4*>(acc);
-        for (int i = tid; i < (n >> 2); i += nthr) a4[i] = make_int4(0, 0, 0, 0);
-        if (tid == 0) acc[n] = 0;
-    } else {
-        for (int i = tid; i <= n; i += nthr) acc[i] = 0;
+        for (int i = tid; i < ((n + 4) >> 2); i += nthr) a4[i] = make_int4(0, 0, 0, 0);
     }
     sync();
     // out-edges of a against G2 in-lists of p(v), then in-edges against out-lists of p(u)
@@ -291,12 +298,11 @@ __device__ __forceinline__ void profit_row_on(const DevView<W16>& g, int a, int*
     }
     sync();
     if (work_total && tid == 0) atomicAdd(work_total, (unsigned long long)*s_terms);
-    int* row = g.S + (size_t)a * (size_t)n;
-    if ((n & 3) == 0) {
-        int4* r4 = reinterpret_cast<int4*>(row);
+    {
+        const int n4 = s_pitch(n) >> 2;
+        int4* r4 = reinterpret_cast<int4*>(g.S + g.at(a, 0));
         const int4* a4 = reinterpret_cast<const int4*>(acc);
         if (is_hub) {
-            const int n4 = n >> 2;
             int i = tid;
             for (; i + 3 * (int)nthr < n4; i += 4 * nthr) {
                 int4 h[4];
@@ -313,11 +319,8 @@ __device__ __forceinline__ void profit_row_on(const DevView<W16>& g, int a, int*
                 r4[i] = make_int4(h.x + v.x, h.y + v.y, h.z + v.z, h.w + v.w);
             }
         } else {
-            for (int i = tid; i < (n >> 2); i += nthr) r4[i] = a4[i];
+            for (int i = tid; i < n4; i += nthr) r4[i] = a4[i];
         }
-    } else {
-        if (is_hub) for (int i = tid; i < n; i += nthr) row[i] += acc[i];
-        else for (int i = tid; i < n; i += nthr) row[i] = acc[i];
     }
     sync();
 }
@@ -336,7 +339,7 @@ template <bool W16>
 __global__ void __launch_bounds__(512, 3)
 k_profit(DevView<W16> g, const int* __restrict__ order, int* __restrict__ counter,
          const unsigned char* __restrict__ is_hub, int hub_thr, unsigned long long* __restrict__ work_total) {
-    extern __shared__ int acc[];
+    extern __shared__ __align__(16) int acc[];
     __shared__ int s_row, s_nlong, s_terms;
     __shared__ int2 s_long[kLongQueue];  // (G2 vertex, w1 | kind << 31)
     for (;;) {

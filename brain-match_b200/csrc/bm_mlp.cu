@@ -257,7 +257,7 @@ __global__ void k_samples(DevView<W16> g, const unsigned long long* __restrict__
     for (int j = 0; j <= extra; j++) {
         int b = j == 0 ? (int)(~(unsigned)(rowbest[a] & 0xffffffffu)) : pool_partner(g, a, j - 1, seed);
         if (b < 0 || b >= n || b == a) b = (a + 1) % n;
-        const int d = S[(size_t)a * n + b] + S[(size_t)b * n + a] - S[(size_t)a * n + a] - S[(size_t)b * n + b];
+        const int d = S[g.at(a, b)] + S[g.at(b, a)] - S[g.at(a, a)] - S[g.at(b, b)];
         const size_t o = (size_t)a * (extra + 1) + j;
         pa[o] = a; pb[o] = b;
         t[o] = (d > 0 ? 1.f : (d < 0 ? -1.f : 0.f)) * log1pf(fabsf((float)d));

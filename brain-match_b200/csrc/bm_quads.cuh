@@ -60,7 +60,7 @@ __device__ int quad_delta_S(const DevView<W16>& g, const unsigned* __restrict__ 
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         if (sg[i] == i) continue;  // a vertex that keeps its image adds nothing from S
-        d += g.S[(size_t)M[i] * n + M[sg[i]]] - g.S[(size_t)M[i] * n + M[i]];
+        d += g.S[g.at(M[i], M[sg[i]])] - g.S[g.at(M[i], M[i])];
     }
     for (int i = 0; i < 4; i++) {
         for (int j = 0; j < 4; j++) {
@@ -185,7 +185,7 @@ __device__ void quad_best(const DevView<W16>& g, const unsigned* __restrict__ ad
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            sm[i][j] = g.S[(size_t)M[i] * n + M[j]];
+            sm[i][j] = g.S[g.at(M[i], M[j])];
             wm[i][j] = g.w2(pm[i], pm[j]);
         }
     for (int q = 1; q < 24; q++) {

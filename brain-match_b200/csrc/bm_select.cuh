@@ -18,91 +18,91 @@ namespace bm {
 
 constexpr int kTile = 64;
 
-// One TxT tile (ti <= tj) of the upper triangle, 256 threads (T = 32 or 64).
 // Shared memory of one combine tile pass.
 template <int T> struct CombineSmem {
+    static constexpr int kSegs = 128 / T;   // threads per owner: the partners in kSegs shares
     int sA[T][T + 1];               // sA[r][c] = S[a0+r][b0+c]
     int sB[T][T + 1];               // sB[r][c] = S[b0+r][a0+c]
     int dA[T], dB[T];
-    unsigned long long cpart[8][T];
+    int2 best[2][kSegs][T];         // (delta + own diagonal, partner) of each owner's share
 };
 
-// One tile pair by 256 threads (tid 0..255 among them; `sync` is a barrier
-// over exactly those threads), staged in `sm`.
+// One TxT tile (ti <= tj) of the upper triangle by 256 threads (tid 0..255 among
+// them; T = 32 or 64; `sync` is a barrier over exactly those threads), staged in
+// `sm`.  A thread owns one vertex of the tile -- a row vertex (threads 0-127) or
+// a column vertex -- and walks a share of its partners in ascending order, so a
+// best is a compare and two moves in registers; reading the other tile
+// transposed costs no more than the tile itself (rows padded by one word).
+// Lanes holding rows, with a shuffle reduction per row and packed 64-bit keys,
+// took 2.3 times the instructions.
 template <int T, typename Sync>
 __device__ __forceinline__ void combine_tile_on(const int* __restrict__ S, int n, int ti, int tj,
                                                 unsigned long long* __restrict__ part, int* __restrict__ all_out,
                                                 CombineSmem<T>& sm, int tid, Sync sync) {
-    constexpr int CL = T / 32;            // columns per lane
+    constexpr int SEGS = CombineSmem<T>::kSegs, L = T / SEGS;   // partners per share
     const int a0 = ti * T, b0 = tj * T;
-    const int lane = tid & 31, wid = tid >> 5;  // 8 warps
-    if ((n & 3) == 0) {
-        // 16-byte streaming loads: with n a multiple of 4 every 4-column group
-        // of a row is aligned and lies wholly inside or outside the matrix
-        for (int i = tid; i < T * T / 4; i += 256) {
-            const int r = i / (T / 4), c = (i % (T / 4)) * 4;
-            const int a = a0 + r, b = b0 + c;
-            const int bb = b0 + r, aa = a0 + c;
-            int4 va = make_int4(0, 0, 0, 0), vb = make_int4(0, 0, 0, 0);
-            if (a < n && b < n) va = __ldcs(reinterpret_cast<const int4*>(S + (size_t)a * n + b));
-            if (bb < n && aa < n) vb = __ldcs(reinterpret_cast<const int4*>(S + (size_t)bb * n + aa));
-            sm.sA[r][c] = va.x; sm.sA[r][c + 1] = va.y; sm.sA[r][c + 2] = va.z; sm.sA[r][c + 3] = va.w;
-            sm.sB[r][c] = vb.x; sm.sB[r][c + 1] = vb.y; sm.sB[r][c + 2] = vb.z; sm.sB[r][c + 3] = vb.w;
-        }
-    } else {
-        for (int i = tid; i < T * T; i += 256) {
-            const int r = i / T, c = i % T;
-            const int a = a0 + r, b = b0 + c;
-            sm.sA[r][c] = (a < n && b < n) ? S[(size_t)a * n + b] : 0;
-            const int bb = b0 + r, aa = a0 + c;
-            sm.sB[r][c] = (bb < n && aa < n) ? S[(size_t)bb * n + aa] : 0;
-        }
+    const size_t ld = s_pitch(n);
+    // 16-byte streaming loads: a 4-column group that starts inside the matrix
+    // lies inside its row's pitch
+    for (int i = tid; i < T * T / 4; i += 256) {
+        const int r = i / (T / 4), c = (i % (T / 4)) * 4;
+        const int a = a0 + r, b = b0 + c;
+        const int bb = b0 + r, aa = a0 + c;
+        int4 va = make_int4(0, 0, 0, 0), vb = make_int4(0, 0, 0, 0);
+        if (a < n && b < n) va = __ldcs(reinterpret_cast<const int4*>(S + a * ld + b));
+        if (bb < n && aa < n) vb = __ldcs(reinterpret_cast<const int4*>(S + bb * ld + aa));
+        sm.sA[r][c] = va.x; sm.sA[r][c + 1] = va.y; sm.sA[r][c + 2] = va.z; sm.sA[r][c + 3] = va.w;
+        sm.sB[r][c] = vb.x; sm.sB[r][c + 1] = vb.y; sm.sB[r][c + 2] = vb.z; sm.sB[r][c + 3] = vb.w;
     }
     if (tid < T) {
         const int a = a0 + tid, b = b0 + tid;
-        sm.dA[tid] = a < n ? S[(size_t)a * n + a] : 0;
-        sm.dB[tid] = b < n ? S[(size_t)b * n + b] : 0;
+        sm.dA[tid] = a < n ? S[a * ld + a] : 0;
+        sm.dB[tid] = b < n ? S[b * ld + b] : 0;
     }
     sync();
-    const bool diag = (ti == tj);
-    // bests as 32-bit (delta, partner) pairs -- larger delta, then smaller
-    // partner -- packed into the 64-bit key only for the reductions
-    int cbd[CL], cbi[CL];
-#pragma unroll
-    for (int q = 0; q < CL; q++) { cbd[q] = INT_MIN; cbi[q] = INT_MAX; }
-    for (int r = wid; r < T; r += 8) {
-        const int a = a0 + r;
-        int rd = INT_MIN, ri = INT_MAX;
-        if (a < n) {
-#pragma unroll
-            for (int q = 0; q < CL; q++) {
-                const int c = lane + 32 * q, b = b0 + c;
-                if (b < n && b != a) {
-                    const int d = sm.sA[r][c] + sm.sB[c][r] - sm.dA[r] - sm.dB[c];
-                    if (d > rd || (d == rd && b < ri)) { rd = d; ri = b; }
-                    if (d > cbd[q] || (d == cbd[q] && a < cbi[q])) { cbd[q] = d; cbi[q] = a; }
-                    if (all_out && a < b) all_out[(long long)a * (2LL * n - a - 1) / 2 + (b - a - 1)] = d;
-                }
+    const bool diag = ti == tj;   // its row owners already cover both orders of every pair
+    const int dir = tid >> 7, seg = (tid & 127) / T, o = tid & (T - 1);
+    if (!(dir && diag)) {
+        const int (*X)[T + 1] = dir ? sm.sB : sm.sA;   // X[o][c]: own row
+        const int (*Y)[T + 1] = dir ? sm.sA : sm.sB;   // Y[c][o]: the partner's row
+        const int* dP = dir ? sm.dA : sm.dB;
+        const int p0 = dir ? a0 : b0;                  // partner c is vertex p0 + c
+        const int skip = diag ? o : -1, last = min(L * (seg + 1), n - p0);
+        int bd = INT_MIN, bi = -1;
+        if (!diag && last == L * (seg + 1)) {
+#pragma unroll 8
+            for (int c = L * seg; c < L * (seg + 1); c++) {
+                const int d = X[o][c] + Y[c][o] - dP[c];
+                if (d > bd || bi < 0) { bd = d; bi = c; }
+            }
+        } else {
+            for (int c = L * seg; c < last; c++) {
+                const int d = X[o][c] + Y[c][o] - dP[c];
+                if (c != skip && (d > bd || bi < 0)) { bd = d; bi = c; }
             }
         }
-        unsigned long long rb = ri == INT_MAX ? 0ull : pack_best(rd, ri);
-        for (int o = 16; o; o >>= 1) rb = kmax(rb, __shfl_xor_sync(0xffffffffu, rb, o));
-        if (lane == 0 && a < n) part[(size_t)tj * n + a] = rb;  // row partial of a over this tile
+        sm.best[dir][seg][o] = make_int2(bd, bi);
     }
-    unsigned long long cb[CL];
+    if (all_out) {
+        for (int i = tid; i < T * T; i += 256) {
+            const int r = i / T, c = i % T, a = a0 + r, b = b0 + c;
+            if (a < b && b < n)
+                all_out[(long long)a * (2LL * n - a - 1) / 2 + (b - a - 1)] =
+                    sm.sA[r][c] + sm.sB[c][r] - sm.dA[r] - sm.dB[c];
+        }
+    }
+    sync();
+    if (tid < 2 * T) {
+        const int d = tid / T, q = tid & (T - 1), x = (d ? b0 : a0) + q;
+        if (x < n && !(d && diag)) {
+            int2 k = sm.best[d][0][q];
 #pragma unroll
-    for (int q = 0; q < CL; q++) cb[q] = cbi[q] == INT_MAX ? 0ull : pack_best(cbd[q], cbi[q]);
-    // column partials (vertices b of the tile, over this tile's rows); a
-    // diagonal tile's row partials already cover both orders of every pair
-    if (!diag) {
-#pragma unroll
-        for (int q = 0; q < CL; q++) sm.cpart[wid][lane + 32 * q] = cb[q];
-        sync();
-        if (tid < T) {
-            unsigned long long k = sm.cpart[0][tid];
-            for (int w = 1; w < 8; w++) k = kmax(k, sm.cpart[w][tid]);
-            const int b = b0 + tid;
-            if (b < n) part[(size_t)ti * n + b] = k;
+            for (int g = 1; g < SEGS; g++) {   // the lower share keeps ties: its partners are smaller
+                const int2 y = sm.best[d][g][q];
+                if (y.y >= 0 && (k.y < 0 || y.x > k.x)) k = y;
+            }
+            part[(size_t)(d ? ti : tj) * n + x] =
+                k.y < 0 ? 0ull : pack_best(k.x - (d ? sm.dB[q] : sm.dA[q]), (d ? a0 : b0) + k.y);
         }
     }
 }

@@ -89,7 +89,7 @@ __device__ int triple_delta_S(const DevView<W16>& g, const unsigned* __restrict_
     const int pn[3] = {g.p[sig[0]], g.p[sig[1]], g.p[sig[2]]};
     int d = 0;
     for (int i = 0; i < 3; i++)
-        d += g.S[(size_t)M[i] * n + sig[i]] - g.S[(size_t)M[i] * n + M[i]];
+        d += g.S[g.at(M[i], sig[i])] - g.S[g.at(M[i], M[i])];
     for (int i = 0; i < 3; i++) {
         for (int j = 0; j < 3; j++) {
             if (i == j) continue;
