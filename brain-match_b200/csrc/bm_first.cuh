@@ -17,8 +17,10 @@
 // of their ends' images, and the G2 edges of p(a) against the G1 lists of the
 // vertices they are matched to; an edge between a and b is corrected.  A commit
 // updates C at the neighbours of the two vertices.  Bound by the latency of a
-// step, about 7 us: extents, lists and shared atomics 3, the search 1, the
-// exchange through distributed shared memory and the slowest row 2, C 1.5.
+// step, about 6 us: extents, lists and shared atomics 3, the search 1, the
+// exchange through distributed shared memory and the slowest row 1, C 1.5.  One
+// warp polls the words: with every warp polling, or a cluster barrier instead, a
+// step took 1 us more (n = 600 / E = 12,000: 20.4 ms, now 17.8).
 //
 // k_first (otherwise): the whole grid, a warp per pair (several when the window
 // has fewer pairs than there are warps), the words exchanged through slots in
@@ -28,7 +30,7 @@
 // gathers, one L1 line each, and the exchange (6 us).
 //
 // Three launches, a copy and a host wait per row scan took 189 ms at n = 600 /
-// E = 12,000 (2,171 commits in 6 passes; now 20 ms) and 1,240 ms for one pass at
+// E = 12,000 (2,171 commits in 6 passes; now 18 ms) and 1,240 ms for one pass at
 // n = 3,000 / E = 6e5 (now 423 ms).
 #pragma once
 #include "bm_kernels.cuh"
@@ -42,7 +44,7 @@ constexpr double kFirstLongLists = 1024;     // k_first: average entries of a pa
 constexpr int kRowsCluster = 16;             // k_first_rows: CTAs, rows per step
 constexpr int kRowsThreads = 1024;
 // k_first_rows: average terms of a row.  First pass, rows against grid: n = 600,
-// degree 20 (1,600 terms) 20 / 25 ms for all passes, n = 1,500, degree 30
+// degree 20 (1,600 terms) 18 / 25 ms for all passes, n = 1,500, degree 30
 // (3,600) 79 / 85 ms, degree 60 (14,400) 118 / 93 ms, degree 130 203 / 102 ms.
 constexpr double kRowsTerms = 4096;
 constexpr int kFirstSteps = 1024;            // steps per launch (the host relaunches)
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_first_rows(DevView<W16> g, 
     typedef typename EN::T E;
     constexpr int T = kRowsThreads, NWARP = T / 32;
     extern __shared__ int acc[];                       // n + 1: slot n absorbs terms of unmatched G2 vertices
-    __shared__ unsigned long long s_red[NWARP], s_slot[2][kRowsCluster];
+    __shared__ unsigned long long s_red[NWARP], s_slot[2][kRowsCluster], s_word;
     __shared__ int s_ok;
     const int n = g.n;
     int* C = acc + n + 1;
@@ -304,19 +306,23 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_first_rows(DevView<W16> g, 
             }
         }
         best = kFirstNone;
-        if (lane < kRowsCluster) {   // every warp polls
+        if (wid == 0 && lane < kRowsCluster) {
             const uint32_t here = (uint32_t)__cvta_generic_to_shared(&s_slot[par][lane]);
             unsigned long long v;
             for (unsigned it = 0;;) {
-                asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(here) : "memory");
+                asm volatile("ld.volatile.shared.u64 %0, [%1];" : "=l"(v) : "r"(here) : "memory");
                 if ((v & ~kFirstNone) == tag) break;
                 if (++it > kFirstPolls) { s_ok = 0; v = kFirstNone; break; }
             }
             best = v & kFirstNone;
         }
-        for (int o = 16; o; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
+        if (wid == 0) {
+            for (int o = 16; o; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
+            if (lane == 0) s_word = best;
+        }
         __syncthreads();     // the words are read
         if (!s_ok) break;
+        best = s_word;
         if (best != kFirstNone) {
             // ---- commit: x takes y's image and y x's; C at their neighbours ----
             const int at = (int)(best >> 31), x = m1 + (at >> 16), y = at & 0xffff;

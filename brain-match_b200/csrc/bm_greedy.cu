@@ -27,7 +27,9 @@
 // candidates, and every CTA reduces the published slice bests -- one bounded
 // grid barrier per step (the scatter of step i+1 runs before step i's decision
 // is reduced: only edges to step i's vertex need it, and those are added per
-// slice afterwards).
+// slice afterwards).  Graphs whose steps touch few list entries run in one
+// 16-CTA cluster instead (k_greedy_cluster; n = 3,000 / E = 1.5e5: 22.4 ->
+// 17.6 ms).
 #include <cub/cub.cuh>
 #include <algorithm>
 #include <cstdio>
@@ -403,6 +405,237 @@ __global__ void __launch_bounds__(kGreedyThreads, 1) k_greedy(GreedyArgs a) {
     greedy_decide(a, (a.n - 1) & 1, prev, map_s, taken, a.n, 0, wbest);
 }
 
+// The matching in one cluster of 16 CTAs, for steps of few list entries: a step
+// of the grid kernel is mostly its barrier and the trip of the slice bests
+// through L2 (7.0 us at n = 3,000 / E = 20,000).  Here every CTA adds its share
+// of the list entries into align sums of all candidates in its own shared
+// memory, a cluster barrier follows, each CTA gathers the 16 partial sums of its
+// slice's candidates through distributed shared memory (adding there instead,
+// one remote atomic per entry, took 10 us per step), and writes its slice's best
+// into all CTAs' shared memory, where after a second barrier all decide the
+// same.  The sums and the bests are double-buffered by step parity; a step's
+// vertex, extents and edges are loaded three, two and one step ahead.
+//
+// Bound by latency: 5.9 us per step at n = 3,000 / E = 1.5e5 (35,000 list
+// entries per step), of which the scatter takes 2.5, the gather and the scores
+// 0.9, and the rest, two barriers, prefix sums and reductions, is 4.3 us of a
+// step without entries.  Tagged words that one or all warps of a CTA poll
+// instead of the second barrier took 2.3 us more.
+constexpr int kGreedyCluster = 16;
+// Bound on 2 E1 E2 / n, the list entries of an average step times n (a step's
+// entries and a slice's candidates both grow its time).  ms of all steps,
+// cluster against grid:
+//   n = 200, E = 2,000 (4e4)        0.83 / 1.34
+//   n = 3,000, E = 20,000 (2.7e5)   12.8 / 21.1      E = 1.5e5 (1.5e7)  17.6 / 22.4
+//   n = 4,000, E = 2.4e5 (2.9e7)    26.6 / 30.1      E = 4e5 (8e7)      35.8 / 33.6
+//   n = 3,000, E = 2.5e5 (4.2e7)    20.3 / 22.6      E = 4e5 (1.1e8)    25.7 / 25.8
+//   n = 6,000, E = 3e5 (3e7)        41.5 / 45.1
+//   n = 8,192, E = 1.2e5 (3.5e6)    43.0 / 57.5      E = 5e5 (6.1e7)    71.0 / 65.5
+constexpr double kGreedyClusterWork = 4.8e7;
+
+__host__ __device__ inline int greedy_cluster_slice(int n) { return (n + kGreedyCluster - 1) / kGreedyCluster; }
+__host__ __device__ inline size_t greedy_cluster_smem(int n) {
+    const size_t sl = greedy_cluster_slice(n);
+    return sl * (sizeof(double4) + sizeof(int)) + (5 * (size_t)n + 2) * sizeof(int) + sl;
+}
+
+__device__ __forceinline__ uint32_t cluster_peer(uint32_t addr, int rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kGreedyThreads, 1) k_greedy_cluster(GreedyArgs a) {
+    extern __shared__ double4 gsm4[];
+    const int n = a.n, slice = a.slice;
+    double4* r2_s = gsm4;                                 // slice: ratios of this CTA's candidates
+    int* sums = reinterpret_cast<int*>(r2_s + slice);     // [2][n]: this CTA's align sums, by step parity
+    int* pos_s = sums + 2 * n;                            // slice
+    int* offi = pos_s + slice;                            // n + 1: G2 in-list offsets
+    int* offo = offi + n + 1;                             // n + 1: G2 out-list offsets
+    int* map_s = offo + n + 1;                            // n: G1 -> G2, -1 unmatched
+    unsigned char* taken = reinterpret_cast<unsigned char*>(map_s + n);
+    constexpr int NW = kGreedyThreads / 32;
+    __shared__ GreedyBest wbest[NW];
+    __shared__ __align__(16) GreedyBest s_best[2][kGreedyCluster];   // the CTAs' bests, by step parity
+    __shared__ int s_pre[kGreedyThreads + 1], s_beg[kGreedyThreads], s_w[kGreedyThreads], s_wsum[NW];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, ct = blockIdx.x;
+    const int base = ct * slice, len = max(0, min(slice, n - base));
+    for (int i = tid; i <= n; i += kGreedyThreads) {
+        offi[i] = a.off2i[i];
+        offo[i] = a.off2o[i];
+        if (i < n) map_s[i] = -1;
+    }
+    for (int l = tid; l < slice; l += kGreedyThreads) {
+        taken[l] = l < len ? 0 : 1;
+        pos_s[l] = l < len ? a.pos2[base + l] : 0x7fffffff;
+        r2_s[l] = l < len ? a.ratio2[base + l] : make_double4(0.0, 0.0, 0.0, 0.0);
+    }
+    for (int i = tid; i < 2 * n; i += kGreedyThreads) sums[i] = 0;
+    // heads of steps to come: vertex and extents of step + 1 (h1) and step + 2
+    // (h2), vertex of step + 3 (v3), this thread's first edge and ratios of step + 1
+    struct Head { int v, o0, dout, i0, din; };
+    auto extents = [&](int v) {
+        Head h{v, 0, 0, 0, 0};
+        if (v >= 0) {
+            h.o0 = a.off1o[v]; h.dout = a.off1o[v + 1] - h.o0;
+            h.i0 = a.off1i[v]; h.din = a.off1i[v + 1] - h.i0;
+        }
+        return h;
+    };
+    auto vertex = [&](int step) { return step < n ? a.order1[step] : -1; };
+    int nt = 0, nwt = 0;
+    double4 nr1;
+    auto edge = [&](const Head& h) {
+        if (h.v < 0) return;
+        nr1 = a.ratio1[h.v];
+        if (tid < h.dout + h.din) {
+            nt = tid < h.dout ? a.id1o[h.o0 + tid] : a.id1i[h.i0 + tid - h.dout];
+            nwt = tid < h.dout ? a.w1o[h.o0 + tid] : a.w1i[h.i0 + tid - h.dout];
+        }
+    };
+    Head h1 = extents(vertex(0)), h2 = extents(vertex(1));
+    int v3 = vertex(2);
+    edge(h1);
+    __syncthreads();
+    cluster_sync();   // every CTA's sums and words are cleared
+    int prev = -1, prev_g = -1;
+    for (int step = 0; step < n; step++) {
+        const int o0 = h1.o0, dout = h1.dout, i0 = h1.i0, din = h1.din, v1 = h1.v;
+        const int par = step & 1;
+        const double4 r1 = nr1;
+        int* acc = sums + par * n;
+        // ---- align terms: v1's edges in chunks of one per thread, the chunk's
+        // list entries spread evenly over all threads of the cluster ----
+        for (int c0 = 0; c0 < dout + din; c0 += kGreedyThreads) {
+            const int j = c0 + tid;
+            int beg = 0, cnt = 0, wv = 0;
+            if (j < dout + din) {
+                const bool out = j < dout;
+                const int t = c0 == 0 ? nt : out ? a.id1o[o0 + j] : a.id1i[i0 + j - dout];
+                const int w = c0 == 0 ? nwt : out ? a.w1o[o0 + j] : a.w1i[i0 + j - dout];
+                const int f = t == prev ? prev_g : map_s[t];
+                if (f >= 0 && w > 0) {
+                    const int* off = out ? offi : offo;
+                    beg = off[f];
+                    cnt = off[f + 1] - beg;
+                    wv = out ? w : (w | (int)0x80000000);
+                }
+            }
+            int incl = cnt;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            if (lane == 31) s_wsum[wid] = incl;
+            __syncthreads();
+            int w16 = lane < NW ? s_wsum[lane] : 0;
+            for (int o = 1; o < NW; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, w16, o);
+                if (lane >= o) w16 += y;
+            }
+            const int total = __shfl_sync(0xffffffffu, w16, NW - 1);
+            const int before = __shfl_sync(0xffffffffu, w16, (wid + 31) & 31);
+            s_pre[tid] = incl - cnt + (wid ? before : 0);
+            s_beg[tid] = beg;
+            s_w[tid] = wv;
+            if (tid == 0) s_pre[kGreedyThreads] = total;
+            __syncthreads();
+            const int top = 1 << (31 - __clz(max(min(dout + din - c0, kGreedyThreads) - 1, 1)));
+            constexpr int kAll = kGreedyCluster * kGreedyThreads;
+            for (int q0 = ct * kGreedyThreads + tid; q0 < total; q0 += kGreedyUnroll * kAll) {
+                int g2[kGreedyUnroll], c[kGreedyUnroll], k[kGreedyUnroll], wl[kGreedyUnroll];
+                // last edge with s_pre <= q, the searches side by side
+                int lo[kGreedyUnroll];
+#pragma unroll
+                for (int u = 0; u < kGreedyUnroll; u++) lo[u] = 0;
+                for (int half = top; half; half >>= 1)
+#pragma unroll
+                    for (int u = 0; u < kGreedyUnroll; u++)
+                        if (s_pre[lo[u] + half] <= q0 + u * kAll) lo[u] += half;
+#pragma unroll
+                for (int u = 0; u < kGreedyUnroll; u++) {
+                    const int q = q0 + u * kAll;
+                    k[u] = q < total ? s_beg[lo[u]] + q - s_pre[lo[u]] : -1;
+                    wl[u] = s_w[lo[u]];
+                }
+#pragma unroll
+                for (int u = 0; u < kGreedyUnroll; u++) {
+                    g2[u] = c[u] = 0;
+                    if (k[u] < 0) continue;
+                    const bool out = wl[u] >= 0;
+                    g2[u] = out ? a.id2i[k[u]] : a.id2o[k[u]];
+                    c[u] = min(wl[u] & 0x7fffffff, out ? a.w2i[k[u]] : a.w2o[k[u]]);
+                }
+#pragma unroll
+                for (int u = 0; u < kGreedyUnroll; u++)
+                    if (c[u] > 0) atomicAdd(&acc[g2[u]], c[u]);
+            }
+            __syncthreads();
+        }
+        cluster_sync();       // the step's sums are complete
+        h1 = h2;
+        edge(h1);
+        h2 = extents(v3);
+        v3 = vertex(step + 3);
+        // ---- this CTA's best candidate; the other parity's sums, which every CTA
+        // read before this step's barrier, are cleared for the next step ----
+        for (int i = tid; i < n; i += kGreedyThreads) sums[(par ^ 1) * n + i] = 0;
+        GreedyBest best{-1.0 / 0.0, 0x7fffffff, -1};
+        for (int l = tid; l < len; l += kGreedyThreads) {
+            if (taken[l]) continue;
+            const uint32_t mine = (uint32_t)__cvta_generic_to_shared(acc + base + l);
+            int part[kGreedyCluster], al = 0;
+#pragma unroll
+            for (int r = 0; r < kGreedyCluster; r++)
+                asm volatile("ld.relaxed.cluster.shared::cluster.u32 %0, [%1];" : "=r"(part[r]) : "r"(cluster_peer(mine, r)) : "memory");
+#pragma unroll
+            for (int r = 0; r < kGreedyCluster; r++) al += part[r];
+            const GreedyBest c{greedy_score(r1, r2_s[l], al), pos_s[l], base + l};
+            if (better(c, best)) best = c;
+        }
+        auto reduce = [&](GreedyBest& b, int width) {
+            for (int o = width / 2; o; o >>= 1) {
+                GreedyBest y;
+                y.score = __shfl_xor_sync(0xffffffffu, b.score, o);
+                y.pos = __shfl_xor_sync(0xffffffffu, b.pos, o);
+                y.g = __shfl_xor_sync(0xffffffffu, b.g, o);
+                if (better(y, b)) b = y;
+            }
+        };
+        reduce(best, 32);
+        if (lane == 0) wbest[wid] = best;
+        __syncthreads();
+        // ---- every CTA's best into every CTA ----
+        if (wid == 0) {
+            best = wbest[lane & (NW - 1)];
+            reduce(best, NW);
+            if (lane < kGreedyCluster) {
+                const uint32_t dst = cluster_peer((uint32_t)__cvta_generic_to_shared(&s_best[par][ct]), lane);
+                asm volatile("st.relaxed.cluster.shared::cluster.v2.u64 [%0], {%1, %2};" :: "r"(dst),
+                             "l"(__double_as_longlong(best.score)),
+                             "l"((long long)best.g << 32 | (unsigned)best.pos) : "memory");
+            }
+        }
+        cluster_sync();
+        best = s_best[par][lane & (kGreedyCluster - 1)];
+        reduce(best, kGreedyCluster);
+        best.g = __shfl_sync(0xffffffffu, best.g, 0);
+        prev = v1;
+        prev_g = best.g;
+        if (tid == 0) {
+            map_s[v1] = prev_g;
+            if (prev_g >= base && prev_g < base + len) taken[prev_g - base] = 1;
+            if (ct == 0) a.map[v1] = prev_g;
+        }
+    }
+    cluster_sync();   // no CTA leaves while another may still write into its shared memory
+}
+
 struct GreedyDev {
     std::vector<void*> bufs;
     ~GreedyDev() { for (void* p : bufs) cudaFree(p); }
@@ -683,8 +916,33 @@ extern "C" bm_status bm_greedy_match(int32_t n, int64_t e1, const int32_t* src1,
     A.order1 = order1; A.pos2 = pos2; A.ratio1 = ratio1; A.ratio2 = ratio2;
     A.acc = acc; A.bests = bests; A.bar = bar; A.map = mapd;
     A.stall = take_stall(BM_STALL_GREEDY);
-    void* kargs[] = {&A};
-    GK(cudaLaunchCooperativeKernel((const void*)k_greedy, dim3(grid), dim3(kGreedyThreads), kargs, smem, st));
+    // few list entries per step: one cluster, where a step's exchange is short
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(kGreedyCluster);
+    cfg.blockDim = dim3(kGreedyThreads);
+    cfg.dynamicSmemBytes = greedy_cluster_smem(n);
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kGreedyCluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    const bool cluster =
+        2.0 * (double)e1 * (double)mk / n <= kGreedyClusterWork &&
+        cfg.dynamicSmemBytes + 12288 <= (size_t)optin &&
+        cudaFuncSetAttribute(k_greedy_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) == cudaSuccess &&
+        cudaFuncSetAttribute(k_greedy_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, k_greedy_cluster, &cfg) == cudaSuccess && clusters > 0;
+    cudaGetLastError();   // a refused attribute is not an error of the launch
+    if (cluster && !A.stall) {   // no wait of the cluster kernel can be made to run out
+        A.slice = greedy_cluster_slice(n);
+        GK(cudaLaunchKernelEx(&cfg, k_greedy_cluster, A));
+    } else {
+        void* kargs[] = {&A};
+        GK(cudaLaunchCooperativeKernel((const void*)k_greedy, dim3(grid), dim3(kGreedyThreads), kargs, smem, st));
+    }
     GK(cudaEventRecord(ev[2], st));
     unsigned herr[4] = {0, 0, 0, 0};
     GK(cudaMemcpyAsync(herr, bar, sizeof herr, cudaMemcpyDeviceToHost, st));
