@@ -11,12 +11,14 @@
 //     (instance, tile) item -> reduce -> candidates -> one segmented sort ->
 //     one commit launch (a CTA per instance);
 //   * one persistent launch (k_b_sweep): the same phases in one cooperative
-//     grid behind grid barriers, the candidate sort in shared memory.
+//     grid, the candidate sort in shared memory, and sparse instances' row
+//     bests without their profit matrix (direct_row).
 // One sweep of the whole batch is captured once as a CUDA graph and replayed.
 // The schedule and its launch shapes (profit-row block size, combine tile)
 // are picked by bm_batch_autotune, which times the candidates on the batch
 // itself; results do not depend on the choice.  Hub tensor-core terms are
 // not used here: the instances are built with BM_FLAG_NO_HUB_GEMM.
+#include <climits>
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -42,6 +44,7 @@ struct BatchInst {
     unsigned long long* part;
     unsigned long long* keys;
     unsigned long long* keys_sorted;
+    int* diag;            // direct instances: S[x][x]
 };
 
 __device__ __forceinline__ int find_inst(const int* __restrict__ base, int nb, long long it) {
@@ -198,6 +201,184 @@ k_b_commit(const DevView<W16>* __restrict__ views, const BatchInst* __restrict__
 }
 
 // ---------------------------------------------------------------------------
+// Direct rows (persistent schedule): a sparse instance's row bests without the
+// profit matrix.  delta(a,b) + S[a][a] = S[a][b] + S[b][a] - S[b][b], and both
+// S[a][.] and S[.][a] are sums over short lists: S[a][.] as in profit_row_on,
+// and S[b][a] over G2's lists of p(a) -- a G2 edge p(a) -> g of weight x meets
+// every G1 in-edge (b, w) of pinv(g) with min(w, x), and likewise with both
+// directions turned.  So a group of threads adds all four kinds into one
+// shared-memory row that starts at -S[b][b], takes its maximum, and neither
+// writes n^2 profits nor reads them back in tiles.  Every min term is computed
+// twice (for a and for b), which is why only sparse instances take this path
+// (direct_instance).  64 instances of 500 to 8,000 vertices, 20 edges each, three
+// sweeps: 23.9 -> 11.9 ms, with the set commit's wider steps.
+constexpr double kDirectTerms = 1.5;   // most terms per pair of vertices (direct_instance)
+constexpr int kDirectRows = 4;    // rows of a task per accumulator
+constexpr int kDirectLong = 64;   // longer lists take a whole warp instead of 8 lanes,
+constexpr int kDirectAll = 1024;  // and longer ones than this all of the row's threads
+
+// S[a][a], by L lanes of a warp that call it together (mask); all get the sum.
+template <bool W16, int L>
+__device__ __forceinline__ int direct_diag(const DevView<W16>& g, int a, unsigned mask) {
+    const int sub = threadIdx.x & (L - 1);
+    typedef Ent<W16> EN;
+    typedef typename EN::T E;
+    const int pa = g.p[a];
+    const int so = g.off1o[a], lo = g.off1o[a + 1] - so;
+    const int si = g.off1i[a], tot = lo + g.off1i[a + 1] - si;
+    int d = 0;
+    for (int j0 = sub; j0 < tot; j0 += 4 * L) {
+        int w[4], f[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int j = j0 + L * u;
+            w[u] = 0; f[u] = g.n;
+            if (j < tot) {
+                const E e = j < lo ? g.ent1o[so + j] : g.ent1i[si + (j - lo)];
+                w[u] = EN::w(e);
+                f[u] = g.p[EN::id(e)];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)   // both from row p(a): of W2 for out-edges, of its transpose for in-edges
+            d += imin(w[u], j0 + L * u < lo ? g.w2(pa, f[u]) : g.w2t(f[u], pa));
+    }
+    for (int q = g.offs[a] + sub; q < g.offs[a + 1]; q += L) d += imin(g.selfw[q], g.w2d(pa));
+    for (int o = L / 2; o; o >>= 1) d += __shfl_xor_sync(mask, d, o);
+    return d;
+}
+
+// A list to add: its entries, their number, and the weight they are capped by.
+struct __align__(16) DirectHead {
+    const void* list;
+    int len, w;
+};
+constexpr int kDirectHeads = 128;   // per 128 threads, one each
+static_assert(sizeof(DirectHead) * kDirectHeads >= sizeof(int2) * kLongQueue, "profit_row_on's queue fits the heads");
+
+// Best partner of vertex a (packed key, 0 if it has none) by NT threads of the
+// block's NT-aligned group; `sync` is a barrier over exactly those threads.
+// acc: row_smem(n) bytes of shared memory; head, longs: NT of each; nlong: 2;
+// red: NT / 32 keys.  Thread 0 of the group gets the key; the group may start
+// another row at once.
+//
+// What bounds it: latency and issue, not bytes -- a row of a 20-edge-per-vertex
+// instance is about 80 lists of 20 entries.  So every thread first sets up one
+// list (entry, extent and corner: three dependent loads, taken while the
+// accumulator is started), and the lists are then added from shared memory by 8
+// lanes each, two lists of up to 32 entries in flight.
+template <bool W16, int NT, typename Sync>
+__device__ __forceinline__ unsigned long long direct_row(const DevView<W16>& g, const int* __restrict__ diag, int a,
+                                                         int* acc, DirectHead* head, uint16_t* longs, int* nlong,
+                                                         unsigned long long* red, Sync sync) {
+    typedef Ent<W16> EN;
+    typedef typename EN::T E;
+    constexpr int nw = NT / 32, ng = NT / 8;
+    const int n = g.n;
+    const int tid = (int)(threadIdx.x & (NT - 1)), lane = tid & 31, wid = tid >> 5, sub = lane & 7;
+    const int pa = g.p[a];
+    // list heads: 0 G1 out-edges of a, 1 its in-edges, 2 G2 out-edges of p(a), 3 its in-edges
+    const int h0 = g.off1o[a], h1 = g.off1i[a], h2 = g.off2o[pa], h3 = g.off2i[pa];
+    const int c0 = g.off1o[a + 1] - h0, c1 = c0 + g.off1i[a + 1] - h1;
+    const int c2 = c1 + g.off2o[pa + 1] - h2, tot = c2 + g.off2i[pa + 1] - h3;
+    if (tid == 0) nlong[0] = nlong[1] = 0;
+    int base = 0, par = 0;
+    do {
+        const int j = base + tid;
+        DirectHead h = {nullptr, 0, 0};
+        int cb = 0, cv = 0;   // corner of a G1 edge between a and b: in S[a][b] for a -> b, in S[b][a] for b -> a
+        if (j < tot) {
+            const int kind = j < c0 ? 0 : j < c1 ? 1 : j < c2 ? 2 : 3;
+            const int at = kind == 0 ? h0 + j : kind == 1 ? h1 + (j - c0) : kind == 2 ? h2 + (j - c1) : h3 + (j - c2);
+            const E e = (kind == 0 ? g.ent1oP : kind == 1 ? g.ent1iP : kind == 2 ? g.ent2oP : g.ent2iP)[at];
+            const int f = EN::id(e);
+            h.w = EN::w(e);
+            const int* off = kind == 0 ? g.off2i : kind == 1 ? g.off2o : kind == 2 ? g.off1i : g.off1o;
+            const int b0 = off[f];
+            h.len = off[f + 1] - b0;
+            h.list = (kind == 0 ? g.ent2iP : kind == 1 ? g.ent2oP : kind == 2 ? g.ent1i : g.ent1o) + b0;
+            if (kind < 2) {
+                cb = EN::id((kind == 0 ? g.ent1o : g.ent1i)[at]);
+                cv = imin(h.w, g.w2(pa, f)) + imin(h.w, g.w2t(f, pa)) - imin(h.w, g.w2d(pa)) - imin(h.w, g.w2d(f));
+            }
+        }
+        if (base == 0)
+            for (int i = tid; i < (n + 4) >> 2; i += NT) {   // diag is padded to whole 16-byte words
+                const int4 v = __ldcg(reinterpret_cast<const int4*>(diag) + i);
+                reinterpret_cast<int4*>(acc)[i] = make_int4(-v.x, -v.y, -v.z, -v.w);
+            }
+        sync();   // the accumulator is started, the heads before these are done
+        head[tid] = h;
+        if (cv) atomicAdd(&acc[cb], cv);
+        if (h.len > kDirectLong) longs[atomicAdd(&nlong[par], 1)] = (uint16_t)tid;
+        if (tid == 0) nlong[par ^ 1] = 0;
+        sync();
+        const int cnt = min(NT, tot - base);
+        for (int t = tid >> 3; t < cnt; t += 2 * ng) {
+            DirectHead q[2];
+            E x[2][4];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                q[k].len = 0;
+                if (t + k * ng < cnt) q[k] = head[t + k * ng];
+                if (q[k].len > kDirectLong) q[k].len = 0;
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (sub + 8 * u < q[k].len) x[k][u] = static_cast<const E*>(q[k].list)[sub + 8 * u];
+            }
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (sub + 8 * u < q[k].len) atomicAdd(&acc[EN::id(x[k][u])], imin(q[k].w, EN::w(x[k][u])));
+                for (int i = sub + 32; i < q[k].len; i += 8) {
+                    const E e = static_cast<const E*>(q[k].list)[i];
+                    atomicAdd(&acc[EN::id(e)], imin(q[k].w, EN::w(e)));
+                }
+            }
+        }
+        __syncwarp();
+        const int nl = nlong[par];
+        for (int q = 0; q < nl; q++) {   // a warp each, the longest by all
+            const DirectHead x = head[longs[q]];
+            if (x.len > kDirectAll) scatter_list<W16>(acc, static_cast<const E*>(x.list), 0, x.len, x.w, tid, NT);
+            else if (q % nw == wid) scatter_list<W16>(acc, static_cast<const E*>(x.list), 0, x.len, x.w, lane, 32);
+        }
+        base += NT;
+        par ^= 1;
+    } while (base < tot);
+    if (g.offs[n] > 0) {   // self-loops: of a in S[a][b], of b in S[b][a]
+        const int dpa = g.w2d(pa);
+        for (int b = tid; b < n; b += NT) {
+            int t = 0;
+            const int d = g.w2d(g.p[b]);
+            for (int q = g.offs[a]; q < g.offs[a + 1]; q++) t += imin(g.selfw[q], d);
+            for (int q = g.offs[b]; q < g.offs[b + 1]; q++) t += imin(g.selfw[q], dpa);
+            if (t) atomicAdd(&acc[b], t);
+        }
+    }
+    sync();
+    // the best partner: largest delta, then smallest id
+    int bd = INT_MIN, bi = -1;
+    for (int i = tid; i < (n + 3) >> 2; i += NT) {
+        const int4 v = reinterpret_cast<const int4*>(acc)[i];
+        const int x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int b = 4 * i + e;
+            if (b < n && b != a && (bi < 0 || x[e] > bd)) { bd = x[e]; bi = b; }
+        }
+    }
+    unsigned long long k = bi < 0 ? 0ull : pack_best(bd - __ldcg(&diag[a]), bi);
+    for (int o = 16; o; o >>= 1) k = kmax(k, __shfl_xor_sync(0xffffffffu, k, o));
+    if (lane == 0) red[wid] = k;
+    sync();
+    if (tid == 0)
+        for (int q = 1; q < nw; q++) k = kmax(k, red[q]);
+    return k;
+}
+
+// ---------------------------------------------------------------------------
 // One batch sweep as one persistent launch: a cooperative grid of one
 // 1024-thread CTA per SM.  The relabel of every list of every instance comes
 // first, behind one bounded grid barrier; then a dataflow over the instances
@@ -220,9 +401,13 @@ struct BSweepArgs {
     const typename Ent<W16>::T* const* lists;
     int nb;
     const int* iorder;     // instances, largest first: the order of their tasks
-    const int* rpt;        // rows per row task: 2 when two of the instance's rows fit a group's shared memory
+    const int* rpt;        // rows per row task
+    const int* ways;       // accumulators the task uses: 2 when two of the instance's rows fit a group's
+                           // shared memory; negative for direct rows
     const long long* tbase;   // 2 (count + 1): first row task, then first tile-pair task (from the
                               // first tile-pair task) of each instance in that order
+    const int* row_base;   // first vertex of each instance, laid end to end; rows_total vertices
+    int rows_total;
     int total_tasks;       // every instance's rows and tile pairs
     size_t group_bytes;    // shared memory of one 256-thread group (a row accumulator or a tile stage)
     int* counter;          // tasks taken
@@ -292,17 +477,56 @@ __global__ void __launch_bounds__(kBThreads, 1) k_b_sweep(BSweepArgs<W16> a) {
         const long long tot = a.ebase[4 * a.nb];
         const long long per = (tot + gridDim.x - 1) / gridDim.x;
         const long long lo = (long long)blockIdx.x * per, hi = min(tot, lo + per);
-        for (int sg = 0; sg < 4 * a.nb && lo < hi; sg++) {
+        for (int sg = lo < hi ? find_inst_ll(a.ebase, 4 * a.nb, lo) : 4 * a.nb; sg < 4 * a.nb; sg++) {
             const long long s0 = max(lo, a.ebase[sg]), s1 = min(hi, a.ebase[sg + 1]);
+            if (s0 >= hi) break;
             if (s0 >= s1) continue;
             const int b = sg >> 2, lst = sg & 3;
             const DevView<W16>& g = a.views[b];
             const typename EN::T* in = a.lists[sg];
             typename EN::T* out = lst == 0 ? g.ent1oP : lst == 1 ? g.ent1iP : lst == 2 ? g.ent2oP : g.ent2iP;
             const int* map = lst < 2 ? g.p : g.pinv;
-            for (long long i = s0 - a.ebase[sg] + tid; i < s1 - a.ebase[sg]; i += blockDim.x) {
-                const typename EN::T e = in[i];
-                out[i] = EN::make(map[EN::id(e)], EN::w(e));
+            const long long end = s1 - a.ebase[sg];
+            for (long long i = s0 - a.ebase[sg] + tid; i < end; i += 4 * kBThreads) {   // four entries in flight
+                typename EN::T e[4];
+                int f[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (i + u * kBThreads < end) e[u] = in[i + u * kBThreads];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (i + u * kBThreads < end) f[u] = map[EN::id(e[u])];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (i + u * kBThreads < end) out[i + u * kBThreads] = EN::make(f[u], EN::w(e[u]));
+            }
+        }
+    }
+    // S[x][x] of the direct instances, 8 lanes per vertex; a warp takes its
+    // vertices of many edges with all lanes (8 lanes took 0.2 ms for the largest hub)
+    {
+        const int gw = (blockIdx.x * kBThreads + tid) >> 5, nw = gridDim.x * (kBThreads / 32), q = (tid & 31) >> 3;
+        for (int it0 = 4 * gw; it0 < a.rows_total; it0 += 4 * nw) {
+            const int it = it0 + q;
+            int b = -1, v = 0, deg = 0;
+            if (it < a.rows_total) {
+                b = find_inst(a.row_base, a.nb, it);
+                v = it - a.row_base[b];
+                if (a.ways[b] >= 0) b = -1;
+            }
+            if (b >= 0) {
+                const DevView<W16>& g = a.views[b];
+                deg = g.off1o[v + 1] - g.off1o[v] + g.off1i[v + 1] - g.off1i[v];
+                if (deg <= 256) {
+                    const int d = direct_diag<W16, 8>(g, v, 0xffu << (8 * q));
+                    if ((tid & 7) == 0) a.inst[b].diag[v] = d;
+                }
+            }
+            for (unsigned m = __ballot_sync(0xffffffffu, deg > 256 && (tid & 7) == 0); m; m &= m - 1) {
+                const int src = __ffs(m) - 1;
+                const int bb = __shfl_sync(0xffffffffu, b, src), vv = __shfl_sync(0xffffffffu, v, src);
+                const int d = direct_diag<W16, 32>(a.views[bb], vv, 0xffffffffu);
+                if ((tid & 31) == 0) a.inst[bb].diag[vv] = d;
             }
         }
     }
@@ -330,15 +554,21 @@ __global__ void __launch_bounds__(kBThreads, 1) k_b_sweep(BSweepArgs<W16> a) {
     int* acc = reinterpret_cast<int*>(gsm);
     CombineSmem<T>& cs = *reinterpret_cast<CombineSmem<T>*>(gsm);
     __shared__ int s_task[4], s_go[4];
-    __shared__ int s_nlong[8];
-    __shared__ int2 s_long[8][kLongQueue];   // per group, or per half-group for paired rows
+    __shared__ int s_nlong[16];
+    __shared__ DirectHead s_head[8][kDirectHeads];   // per half-group (a group uses two)
+    __shared__ uint16_t s_longs[8][kDirectHeads];
+    int2* s_long = reinterpret_cast<int2*>(s_head[2 * grp + (gtid >> 7)]);   // profit rows: their long lists
+    __shared__ unsigned long long s_red[kBThreads / 32];
     __shared__ int s_stop;
     for (int own = blockIdx.x;; own += gridDim.x) {
-        const int target = own < a.nb ? a.inst[own].tiles * (a.inst[own].tiles + 1) / 2 : 0;
+        // what the commit of `own` waits for: its tile pairs, or its direct rows
+        const bool odir = own < a.nb && a.ways[own] < 0;
+        const int target = own >= a.nb ? 0 : odir ? a.inst[own].n : a.inst[own].tiles * (a.inst[own].tiles + 1) / 2;
+        const unsigned* fin = (const unsigned*)(odir ? rows_done : tiles_done) + own;
         for (;;) {
             if (gtid == 0) {
                 int go = !b_ld_acquire(&a.bar[2]);
-                if (go && own < a.nb && (int)b_ld_acquire((const unsigned*)&tiles_done[own]) >= target) go = 0;
+                if (go && own < a.nb && (int)b_ld_acquire(fin) >= target) go = 0;
                 int t = -1;
                 if (go && (t = atomicAdd(a.counter, 1)) >= a.total_tasks) go = 0;
                 s_task[grp] = t;
@@ -354,10 +584,34 @@ __global__ void __launch_bounds__(kBThreads, 1) k_b_sweep(BSweepArgs<W16> a) {
             const BatchInst I = a.inst[i];
             const int local = (row ? t : t - (int)a.tbase[a.nb]) - (int)base[k] + (row ? 0 : I.n);
             if (row) {
-                const DevView<W16> g = a.views[i];
-                if (a.rpt[i] == 1) {   // profit row `local` of instance i by the whole group
-                    // (the long-list queue of the group's first half: halves of other groups use theirs)
-                    profit_row_on<W16, 256>(g, local, acc, s_long[2 * grp], &s_nlong[2 * grp], nullptr, 0,
+                const DevView<W16>& g = a.views[i];
+                const int ways = a.ways[i], rpt = a.rpt[i];
+                if (ways < 0) {        // direct rows, by the whole group or by each 128-thread half
+                    const int per = rpt / -ways, end = min(I.n, (local + 1) * rpt);
+                    if (ways == -1) {
+                        for (int r = local * rpt; r < end; r++) {
+                            const unsigned long long k = direct_row<W16, 256>(
+                                a.views[i], I.diag, r, acc, s_head[2 * grp], s_longs[2 * grp], &s_nlong[4 * grp],
+                                s_red + 8 * grp,
+                                [grp] { b_group_sync(grp); });
+                            if (gtid == 0) I.rowbest[r] = k;
+                        }
+                    } else {
+                        const int half = gtid >> 7, hb = 2 * grp + half;
+                        const int r0 = local * rpt + half * per, r1 = min(end, r0 + per);
+                        int* hacc = acc + half * (row_smem(I.n) / sizeof(int));
+                        for (int r = r0; r < r1; r++) {
+                            const unsigned long long k = direct_row<W16, 128>(
+                                a.views[i], I.diag, r, hacc, s_head[hb], s_longs[hb], &s_nlong[2 * hb], s_red + 4 * hb,
+                                [hb] { asm volatile("bar.sync %0, 128;" :: "r"(5 + hb) : "memory"); });
+                            if ((gtid & 127) == 0) I.rowbest[r] = k;
+                        }
+                    }
+                    __threadfence();
+                    b_group_sync(grp);
+                    if (gtid == 0) atomicAdd(&rows_done[i], end - local * rpt);
+                } else if (ways == 1) {   // profit row `local` of instance i by the whole group
+                            profit_row_on<W16, 256>(g, local, acc, reinterpret_cast<int2*>(s_head[2 * grp]), &s_nlong[4 * grp], nullptr, 0,
                                             nullptr, nullptr, [grp] { b_group_sync(grp); });
                     __threadfence();     // every thread's part of the row is visible before it counts
                     b_group_sync(grp);
@@ -366,7 +620,7 @@ __global__ void __launch_bounds__(kBThreads, 1) k_b_sweep(BSweepArgs<W16> a) {
                     const int half = gtid >> 7, r = 2 * local + half;
                     const int hb = 2 * grp + half;   // the half's barrier: 5 + hb, 128 threads
                     if (r < I.n)
-                        profit_row_on<W16, 128>(g, r, acc + half * (row_smem(I.n) / sizeof(int)), s_long[hb], &s_nlong[hb],
+                        profit_row_on<W16, 128>(g, r, acc + half * (row_smem(I.n) / sizeof(int)), s_long, &s_nlong[2 * hb],
                                                 nullptr, 0, nullptr, nullptr, [hb] {
                                                     asm volatile("bar.sync %0, 128;" :: "r"(5 + hb) : "memory");
                                                 });
@@ -399,7 +653,7 @@ __global__ void __launch_bounds__(kBThreads, 1) k_b_sweep(BSweepArgs<W16> a) {
         // ---- instance `own`: wait for its tile pairs, then its bests, candidates, sort and commit
         if (tid == 0) {
             unsigned it = 0;
-            while ((int)b_ld_acquire((const unsigned*)&tiles_done[own]) < target) {
+            while ((int)b_ld_acquire(fin) < target) {
                 if (b_ld_acquire(&a.bar[2]) || ++it > kBSpinLimit) { atomicExch(&a.bar[2], 1u); break; }
                 __nanosleep(64);
             }
@@ -409,7 +663,7 @@ __global__ void __launch_bounds__(kBThreads, 1) k_b_sweep(BSweepArgs<W16> a) {
         __syncthreads();
         if (s_stop) break;
         const BatchInst I = a.inst[own];
-        for (int x = tid; x < I.n; x += blockDim.x) {
+        for (int x = tid; x < I.n && !odir; x += blockDim.x) {
             unsigned long long k = 0;
             for (int tt = 0; tt < I.tiles; tt++) k = kmax(k, __ldcg(&I.part[(size_t)tt * I.n + x]));
             I.rowbest[x] = k;
@@ -417,13 +671,13 @@ __global__ void __launch_bounds__(kBThreads, 1) k_b_sweep(BSweepArgs<W16> a) {
         __syncthreads();
         // candidate keys (the single-instance rule, k_candidates)
         for (int xa = tid; xa < I.n; xa += blockDim.x) {
-            const unsigned long long k = I.rowbest[xa];
+            const unsigned long long k = __ldcg(&I.rowbest[xa]);   // direct rows: written by other CTAs
             unsigned long long out = ~0ull;
             if (k) {
                 const int d = (int)((unsigned)(k >> 32) - 0x80000000u);
                 const int q = (int)(~(unsigned)(k & 0xffffffffu));
                 if (d > 0) {
-                    const unsigned long long kb = I.rowbest[q];
+                    const unsigned long long kb = __ldcg(&I.rowbest[q]);
                     const int qq = (int)(~(unsigned)(kb & 0xffffffffu));
                     const bool mutual = (kb != 0) && (qq == xa);
                     if (!mutual || xa < q) {
@@ -486,7 +740,9 @@ struct bm_batch {
     // row task and tile-pair task of each in that order, per-instance
     // finished rows and tile pairs
     int* iorder = nullptr;
-    int* rpt = nullptr;                   // rows per row task of each instance (1 or 2)
+    int* rpt = nullptr;                   // rows per row task of each instance
+    int* ways = nullptr;                  // accumulators of its row tasks, negative for direct rows
+    int* diag = nullptr;
     long long* tbase = nullptr;
     long long total_tasks = 0;
     int* done = nullptr;
@@ -505,7 +761,7 @@ struct bm_batch {
     // every instance's candidates fit its in-kernel sort) or the launch
     // sequence above; the autotuner times both and keeps the faster
     bool can_persist = false, use_persist = false;
-    size_t psmem = 0;
+    size_t group_cap = 0;                 // most shared memory a 256-thread group of it can have
     unsigned* gbar = nullptr;             // its grid barrier
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -517,8 +773,19 @@ static thread_local char g_batch_create_err[512];
 
 template <bool W16>
 static bm_status persistent_setup(bm_batch* B);
-template <int T>
-static size_t persistent_group_bytes(int max_n);
+static size_t persistent_group_bytes(const bm_batch* B);
+
+// Whether the persistent schedule finds an instance's row bests without its
+// profit matrix (direct_row).  That computes each of the about 2 e1 e2 / n min
+// terms of the matrix twice, and saves writing n^2 profits and reading them in
+// tiles: the line is a number of terms per pair, 4 e1 e2 / n^3.  Measured, ms per
+// sweep of 64 instances (24 at n = 4,000) through the matrix / direct: n = 1,600,
+// 24 edges per vertex (1.4 terms) 2.5 / 2.3, 32 edges (2.6) 2.78 / 2.79, 40 edges
+// (4.0) 3.21 / 3.45; n = 4,000, 40 edges (1.6) 4.39 / 4.45, 50 edges (2.5) 5.05 /
+// 5.95, 63 edges (4.0) 5.8 / 9.4; n = 800, 24 edges (2.9) 1.10 / 1.03.
+static bool direct_instance(const bm_ctx* c) {
+    return 4.0 * (double)c->e1 * (double)c->e2 <= kDirectTerms * (double)c->n * c->n * c->n;
+}
 
 #define BK(call)                                                                         \
     do {                                                                                 \
@@ -537,7 +804,7 @@ static void batch_free(bm_batch* B) {
     void* bufs[] = {B->views, B->inst, B->row_base, B->tile_base, B->e1, B->e2, B->lists, B->wkeys,
                     B->wkeys_sorted, B->ckeys, B->ckeys_sorted, B->wvals, B->order, B->rowbest, B->part,
                     B->cub_tmp, B->counter, B->cstats, B->acc_delta, B->acc_commits, B->gbar, B->ebase,
-                    B->iorder, B->tbase, B->done, B->rpt};
+                    B->iorder, B->tbase, B->done, B->rpt, B->ways, B->diag};
     for (void* p : bufs) if (p) cudaFree(p);
     if (B->ev0) cudaEventDestroy(B->ev0);
     if (B->ev1) cudaEventDestroy(B->ev1);
@@ -564,22 +831,29 @@ static bm_status batch_tiles(bm_batch* B) {
         std::vector<int> ord(B->count);
         for (int i = 0; i < B->count; i++) ord[i] = i;
         std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return B->hinst[x].n > B->hinst[y].n; });
-        // two rows per row task where both accumulators fit a group's shared memory
-        const size_t gb = B->tile == 32 ? persistent_group_bytes<32>(B->max_n) : persistent_group_bytes<64>(B->max_n);
-        std::vector<int> rpt(B->count);
-        for (int i = 0; i < B->count; i++)
-            rpt[i] = 2 * (size_t)((B->hinst[i].n + 1 + 3) & ~3) * sizeof(int) <= gb ? 2 : 1;
+        // two rows at a time where both accumulators fit a group's shared memory; a
+        // task of direct rows has several rows per accumulator (they are short)
+        const size_t gb = persistent_group_bytes(B);
+        std::vector<int> rpt(B->count), ways(B->count);
+        for (int i = 0; i < B->count; i++) {
+            const int w = 2 * row_smem(B->hinst[i].n) <= gb ? 2 : 1;
+            const bool dir = direct_instance(B->ctx[i]);
+            ways[i] = dir ? -w : w;
+            rpt[i] = dir ? w * kDirectRows : w;
+        }
         // [rows prefix (count + 1)][tile-pair prefix (count + 1)]
         std::vector<long long> tbase(2 * (size_t)B->count + 2, 0);
         for (int k = 0; k < B->count; k++) {
             const BatchInst& I = B->hinst[ord[k]];
             tbase[k + 1] = tbase[k] + (I.n + rpt[ord[k]] - 1) / rpt[ord[k]];
-            tbase[B->count + 1 + k + 1] = tbase[B->count + 1 + k] + (long long)I.tiles * (I.tiles + 1) / 2;
+            tbase[B->count + 1 + k + 1] = tbase[B->count + 1 + k] +
+                (ways[ord[k]] < 0 ? 0 : (long long)I.tiles * (I.tiles + 1) / 2);
         }
         B->total_tasks = tbase[B->count] + tbase[2 * (size_t)B->count + 1];
         if (B->total_tasks > 0x7fffffffLL) B->can_persist = B->use_persist = false;   // 32-bit task indices
         BK(cudaMemcpy(B->iorder, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice));
         BK(cudaMemcpy(B->rpt, rpt.data(), rpt.size() * sizeof(int), cudaMemcpyHostToDevice));
+        BK(cudaMemcpy(B->ways, ways.data(), ways.size() * sizeof(int), cudaMemcpyHostToDevice));
         BK(cudaMemcpy(B->tbase, tbase.data(), tbase.size() * sizeof(long long), cudaMemcpyHostToDevice));
     }
     BK(cudaMemcpy(B->inst, B->hinst.data(), B->hinst.size() * sizeof(BatchInst), cudaMemcpyHostToDevice));
@@ -695,7 +969,11 @@ extern "C" bm_status bm_batch_create(bm_batch** out, int32_t count, const int32_
         B->cub_bytes = std::max(b1, b2);
         BK(cudaMalloc(&B->cub_tmp, B->cub_bytes));
         B->hinst.resize(count);
-        long long poff = 0;
+        long long poff = 0, doff = 0;
+        for (int i = 0; i < count; i++) doff += row_smem(B->ctx[i]->n) / sizeof(int);
+        BK(cudaMalloc(&B->diag, (size_t)doff * sizeof(int)));
+        BK(cudaMemset(B->diag, 0, (size_t)doff * sizeof(int)));   // the padding is read
+        doff = 0;
         for (int i = 0; i < count; i++) {
             BatchInst& I = B->hinst[i];
             I.n = B->ctx[i]->n;
@@ -704,6 +982,8 @@ extern "C" bm_status bm_batch_create(bm_batch** out, int32_t count, const int32_
             I.rowbest = B->rowbest + rb[i];
             I.part = B->part + poff;
             poff += (long long)((I.n + 31) / 32) * I.n;
+            I.diag = B->diag + doff;
+            doff += row_smem(I.n) / sizeof(int);
             I.keys = B->ckeys + rb[i];
             I.keys_sorted = B->ckeys_sorted + rb[i];
         }
@@ -713,6 +993,7 @@ extern "C" bm_status bm_batch_create(bm_batch** out, int32_t count, const int32_
         BK(cudaMemset(B->gbar, 0, 4 * sizeof(unsigned)));
         BK(cudaMalloc(&B->iorder, count * sizeof(int)));
         BK(cudaMalloc(&B->rpt, count * sizeof(int)));
+        BK(cudaMalloc(&B->ways, count * sizeof(int)));
         BK(cudaMalloc(&B->tbase, 2 * (count + 1) * sizeof(long long)));
         BK(cudaMalloc(&B->done, 2 * count * sizeof(int)));
         s2 = B->w16 ? persistent_setup<true>(B) : persistent_setup<false>(B);
@@ -756,26 +1037,36 @@ extern "C" bm_status bm_batch_scores(bm_batch* B, int64_t* scores) {
     return BM_OK;
 }
 
-// Shared memory of k_b_sweep: the largest of its phases' needs.
 // Shared memory of one 256-thread group of k_b_sweep: a row accumulator or a
-// tile stage, whichever is larger.
-template <int T>
-static size_t persistent_group_bytes(int max_n) {
-    return (std::max(row_smem(max_n), sizeof(CombineSmem<T>)) + 15) & ~(size_t)15;
+// tile stage, whichever is larger, and room for two accumulators of the
+// direct instances as far as the SM has it.
+static size_t persistent_group_bytes(const bm_batch* B) {
+    size_t m = std::max(row_smem(B->max_n), B->tile == 32 ? sizeof(CombineSmem<32>) : sizeof(CombineSmem<64>));
+    m = (m + 15) & ~(size_t)15;
+    for (const bm_ctx* c : B->ctx)
+        if (direct_instance(c) && 2 * row_smem(c->n) <= B->group_cap) m = std::max(m, 2 * row_smem(c->n));
+    return m;
 }
 
-template <int T>
-static size_t persistent_smem(int max_n) {
-    size_t m = 4 * persistent_group_bytes<T>(max_n);                      // four groups
+// Shared memory of k_b_sweep: the largest of its phases' needs.
+static size_t persistent_smem(const bm_batch* B) {
+    size_t m = 4 * persistent_group_bytes(B);                              // four groups
     m = std::max(m, sizeof(typename BSort::TempStorage));                  // the candidate sort
-    m = std::max(m, commit_group_smem(max_n));                             // the set commit
+    m = std::max(m, commit_group_smem(B->max_n));                          // the set commit
     return (m + 15) & ~(size_t)15;
 }
 
 template <bool W16, int T>
-static bool persistent_fits(bm_batch* B, size_t* smem) {
-    const size_t sm = persistent_smem<T>(B->max_n);
-    if (cudaFuncSetAttribute(k_b_sweep<W16, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) {
+static bool persistent_fits(bm_batch* B) {
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, k_b_sweep<W16, T>) != cudaSuccess) { cudaGetLastError(); return false; }
+    B->tile = T;
+    const size_t room = B->ctx[0]->smem_optin - std::min(B->ctx[0]->smem_optin, fa.sharedSizeBytes);
+    B->group_cap = (room / 4) & ~(size_t)15;
+    const size_t sm = persistent_smem(B);
+    // the limit is the same for every batch: one with smaller instances must not lower another's
+    if (sm > room ||
+        cudaFuncSetAttribute(k_b_sweep<W16, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -785,7 +1076,6 @@ static bool persistent_fits(bm_batch* B, size_t* smem) {
         cudaGetLastError();
         return false;
     }
-    *smem = sm;
     return true;
 }
 
@@ -794,9 +1084,9 @@ static bool persistent_fits(bm_batch* B, size_t* smem) {
 // either combine tile.
 template <bool W16>
 static bm_status persistent_setup(bm_batch* B) {
-    size_t s32 = 0, s64 = 0;
-    B->can_persist = B->max_n <= kBSortMax && persistent_fits<W16, 32>(B, &s32) && persistent_fits<W16, 64>(B, &s64);
-    B->psmem = std::max(s32, s64);
+    const int tile = B->tile;
+    B->can_persist = B->max_n <= kBSortMax && persistent_fits<W16, 32>(B) && persistent_fits<W16, 64>(B);
+    B->tile = tile;
     return BM_OK;
 }
 
@@ -810,9 +1100,12 @@ static bm_status enqueue_persistent(bm_batch* B, int max_scan, int max_verify, i
     a.nb = B->count;
     a.iorder = B->iorder;
     a.rpt = B->rpt;
+    a.ways = B->ways;
+    a.row_base = B->row_base;
+    a.rows_total = B->total;
     a.tbase = B->tbase;
     a.total_tasks = (int)B->total_tasks;
-    a.group_bytes = B->tile == 32 ? persistent_group_bytes<32>(B->max_n) : persistent_group_bytes<64>(B->max_n);
+    a.group_bytes = persistent_group_bytes(B);
     a.counter = B->counter;
     a.done = B->done;
     a.bar = B->gbar;
@@ -825,7 +1118,7 @@ static bm_status enqueue_persistent(bm_batch* B, int max_scan, int max_verify, i
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(B->ctx[0]->num_sms);
     cfg.blockDim = dim3(kBThreads);
-    cfg.dynamicSmemBytes = B->tile == 32 ? persistent_smem<32>(B->max_n) : persistent_smem<64>(B->max_n);
+    cfg.dynamicSmemBytes = persistent_smem(B);
     cfg.stream = B->st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
