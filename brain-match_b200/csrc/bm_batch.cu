@@ -83,6 +83,34 @@ __global__ void k_b_relabel(const DevView<W16>* __restrict__ views, const long l
     }
 }
 
+// Matchings of the instances in and out of one staging buffer: p, then pinv, of
+// instance b from 2 (row_base[b] + b).  64 instances took 4 ms per set and get
+// as copies, scores and waits of their own (8 sweeps of the smallest).
+template <bool W16>
+__global__ void k_b_maps_in(const DevView<W16>* __restrict__ views, const int* __restrict__ row_base,
+                            const int* __restrict__ stage) {
+    const int b = blockIdx.y;
+    const DevView<W16>& g = views[b];
+    const int* s = stage + 2 * ((size_t)row_base[b] + b);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= g.n; i += gridDim.x * blockDim.x) {
+        g.p[i] = s[i];
+        g.pinv[i] = s[g.n + 1 + i];
+    }
+}
+template <bool W16>
+__global__ void k_b_maps_out(const DevView<W16>* __restrict__ views, const int* __restrict__ row_base,
+                             int* __restrict__ stage) {
+    const int b = blockIdx.y;
+    const DevView<W16>& g = views[b];
+    int* s = stage + 2 * ((size_t)row_base[b] + b);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= g.n; i += gridDim.x * blockDim.x) s[i] = g.p[i];
+}
+template <bool W16>
+__global__ void k_b_score(const DevView<W16>* __restrict__ views, const long long* __restrict__ e1,
+                          unsigned long long* __restrict__ out) {
+    add_score<W16>(views[blockIdx.y], (int)e1[blockIdx.y], out + blockIdx.y);
+}
+
 template <bool W16>
 __global__ void k_b_row_work(const DevView<W16>* __restrict__ views, const int* __restrict__ row_base, int nb,
                              int total, unsigned long long* __restrict__ key, int* __restrict__ val) {
@@ -743,6 +771,8 @@ struct bm_batch {
     int* rpt = nullptr;                   // rows per row task of each instance
     int* ways = nullptr;                  // accumulators of its row tasks, negative for direct rows
     int* diag = nullptr;
+    int *stage = nullptr, *hstage = nullptr;                       // matchings, device and pinned host
+    unsigned long long *scores = nullptr, *hscores = nullptr;
     long long* tbase = nullptr;
     long long total_tasks = 0;
     int* done = nullptr;
@@ -804,8 +834,10 @@ static void batch_free(bm_batch* B) {
     void* bufs[] = {B->views, B->inst, B->row_base, B->tile_base, B->e1, B->e2, B->lists, B->wkeys,
                     B->wkeys_sorted, B->ckeys, B->ckeys_sorted, B->wvals, B->order, B->rowbest, B->part,
                     B->cub_tmp, B->counter, B->cstats, B->acc_delta, B->acc_commits, B->gbar, B->ebase,
-                    B->iorder, B->tbase, B->done, B->rpt, B->ways, B->diag};
+                    B->iorder, B->tbase, B->done, B->rpt, B->ways, B->diag, B->stage, B->scores};
     for (void* p : bufs) if (p) cudaFree(p);
+    if (B->hstage) cudaFreeHost(B->hstage);
+    if (B->hscores) cudaFreeHost(B->hscores);
     if (B->ev0) cudaEventDestroy(B->ev0);
     if (B->ev1) cudaEventDestroy(B->ev1);
     if (B->st) cudaStreamDestroy(B->st);
@@ -959,6 +991,10 @@ extern "C" bm_status bm_batch_create(bm_batch** out, int32_t count, const int32_
         BK(cudaMalloc(&B->part, (size_t)part_total * sizeof(unsigned long long)));
         BK(cudaMalloc(&B->counter, sizeof(int)));
         BK(cudaMalloc(&B->cstats, count * sizeof(CommitStats)));
+        BK(cudaMalloc(&B->stage, 2 * (tot + count) * sizeof(int)));
+        BK(cudaMallocHost(&B->hstage, 2 * (tot + count) * sizeof(int)));
+        BK(cudaMalloc(&B->scores, count * sizeof(unsigned long long)));
+        BK(cudaMallocHost(&B->hscores, count * sizeof(unsigned long long)));
         BK(cudaMalloc(&B->acc_delta, count * sizeof(long long)));
         BK(cudaMalloc(&B->acc_commits, count * sizeof(long long)));
         size_t b1 = 0, b2 = 0;
@@ -1010,22 +1046,67 @@ extern "C" bm_status bm_batch_create(bm_batch** out, int32_t count, const int32_
     return BM_OK;
 }
 
+template <bool W16>
+static bm_status batch_maps_in(bm_batch* B, int k, size_t ints) {
+    const DevView<W16>* views = (const DevView<W16>*)B->views;
+    const dim3 grid((B->max_n + 1024) / 1024, k);
+    BK(cudaMemcpyAsync(B->stage, B->hstage, ints * sizeof(int), cudaMemcpyHostToDevice, B->st));
+    BK(cudaMemsetAsync(B->scores, 0, k * sizeof(unsigned long long), B->st));
+    k_b_maps_in<W16><<<grid, 256, 0, B->st>>>(views, B->row_base, B->stage);
+    BK(cudaGetLastError());
+    k_b_score<W16><<<dim3(16, k), 256, 0, B->st>>>(views, B->e1, B->scores);
+    BK(cudaGetLastError());
+    BK(cudaMemcpyAsync(B->hscores, B->scores, k * sizeof(unsigned long long), cudaMemcpyDeviceToHost, B->st));
+    BK(cudaStreamSynchronize(B->st));
+    return BM_OK;
+}
+
 extern "C" bm_status bm_batch_set_mappings(bm_batch* B, const int32_t* const* maps) {
     if (!B || !maps) return BM_E_INPUT;
-    for (int i = 0; i < B->count; i++) {
-        bm_status s = bm_set_mapping(B->ctx[i], maps[i]);
-        if (s) { snprintf(B->err, sizeof B->err, "instance %d: %.480s", i, B->ctx[i]->err); return s; }
+    bm_status bad = BM_OK;
+    size_t at = 0;
+    int k = 0;   // the instances before the first bad matching are set
+    for (; k < B->count; k++) {
+        const size_t n1 = (size_t)B->ctx[k]->n + 1;
+        if ((bad = decode_mapping(B->ctx[k], maps[k], B->hstage + at, B->hstage + at + n1))) break;
+        at += 2 * n1;
     }
-    return BM_OK;
+    if (k) {
+        bm_status s = B->w16 ? batch_maps_in<true>(B, k, at) : batch_maps_in<false>(B, k, at);
+        if (s) return s;
+        for (int i = 0; i < k; i++) {
+            B->ctx[i]->mapped = true;
+            B->ctx[i]->score = (long long)B->hscores[i];
+        }
+    }
+    if (bad) snprintf(B->err, sizeof B->err, "instance %d: %.480s", k, B->ctx[k]->err);
+    return bad;
 }
 
 extern "C" bm_status bm_batch_get_mappings(bm_batch* B, int32_t* const* maps) {
     if (!B || !maps) return BM_E_INPUT;
-    for (int i = 0; i < B->count; i++) {
-        bm_status s = bm_get_mapping(B->ctx[i], maps[i]);
-        if (s) { snprintf(B->err, sizeof B->err, "instance %d: %.480s", i, B->ctx[i]->err); return s; }
+    size_t at = 0;
+    int k = 0;
+    for (; k < B->count && B->ctx[k]->mapped && maps[k]; k++) at += 2 * ((size_t)B->ctx[k]->n + 1);
+    if (k) {
+        const dim3 grid((B->max_n + 1024) / 1024, k);
+        if (B->w16) k_b_maps_out<true><<<grid, 256, 0, B->st>>>((const DevView<true>*)B->views, B->row_base, B->stage);
+        else k_b_maps_out<false><<<grid, 256, 0, B->st>>>((const DevView<false>*)B->views, B->row_base, B->stage);
+        BK(cudaGetLastError());
+        BK(cudaMemcpyAsync(B->hstage, B->stage, at * sizeof(int), cudaMemcpyDeviceToHost, B->st));
+        BK(cudaStreamSynchronize(B->st));
     }
-    return BM_OK;
+    const int* p = B->hstage;
+    for (int i = 0; i < k; i++) {
+        const int n = B->ctx[i]->n;
+        maps[i][0] = 0;
+        for (int a = 0; a < n; a++) maps[i][a + 1] = p[a] == n ? 0 : p[a] + 1;
+        p += 2 * ((size_t)n + 1);
+    }
+    if (k == B->count) return BM_OK;
+    bm_status s = bm_get_mapping(B->ctx[k], maps[k]);   // the error of the first it cannot get
+    snprintf(B->err, sizeof B->err, "instance %d: %.480s", k, B->ctx[k]->err);
+    return s;
 }
 
 extern "C" bm_status bm_batch_scores(bm_batch* B, int64_t* scores) {
@@ -1205,18 +1286,14 @@ extern "C" bm_status bm_batch_autotune(bm_batch* B, int32_t* profit_threads, int
     for (int pt : {256, 512})
         for (int tl : {32, 64}) cand.push_back({false, pt, tl});
     std::vector<std::vector<int32_t>> saved(B->count);
+    std::vector<int32_t*> maps(B->count);
     for (int i = 0; i < B->count; i++) {
         saved[i].resize((size_t)B->ctx[i]->n + 1);
-        bm_status s = bm_get_mapping(B->ctx[i], saved[i].data());
-        if (s) return s;
+        maps[i] = saved[i].data();
     }
-    auto restore = [&]() -> bm_status {
-        for (int i = 0; i < B->count; i++) {
-            bm_status s = bm_set_mapping(B->ctx[i], saved[i].data());
-            if (s) return s;
-        }
-        return BM_OK;
-    };
+    bm_status got = bm_batch_get_mappings(B, maps.data());
+    if (got) return got;
+    auto restore = [&]() { return bm_batch_set_mappings(B, maps.data()); };
     float best = 1e30f;
     Sched pick = cand[0];
     for (const Sched& c : cand) {

@@ -437,11 +437,10 @@ static bm_status compute_score(bm_ctx* ctx, long long* out) {
     return BM_OK;
 }
 
-extern "C" bm_status bm_set_mapping(bm_ctx* ctx, const int32_t* map) {
-    if (!ctx) return BM_E_INPUT;
+bm_status decode_mapping(bm_ctx* ctx, const int32_t* map, int* p, int* pinv) {
     if (!map) { set_err(ctx, "bm_set_mapping: map is NULL"); return BM_E_INPUT; }
     const int n = ctx->n;
-    std::vector<int> p(n + 1), pinv(n + 1, n);
+    std::fill(pinv, pinv + n + 1, n);
     for (int a = 0; a < n; a++) {
         const int f = map[a + 1];
         if (f < 0 || f > n) { set_err(ctx, "bm_set_mapping: map[%d]=%d outside 0..%d", a + 1, f, n); return BM_E_INPUT; }
@@ -451,7 +450,15 @@ extern "C" bm_status bm_set_mapping(bm_ctx* ctx, const int32_t* map) {
         pinv[f - 1] = a;
     }
     p[n] = n;
-    pinv[n] = n;
+    return BM_OK;
+}
+
+extern "C" bm_status bm_set_mapping(bm_ctx* ctx, const int32_t* map) {
+    if (!ctx) return BM_E_INPUT;
+    const int n = ctx->n;
+    std::vector<int> p(n + 1), pinv(n + 1);
+    bm_status s = decode_mapping(ctx, map, p.data(), pinv.data());
+    if (s) return s;
     CK(cudaMemcpyAsync(ctx->p, p.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(ctx->pinv, pinv.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
     ctx->mapped = true;

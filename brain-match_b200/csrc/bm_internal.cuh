@@ -139,6 +139,8 @@ template <bool W16> bm_status stage_profit(bm_ctx* ctx);
 // stage_profit.  *mode: 0 rebuilt, 1 updated, 2 already exact.
 template <bool W16> bm_status stage_refresh(bm_ctx* ctx, int* mode);
 bm_status stage_combine(bm_ctx* ctx, int* all_out);
+// The engine's p and pinv (n + 1 each) of a 1-based matching; checks it.
+bm_status decode_mapping(bm_ctx* ctx, const int32_t* map, int* p, int* pinv);
 // Enqueues the set commit of the first lim sorted candidate keys (K = 2: pairs
 // in the keys; K = 3, 4: the sets in `sets`) on ctx's stream; statistics go to
 // ctx->cstats.  ctas <= 0: as many CTAs as the window's lists need; ctl_clear:

@@ -535,7 +535,7 @@ __device__ __forceinline__ int row_of(const int* __restrict__ off, int n, int i)
 // the power-law rows' longest held the launch (54 us at n = 8,192 / E = 1e6).
 constexpr int kScoreRun = 128;
 template <bool W16>
-__global__ void k_score(DevView<W16> g, int m, unsigned long long* __restrict__ out) {
+__device__ __forceinline__ void add_score(const DevView<W16>& g, int m, unsigned long long* __restrict__ out) {
     typedef Ent<W16> EN;
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -559,6 +559,8 @@ __global__ void k_score(DevView<W16> g, int m, unsigned long long* __restrict__ 
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0 && s) atomicAdd(out, (unsigned long long)s);
 }
+template <bool W16>
+__global__ void k_score(DevView<W16> g, int m, unsigned long long* __restrict__ out) { add_score<W16>(g, m, out); }
 
 // C[a] += what vertex a's G1 edges and self-loops earn now; one pass over the
 // G1 entries, dealt as in k_score (C zero before).  Most terms of an early

@@ -62,3 +62,21 @@ def test_instances_end_where_they_end_alone(name, flags):
             want = sum(E.sweep()["committed"] for _ in range(3))
             assert c == want, g["n"]
             np.testing.assert_array_equal(m, E.get_mapping())
+
+
+def test_a_bad_matching_stops_at_its_instance():
+    pairs = [_pair(n, 4, n, unmatched=2) for n in (40, 70, 55)]
+    first = [g["map0"] for g in pairs]
+    with bm.Batch(pairs) as B:
+        with pytest.raises(bm.BMError):
+            B.get_mappings()
+        B.set_mappings(first)
+        scores = B.scores()
+        other = [np.concatenate([m[:1], np.roll(m[1:], 3)]) for m in first]
+        other[1] = other[1].copy()
+        other[1][1] = other[1][2] = 7
+        with pytest.raises(bm.BMError, match="instance 1: .*matched twice"):
+            B.set_mappings(other)
+        for want, m in zip((other[0], first[1], first[2]), B.get_mappings()):
+            np.testing.assert_array_equal(m, want)
+        assert (B.scores()[1:] == scores[1:]).all()
