@@ -623,13 +623,18 @@ static bm_status ensure_moved(bm_ctx* ctx) {
     return BM_OK;
 }
 
-// Step 3's row path (k_terms_rows): up to 256 edge slots per moved vertex.
+// Step 3's row path (k_terms_rows): up to 256 edge slots per moved vertex, or as
+// many as the GPU holds for a swap.  Both vertices of a swap have the same two
+// lists, but the one with many edges has nearly all of the rows: 256 slots left
+// half of the GPU idle (n = 8,192 / E = 1e6, 64 swaps from a random matching: 86 us a
+// swap, now 61 with four entries of a list in flight per thread).
 template <bool W16>
 static cudaError_t launch_terms_rows(bm_ctx* ctx, const DevView<W16>& g, int count, const int* dcount, int maxd) {
     const size_t smem = (size_t)(ctx->n + 1) * sizeof(int);
     cudaError_t e = cudaFuncSetAttribute(k_terms_rows<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    dim3 grid(count, std::min(maxd, 256));
+    const int held = ctx->num_sms * (int)std::max<size_t>(1, std::min<size_t>(4, ctx->smem_optin / (smem + 1024)));
+    dim3 grid(count, std::min(maxd, std::max(256, 2 * held / count)));
     k_terms_rows<W16><<<grid, kIncrRowThreads, smem, ctx->st>>>(g, ctx->pS, ctx->moved, count, dcount);
     return cudaGetLastError();
 }

@@ -159,6 +159,30 @@ __global__ void k_perm_cols(int* __restrict__ S, int n, const int* __restrict__ 
     }
 }
 
+// Adds sign * min(w1, w2) of list[i0, i1) at the columns its G2 vertices are
+// matched to, four entries of a thread in flight (two dependent loads each: a
+// swap of hubs walks lists of thousands: k_terms 37 -> 26 us a swap at n = 8,192 /
+// E = 1e6).  FULL: acc has a column n for the
+// unmatched, else they are skipped.
+template <bool W16, bool FULL>
+__device__ __forceinline__ void add_terms(int* acc, const typename Ent<W16>::T* __restrict__ list, int i0, int i1,
+                                          const int* __restrict__ pinv, int n, int w1, int sign, int first, int step) {
+    typedef Ent<W16> EN;
+    for (int k = i0 + first; k < i1; k += 4 * step) {
+        typename EN::T e[4];
+        int col[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (k + u * step < i1) e[u] = list[k + u * step];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (k + u * step < i1) col[u] = pinv[EN::id(e[u])];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (k + u * step < i1 && (FULL || col[u] < n)) atomicAdd(&acc[col[u]], sign * imin(w1, EN::w(e[u])));
+    }
+}
+
 // Step 3: the T terms of every G1 edge at a moved vertex, old image out, new
 // image in.  grid = (count, ceil(max degree / kIncrEdgesPerBlock)), 256
 // threads: each warp takes an edge and its lanes walk the two G2 lists.
@@ -194,23 +218,15 @@ __global__ void __launch_bounds__(256) k_terms(DevView<W16> g, const int* __rest
             off = g.off2o; list = g.ent2o;
         }
         int* srow = g.S + g.at(row, 0);
-        for (int k = off[fo] + lane; k < off[fo + 1]; k += 32) {
-            const E e = list[k];
-            const int col = g.pinv[EN::id(e)];
-            if (col < n) atomicAdd(&srow[col], -imin(w1, EN::w(e)));
-        }
-        for (int k = off[fn] + lane; k < off[fn + 1]; k += 32) {
-            const E e = list[k];
-            const int col = g.pinv[EN::id(e)];
-            if (col < n) atomicAdd(&srow[col], imin(w1, EN::w(e)));
-        }
+        add_terms<W16, false>(srow, list, off[fo], off[fo + 1], g.pinv, n, w1, -1, lane, 32);
+        add_terms<W16, false>(srow, list, off[fn], off[fn + 1], g.pinv, n, w1, 1, lane, 32);
     }
 }
 
 // Step 3 for the edges whose lists cover much of their row (incr_heavy): a
 // block per edge sums its terms in a shared-memory row, then adds the nonzero
-// entries to S in column order.  grid = (count, up to 256 edge slots per
-// moved vertex), dynamic shared memory (n+1) ints.
+// entries to S in column order.  grid = (count, edge slots per moved
+// vertex), dynamic shared memory (n+1) ints.
 template <bool W16>
 __global__ void __launch_bounds__(kIncrRowThreads) k_terms_rows(DevView<W16> g, const int* __restrict__ pS,
                                                                const int* __restrict__ moved, int count,
@@ -244,14 +260,9 @@ __global__ void __launch_bounds__(kIncrRowThreads) k_terms_rows(DevView<W16> g, 
             off = g.off2o; list = g.ent2o;
         }
         __syncthreads();
-        for (int k = off[fo] + threadIdx.x; k < off[fo + 1]; k += blockDim.x) {
-            const E e = list[k];
-            atomicAdd(&rowbuf[g.pinv[EN::id(e)]], -imin(w1, EN::w(e)));   // column n: unmatched, dropped
-        }
-        for (int k = off[fn] + threadIdx.x; k < off[fn + 1]; k += blockDim.x) {
-            const E e = list[k];
-            atomicAdd(&rowbuf[g.pinv[EN::id(e)]], imin(w1, EN::w(e)));
-        }
+        // column n: unmatched, dropped
+        add_terms<W16, true>(rowbuf, list, off[fo], off[fo + 1], g.pinv, n, w1, -1, threadIdx.x, blockDim.x);
+        add_terms<W16, true>(rowbuf, list, off[fn], off[fn + 1], g.pinv, n, w1, 1, threadIdx.x, blockDim.x);
         __syncthreads();
         int* srow = g.S + g.at(row, 0);
         for (int c = threadIdx.x; c < n; c += blockDim.x) {
