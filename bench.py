@@ -37,21 +37,20 @@ WORKLOADS = {
     # smaller pair for ncu captures (S = 268 MB, still above L2)
     "n8192_e1m": dict(n=8192, e=1_000_000, wmax=30000, tail_prob=1e-3, seed=20261206),
 }
-OWN_KERNELS_PER_SWEEP = 18  # relabel x5, hub B build, hub GEMM, profit, diagonal, combine, reduce, candidates,
-#                             4 L2 prefetches, candidate extents, commit (row work only after a new matching)
+OWN_KERNELS_PER_SWEEP = 10  # relabel, hub B build, hub GEMM, profit, diagonal, combine, reduce, candidates,
+#                             candidate sort, commit
 # batch sweep, launch sequence: relabel, row work, profit, combine, reduce, candidates, commit
 # (+ 21 CUB launches: the row sort and the segmented candidate sort); the persistent schedule is one launch
 OWN_KERNELS_PER_BATCH_SWEEP = 7
-CUB_KERNELS_PER_SWEEP = 16  # two radix sorts: histogram + exclusive sum + 6 onesweep passes each
 # learned sweep: contribution, dynamic features, column stats, normalise, pool, U/V, fused ranking,
-# score keys, gather, exact deltas, candidate keys, candidate extents, commit (plus two CUB radix sorts)
+# score keys, gather, exact deltas, candidate keys, candidate sort, commit (plus a CUB radix sort)
 OWN_KERNELS_PER_LEARNED_SWEEP = 13
 # greedy matching: 2 id conversions, 6 list builds (histogram + scatter), pair keys, last-of-run,
 # gather, 4 two-hop counts, 2 feature kernels, positions, the matching kernel (plus CUB sorts/scans)
 OWN_KERNELS_PER_GREEDY = 25
-# best swap: combine + per-row reduce, pick/commit, corner x2, column permutation, term update (scatter
+# best swap: diagonal, combine + per-row reduce, pick/commit, corner x2, column permutation, term update (scatter
 # and row paths), pS sync
-OWN_KERNELS_PER_LOOKUP_SWAP = 9
+OWN_KERNELS_PER_LOOKUP_SWAP = 10
 
 
 def peaks():
@@ -364,7 +363,7 @@ def run_engine(args, g, world, rank, local, pg):
             "profit_smem_atomics": profit_atomics,
             "descent": descent,
             "cpu_baseline": cpu,
-            "gpu_launches": args.steps * (OWN_KERNELS_PER_SWEEP + CUB_KERNELS_PER_SWEEP),
+            "gpu_launches": args.steps * OWN_KERNELS_PER_SWEEP,
             "clocks": clk.summary(),
             "sweeps": [{k: s[k] for k in ("score_before", "score_after", "committed", "verified", "candidates",
                                          "ms_prep", "ms_hub", "ms_profit", "ms_combine", "ms_commit",
