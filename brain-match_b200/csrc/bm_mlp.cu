@@ -458,7 +458,11 @@ extern "C" bm_status bm_mlp_create(bm_mlp** out, uint64_t seed) {
         MK(cudaMalloc(&M->W2b, kMlpHid * kMlpHid * sizeof(__nv_bfloat16)));
         MK(cudaMalloc(&M->W2Tb, kMlpHid * kMlpHid * sizeof(__nv_bfloat16)));
         MK(cudaMalloc(&M->err_d, sizeof(int)));
-        MK(cudaMemset(M->err_d, 0, sizeof(int)));
+        // on the network's own stream, as everything that follows: it does not wait
+        // for the legacy stream, and a copy from pageable memory there may still be
+        // under way when cudaMemcpy returns (2 of 600 new networks read weights that
+        // had not arrived)
+        MK(cudaMemsetAsync(M->err_d, 0, sizeof(int), M->cs));
         // He-uniform initialisation from a seeded generator; zero biases
         std::mt19937_64 rng(seed);
         std::vector<float> h(kParams, 0.f);
@@ -470,7 +474,7 @@ extern "C" bm_status bm_mlp_create(bm_mlp** out, uint64_t seed) {
         fill(oW1, kMlpHid * kMlpIn, kMlpIn);
         fill(oW2, kMlpHid * kMlpHid, kMlpHid);
         fill(oW3, kMlpHid, kMlpHid);
-        MK(cudaMemcpy(M->P, h.data(), kParams * sizeof(float), cudaMemcpyHostToDevice));
+        MK(cudaMemcpyAsync(M->P, h.data(), kParams * sizeof(float), cudaMemcpyHostToDevice, M->cs));
         bm_status s = mlp_update(M, nullptr, 0.f);
         if (s) return s;
         MK(cudaStreamSynchronize(M->cs));
@@ -553,7 +557,8 @@ static bm_status check_err(bm_mlp* M) {
     if (e) {
         // the call's results are not trusted; the network object stays usable
         snprintf(M->err, sizeof M->err, "tensor-core GEMM wait timed out");
-        MK(cudaMemset(M->err_d, 0, sizeof(int)));
+        MK(cudaMemsetAsync(M->err_d, 0, sizeof(int), M->cs));
+        MK(cudaStreamSynchronize(M->cs));   // the next call may be on another stream
         return BM_E_TIMEOUT;
     }
     return BM_OK;
