@@ -848,7 +848,9 @@ static void batch_free(bm_batch* B) {
 extern "C" void bm_batch_destroy(bm_batch* B) { batch_free(B); }
 extern "C" const char* bm_batch_last_error(const bm_batch* B) { return B ? B->err : g_batch_create_err; }
 
-// (Re)builds the per-instance tile tables for the current tile size.
+// (Re)builds the per-instance tile tables for the current tile size.  Every table
+// is copied on the batch's stream: its launches do not wait for the legacy
+// stream, where a copy from pageable memory may still be under way on return.
 static bm_status batch_tiles(bm_batch* B) {
     std::vector<long long> tb(B->count + 1, 0);
     for (int i = 0; i < B->count; i++) {
@@ -858,7 +860,7 @@ static bm_status batch_tiles(bm_batch* B) {
         tb[i + 1] = tb[i] + (long long)T * (T + 1) / 2;
     }
     B->total_tiles = tb[B->count];
-    BK(cudaMemcpy(B->tile_base, tb.data(), tb.size() * sizeof(long long), cudaMemcpyHostToDevice));
+    BK(cudaMemcpyAsync(B->tile_base, tb.data(), tb.size() * sizeof(long long), cudaMemcpyHostToDevice, B->st));
     if (B->iorder) {   // the persistent schedule's task layout: per instance, largest first, rows then tile pairs
         std::vector<int> ord(B->count);
         for (int i = 0; i < B->count; i++) ord[i] = i;
@@ -883,12 +885,12 @@ static bm_status batch_tiles(bm_batch* B) {
         }
         B->total_tasks = tbase[B->count] + tbase[2 * (size_t)B->count + 1];
         if (B->total_tasks > 0x7fffffffLL) B->can_persist = B->use_persist = false;   // 32-bit task indices
-        BK(cudaMemcpy(B->iorder, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice));
-        BK(cudaMemcpy(B->rpt, rpt.data(), rpt.size() * sizeof(int), cudaMemcpyHostToDevice));
-        BK(cudaMemcpy(B->ways, ways.data(), ways.size() * sizeof(int), cudaMemcpyHostToDevice));
-        BK(cudaMemcpy(B->tbase, tbase.data(), tbase.size() * sizeof(long long), cudaMemcpyHostToDevice));
+        BK(cudaMemcpyAsync(B->iorder, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice, B->st));
+        BK(cudaMemcpyAsync(B->rpt, rpt.data(), rpt.size() * sizeof(int), cudaMemcpyHostToDevice, B->st));
+        BK(cudaMemcpyAsync(B->ways, ways.data(), ways.size() * sizeof(int), cudaMemcpyHostToDevice, B->st));
+        BK(cudaMemcpyAsync(B->tbase, tbase.data(), tbase.size() * sizeof(long long), cudaMemcpyHostToDevice, B->st));
     }
-    BK(cudaMemcpy(B->inst, B->hinst.data(), B->hinst.size() * sizeof(BatchInst), cudaMemcpyHostToDevice));
+    BK(cudaMemcpyAsync(B->inst, B->hinst.data(), B->hinst.size() * sizeof(BatchInst), cudaMemcpyHostToDevice, B->st));
     return BM_OK;
 }
 
@@ -907,18 +909,18 @@ static bm_status batch_tables(bm_batch* B) {
         e2[i] = B->ctx[i]->e2;
     }
     BK(cudaMalloc(&B->views, v.size() * sizeof(DevView<W16>)));
-    BK(cudaMemcpy(B->views, v.data(), v.size() * sizeof(DevView<W16>), cudaMemcpyHostToDevice));
+    BK(cudaMemcpyAsync(B->views, v.data(), v.size() * sizeof(DevView<W16>), cudaMemcpyHostToDevice, B->st));
     BK(cudaMalloc(&B->lists, lists.size() * sizeof(void*)));
-    BK(cudaMemcpy(B->lists, lists.data(), lists.size() * sizeof(void*), cudaMemcpyHostToDevice));
+    BK(cudaMemcpyAsync(B->lists, lists.data(), lists.size() * sizeof(void*), cudaMemcpyHostToDevice, B->st));
     BK(cudaMalloc(&B->e1, B->count * sizeof(long long)));
     BK(cudaMalloc(&B->e2, B->count * sizeof(long long)));
-    BK(cudaMemcpy(B->e1, e1.data(), B->count * sizeof(long long), cudaMemcpyHostToDevice));
-    BK(cudaMemcpy(B->e2, e2.data(), B->count * sizeof(long long), cudaMemcpyHostToDevice));
+    BK(cudaMemcpyAsync(B->e1, e1.data(), B->count * sizeof(long long), cudaMemcpyHostToDevice, B->st));
+    BK(cudaMemcpyAsync(B->e2, e2.data(), B->count * sizeof(long long), cudaMemcpyHostToDevice, B->st));
     std::vector<long long> eb(4 * (size_t)B->count + 1, 0);
     for (int i = 0; i < B->count; i++)
         for (int l = 0; l < 4; l++) eb[4 * i + l + 1] = eb[4 * i + l] + (l < 2 ? e1[i] : e2[i]);
     BK(cudaMalloc(&B->ebase, eb.size() * sizeof(long long)));
-    BK(cudaMemcpy(B->ebase, eb.data(), eb.size() * sizeof(long long), cudaMemcpyHostToDevice));
+    BK(cudaMemcpyAsync(B->ebase, eb.data(), eb.size() * sizeof(long long), cudaMemcpyHostToDevice, B->st));
     return BM_OK;
 }
 
@@ -977,7 +979,7 @@ extern "C" bm_status bm_batch_create(bm_batch** out, int32_t count, const int32_
             part_total += (long long)((B->ctx[i]->n + 31) / 32) * B->ctx[i]->n;
         }
         BK(cudaMalloc(&B->row_base, rb.size() * sizeof(int)));
-        BK(cudaMemcpy(B->row_base, rb.data(), rb.size() * sizeof(int), cudaMemcpyHostToDevice));
+        BK(cudaMemcpyAsync(B->row_base, rb.data(), rb.size() * sizeof(int), cudaMemcpyHostToDevice, B->st));
         BK(cudaMalloc(&B->tile_base, (count + 1) * sizeof(long long)));
         BK(cudaMalloc(&B->inst, count * sizeof(BatchInst)));
         const size_t tot = (size_t)B->total;
@@ -1008,7 +1010,7 @@ extern "C" bm_status bm_batch_create(bm_batch** out, int32_t count, const int32_
         long long poff = 0, doff = 0;
         for (int i = 0; i < count; i++) doff += row_smem(B->ctx[i]->n) / sizeof(int);
         BK(cudaMalloc(&B->diag, (size_t)doff * sizeof(int)));
-        BK(cudaMemset(B->diag, 0, (size_t)doff * sizeof(int)));   // the padding is read
+        BK(cudaMemsetAsync(B->diag, 0, (size_t)doff * sizeof(int), B->st));   // the padding is read
         doff = 0;
         for (int i = 0; i < count; i++) {
             BatchInst& I = B->hinst[i];
@@ -1026,7 +1028,7 @@ extern "C" bm_status bm_batch_create(bm_batch** out, int32_t count, const int32_
         bm_status s2 = B->w16 ? batch_tables<true>(B) : batch_tables<false>(B);
         if (s2) return s2;
         BK(cudaMalloc(&B->gbar, 4 * sizeof(unsigned)));
-        BK(cudaMemset(B->gbar, 0, 4 * sizeof(unsigned)));
+        BK(cudaMemsetAsync(B->gbar, 0, 4 * sizeof(unsigned), B->st));
         BK(cudaMalloc(&B->iorder, count * sizeof(int)));
         BK(cudaMalloc(&B->rpt, count * sizeof(int)));
         BK(cudaMalloc(&B->ways, count * sizeof(int)));
@@ -1402,7 +1404,7 @@ extern "C" bm_status bm_batch_sweeps(bm_batch* B, int32_t sweeps, const bm_sweep
     if (gerr) {
         // a grid-barrier wait of the persistent sweep ran out: the matchings
         // may be partly committed; the caller sets them again
-        BK(cudaMemset(B->gbar, 0, 4 * sizeof(unsigned)));
+        BK(cudaMemsetAsync(B->gbar, 0, 4 * sizeof(unsigned), B->st));
         for (bm_ctx* c : B->ctx) { c->mapped = false; c->S_exact = false; }
         snprintf(B->err, sizeof B->err, "bm_batch_sweeps: persistent sweep grid barrier wait timed out");
         return BM_E_TIMEOUT;

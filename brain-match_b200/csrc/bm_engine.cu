@@ -977,7 +977,7 @@ extern "C" bm_status bm_sweep(bm_ctx* ctx, const bm_sweep_opts* opts, bm_sweep_s
                                                                         : "set commit cluster barrier");
         ctx->mapped = false;
         ctx->S_exact = false;
-        if (herr) CK(cudaMemset(ctx->hub_err, 0, sizeof(int)));
+        if (herr) CK(cudaMemsetAsync(ctx->hub_err, 0, sizeof(int), ctx->st));
         if (cerr && (s = set_commit_reset(ctx))) return s;
         return BM_E_TIMEOUT;
     }
@@ -1089,7 +1089,7 @@ static bm_status lookup_descent_impl(bm_ctx* ctx, int max_swaps, bm_lookup_stats
         CK(cudaMemcpy(&herr, ctx->hub_err, sizeof herr, cudaMemcpyDeviceToHost));
         if (herr & (1 << kCmbErrBit)) {
             set_err(ctx, "bm_lookup_descent: pair combine tile wait timed out");
-            CK(cudaMemset(ctx->hub_err, 0, sizeof(int)));
+            CK(cudaMemsetAsync(ctx->hub_err, 0, sizeof(int), ctx->st));
             ctx->mapped = false;
             ctx->S_exact = false;
             return BM_E_TIMEOUT;
