@@ -502,13 +502,11 @@ extern "C" bm_status bm_mlp_set_params(bm_mlp* M, const float* params) {
     return BM_OK;
 }
 
-// A (m x k) times B (n x k) transposed; `splits` shares of K (their results must
-// be added: o.add).
+// A (m x k) times B (n x k) transposed.
 template <int BN>
-static bm_status gemm(bm_mlp* M, const __nv_bfloat16* A, const __nv_bfloat16* B, int m, int n, int k, const GemmOut& o,
-                      int splits = 1) {
+static bm_status gemm(bm_mlp* M, const __nv_bfloat16* A, const __nv_bfloat16* B, int m, int n, int k, const GemmOut& o) {
     MK(cudaFuncSetAttribute(k_gemm_bf16<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_bf16_smem<BN>()));
-    k_gemm_bf16<BN><<<dim3(n / BN, m / kGemmM, splits), kGemmThreads, gemm_bf16_smem<BN>(), M->cs>>>(
+    k_gemm_bf16<BN><<<dim3(n / BN, m / kGemmM), kGemmThreads, gemm_bf16_smem<BN>(), M->cs>>>(
         A, B, m, n, k, o, M->err_d, take_stall(BM_STALL_MLP_GEMM));
     MK(cudaGetLastError());
     return BM_OK;
@@ -527,6 +525,14 @@ static bm_status mlp_forward_dev(bm_mlp* M, int kpad, bool backward) {
     return BM_OK;
 }
 
+// Columns per CTA of the weight gradients' GEMMs.  Their sums over all rows stay
+// in one accumulator each, in row order: shares of 512 rows, added with float
+// atomics, were up to 6.8e-6 (2-norm) off these sums at 8,000 rows and did not
+// repeat from three shares on.  So a layer has few CTAs and a long serial chain,
+// and narrower ones help (a step of 1,024 rows 248 -> 241 us with 32 columns instead of
+// 64, of 8,000 rows 570 -> 555; 445 with the shares).
+constexpr int kGradBN = 32;
+
 // One forward + backward on rows [0,k) of X (XT its transpose) with targets t;
 // gradients into M->G.
 static bm_status mlp_fwd_bwd_dev(bm_mlp* M, int k) {
@@ -541,12 +547,11 @@ static bm_status mlp_fwd_bwd_dev(bm_mlp* M, int k) {
     GemmOut oh, o2, o1;
     oh.mask = M->H1f; oh.CbT = M->dH1T; oh.colsum = M->G + oB1;
     if ((s = gemm<64>(M, M->dH2b, M->W2Tb, kpad, kMlpHid, kMlpHid, oh))) return s;
-    // dW2 = dH2^T H1, dW1 = dH1^T X, over shares of 512 rows
-    const int splits = std::max(1, kpad / 512);
-    o2.add = M->G + oW2;
-    if ((s = gemm<64>(M, M->dH2T, M->H1T, kMlpHid, kMlpHid, kpad, o2, splits))) return s;
-    o1.add = M->G + oW1;
-    if ((s = gemm<64>(M, M->dH1T, M->XT, kMlpHid, kMlpIn, kpad, o1, splits))) return s;
+    // dW2 = dH2^T H1, dW1 = dH1^T X
+    o2.C = M->G + oW2;
+    if ((s = gemm<kGradBN>(M, M->dH2T, M->H1T, kMlpHid, kMlpHid, kpad, o2))) return s;
+    o1.C = M->G + oW1;
+    if ((s = gemm<kGradBN>(M, M->dH1T, M->XT, kMlpHid, kMlpIn, kpad, o1))) return s;
     return BM_OK;
 }
 

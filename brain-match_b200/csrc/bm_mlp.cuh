@@ -22,13 +22,12 @@ struct GemmOut {
     int relu = 0;                     // max(., 0)
     const float* mask = nullptr;      // M x N: 0 where mask <= 0
     float* C = nullptr;               // M x N fp32
-    float* add = nullptr;             // M x N fp32, added atomically (split K)
     float* colsum = nullptr;          // N: += column sums
     __nv_bfloat16* Cb = nullptr;      // M x N bf16
     __nv_bfloat16* CbT = nullptr;     // N x M bf16, transposed
 };
 
-// M % 128 == 0, N % BN == 0, K % 64 == 0; grid (N / BN, M / 128, splits of K).
+// M % 128 == 0, N % BN == 0, K % 64 == 0; grid (N / BN, M / 128).
 // The network's GEMMs are small (1,024 x 256 x 256 for a training batch), so a
 // launch is bound by its latency and by how many SMs it uses: 64 columns per
 // CTA (32 CTAs per batch instead of 8 with whole rows), the four K-chunks of a
@@ -53,9 +52,7 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int b0 = blockIdx.x * BN, a0 = blockIdx.y * kGemmM;
     const int KB = K * 2;                        // bytes per row
-    const int all = KB / kGemmKC;                // 128-byte chunks; this split's are [k0, k0 + KC)
-    const int k0 = (int)((long long)all * blockIdx.z / gridDim.z);
-    const int KC = (int)((long long)all * (blockIdx.z + 1) / gridDim.z) - k0;
+    const int KC = KB / kGemmKC;                 // 128-byte chunks
     const uint8_t* Ab = reinterpret_cast<const uint8_t*>(A);
     const uint8_t* Bb = reinterpret_cast<const uint8_t*>(B);
 
@@ -76,7 +73,7 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
 
     auto load = [&](int st, int kc) {
         const uint32_t sA = base + st * kStage, sB = sA + kGemmM * kGemmKC;
-        const size_t koff = (size_t)(k0 + kc) * kGemmKC;
+        const size_t koff = (size_t)kc * kGemmKC;
         for (int i = tid; i < kGemmM * 8; i += kGemmThreads) {
             const int r = i >> 3, c = i & 7;
             cp_async16(sA + r * 128 + ((c ^ (r & 7)) << 4), Ab + (size_t)(a0 + r) * KB + koff + c * 16);
@@ -126,7 +123,7 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
         const int last = KC - 1;
         ok = ok && mbar_wait_bounded(bars + 8 * (last % kMlpStages), (last / kMlpStages) & 1, err);
         // test hook (bm_test_stall): the barrier's next phase never completes
-        if (stall && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
+        if (stall && blockIdx.x == 0 && blockIdx.y == 0)
             ok = ok && mbar_wait_bounded(bars + 8 * (last % kMlpStages), ((last / kMlpStages) + 1) & 1, err,
                                          kStallPolls);
     }
@@ -171,10 +168,6 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
             float4* d4 = reinterpret_cast<float4*>(o.C + (size_t)row * N + c0);
 #pragma unroll
             for (int q = 0; q < 8; q++) d4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        }
-        if (o.add) {
-#pragma unroll
-            for (int q = 0; q < 32; q++) atomicAdd(o.add + (size_t)row * N + c0 + q, v[q]);
         }
         if (o.Cb) {
             __nv_bfloat162* d2 = reinterpret_cast<__nv_bfloat162*>(o.Cb + (size_t)row * N + c0);
