@@ -270,7 +270,7 @@ static __global__ void __launch_bounds__(kMlpHid) k_head(const float* __restrict
         const float hv = H2[(size_t)(r0 + r) * kMlpHid + c], dy = s_dy[r];
         col[r] = __float2bfloat16(hv > 0.f ? dy * w : 0.f);
         dH2[(size_t)(r0 + r) * kMlpHid + c] = col[r];
-        g3 += hv * dy;
+        if (dy != 0.f) g3 += hv * dy;   // a padded row's activation may be infinite: it adds nothing
         g2 += __bfloat162float(col[r]);
     }
     uint4* dst = reinterpret_cast<uint4*>(dH2T + (size_t)c * Bpad + r0);
