@@ -670,7 +670,8 @@ static bm_status rank_pairs_dev(bm_ctx* ctx, bm_mlp* M, const int* pa, const int
     const long long tiles = (k + kGemmM - 1) / kGemmM;
     const int grid = (int)std::min<long long>(tiles, ctx->num_sms);
     k_mlp_rank<<<grid, kRankThreads, kRankSmem, M->cs>>>(M->U.as<float>(), M->V.as<float>(), pa, pb, k, M->W2b,
-                                                         M->P + oB2, M->P + oW3, M->P + oB3, y, M->err_d);
+                                                         M->P + oB2, M->P + oW3, M->P + oB3, y, M->err_d,
+                                                         take_stall(BM_STALL_RANK));
     MK(cudaGetLastError());
     return BM_OK;
 }
@@ -900,7 +901,7 @@ static bm_status learned_impl(bm_ctx* ctx, bm_mlp* M, const bm_learned_opts* o, 
                      smem, n);
             return BM_E_INPUT;
         }
-        if ((r = launch_set_commit<W16, 2>(ctx, ck + top, nullptr, top, -1, 0, 0))) {
+        if ((r = launch_set_commit<W16, 2>(ctx, ck + top, nullptr, top, -1, 0, take_stall(BM_STALL_COMMIT)))) {
             snprintf(M->err, sizeof M->err, "%s", ctx->err);
             return r;
         }
@@ -908,11 +909,20 @@ static bm_status learned_impl(bm_ctx* ctx, bm_mlp* M, const bm_learned_opts* o, 
         int cerr = 0;
         MK(cudaMemcpyAsync(&cerr, set_commit_err(ctx), sizeof cerr, cudaMemcpyDeviceToHost, M->cs));
         MK(cudaEventRecord(M->e1, M->cs));
-        if ((r = check_err(M))) return r;
-        if (cerr) {
-            set_commit_reset(ctx);
-            snprintf(M->err, sizeof M->err, "set commit grid barrier wait timed out");
-            return BM_E_TIMEOUT;
+        r = check_err(M);
+        if (r || cerr) {
+            // the commit has run on what the ranking gave, or stopped in part: the
+            // caller sets a matching again before the next call
+            ctx->mapped = false;
+            ctx->S_exact = false;
+            if (cerr) {
+                const bm_status rs = set_commit_reset(ctx);
+                if (!r) {
+                    snprintf(M->err, sizeof M->err, "%s", rs ? ctx->err : "set commit wait timed out");
+                    r = rs ? rs : BM_E_TIMEOUT;
+                }
+            }
+            return r;
         }
         if (stats) {
             float t[5];

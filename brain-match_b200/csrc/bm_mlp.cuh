@@ -408,7 +408,7 @@ static __global__ void __launch_bounds__(kRankThreads, 1)
 k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* __restrict__ pa,
            const int* __restrict__ pb, long long k, const __nv_bfloat16* __restrict__ W2b,
            const float* __restrict__ b2, const float* __restrict__ w3, const float* __restrict__ b3,
-           float* __restrict__ y, int* __restrict__ err) {
+           float* __restrict__ y, int* __restrict__ err, int stall) {
     constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kMlpHid >> 3) << 17) |
                                 ((uint32_t)(kGemmM >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
@@ -452,6 +452,7 @@ k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* 
     const uint32_t tmem = *tslot_ptr;
 
     const long long tiles = (k + kGemmM - 1) / kGemmM;
+    const int limit = stall ? kStallPolls : 1 << 22;   // polls of a wait
     int it = 0, issued = 0;   // tiles begun; tiles handed to the tensor cores (thread 0)
     bool ok = true;
     if (wid < kRankBuilders / 32) {
@@ -464,7 +465,7 @@ k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* 
             const int h = it & 1;
             const long long row0 = t * kGemmM;
             // the previous tile's MMA has read A
-            if (ok && it > 0) ok = mbar_wait_bounded(bar_mma(h ^ 1), ((it - 1) >> 1) & 1, err);
+            if (ok && it > 0) ok = mbar_wait_bounded(bar_mma(h ^ 1), ((it - 1) >> 1) & 1, err, limit);
             // A tile: warp w builds rows 8 w .. 8 w + 7 (four rows per pass, their
             // loads all issued before any store); lane = 16-byte chunk (8 units).
             // Lane q holds row q's pair, loaded a tile ahead.
@@ -508,7 +509,7 @@ k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* 
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("bar.sync 1, %0;" :: "n"(kRankBuilders) : "memory");
             // the accumulator's previous tile has been reduced
-            if (tid == 0 && ok && it >= 2) ok = mbar_wait_bounded(bar_free(h), ((it >> 1) - 1) & 1, err);
+            if (tid == 0 && ok && it >= 2) ok = mbar_wait_bounded(bar_free(h), ((it >> 1) - 1) & 1, err, limit);
             if (tid == 0 && ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -535,7 +536,11 @@ k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* 
         const int q4 = wid & 3;   // the TMEM lane quarter a warp may read
         for (long long t = blockIdx.x; t < tiles; t += gridDim.x, it++) {
             const int h = it & 1;
-            ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(bar_mma(h), (it >> 1) & 1, err));
+            bool here = ok && mbar_wait_bounded(bar_mma(h), (it >> 1) & 1, err, limit);
+            // test hook (bm_test_stall): CTA 0's first tile also waits for the
+            // accumulator's next tile, which needs this one reduced first
+            if (here && stall && blockIdx.x == 0 && it == 0) here = mbar_wait_bounded(bar_mma(h), 1, err, limit);
+            ok = __all_sync(0xffffffffu, here);
             if (!ok) continue;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const long long i = t * kGemmM + q4 * 32 + lane;
