@@ -19,7 +19,7 @@ BM_FLAG_NO_HUB_GEMM = 2
 BM_STATIC_MAX_PAIRS = 65536
 BM_STALL_HUB_GEMM, BM_STALL_COMMIT, BM_STALL_COMBINE, BM_STALL_GREEDY, BM_STALL_MLP_GEMM, BM_STALL_BATCH = (
     1, 2, 3, 4, 5, 6)
-BM_STALL_RANK = 7
+BM_STALL_RANK, BM_STALL_FIRST = 7, 8
 
 
 class GenParams(C.Structure):

@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(kSetThreads, 1) k_commit_sets(DevView<W16> g, 
             __threadfence();
             if (!(A.stall && step == 0 && nct > 1 && ct == nct - 1)) atomicAdd(&A.ctl->arrived, 1u);
             if (ct == 0) {
-                const unsigned want = (unsigned)nct * (step + 1), limit = A.stall ? 1u << 12 : kSetPolls;
+                const unsigned want = (unsigned)nct * (step + 1), limit = A.stall ? kStallPolls : kSetPolls;
                 unsigned it = 0;
                 while (set_ld_acquire(&A.ctl->arrived) != want)
                     if (++it > limit) { s_ok = 0; break; }

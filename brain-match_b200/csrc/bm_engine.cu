@@ -44,7 +44,7 @@ int take_stall(int site) {
 }
 
 extern "C" bm_status bm_test_stall(int32_t site) {
-    if (site < 0 || site > BM_STALL_RANK) return BM_E_INPUT;
+    if (site < 0 || site > BM_STALL_FIRST) return BM_E_INPUT;
     g_stall.store(site);
     return BM_OK;
 }
@@ -1206,12 +1206,13 @@ static bm_status first_improvement_impl(bm_ctx* ctx, int max_passes, long long* 
         CK(cudaGetLastError());
     }
     FirstState h;
+    int stall = take_stall(BM_STALL_FIRST);
     do {
         if (rows) {
-            CK(cudaLaunchKernelEx(&cfg, k_first_rows<W16>, g, st, contrib, max_passes));
+            CK(cudaLaunchKernelEx(&cfg, k_first_rows<W16>, g, st, contrib, max_passes, stall));
         } else {
             CK(cudaMemsetAsync(slots, 0, slot_bytes, ctx->st));   // a launch starts again at tag 1
-            void* args[] = {&g, &st, &slots, &max_passes};
+            void* args[] = {&g, &st, &slots, &max_passes, &stall};
             CK(cudaLaunchCooperativeKernel((const void*)k_first<W16>, dim3(grid), dim3(kFirstThreads), args, smem, ctx->st));
         }
         CK(cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, ctx->st));
@@ -1310,7 +1311,8 @@ static bm_status triple_round_impl(bm_ctx* ctx, const bm_triple_opts* o, bm_trip
     k_triple_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets);
     CK(cudaGetLastError());
     const int lim = o->max_candidates > 0 ? std::min(o->max_candidates, n) : n;
-    if ((s = launch_set_commit<W16, 3>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0, 0, false))) return s;
+    if ((s = launch_set_commit<W16, 3>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0,
+                                       take_stall(BM_STALL_COMMIT), false))) return s;
     CK(cudaEventRecord(ctx->ev[3], ctx->st));
     CommitStats cs;
     unsigned long long cnt[2], top = 0;
@@ -1411,7 +1413,8 @@ static bm_status quad_round_impl(bm_ctx* ctx, const bm_quad_opts* o, bm_quad_sta
     k_quad_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets);
     CK(cudaGetLastError());
     const int lim = o->max_candidates > 0 ? std::min(o->max_candidates, n) : n;
-    if ((s = launch_set_commit<W16, 4>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0, 0, false))) return s;
+    if ((s = launch_set_commit<W16, 4>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0,
+                                       take_stall(BM_STALL_COMMIT), false))) return s;
     CK(cudaEventRecord(ctx->ev[3], ctx->st));
     CommitStats cs;
     unsigned long long cnt[2], top = 0;

@@ -61,7 +61,7 @@ struct FirstState {
 
 template <bool W16>
 __global__ void __launch_bounds__(kFirstThreads) k_first(DevView<W16> g, FirstState* __restrict__ st,
-                                                         unsigned long long* slots, int max_passes) {
+                                                         unsigned long long* slots, int max_passes, int stall) {
     constexpr int NWARP = kFirstThreads / 32;
     extern __shared__ unsigned short p16[];   // the matching; unmatched = n
     __shared__ unsigned long long s_red[NWARP];
@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(kFirstThreads) k_first(DevView<W16> g, FirstSt
     const int G = gridDim.x, nw = G * NWARP;
     for (int v = tid; v < n; v += kFirstThreads) p16[v] = (unsigned short)g.p[v];
     if (tid == 0) s_ok = 1;
+    const unsigned polls = stall ? kStallPolls : kFirstPolls;   // stall (bm_test_stall): the last CTA keeps its words
     const int most = nw * kFirstMult;
     int want = kFirstMin;
     int m1 = st->m1, m2 = st->m2, in_pass = st->in_pass, passes = st->passes, done = 0;
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(kFirstThreads) k_first(DevView<W16> g, FirstSt
         if (wid == 0) {
             best = lane < NWARP ? s_red[lane] : kFirstNone;
             for (int o = 16; o; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-            if (lane == 0)
+            if (lane == 0 && !(stall && blockIdx.x == G - 1))
                 asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(sl + blockIdx.x), "l"(tag | best) : "memory");
         }
         best = kFirstNone;
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(kFirstThreads) k_first(DevView<W16> g, FirstSt
             for (unsigned it = 0;;) {
                 asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(sl + s) : "memory");
                 if ((v & ~kFirstNone) == tag) break;
-                if (++it > kFirstPolls) { s_ok = 0; v = kFirstNone; break; }
+                if (++it > polls) { s_ok = 0; v = kFirstNone; break; }
             }
             best = min(best, v & kFirstNone);
         }
@@ -183,7 +184,7 @@ __host__ __device__ inline size_t first_rows_smem(int n) {
 
 template <bool W16>
 __global__ void __launch_bounds__(kRowsThreads, 1) k_first_rows(DevView<W16> g, FirstState* __restrict__ st,
-                                                                int* __restrict__ Cg, int max_passes) {
+                                                                int* __restrict__ Cg, int max_passes, int stall) {
     typedef Ent<W16> EN;
     typedef typename EN::T E;
     constexpr int T = kRowsThreads, NWARP = T / 32;
@@ -204,6 +205,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_first_rows(DevView<W16> g, 
     if (tid == 0) s_ok = 1;
     if (tid < 2 * kRowsCluster) (&s_slot[0][0])[tid] = 0;
     const bool loops = g.offs[n] > 0;
+    const unsigned polls = stall ? kStallPolls : kFirstPolls;   // stall (bm_test_stall): the last CTA keeps its words
     int m1 = st->m1, m2 = st->m2, in_pass = st->in_pass, passes = st->passes, done = 0;
     long long delta = st->delta, commits = st->commits;
     int rows = 1, seen = 0;   // rows of this step; rows since the last commit
@@ -298,7 +300,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_first_rows(DevView<W16> g, 
         if (wid == 0) {
             best = lane < NWARP ? s_red[lane] : kFirstNone;
             for (int o = 16; o; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-            if (lane < kRowsCluster) {
+            if (lane < kRowsCluster && !(stall && blockIdx.x == kRowsCluster - 1)) {
                 const uint32_t mine = (uint32_t)__cvta_generic_to_shared(&s_slot[par][blockIdx.x]);
                 uint32_t peer;
                 asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(mine), "r"(lane));
@@ -312,7 +314,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_first_rows(DevView<W16> g, 
             for (unsigned it = 0;;) {
                 asm volatile("ld.volatile.shared.u64 %0, [%1];" : "=l"(v) : "r"(here) : "memory");
                 if ((v & ~kFirstNone) == tag) break;
-                if (++it > kFirstPolls) { s_ok = 0; v = kFirstNone; break; }
+                if (++it > polls) { s_ok = 0; v = kFirstNone; break; }
             }
             best = v & kFirstNone;
         }

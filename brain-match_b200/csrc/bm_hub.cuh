@@ -66,9 +66,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
     return false;
 }
 
-// Polls of a wait that the stall test hook (bm_test_stall) makes run out.
-constexpr int kStallPolls = 1 << 12;
-
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
 }

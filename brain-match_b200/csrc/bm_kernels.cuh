@@ -86,6 +86,9 @@ template <bool W16> struct DevView {
     __device__ __forceinline__ int w2d(int f) const { return W2D[f]; }
 };
 
+// Polls of a wait that the stall test hook (bm_test_stall) makes run out.
+constexpr int kStallPolls = 1 << 12;
+
 __device__ __forceinline__ int imin(int a, int b) { return a < b ? a : b; }
 
 // ---------------------------------------------------------------------------

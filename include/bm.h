@@ -264,12 +264,14 @@ bm_status bm_measure_peaks(int32_t n, double* red_per_s, double* minadd_per_s);
  * may be partly committed: set a matching again before the next call.
  */
 #define BM_STALL_HUB_GEMM   1   /* bm_sweep: tensor-core hub GEMM          */
-#define BM_STALL_COMMIT     2   /* bm_sweep, bm_learned_sweep: set commit  */
+#define BM_STALL_COMMIT     2   /* bm_sweep, bm_triple_round, bm_quad_round,
+                                   bm_learned_sweep: set commit            */
 #define BM_STALL_COMBINE    3   /* bm_sweep: TMA-fed pair combine          */
 #define BM_STALL_GREEDY     4   /* bm_greedy_match: grid barrier           */
 #define BM_STALL_MLP_GEMM   5   /* bm_mlp_*: tensor-core GEMM              */
 #define BM_STALL_BATCH      6   /* bm_batch_sweeps: persistent sweep grid barrier */
 #define BM_STALL_RANK       7   /* bm_learned_sweep, bm_mlp_rank_pairs: ranking */
+#define BM_STALL_FIRST      8   /* bm_first_improvement: exchange          */
 bm_status bm_test_stall(int32_t site);
 
 /* ---- Exact swap-lookup table ----
