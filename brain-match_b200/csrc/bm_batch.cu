@@ -1231,7 +1231,7 @@ static bm_status enqueue_eval(bm_batch* B) {
                                                  B->total, 0, 64, B->st));
     BK(cudaMemsetAsync(B->counter, 0, sizeof(int), B->st));
     const size_t smem = row_smem(B->max_n);
-    BK(cudaFuncSetAttribute(k_b_profit<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BK(allow_smem<k_b_profit<W16>>(smem));
     int per_sm = 0, sms = B->ctx[0]->num_sms;
     BK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_b_profit<W16>, B->profit_threads, smem));
     if (per_sm < 1) { snprintf(B->err, sizeof B->err, "profit kernel does not fit (max n %d)", B->max_n); return BM_E_INPUT; }
@@ -1257,7 +1257,7 @@ static bm_status enqueue_select_commit(bm_batch* B, int max_scan, int max_verify
     BK(cub::DeviceSegmentedRadixSort::SortKeys(B->cub_tmp, tb, B->ckeys, B->ckeys_sorted, B->total, B->count,
                                                B->row_base, B->row_base + 1, 0, 64, B->st));
     const size_t smem = commit_group_smem(B->max_n);
-    BK(cudaFuncSetAttribute(k_b_commit<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BK(allow_smem<k_b_commit<W16>>(smem));
     k_b_commit<W16><<<B->count, 1024, smem, B->st>>>((const DevView<W16>*)B->views, B->inst, max_scan, max_verify,
                                                      B->cstats, B->acc_delta, B->acc_commits);
     BK(cudaGetLastError());

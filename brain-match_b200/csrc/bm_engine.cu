@@ -599,7 +599,7 @@ bm_status stage_profit(bm_ctx* ctx) {
         CK(cudaGetLastError());
     }
     const size_t smem = row_smem(n);
-    CK(cudaFuncSetAttribute(k_profit<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(allow_smem<k_profit<W16>>(smem));
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_profit<W16>, 512, smem));
     if (per_sm < 1) { set_err(ctx, "profit kernel does not fit (n=%d)", n); return BM_E_INPUT; }
@@ -631,7 +631,7 @@ static bm_status ensure_moved(bm_ctx* ctx) {
 template <bool W16>
 static cudaError_t launch_terms_rows(bm_ctx* ctx, const DevView<W16>& g, int count, const int* dcount, int maxd) {
     const size_t smem = (size_t)(ctx->n + 1) * sizeof(int);
-    cudaError_t e = cudaFuncSetAttribute(k_terms_rows<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem<k_terms_rows<W16>>(smem);
     if (e != cudaSuccess) return e;
     const int held = ctx->num_sms * (int)std::max<size_t>(1, std::min<size_t>(4, ctx->smem_optin / (smem + 1024)));
     dim3 grid(count, std::min(maxd, std::max(256, 2 * held / count)));
@@ -685,7 +685,7 @@ bm_status stage_refresh(bm_ctx* ctx, int* mode) {
     }
     {
         const size_t smem = 3 * (size_t)count * sizeof(int);
-        CK(cudaFuncSetAttribute(k_perm_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(allow_smem<k_perm_cols>(smem));
         const int blocks = std::min(n, ctx->num_sms * (smem <= 48 * 1024 ? 4 : 1));
         k_perm_cols<<<blocks, 512, smem, ctx->st>>>(ctx->S, n, ctx->moved, count, ctx->p, ctx->pinvS);
         CK(cudaGetLastError());
@@ -861,7 +861,7 @@ bm_status launch_set_commit(bm_ctx* ctx, const unsigned long long* keys, const i
     }
     grid = std::min(grid, ctx->num_sms);
     const size_t smem = SetSmem<K>::bytes(n);
-    CK(cudaFuncSetAttribute(k_commit_sets<W16, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK((allow_smem<k_commit_sets<W16, K>>(smem)));
     DevView<W16> g = view<W16>(ctx);
     void* args[] = {&g, &a};
     CK(cudaLaunchCooperativeKernel((const void*)k_commit_sets<W16, K>, dim3(grid), dim3(kSetThreads), args, smem,
@@ -1156,7 +1156,7 @@ static bool first_rows_fit(bm_ctx* ctx, cudaLaunchConfig_t* cfg) {
     cfg->dynamicSmemBytes = smem;
     int clusters = 0;
     const bool ok =
-        cudaFuncSetAttribute(k_first_rows<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+        allow_smem<k_first_rows<W16>>(smem) == cudaSuccess &&
         cudaFuncSetAttribute(k_first_rows<W16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
         cudaOccupancyMaxActiveClusters(&clusters, k_first_rows<W16>, cfg) == cudaSuccess && clusters > 0;
     cudaGetLastError();   // a refused attribute is not an error of the launches
@@ -1182,7 +1182,7 @@ static bm_status first_improvement_impl(bm_ctx* ctx, int max_passes, long long* 
     int grid = 0;
     const size_t smem = (size_t)n * sizeof(unsigned short);
     if (!rows) {
-        CK(cudaFuncSetAttribute(k_first<W16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(allow_smem<k_first<W16>>(smem));
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_first<W16>, kFirstThreads, smem));
         if (per_sm < 1) { set_err(ctx, "first-improvement kernel does not fit (n=%d)", n); return BM_E_INPUT; }

@@ -794,7 +794,7 @@ bm_status device_features(const char* fn, GreedyDev& D, int n, const DevLists& l
     GK(D.alloc(&r2, n)); GK(D.alloc(&c2, n));
     GK(D.alloc(&key, n)); GK(D.alloc(&key2, n)); GK(D.alloc(&val, n)); GK(D.alloc(&val2, n));
     const size_t bm = (size_t)((n + 31) / 32) * sizeof(unsigned);
-    GK(cudaFuncSetAttribute(k_two_hop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bm));
+    GK(allow_smem<k_two_hop>(bm));
     k_two_hop<<<sms * 4, 512, bm, st>>>(lo.off, lo.id, n, r2);
     k_two_hop<<<sms * 4, 512, bm, st>>>(li.off, li.id, n, c2);
     k_features<<<(n + 255) / 256, 256, 0, st>>>(lo.off, li.off, r2, c2, n, feat, ratio, key, val);
@@ -864,7 +864,7 @@ extern "C" bm_status bm_greedy_match(int32_t n, int64_t e1, const int32_t* src1,
         set_err(nullptr, "%s: n=%d needs %zu bytes of shared memory per CTA (limit %d)", fn, n, smem, optin);
         return BM_E_INPUT;
     }
-    GK(cudaFuncSetAttribute(k_greedy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GK(allow_smem<k_greedy>(smem));
     GK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_greedy, kGreedyThreads, smem));
     if (per_sm < 1) { set_err(nullptr, "%s: the matching kernel does not fit on an SM", fn); return BM_E_INPUT; }
     const int grid = sms;
@@ -932,7 +932,7 @@ extern "C" bm_status bm_greedy_match(int32_t n, int64_t e1, const int32_t* src1,
     const bool cluster =
         2.0 * (double)e1 * (double)mk / n <= kGreedyClusterWork &&
         cfg.dynamicSmemBytes + 12288 <= (size_t)optin &&
-        cudaFuncSetAttribute(k_greedy_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) == cudaSuccess &&
+        allow_smem<k_greedy_cluster>(cfg.dynamicSmemBytes) == cudaSuccess &&
         cudaFuncSetAttribute(k_greedy_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
         cudaOccupancyMaxActiveClusters(&clusters, k_greedy_cluster, &cfg) == cudaSuccess && clusters > 0;
     cudaGetLastError();   // a refused attribute is not an error of the launch

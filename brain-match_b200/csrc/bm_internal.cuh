@@ -3,6 +3,7 @@
 #pragma once
 #include <cstdio>
 #include <cstdarg>
+#include <atomic>
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include "bm.h"
@@ -13,6 +14,28 @@ using namespace bm;
 // Test hook (bm_test_stall): 1 if the next launch at `site` is to make one of
 // its bounded waits run out, clearing the request.
 int take_stall(int site);
+
+// cudaSuccess if a launch of Kernel may use `bytes` of dynamic shared memory.  The
+// limit of a kernel belongs to the process, so it is set once per device to all
+// that a block can have: set to each launch's own need, a thread with a smaller
+// engine lowered it between another thread's setting and launch, and that launch
+// was refused.
+template <auto Kernel> cudaError_t allow_smem(size_t bytes) {
+    static std::atomic<int> limit[64];   // 0: not set
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    int most = dev < 64 ? limit[dev].load() : 0;
+    if (!most) {
+        cudaFuncAttributes fa;
+        if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+        if ((e = cudaFuncGetAttributes(&fa, Kernel)) != cudaSuccess) return e;
+        most -= (int)fa.sharedSizeBytes;
+        if ((e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most)) != cudaSuccess) return e;
+        if (dev < 64) limit[dev].store(most);
+    }
+    return bytes <= (size_t)most ? cudaSuccess : cudaErrorInvalidValue;
+}
 
 struct bm_ctx {
     int n = 0;
