@@ -666,12 +666,12 @@ static bm_status rank_pairs_dev(bm_ctx* ctx, bm_mlp* M, const int* pa, const int
         MK(cudaGetLastError());
     }
     if (k == 0) return BM_OK;
-    MK(cudaFuncSetAttribute(k_mlp_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, kRankSmem));
+    const auto rank = take_stall(BM_STALL_RANK) ? k_mlp_rank<true> : k_mlp_rank<false>;
+    MK(cudaFuncSetAttribute(rank, cudaFuncAttributeMaxDynamicSharedMemorySize, kRankSmem));
     const long long tiles = (k + kGemmM - 1) / kGemmM;
     const int grid = (int)std::min<long long>(tiles, ctx->num_sms);
-    k_mlp_rank<<<grid, kRankThreads, kRankSmem, M->cs>>>(M->U.as<float>(), M->V.as<float>(), pa, pb, k, M->W2b,
-                                                         M->P + oB2, M->P + oW3, M->P + oB3, y, M->err_d,
-                                                         take_stall(BM_STALL_RANK));
+    rank<<<grid, kRankThreads, kRankSmem, M->cs>>>(M->U.as<float>(), M->V.as<float>(), pa, pb, k, M->W2b,
+                                                   M->P + oB2, M->P + oW3, M->P + oB3, y, M->err_d);
     MK(cudaGetLastError());
     return BM_OK;
 }

@@ -404,11 +404,14 @@ constexpr int kRankSmem = kRankA + kRankB + 2 * kMlpHid * 4 + 1024 + 256;
 // build, 2 KB of fp32 U and V per pair.
 // Every wait is bounded: after a timeout (err set) a thread waits no more, no
 // further MMA is issued or accumulator read, and the warps run out their loops.
+// STALL: the test hook's form, in a kernel of its own because the registers of
+// this one are all taken (a run-time switch cost the learned sweep 1.7%).
+template <bool STALL>
 static __global__ void __launch_bounds__(kRankThreads, 1)
 k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* __restrict__ pa,
            const int* __restrict__ pb, long long k, const __nv_bfloat16* __restrict__ W2b,
            const float* __restrict__ b2, const float* __restrict__ w3, const float* __restrict__ b3,
-           float* __restrict__ y, int* __restrict__ err, int stall) {
+           float* __restrict__ y, int* __restrict__ err) {
     constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kMlpHid >> 3) << 17) |
                                 ((uint32_t)(kGemmM >> 4) << 24);
     extern __shared__ uint8_t smem_raw[];
@@ -452,7 +455,7 @@ k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* 
     const uint32_t tmem = *tslot_ptr;
 
     const long long tiles = (k + kGemmM - 1) / kGemmM;
-    const int limit = stall ? kStallPolls : 1 << 22;   // polls of a wait
+    constexpr int limit = STALL ? kStallPolls : 1 << 22;   // polls of a wait
     int it = 0, issued = 0;   // tiles begun; tiles handed to the tensor cores (thread 0)
     bool ok = true;
     if (wid < kRankBuilders / 32) {
@@ -539,7 +542,7 @@ k_mlp_rank(const float* __restrict__ U, const float* __restrict__ V, const int* 
             bool here = ok && mbar_wait_bounded(bar_mma(h), (it >> 1) & 1, err, limit);
             // test hook (bm_test_stall): CTA 0's first tile also waits for the
             // accumulator's next tile, which needs this one reduced first
-            if (here && stall && blockIdx.x == 0 && it == 0) here = mbar_wait_bounded(bar_mma(h), 1, err, limit);
+            if (here && STALL && blockIdx.x == 0 && it == 0) here = mbar_wait_bounded(bar_mma(h), 1, err, limit);
             ok = __all_sync(0xffffffffu, here);
             if (!ok) continue;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
