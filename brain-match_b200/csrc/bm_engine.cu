@@ -1148,7 +1148,7 @@ extern "C" bm_status bm_hillclimb(bm_ctx* ctx, int32_t max_sweeps, const bm_swee
 // Whether k_first_rows runs: its row, contributions and matchings fit a CTA's
 // shared memory, a 16-CTA cluster of them can be placed, and a row's terms
 // (which one CTA sums) are few enough to beat the grid's pairs.
-template <bool W16>
+template <bool W16, bool STALL>
 static bool first_rows_fit(bm_ctx* ctx, cudaLaunchConfig_t* cfg) {
     const size_t smem = first_rows_smem(ctx->n);
     const double terms = 4.0 * (double)ctx->e1 / ctx->n * (double)ctx->e2 / ctx->n;
@@ -1156,14 +1156,14 @@ static bool first_rows_fit(bm_ctx* ctx, cudaLaunchConfig_t* cfg) {
     cfg->dynamicSmemBytes = smem;
     int clusters = 0;
     const bool ok =
-        allow_smem<k_first_rows<W16>>(smem) == cudaSuccess &&
-        cudaFuncSetAttribute(k_first_rows<W16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&clusters, k_first_rows<W16>, cfg) == cudaSuccess && clusters > 0;
+        (allow_smem<k_first_rows<W16, STALL>>(smem)) == cudaSuccess &&
+        cudaFuncSetAttribute(k_first_rows<W16, STALL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, k_first_rows<W16, STALL>, cfg) == cudaSuccess && clusters > 0;
     cudaGetLastError();   // a refused attribute is not an error of the launches
     return ok;
 }
 
-template <bool W16>
+template <bool W16, bool STALL>
 static bm_status first_improvement_impl(bm_ctx* ctx, int max_passes, long long* commits, int* passes) {
     if (max_passes == 0) return BM_OK;
     const int n = ctx->n;
@@ -1178,13 +1178,13 @@ static bm_status first_improvement_impl(bm_ctx* ctx, int max_passes, long long* 
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const bool rows = first_rows_fit<W16>(ctx, &cfg);
+    const bool rows = first_rows_fit<W16, STALL>(ctx, &cfg);
     int grid = 0;
     const size_t smem = (size_t)n * sizeof(unsigned short);
     if (!rows) {
-        CK(allow_smem<k_first<W16>>(smem));
+        CK((allow_smem<k_first<W16, STALL>>(smem)));
         int per_sm = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_first<W16>, kFirstThreads, smem));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (k_first<W16, STALL>), kFirstThreads, smem));
         if (per_sm < 1) { set_err(ctx, "first-improvement kernel does not fit (n=%d)", n); return BM_E_INPUT; }
         // short lists are bound by the step's latency, which more CTAs lengthen
         // (n = 600: one CTA per SM 24.6, two 28.5 ms); long ones by the loads in flight
@@ -1193,8 +1193,10 @@ static bm_status first_improvement_impl(bm_ctx* ctx, int max_passes, long long* 
     // behind the state: the contributions of k_first_rows or the slots of k_first
     const size_t slot_bytes = 2 * (size_t)grid * sizeof(unsigned long long);
     static_assert(sizeof(FirstState) % sizeof(unsigned long long) == 0, "the slots follow the state");
-    if (!ctx->first)   // the path depends on the context alone
-        CK(dalloc(ctx, (char**)&ctx->first, sizeof(FirstState) + (rows ? (size_t)n * sizeof(int) : slot_bytes)));
+    if (!ctx->first) {   // either path, and every grid that fits the GPU
+        const size_t most = 2 * (size_t)ctx->num_sms * (2048 / kFirstThreads) * sizeof(unsigned long long);
+        CK(dalloc(ctx, (char**)&ctx->first, sizeof(FirstState) + std::max((size_t)n * sizeof(int), most)));
+    }
     CK(cudaMemsetAsync(ctx->first, 0, sizeof(FirstState), ctx->st));
     FirstState* st = static_cast<FirstState*>(ctx->first);
     unsigned long long* slots = reinterpret_cast<unsigned long long*>(st + 1);
@@ -1206,14 +1208,13 @@ static bm_status first_improvement_impl(bm_ctx* ctx, int max_passes, long long* 
         CK(cudaGetLastError());
     }
     FirstState h;
-    int stall = take_stall(BM_STALL_FIRST);
     do {
         if (rows) {
-            CK(cudaLaunchKernelEx(&cfg, k_first_rows<W16>, g, st, contrib, max_passes, stall));
+            CK(cudaLaunchKernelEx(&cfg, (k_first_rows<W16, STALL>), g, st, contrib, max_passes));
         } else {
             CK(cudaMemsetAsync(slots, 0, slot_bytes, ctx->st));   // a launch starts again at tag 1
-            void* args[] = {&g, &st, &slots, &max_passes, &stall};
-            CK(cudaLaunchCooperativeKernel((const void*)k_first<W16>, dim3(grid), dim3(kFirstThreads), args, smem, ctx->st));
+            void* args[] = {&g, &st, &slots, &max_passes};
+            CK(cudaLaunchCooperativeKernel((const void*)(k_first<W16, STALL>), dim3(grid), dim3(kFirstThreads), args, smem, ctx->st));
         }
         CK(cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, ctx->st));
         CK(cudaStreamSynchronize(ctx->st));
@@ -1235,8 +1236,10 @@ extern "C" bm_status bm_first_improvement(bm_ctx* ctx, int32_t max_passes, int64
     if (!ctx->mapped) { set_err(ctx, "bm_first_improvement: no mapping set"); return BM_E_STATE; }
     long long c = 0;
     int p = 0;
-    bm_status s = ctx->w16 ? first_improvement_impl<true>(ctx, max_passes, &c, &p)
-                           : first_improvement_impl<false>(ctx, max_passes, &c, &p);
+    const bool stall = max_passes && take_stall(BM_STALL_FIRST);
+    auto impl = ctx->w16 ? (stall ? first_improvement_impl<true, true> : first_improvement_impl<true, false>)
+                         : (stall ? first_improvement_impl<false, true> : first_improvement_impl<false, false>);
+    const bm_status s = impl(ctx, max_passes, &c, &p);
     if (commits) *commits = c;
     if (passes_done) *passes_done = p;
     return s;

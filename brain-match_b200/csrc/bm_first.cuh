@@ -48,7 +48,10 @@ constexpr int kRowsThreads = 1024;
 // (3,600) 79 / 85 ms, degree 60 (14,400) 118 / 93 ms, degree 130 203 / 102 ms.
 constexpr double kRowsTerms = 4096;
 constexpr int kFirstSteps = 1024;            // steps per launch (the host relaunches)
-constexpr unsigned kFirstPolls = 1u << 22;   // polls of one slot (seconds)
+// Polls of one slot (seconds).  The kernels' STALL forms (bm_test_stall) poll a
+// few thousand times, and their last CTA keeps its words to itself; they are
+// kernels of their own because a run-time switch took 0.3 to 1.3%.
+constexpr unsigned kFirstPolls = 1u << 22;
 constexpr unsigned long long kFirstNone = (1ull << 51) - 1;   // (place << 31 | delta) of no pair
 
 // The scan between launches; zero at the start.
@@ -59,9 +62,9 @@ struct FirstState {
     long long delta, commits;
 };
 
-template <bool W16>
+template <bool W16, bool STALL>
 __global__ void __launch_bounds__(kFirstThreads) k_first(DevView<W16> g, FirstState* __restrict__ st,
-                                                         unsigned long long* slots, int max_passes, int stall) {
+                                                         unsigned long long* slots, int max_passes) {
     constexpr int NWARP = kFirstThreads / 32;
     extern __shared__ unsigned short p16[];   // the matching; unmatched = n
     __shared__ unsigned long long s_red[NWARP];
@@ -72,7 +75,7 @@ __global__ void __launch_bounds__(kFirstThreads) k_first(DevView<W16> g, FirstSt
     const int G = gridDim.x, nw = G * NWARP;
     for (int v = tid; v < n; v += kFirstThreads) p16[v] = (unsigned short)g.p[v];
     if (tid == 0) s_ok = 1;
-    const unsigned polls = stall ? kStallPolls : kFirstPolls;   // stall (bm_test_stall): the last CTA keeps its words
+    constexpr unsigned polls = STALL ? kStallPolls : kFirstPolls;
     const int most = nw * kFirstMult;
     int want = kFirstMin;
     int m1 = st->m1, m2 = st->m2, in_pass = st->in_pass, passes = st->passes, done = 0;
@@ -114,7 +117,7 @@ __global__ void __launch_bounds__(kFirstThreads) k_first(DevView<W16> g, FirstSt
         if (wid == 0) {
             best = lane < NWARP ? s_red[lane] : kFirstNone;
             for (int o = 16; o; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-            if (lane == 0 && !(stall && blockIdx.x == G - 1))
+            if (lane == 0 && !(STALL && (int)blockIdx.x == G - 1))
                 asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(sl + blockIdx.x), "l"(tag | best) : "memory");
         }
         best = kFirstNone;
@@ -182,9 +185,9 @@ __host__ __device__ inline size_t first_rows_smem(int n) {
     return (2 * (size_t)n + 1) * sizeof(int) + 2 * ((size_t)n + 1) * sizeof(unsigned short);
 }
 
-template <bool W16>
+template <bool W16, bool STALL>
 __global__ void __launch_bounds__(kRowsThreads, 1) k_first_rows(DevView<W16> g, FirstState* __restrict__ st,
-                                                                int* __restrict__ Cg, int max_passes, int stall) {
+                                                                int* __restrict__ Cg, int max_passes) {
     typedef Ent<W16> EN;
     typedef typename EN::T E;
     constexpr int T = kRowsThreads, NWARP = T / 32;
@@ -205,7 +208,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_first_rows(DevView<W16> g, 
     if (tid == 0) s_ok = 1;
     if (tid < 2 * kRowsCluster) (&s_slot[0][0])[tid] = 0;
     const bool loops = g.offs[n] > 0;
-    const unsigned polls = stall ? kStallPolls : kFirstPolls;   // stall (bm_test_stall): the last CTA keeps its words
+    constexpr unsigned polls = STALL ? kStallPolls : kFirstPolls;
     int m1 = st->m1, m2 = st->m2, in_pass = st->in_pass, passes = st->passes, done = 0;
     long long delta = st->delta, commits = st->commits;
     int rows = 1, seen = 0;   // rows of this step; rows since the last commit
@@ -300,7 +303,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) k_first_rows(DevView<W16> g, 
         if (wid == 0) {
             best = lane < NWARP ? s_red[lane] : kFirstNone;
             for (int o = 16; o; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-            if (lane < kRowsCluster && !(stall && blockIdx.x == kRowsCluster - 1)) {
+            if (lane < kRowsCluster && !(STALL && (int)blockIdx.x == kRowsCluster - 1)) {
                 const uint32_t mine = (uint32_t)__cvta_generic_to_shared(&s_slot[par][blockIdx.x]);
                 uint32_t peer;
                 asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(mine), "r"(lane));
