@@ -329,7 +329,6 @@ extern "C" bm_status bm_create(bm_ctx** out, int32_t n, int64_t e1, const int32_
         CK(cudaEventCreate(&ctx->ev_hub));
         CK(dalloc(ctx, &ctx->hub_err, sizeof(int)));
         CK(cudaMemset(ctx->hub_err, 0, sizeof(int)));
-        std::vector<int> hub_list;
         if (!(flags & BM_FLAG_NO_HUB_GEMM)) {
             // hubs: G1 vertices of out-degree >= max(64, n/9), at most kHubMaxHubs,
             // topped up by the next-largest out-degrees to a multiple of 16 so the
@@ -351,7 +350,6 @@ extern "C" bm_status bm_create(bm_ctx** out, int32_t n, int64_t e1, const int32_
                     std::vector<unsigned char> flag(n, 0);
                     std::vector<int> hv(byd.begin(), byd.begin() + nh);
                     for (int v : hv) flag[v] = 1;
-                    hub_list = hv;
                     ctx->nh = nh;
                     ctx->hubK = nh * kHubT;
                     ctx->Mpad = (n + 2 * kGemmM - 1) / (2 * kGemmM) * (2 * kGemmM);  // whole 256-row tiles
@@ -368,30 +366,6 @@ extern "C" bm_status bm_create(bm_ctx** out, int32_t n, int64_t e1, const int32_
         CK(dalloc(ctx, &ctx->rowbest, n * sizeof(unsigned long long)));
         CK(dalloc(ctx, &ctx->ckeys, n * sizeof(unsigned long long)));
         CK(dalloc(ctx, &ctx->ckeys_sorted, n * sizeof(unsigned long long)));
-        {   // profit rows, heaviest first: the terms of a row, half on a random
-            // matching and half on one that matches degrees
-            const double mean = (double)ctx->e2 / n;
-            std::vector<char> hub(n, 0);
-            for (int v : hub_list) hub[v] = 1;
-            std::vector<std::pair<float, int>> w(n);
-            for (int a = 0; a < n; a++) {
-                double t = 0;
-                for (int i = g1o.off[a]; i < g1o.off[a + 1]; i++) {
-                    const int v = g1o.id[i];
-                    t += mean + (g1i.off[v + 1] - g1i.off[v]);
-                }
-                for (int i = g1i.off[a]; i < g1i.off[a + 1]; i++) {
-                    const int u = g1i.id[i];
-                    if (!hub[u]) t += mean + (g1o.off[u + 1] - g1o.off[u]);
-                }
-                w[a] = {(float)-t, a};
-            }
-            std::sort(w.begin(), w.end());
-            std::vector<int> order(n);
-            for (int a = 0; a < n; a++) order[a] = w[a].second;
-            CK(dalloc(ctx, &ctx->order, n * sizeof(int)));
-            CK(cudaMemcpy(ctx->order, order.data(), n * sizeof(int), cudaMemcpyHostToDevice));
-        }
         CK(dalloc(ctx, &ctx->small, 16 * sizeof(int)));
         CK(dalloc(ctx, &ctx->score_acc, sizeof(unsigned long long)));
         CK(dalloc(ctx, &ctx->cstats, sizeof(CommitStats)));
@@ -549,12 +523,44 @@ bm_status ensure_S(bm_ctx* ctx) {
     return BM_OK;
 }
 
+// ctx->ckeys[0, *count) sorted into ctx->ckeys_sorted, ~0 behind (with n >
+// kRankMax, ckeys holds ~0 behind its keys).
+static cudaError_t sort_keys(bm_ctx* ctx, const int* count) {
+    const int n = ctx->n;
+    if (n <= kRankMax) {
+        k_rank_sort<false><<<(n + 31) / 32, 256, 0, ctx->st>>>(ctx->ckeys, count, n, ctx->ckeys_sorted);
+        return cudaGetLastError();
+    }
+    size_t tb = ctx->cub_bytes;
+    return cub::DeviceRadixSort::SortKeys(ctx->cub_tmp, tb, ctx->ckeys, ctx->ckeys_sorted, n, 0, 64, ctx->st);
+}
+
+// The order in which k_profit takes the rows, made with a context's first profit
+// matrix: an engine that never builds one, and the instances of a batch, need
+// none.  (A loop over the edges and a sort on the host, for every engine, took 1
+// of 18 ms of creation at n = 3,001 and 6 of 130 at n = 8,192 / E = 1e6.)
+template <bool W16>
+static bm_status ensure_order(bm_ctx* ctx) {
+    if (ctx->order) return BM_OK;
+    const int n = ctx->n;
+    CK(dalloc(ctx, &ctx->order, n * sizeof(int)));
+    k_row_keys<W16><<<(n + 7) / 8, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->nh ? ctx->is_hub : nullptr,
+                                                      (float)ctx->e2 / n, ctx->ckeys, ctx->small + 1);
+    CK(cudaGetLastError());
+    CK(sort_keys(ctx, ctx->small + 1));
+    k_row_order<<<(n + 255) / 256, 256, 0, ctx->st>>>(ctx->ckeys_sorted, n, ctx->order);
+    CK(cudaGetLastError());
+    return BM_OK;
+}
+
 template <bool W16>
 bm_status stage_profit(bm_ctx* ctx) {
     typedef typename Ent<W16>::T E;
     DevView<W16> g = view<W16>(ctx);
     const int n = ctx->n;
     ctx->S_exact = false;
+    const bm_status so = ensure_order<W16>(ctx);
+    if (so) return so;
     RelabelLists<W16> rl = {};
     auto list = [&](int l, const void* in, void* out, const int* map, long long len) {
         rl.in[l] = (const E*)in; rl.out[l] = (E*)out; rl.map[l] = map; rl.len[l] = len;
@@ -822,18 +828,6 @@ static cudaError_t ensure_set(bm_ctx* ctx) {
     const size_t bytes = (kSetCtlInts + kSetBufInts + (size_t)ctx->n) * sizeof(int);
     const cudaError_t e = dalloc(ctx, &ctx->cset, bytes);
     return e != cudaSuccess ? e : cudaMemsetAsync(ctx->cset, 0, bytes, ctx->st);
-}
-
-// ctx->ckeys[0, *count) sorted into ctx->ckeys_sorted, ~0 behind (with n >
-// kRankMax, ckeys holds ~0 behind its keys).
-static cudaError_t sort_keys(bm_ctx* ctx, const int* count) {
-    const int n = ctx->n;
-    if (n <= kRankMax) {
-        k_rank_sort<false><<<(n + 31) / 32, 256, 0, ctx->st>>>(ctx->ckeys, count, n, ctx->ckeys_sorted);
-        return cudaGetLastError();
-    }
-    size_t tb = ctx->cub_bytes;
-    return cub::DeviceRadixSort::SortKeys(ctx->cub_tmp, tb, ctx->ckeys, ctx->ckeys_sorted, n, 0, 64, ctx->st);
 }
 
 template <bool W16, int K>

@@ -63,7 +63,7 @@ struct bm_ctx {
     int* S = nullptr;
     unsigned long long* rowbest = nullptr;
     unsigned long long *ckeys = nullptr, *ckeys_sorted = nullptr;
-    int* order = nullptr;          // profit rows, heaviest first
+    int* order = nullptr;          // profit rows, heaviest first (made with the first profit matrix)
     void* cub_tmp = nullptr;
     size_t cub_bytes = 0;
     int* small = nullptr;          // [0]=row counter [1]=ncand [2]=best delta

@@ -409,6 +409,42 @@ static __global__ void k_candidates(const unsigned long long* __restrict__ rowbe
     append_key(out != ~0ull, out, keys, ncand);
 }
 
+// Sort key of every profit row, heaviest first: (2^32 - 1 - terms) << 32 | row, a
+// warp per row.  The terms of a row are half those on a random matching (`mean`
+// G2 entries per G1 edge) and half those on one that matches degrees; in-edges
+// from hubs are the tensor cores'.  *count = n.
+template <bool W16>
+__global__ void __launch_bounds__(256) k_row_keys(DevView<W16> g, const unsigned char* __restrict__ is_hub, float mean,
+                                                  unsigned long long* __restrict__ keys, int* __restrict__ count) {
+    typedef Ent<W16> EN;
+    const int lane = threadIdx.x & 31, a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *count = g.n;
+    if (a >= g.n) return;
+    unsigned long long t = 0;   // entries of the lists the row's edges meet, and the edges
+    unsigned edges = 0;
+#pragma unroll 4
+    for (int i = g.off1o[a] + lane; i < g.off1o[a + 1]; i += 32) {
+        const int v = EN::id(g.ent1o[i]);
+        t += g.off1i[v + 1] - g.off1i[v];
+        edges++;
+    }
+#pragma unroll 4
+    for (int i = g.off1i[a] + lane; i < g.off1i[a + 1]; i += 32) {
+        const int u = EN::id(g.ent1i[i]);
+        if (is_hub && is_hub[u]) continue;
+        t += g.off1o[u + 1] - g.off1o[u];
+        edges++;
+    }
+    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    edges = __reduce_add_sync(0xffffffffu, edges);
+    t = min(t + (unsigned long long)(mean * edges), 0xffffffffull);
+    if (lane == 0) keys[a] = (0xffffffffull - t) << 32 | (unsigned)a;
+}
+static __global__ void k_row_order(const unsigned long long* __restrict__ keys, int n, int* __restrict__ order) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) order[i] = (int)(unsigned)keys[i];
+}
+
 // Sorts keys[0, *count) (distinct, or with DUP any) into sorted[0, *count) and
 // fills sorted[*count, n) with ~0: each key's place is the number of smaller
 // keys (equal ones by index), a warp counting for kRankKeys keys at once.  Quadratic, but one launch that
