@@ -506,7 +506,7 @@ extern "C" bm_status bm_mlp_set_params(bm_mlp* M, const float* params) {
 template <int BN>
 static bm_status gemm(bm_mlp* M, const __nv_bfloat16* A, const __nv_bfloat16* B, int m, int n, int k, const GemmOut& o) {
     MK(cudaFuncSetAttribute(k_gemm_bf16<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_bf16_smem<BN>()));
-    k_gemm_bf16<BN><<<dim3(n / BN, m / kGemmM), kGemmThreads, gemm_bf16_smem<BN>(), M->cs>>>(
+    k_gemm_bf16<BN><<<n / BN * (m / kGemmM), kGemmThreads, gemm_bf16_smem<BN>(), M->cs>>>(
         A, B, m, n, k, o, M->err_d, take_stall(BM_STALL_MLP_GEMM));
     MK(cudaGetLastError());
     return BM_OK;

@@ -27,7 +27,8 @@ struct GemmOut {
     __nv_bfloat16* CbT = nullptr;     // N x M bf16, transposed
 };
 
-// M % 128 == 0, N % BN == 0, K % 64 == 0; grid (N / BN, M / 128).
+// M % 128 == 0, N % BN == 0, K % 64 == 0; N / BN * M / 128 CTAs along x (the
+// other dimensions end at 65,535), a row tile's columns side by side.
 // The network's GEMMs are small (1,024 x 256 x 256 for a training batch), so a
 // launch is bound by its latency and by how many SMs it uses: 64 columns per
 // CTA (32 CTAs per batch instead of 8 with whole rows), the four K-chunks of a
@@ -50,7 +51,7 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
     const uint32_t tslot = bars + 8 * kMlpStages;
     uint32_t* tslot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tslot - raw));
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
-    const int b0 = blockIdx.x * BN, a0 = blockIdx.y * kGemmM;
+    const int cols = N / BN, b0 = (blockIdx.x % cols) * BN, a0 = (blockIdx.x / cols) * kGemmM;
     const int KB = K * 2;                        // bytes per row
     const int KC = KB / kGemmKC;                 // 128-byte chunks
     const uint8_t* Ab = reinterpret_cast<const uint8_t*>(A);
@@ -123,7 +124,7 @@ k_gemm_bf16(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict
         const int last = KC - 1;
         ok = ok && mbar_wait_bounded(bars + 8 * (last % kMlpStages), (last / kMlpStages) & 1, err);
         // test hook (bm_test_stall): the barrier's next phase never completes
-        if (stall && blockIdx.x == 0 && blockIdx.y == 0)
+        if (stall && blockIdx.x == 0)
             ok = ok && mbar_wait_bounded(bars + 8 * (last % kMlpStages), ((last / kMlpStages) + 1) & 1, err,
                                          kStallPolls);
     }
