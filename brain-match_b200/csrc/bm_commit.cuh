@@ -40,7 +40,6 @@ constexpr int kSetThreads = 1024;
 // memory at every n.  256 took 16 steps of 45 us at n = 18,524 / E = 5e6 where
 // 128 take 29 of 20 us (more dead sets scanned, a longer decision).
 constexpr int kSetW = 128, kSetWords = kSetW / 32;
-constexpr int kCommitMaxCtas = 8;         // bm_sweep_opts.commit_ctas
 constexpr unsigned kSetPolls = 1u << 22;    // polls of one wait (seconds)
 constexpr unsigned kSetAbort = 0xffffffffu;
 

@@ -847,13 +847,12 @@ bm_status launch_set_commit(bm_ctx* ctx, const unsigned long long* keys, const i
     // windows of hub pairs scan several times the average, and the grid
     // barrier of 148 CTAs costs about 1 us more than that of 8 (n = 1,000 /
     // E = 2e4: 16, 64 and 148 CTAs 113, 107 and 109 us; n = 18,524 / E = 5e6:
-    // 1,188, 682 and 627 us)
-    int grid = ctas;
-    if (grid <= 0) {
-        const double per_step = 2.0 * (double)ctx->e1 / n * K * kSetW;
-        grid = (int)std::min<double>(ctx->num_sms, std::max(8.0, per_step / 256));
-    }
-    grid = std::min(grid, ctx->num_sms);
+    // 1,188, 682 and 627 us).  Fewer than 8 are slower at every size (the first
+    // sweep of the same two pairs with 1, 2 and 8 CTAs: 292, 189 and 112 us; 5.7,
+    // 3.0 and 1.0 ms; 97 us and 0.26 ms by this rule).
+    const double per_step = 2.0 * (double)ctx->e1 / n * K * kSetW;
+    int grid = (int)std::min<double>(ctx->num_sms, std::max(8.0, per_step / 256));
+    grid = std::min(std::max(grid, ctas), ctx->num_sms);
     const size_t smem = SetSmem<K>::bytes(n);
     CK((allow_smem<k_commit_sets<W16, K>>(smem)));
     DevView<W16> g = view<W16>(ctx);
@@ -896,9 +895,8 @@ static bm_status stage_commit(bm_ctx* ctx, const bm_sweep_opts* o) {
                 smem, n, ctx->smem_optin);
         return BM_E_INPUT;
     }
-    const int ctas = o && o->commit_ctas > 0 ? std::min(o->commit_ctas, kCommitMaxCtas) : 0;
-    return launch_set_commit<W16, 2>(ctx, ctx->ckeys_sorted, nullptr, lim, max_verify, ctas,
-                                     ctas != 1 ? take_stall(BM_STALL_COMMIT) : 0, true);
+    return launch_set_commit<W16, 2>(ctx, ctx->ckeys_sorted, nullptr, lim, max_verify, o ? o->commit_ctas : 0,
+                                     take_stall(BM_STALL_COMMIT), true);
 }
 
 extern "C" bm_status bm_all_deltas(bm_ctx* ctx, int32_t* out) {

@@ -166,7 +166,7 @@ bm_status stage_combine(bm_ctx* ctx, int* all_out);
 bm_status decode_mapping(bm_ctx* ctx, const int32_t* map, int* p, int* pinv);
 // Enqueues the set commit of the first lim sorted candidate keys (K = 2: pairs
 // in the keys; K = 3, 4: the sets in `sets`) on ctx's stream; statistics go to
-// ctx->cstats.  ctas <= 0: as many CTAs as the window's lists need; ctl_clear:
+// ctx->cstats.  ctas: fewest CTAs, more where the window's lists need them; ctl_clear:
 // an earlier kernel cleared the control words (ctx->cset).
 template <bool W16, int K>
 bm_status launch_set_commit(bm_ctx* ctx, const unsigned long long* keys, const int4* sets, int lim, int max_verify,

@@ -171,9 +171,9 @@ bm_status bm_profit_row(bm_ctx* ctx, int32_t a, int32_t* out);
 typedef struct {
     int32_t max_candidates;  /* sorted candidates scanned per sweep (<=0: all)   */
     int32_t max_verify;      /* re-verifications of tainted candidates (<0: all) */
-    int32_t commit_ctas;     /* CTAs (one thread-block cluster) sharing the set
-                                commit's list scans: 0 = default (8), 1..8;
-                                results never depend on it                      */
+    int32_t commit_ctas;     /* fewest CTAs sharing the set commit's list scans
+                                (<=0: 8); it takes more, up to one per SM, where
+                                the lists are long; results never depend on it   */
     int32_t incremental;     /* 1: keep the profit matrix exact across sweeps and
                                 update it from the vertices the last commit moved
                                 when that is cheaper than a rebuild; results never
@@ -203,7 +203,8 @@ typedef struct {
                                    list entries applied by an update       */
     int64_t commit_entries;     /* edge-list entries read by the commit   */
     int32_t commit_steps;       /* commit steps (pairs decided per step)  */
-    int32_t commit_carried;     /* pairs carried into a later step        */
+    int32_t commit_carried;     /* 0: every pair is decided in the step
+                                   that scans it                          */
 } bm_sweep_stats;
 
 /*
