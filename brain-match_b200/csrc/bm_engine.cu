@@ -400,7 +400,7 @@ extern "C" bm_status bm_get_info(const bm_ctx* ctx, bm_info* info) {
 // ---------------------------------------------------------------------------
 static bm_status compute_score(bm_ctx* ctx, long long* out) {
     CK(cudaMemsetAsync(ctx->score_acc, 0, sizeof(unsigned long long), ctx->st));
-    const int blocks = (int)std::min<long long>(ctx->num_sms * 8LL, ctx->e1 / (8 * kScoreRun) + 1);
+    const int blocks = score_blocks(ctx->e1, ctx->num_sms * 8);
     if (ctx->w16) k_score<true><<<blocks, 256, 0, ctx->st>>>(view<true>(ctx), (int)ctx->e1, ctx->score_acc);
     else k_score<false><<<blocks, 256, 0, ctx->st>>>(view<false>(ctx), (int)ctx->e1, ctx->score_acc);
     CK(cudaGetLastError());
@@ -1195,7 +1195,7 @@ static bm_status first_improvement_impl(bm_ctx* ctx, int max_passes, long long* 
     int* contrib = reinterpret_cast<int*>(st + 1);
     if (rows) {
         CK(cudaMemsetAsync(contrib, 0, (size_t)n * sizeof(int), ctx->st));
-        k_contrib<W16><<<(int)std::min<long long>(ctx->num_sms * 8LL, ctx->e1 / (8 * kScoreRun) + 1), 256, 0, ctx->st>>>(
+        k_contrib<W16><<<score_blocks(ctx->e1, ctx->num_sms * 8), 256, 0, ctx->st>>>(
             g, (int)ctx->e1, contrib);
         CK(cudaGetLastError());
     }

@@ -569,10 +569,31 @@ __device__ __forceinline__ int row_of(const int* __restrict__ off, int n, int i)
     return lo;
 }
 
-// Alignment score (src/graph-alignment-optimized.c:292-307).  A warp takes
-// kScoreRun consecutive G1 entries, whatever their rows: with a warp per row
-// the power-law rows' longest held the launch (54 us at n = 8,192 / E = 1e6).
+// The same, one i for a warp: its lanes try 32 rows at once, so n = 1,000 takes two
+// dependent loads instead of ten.
+__device__ __forceinline__ int row_of_warp(const int* __restrict__ off, int n, int i, int lane) {
+    int lo = 0, hi = n;   // off[lo] <= i < off[hi]
+    while (hi - lo > 1) {
+        const int step = (hi - lo + 32) / 33, x = lo + (lane + 1) * step;
+        lo += step * __popc(__ballot_sync(0xffffffffu, x < hi && off[x] <= i));
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
+// Alignment score (src/graph-alignment-optimized.c:292-307).  A warp takes a run of
+// consecutive G1 entries, whatever their rows: with a warp per row the
+// power-law rows' longest held the launch (54 us at n = 8,192 / E = 1e6).  Runs
+// of 128 entries, or of 32 where that leaves warps without one (each entry's row
+// is walked to from the run's first: n = 500 / E = 7,500, 23.3 us a call with a binary
+// search and runs of 128, 20.2 with a warp per row, now 19.4).
 constexpr int kScoreRun = 128;
+__host__ __device__ __forceinline__ int score_blocks(long long m, int most) {   // of 256 threads
+    return m / 256 + 1 < most ? (int)(m / 256 + 1) : most;
+}
+__device__ __forceinline__ int score_run(int m, int nwarps) {
+    return min(kScoreRun, (m / nwarps + 32) & ~31);
+}
 template <bool W16>
 __device__ __forceinline__ void add_score(const DevView<W16>& g, int m, unsigned long long* __restrict__ out) {
     typedef Ent<W16> EN;
@@ -580,9 +601,10 @@ __device__ __forceinline__ void add_score(const DevView<W16>& g, int m, unsigned
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     long long s = 0;
-    for (long long r0 = (long long)warp * kScoreRun; r0 < m; r0 += (long long)nwarps * kScoreRun) {
-        int a = row_of(g.off1o, g.n, (int)r0), end = g.off1o[a + 1];
-        const int r1 = (int)min((long long)m, r0 + kScoreRun);
+    const int run = score_run(m, nwarps);
+    for (long long r0 = (long long)warp * run; r0 < m; r0 += (long long)nwarps * run) {
+        int a = row_of_warp(g.off1o, g.n, (int)r0, lane), end = g.off1o[a + 1];
+        const int r1 = (int)min((long long)m, r0 + run);
 #pragma unroll
         for (int u = 0; u < kScoreRun / 32; u++) {
             const int i = (int)r0 + 32 * u + lane;
@@ -610,9 +632,10 @@ __global__ void k_contrib(DevView<W16> g, int m, int* __restrict__ C) {
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (long long r0 = (long long)warp * kScoreRun; r0 < m; r0 += (long long)nwarps * kScoreRun) {
-        int a = row_of(g.off1o, g.n, (int)r0), end = g.off1o[a + 1];
-        const int r1 = (int)min((long long)m, r0 + kScoreRun);
+    const int run = score_run(m, nwarps);
+    for (long long r0 = (long long)warp * run; r0 < m; r0 += (long long)nwarps * run) {
+        int a = row_of_warp(g.off1o, g.n, (int)r0, lane), end = g.off1o[a + 1];
+        const int r1 = (int)min((long long)m, r0 + run);
 #pragma unroll
         for (int u = 0; u < kScoreRun / 32; u++) {
             const int i = (int)r0 + 32 * u + lane;

@@ -640,7 +640,7 @@ static bm_status features(bm_ctx* ctx, bm_mlp* M) {
     MK(cudaMemcpyAsync(M->F1.p, M->S1.p, fbytes, cudaMemcpyDeviceToDevice, M->cs));
     MK(cudaMemcpyAsync(M->F2.p, M->S2.p, fbytes, cudaMemcpyDeviceToDevice, M->cs));
     MK(cudaMemsetAsync(M->contrib.p, 0, (size_t)n * sizeof(int), M->cs));
-    k_contrib<W16><<<(int)std::min<long long>(ctx->num_sms * 8LL, ctx->e1 / (8 * kScoreRun) + 1), 256, 0, M->cs>>>(
+    k_contrib<W16><<<score_blocks(ctx->e1, ctx->num_sms * 8), 256, 0, M->cs>>>(
         g, (int)ctx->e1, M->contrib.as<int>());
     k_dyn_features<<<(n + 255) / 256, 256, 0, M->cs>>>(M->contrib.as<int>(), ctx->pinv, n, M->F1.as<float>(),
                                                        M->F2.as<float>());
