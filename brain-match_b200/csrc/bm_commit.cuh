@@ -43,13 +43,6 @@ constexpr int kSetW = 128, kSetWords = kSetW / 32;
 constexpr unsigned kSetPolls = 1u << 22;    // polls of one wait (seconds)
 constexpr unsigned kSetAbort = 0xffffffffu;
 
-// Control words of a launch, zeroed before it.
-struct SetCtl {
-    unsigned arrived;    // arrivals of the CTAs, all steps
-    unsigned released;   // steps decided so far, or kSetAbort
-    int err;             // bit 1: a wait ran out
-};
-
 // Step results in global memory, two copies by step parity; zero between uses.
 struct SetBuf {
     static constexpr int W = kSetW, kWords = kSetWords;

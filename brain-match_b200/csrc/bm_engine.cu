@@ -166,7 +166,7 @@ static void free_ctx(bm_ctx* c) {
     void* bufs[] = {c->off1o, c->off1i, c->off2o, c->off2i, c->offs, c->selfw, c->ent1o, c->ent1i,
                     c->ent2o, c->ent2i, c->ent1oP, c->ent1iP, c->ent2oP, c->ent2iP, c->W2, c->p,
                     c->pinv, c->S, c->rowbest, c->ckeys, c->ckeys_sorted, 
-                    c->order, c->cub_tmp, c->small, c->score_acc, c->cstats, c->scratch_pairs,
+                    c->order, c->cub_tmp, c->small, c->score_acc, c->scratch_pairs,
                     c->adj, c->first, c->fi_acc, c->tcount};
     for (void* b : bufs) if (b) cudaFree(b);
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);
@@ -368,7 +368,6 @@ extern "C" bm_status bm_create(bm_ctx** out, int32_t n, int64_t e1, const int32_
         CK(dalloc(ctx, &ctx->ckeys_sorted, n * sizeof(unsigned long long)));
         CK(dalloc(ctx, &ctx->small, 16 * sizeof(int)));
         CK(dalloc(ctx, &ctx->score_acc, sizeof(unsigned long long)));
-        CK(dalloc(ctx, &ctx->cstats, sizeof(CommitStats)));
         size_t b1 = 0;
         CK(cub::DeviceRadixSort::SortKeys(nullptr, b1, ctx->ckeys, ctx->ckeys_sorted, n));
         ctx->cub_bytes = b1;
@@ -825,8 +824,8 @@ static bm_status ensure_adj(bm_ctx* ctx) {
 // The set commit's control words, step results (zero between launches) and images.
 static cudaError_t ensure_set(bm_ctx* ctx) {
     if (ctx->cset) return cudaSuccess;
-    const size_t bytes = (kSetCtlInts + kSetBufInts + (size_t)ctx->n) * sizeof(int);
-    const cudaError_t e = dalloc(ctx, &ctx->cset, bytes);
+    const size_t bytes = sizeof(SetResult) + (kSetBufInts + (size_t)ctx->n) * sizeof(int);
+    const cudaError_t e = dalloc(ctx, (char**)&ctx->cset, bytes);
     return e != cudaSuccess ? e : cudaMemsetAsync(ctx->cset, 0, bytes, ctx->st);
 }
 
@@ -834,13 +833,12 @@ template <bool W16, int K>
 bm_status launch_set_commit(bm_ctx* ctx, const unsigned long long* keys, const int4* sets, int lim, int max_verify,
                             int ctas, int stall, bool ctl_clear) {
     const int n = ctx->n;
-    static_assert(sizeof(SetCtl) <= kSetCtlInts * sizeof(int), "control words");
     CK(ensure_set(ctx));
-    if (!ctl_clear) CK(cudaMemsetAsync(ctx->cset, 0, kSetCtlInts * sizeof(int), ctx->st));
+    if (!ctl_clear) CK(cudaMemsetAsync(&ctx->cset->ctl, 0, sizeof(SetCtl), ctx->st));
     SetArgs a;
-    a.keys = keys; a.sets = sets; a.lim = lim; a.max_verify = max_verify; a.st = ctx->cstats;
-    a.ctl = reinterpret_cast<SetCtl*>(ctx->cset);
-    a.buf = ctx->cset + kSetCtlInts;
+    a.keys = keys; a.sets = sets; a.lim = lim; a.max_verify = max_verify; a.st = &ctx->cset->st;
+    a.ctl = &ctx->cset->ctl;
+    a.buf = reinterpret_cast<int*>(ctx->cset + 1);
     a.newp = a.buf + kSetBufInts;
     a.stall = stall;
     // a quarter of the list entries a step scans on average per CTA's thread:
@@ -869,10 +867,8 @@ template bm_status launch_set_commit<false, 3>(bm_ctx*, const unsigned long long
 template bm_status launch_set_commit<true, 4>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int, bool);
 template bm_status launch_set_commit<false, 4>(bm_ctx*, const unsigned long long*, const int4*, int, int, int, int, bool);
 
-const int* set_commit_err(bm_ctx* ctx) { return &reinterpret_cast<SetCtl*>(ctx->cset)->err; }
-
 bm_status set_commit_reset(bm_ctx* ctx) {
-    CK(cudaMemsetAsync(ctx->cset, 0, (kSetCtlInts + kSetBufInts) * sizeof(int), ctx->st));
+    CK(cudaMemsetAsync(ctx->cset, 0, sizeof(SetResult) + kSetBufInts * sizeof(int), ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
     return BM_OK;
 }
@@ -883,7 +879,7 @@ static bm_status stage_commit(bm_ctx* ctx, const bm_sweep_opts* o) {
     CK(ensure_set(ctx));
     if (n > kRankMax) CK(cudaMemsetAsync(ctx->ckeys, 0xff, n * sizeof(unsigned long long), ctx->st));
     k_candidates<<<(n + 255) / 256, 256, 0, ctx->st>>>(ctx->rowbest, n, ctx->ckeys, ctx->small + 1, ctx->small + 2,
-                                                       ctx->cset);
+                                                       &ctx->cset->ctl);
     CK(cudaGetLastError());
     CK(sort_keys(ctx, ctx->small + 1));
     const int max_scan = o ? o->max_candidates : 0;
@@ -951,16 +947,17 @@ extern "C" bm_status bm_sweep(bm_ctx* ctx, const bm_sweep_opts* opts, bm_sweep_s
     s = ctx->w16 ? stage_commit<true>(ctx, opts) : stage_commit<false>(ctx, opts);
     if (s) return s;
     CK(cudaEventRecord(ctx->ev[3], ctx->st));
-    CommitStats cs;
+    SetResult res;
     int small[3];
     unsigned long long terms = 0;
-    int herr = 0, cerr = 0;
-    CK(cudaMemcpyAsync(&cs, ctx->cstats, sizeof cs, cudaMemcpyDeviceToHost, ctx->st));
+    int herr = 0;
+    CK(cudaMemcpyAsync(&res, ctx->cset, sizeof res, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(small, ctx->small, 3 * sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(&terms, ctx->work_sum, sizeof terms, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(&herr, ctx->hub_err, sizeof herr, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(&cerr, set_commit_err(ctx), sizeof cerr, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
+    const CommitStats& cs = res.st;
+    const int cerr = res.ctl.err;
     if (herr || cerr) {
         // the matching may be partly committed and S is not trusted: the
         // caller sets a matching again before the next call
@@ -1287,7 +1284,7 @@ static bm_status triple_round_impl(bm_ctx* ctx, const bm_triple_opts* o, bm_trip
     if (s) return s;
     s = ensure_adj<W16>(ctx);
     if (s) return s;
-    if (!ctx->tcount) CK(dalloc(ctx, &ctx->tcount, 2 * sizeof(unsigned long long)));
+    if (!ctx->tcount) CK(dalloc(ctx, &ctx->tcount, 3 * sizeof(unsigned long long)));
     const long long before = ctx->score;
     CK(cudaEventRecord(ctx->ev[0], ctx->st));
     int mode = 0;
@@ -1303,21 +1300,21 @@ static bm_status triple_round_impl(bm_ctx* ctx, const bm_triple_opts* o, bm_trip
     CK(cudaEventRecord(ctx->ev[2], ctx->st));
     CK(sort_keys(ctx, reinterpret_cast<int*>(ctx->tcount + 1)));
     if (!ctx->csets) CK(dalloc(ctx, &ctx->csets, (size_t)n * sizeof(int4)));
-    k_triple_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets);
+    CK(ensure_set(ctx));
+    k_triple_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets,
+                                                             ctx->tcount + 2, &ctx->cset->ctl);
     CK(cudaGetLastError());
     const int lim = o->max_candidates > 0 ? std::min(o->max_candidates, n) : n;
     if ((s = launch_set_commit<W16, 3>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0,
-                                       take_stall(BM_STALL_COMMIT), false))) return s;
+                                       take_stall(BM_STALL_COMMIT), true))) return s;
     CK(cudaEventRecord(ctx->ev[3], ctx->st));
-    CommitStats cs;
-    unsigned long long cnt[2], top = 0;
-    int cerr = 0;
-    CK(cudaMemcpyAsync(&cs, ctx->cstats, sizeof cs, cudaMemcpyDeviceToHost, ctx->st));
+    SetResult res;
+    unsigned long long cnt[3];
+    CK(cudaMemcpyAsync(&res, ctx->cset, sizeof res, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(cnt, ctx->tcount, sizeof cnt, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(&top, ctx->ckeys_sorted, sizeof top, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(&cerr, set_commit_err(ctx), sizeof cerr, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
-    if (cerr) return set_commit_timeout(ctx, "bm_triple_round");
+    const CommitStats& cs = res.st;
+    if (res.ctl.err) return set_commit_timeout(ctx, "bm_triple_round");
     ctx->score = before + cs.total_delta;
     if (stats) {
         memset(stats, 0, sizeof *stats);
@@ -1326,7 +1323,7 @@ static bm_status triple_round_impl(bm_ctx* ctx, const bm_triple_opts* o, bm_trip
         stats->triples = (long long)cnt[0];
         stats->rotations = 2 * (long long)cnt[0];
         stats->candidates = (int32_t)cnt[1];
-        stats->best_delta = cnt[1] ? (int)(0x7fffffffu - (unsigned)(top >> 32)) : 0;
+        stats->best_delta = cnt[1] ? (int)(0x7fffffffu - (unsigned)(cnt[2] >> 32)) : 0;
         stats->scanned = cs.scanned;
         stats->verified = cs.verified;
         stats->committed = cs.committed;
@@ -1389,7 +1386,7 @@ static bm_status quad_round_impl(bm_ctx* ctx, const bm_quad_opts* o, bm_quad_sta
     if (s) return s;
     s = ensure_adj<W16>(ctx);
     if (s) return s;
-    if (!ctx->tcount) CK(dalloc(ctx, &ctx->tcount, 2 * sizeof(unsigned long long)));
+    if (!ctx->tcount) CK(dalloc(ctx, &ctx->tcount, 3 * sizeof(unsigned long long)));
     const long long before = ctx->score;
     CK(cudaEventRecord(ctx->ev[0], ctx->st));
     int mode = 0;
@@ -1405,21 +1402,21 @@ static bm_status quad_round_impl(bm_ctx* ctx, const bm_quad_opts* o, bm_quad_sta
     CK(cudaEventRecord(ctx->ev[2], ctx->st));
     CK(sort_keys(ctx, reinterpret_cast<int*>(ctx->tcount + 1)));
     if (!ctx->csets) CK(dalloc(ctx, &ctx->csets, (size_t)n * sizeof(int4)));
-    k_quad_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets);
+    CK(ensure_set(ctx));
+    k_quad_sets<W16><<<(n + 255) / 256, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->ckeys_sorted, o->seed, ctx->csets,
+                                                           ctx->tcount + 2, &ctx->cset->ctl);
     CK(cudaGetLastError());
     const int lim = o->max_candidates > 0 ? std::min(o->max_candidates, n) : n;
     if ((s = launch_set_commit<W16, 4>(ctx, ctx->ckeys_sorted, ctx->csets, lim, o->max_verify, 0,
-                                       take_stall(BM_STALL_COMMIT), false))) return s;
+                                       take_stall(BM_STALL_COMMIT), true))) return s;
     CK(cudaEventRecord(ctx->ev[3], ctx->st));
-    CommitStats cs;
-    unsigned long long cnt[2], top = 0;
-    int cerr = 0;
-    CK(cudaMemcpyAsync(&cs, ctx->cstats, sizeof cs, cudaMemcpyDeviceToHost, ctx->st));
+    SetResult res;
+    unsigned long long cnt[3];
+    CK(cudaMemcpyAsync(&res, ctx->cset, sizeof res, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemcpyAsync(cnt, ctx->tcount, sizeof cnt, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(&top, ctx->ckeys_sorted, sizeof top, cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaMemcpyAsync(&cerr, set_commit_err(ctx), sizeof cerr, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
-    if (cerr) return set_commit_timeout(ctx, "bm_quad_round");
+    const CommitStats& cs = res.st;
+    if (res.ctl.err) return set_commit_timeout(ctx, "bm_quad_round");
     ctx->score = before + cs.total_delta;
     if (stats) {
         memset(stats, 0, sizeof *stats);
@@ -1428,7 +1425,7 @@ static bm_status quad_round_impl(bm_ctx* ctx, const bm_quad_opts* o, bm_quad_sta
         stats->quads = (long long)cnt[0];
         stats->permutations = 23 * (long long)cnt[0];
         stats->candidates = (int32_t)cnt[1];
-        stats->best_delta = cnt[1] ? (int)(0x7fffffffu - (unsigned)(top >> 32)) : 0;
+        stats->best_delta = cnt[1] ? (int)(0x7fffffffu - (unsigned)(cnt[2] >> 32)) : 0;
         stats->scanned = cs.scanned;
         stats->verified = cs.verified;
         stats->committed = cs.committed;

@@ -68,8 +68,7 @@ struct bm_ctx {
     size_t cub_bytes = 0;
     int* small = nullptr;          // [0]=row counter [1]=ncand [2]=best delta
     unsigned long long* score_acc = nullptr;
-    CommitStats* cstats = nullptr;
-    int* cset = nullptr;    // set commit: control words, step results, images of moved vertices
+    SetResult* cset = nullptr;   // set commit: control words and statistics, then step results and images of moved vertices
     int4* csets = nullptr;  // vertices and permutations of the sorted 3- and 4-set candidates
     // S kept exact across commits: the matching it is exact for, and the moved-vertex update
     bool S_exact = false;
@@ -166,12 +165,10 @@ bm_status stage_combine(bm_ctx* ctx, int* all_out);
 bm_status decode_mapping(bm_ctx* ctx, const int32_t* map, int* p, int* pinv);
 // Enqueues the set commit of the first lim sorted candidate keys (K = 2: pairs
 // in the keys; K = 3, 4: the sets in `sets`) on ctx's stream; statistics go to
-// ctx->cstats.  ctas: fewest CTAs, more where the window's lists need them; ctl_clear:
-// an earlier kernel cleared the control words (ctx->cset).
+// ctx->cset.  ctas: fewest CTAs, more where the window's lists need them; ctl_clear:
+// an earlier kernel cleared the control words.
 template <bool W16, int K>
 bm_status launch_set_commit(bm_ctx* ctx, const unsigned long long* keys, const int4* sets, int lim, int max_verify,
                             int ctas, int stall, bool ctl_clear = false);
-// Error word of the last set commit (device), and the clean-up after a wait of
-// it ran out.
-const int* set_commit_err(bm_ctx* ctx);
+// The clean-up after a wait of the last set commit ran out.
 bm_status set_commit_reset(bm_ctx* ctx);

@@ -377,16 +377,36 @@ __device__ __forceinline__ void append_key(bool has, unsigned long long key, uns
     if (has) keys[at + __popc(m & ((1u << lane) - 1u))] = key;
 }
 
+// Counters reported by the commit kernels.
+struct CommitStats {
+    long long total_delta;
+    int scanned, verified, committed, steps;
+    long long entries;
+    int carried, pad;
+};
+
+// Control words of a set commit, zeroed before it.
+struct SetCtl {
+    unsigned arrived;    // arrivals of the CTAs, all steps
+    unsigned released;   // steps decided so far, or kSetAbort
+    int err;             // bit 1: a wait ran out
+    int pad;
+};
+// What the host reads after it, in one copy.
+struct alignas(16) SetResult {
+    SetCtl ctl;
+    CommitStats st;
+};
+
 // Candidate keys: one per row whose best partner improves, deduplicated when
 // two rows pick each other.  Sort key: (0x7fffffff - delta) << 32 | lo << 16 | hi
-// -> ascending order = delta desc, lo asc, hi asc.  ctl: kSetCtlInts words of
-// the set commit that follows, cleared here.
-constexpr int kSetCtlInts = 4;
+// -> ascending order = delta desc, lo asc, hi asc.  ctl: of the set commit that
+// follows, cleared here.
 static __global__ void k_candidates(const unsigned long long* __restrict__ rowbest, int n,
                              unsigned long long* __restrict__ keys, int* __restrict__ ncand,
-                             int* __restrict__ best_delta, int* __restrict__ ctl) {
+                             int* __restrict__ best_delta, SetCtl* __restrict__ ctl) {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a < kSetCtlInts) ctl[a] = 0;
+    if (a == 0) *ctl = SetCtl{};
     const unsigned long long k = a < n ? rowbest[a] : 0ull;
     unsigned long long out = ~0ull;
     int d = 0;
@@ -653,13 +673,5 @@ __global__ void k_contrib(DevView<W16> g, int m, int* __restrict__ C) {
     }
 }
 
-// ---------------------------------------------------------------------------
-// Counters reported by the commit kernels.
-struct CommitStats {
-    long long total_delta;
-    int scanned, verified, committed, steps;
-    long long entries;
-    int carried, pad;
-};
 
 }  // namespace bm

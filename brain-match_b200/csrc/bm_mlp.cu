@@ -905,17 +905,17 @@ static bm_status learned_impl(bm_ctx* ctx, bm_mlp* M, const bm_learned_opts* o, 
             snprintf(M->err, sizeof M->err, "%s", ctx->err);
             return r;
         }
-        MK(cudaMemcpyAsync(&cs, ctx->cstats, sizeof cs, cudaMemcpyDeviceToHost, M->cs));
-        int cerr = 0;
-        MK(cudaMemcpyAsync(&cerr, set_commit_err(ctx), sizeof cerr, cudaMemcpyDeviceToHost, M->cs));
+        SetResult res;
+        MK(cudaMemcpyAsync(&res, ctx->cset, sizeof res, cudaMemcpyDeviceToHost, M->cs));
         MK(cudaEventRecord(M->e1, M->cs));
         r = check_err(M);
-        if (r || cerr) {
+        cs = res.st;
+        if (r || res.ctl.err) {
             // the commit has run on what the ranking gave, or stopped in part: the
             // caller sets a matching again before the next call
             ctx->mapped = false;
             ctx->S_exact = false;
-            if (cerr) {
+            if (res.ctl.err) {
                 const bm_status rs = set_commit_reset(ctx);
                 if (!r) {
                     snprintf(M->err, sizeof M->err, "%s", rs ? ctx->err : "set commit wait timed out");

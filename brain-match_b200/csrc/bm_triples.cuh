@@ -228,12 +228,14 @@ k_triple_eval(DevView<W16> g, const unsigned* __restrict__ adj, int words, int p
     }
 }
 
-// The sets of the sorted 3-cycle candidates for the set commit (SetArgs::sets).
+// The sets of the sorted 3-cycle candidates for the set commit (SetArgs::sets),
+// the first key for the host, and the commit's control words cleared.
 template <bool W16>
 __global__ void k_triple_sets(DevView<W16> g, const unsigned long long* __restrict__ keys, unsigned long long seed,
-                              int4* __restrict__ sets) {
+                              int4* __restrict__ sets, unsigned long long* __restrict__ top, SetCtl* __restrict__ ctl) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned long long key = i < g.n ? keys[i] : ~0ull;
+    if (i == 0) { *top = key; *ctl = SetCtl{}; }
     if (key == ~0ull) return;
     const int a = (int)((key >> 16) & 0xffffu), j = (int)((key >> 1) & 0x7fffu);
     int b = 0, c = 0;
