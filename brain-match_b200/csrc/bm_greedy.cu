@@ -430,8 +430,16 @@ constexpr int kGreedyCluster = 16;
 //   n = 4,000, E = 2.4e5 (2.9e7)    26.6 / 30.1      E = 4e5 (8e7)      35.8 / 33.6
 //   n = 3,000, E = 2.5e5 (4.2e7)    20.3 / 22.6      E = 4e5 (1.1e8)    25.7 / 25.8
 //   n = 6,000, E = 3e5 (3e7)        41.5 / 45.1
+//   n = 6,500, E = 1.6e5 (8.1e6)    39.1 / 48.1      E = 3.6e5 (3.9e7)  49.7 / 49.2
+//   n = 7,600, E = 3e5 (2.4e7)      55.0 / 57.2      E = 4.2e5 (4.6e7)  64.9 / 60.7
 //   n = 8,192, E = 1.2e5 (3.5e6)    43.0 / 57.5      E = 5e5 (6.1e7)    71.0 / 65.5
-constexpr double kGreedyClusterWork = 4.8e7;
+//              E = 3.3e5 (2.6e7)    60.5 / 61.1
+// and with more candidates in a slice than a CTA has threads, which walks them twice:
+//   n = 8,300, E = 2.1e5 (1e7)      59.4 / 59.9      E = 2.5e5 (1.5e7)  61.9 / 60.2
+//   n = 9,000, E = 2.2e5 (1.1e7)    65.2 / 67.4      E = 3.6e5 (2.9e7)  73.0 / 67.9
+inline double greedy_cluster_work(int n) {
+    return n > kGreedyCluster * kGreedyThreads ? 1.0e7 : std::min(4.8e7, 2.0e11 / n);
+}
 
 __host__ __device__ inline int greedy_cluster_slice(int n) { return (n + kGreedyCluster - 1) / kGreedyCluster; }
 __host__ __device__ inline size_t greedy_cluster_smem(int n) {
@@ -930,7 +938,7 @@ extern "C" bm_status bm_greedy_match(int32_t n, int64_t e1, const int32_t* src1,
     cfg.numAttrs = 1;
     int clusters = 0;
     const bool cluster =
-        2.0 * (double)e1 * (double)mk / n <= kGreedyClusterWork &&
+        2.0 * (double)e1 * (double)mk / n <= greedy_cluster_work(n) &&
         cfg.dynamicSmemBytes + 12288 <= (size_t)optin &&
         allow_smem<k_greedy_cluster>(cfg.dynamicSmemBytes) == cudaSuccess &&
         cudaFuncSetAttribute(k_greedy_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
