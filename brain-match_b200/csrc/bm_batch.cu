@@ -238,8 +238,8 @@ k_b_commit(const DevView<W16>* __restrict__ views, const BatchInst* __restrict__
 // shared-memory row that starts at -S[b][b], takes its maximum, and neither
 // writes n^2 profits nor reads them back in tiles.  Every min term is computed
 // twice (for a and for b), which is why only sparse instances take this path
-// (direct_instance).  64 instances of 500 to 8,000 vertices, 20 edges each, three
-// sweeps: 23.9 -> 11.9 ms, with the set commit's wider steps.
+// (direct_instance).  A call of three sweeps of 64 instances of 500 to 8,000
+// vertices, 20 edges each: 23.9 -> 15.9 ms, the set commit's wider steps included.
 constexpr double kDirectTerms = 1.5;   // most terms per pair of vertices (direct_instance)
 constexpr int kDirectRows = 4;    // rows of a task per accumulator
 constexpr int kDirectLong = 64;   // longer lists take a whole warp instead of 8 lanes,
@@ -639,8 +639,8 @@ __global__ void __launch_bounds__(kBThreads, 1) k_b_sweep(BSweepArgs<W16> a) {
                     b_group_sync(grp);
                     if (gtid == 0) atomicAdd(&rows_done[i], end - local * rpt);
                 } else if (ways == 1) {   // profit row `local` of instance i by the whole group
-                            profit_row_on<W16, 256>(g, local, acc, reinterpret_cast<int2*>(s_head[2 * grp]), &s_nlong[4 * grp], nullptr, 0,
-                                            nullptr, nullptr, [grp] { b_group_sync(grp); });
+                    profit_row_on<W16, 256>(g, local, acc, reinterpret_cast<int2*>(s_head[2 * grp]), &s_nlong[4 * grp],
+                                            nullptr, 0, nullptr, nullptr, [grp] { b_group_sync(grp); });
                     __threadfence();     // every thread's part of the row is visible before it counts
                     b_group_sync(grp);
                     if (gtid == 0) atomicAdd(&rows_done[i], 1);

@@ -885,12 +885,7 @@ static bm_status stage_commit(bm_ctx* ctx, const bm_sweep_opts* o) {
     const int max_scan = o ? o->max_candidates : 0;
     const int max_verify = o ? o->max_verify : -1;
     const int lim = (max_scan > 0 && max_scan < n) ? max_scan : n;
-    const size_t smem = commit_group_smem(n);
-    if (smem + 4096 > ctx->smem_optin) {
-        set_err(ctx, "set commit needs %zu bytes of shared memory for n=%d (limit %zu): n too large for a sweep",
-                smem, n, ctx->smem_optin);
-        return BM_E_INPUT;
-    }
+    if (!sweep_takes(n, ctx->smem_optin)) { set_err(ctx, "n=%d is too large for a sweep", n); return BM_E_INPUT; }
     return launch_set_commit<W16, 2>(ctx, ctx->ckeys_sorted, nullptr, lim, max_verify, o ? o->commit_ctas : 0,
                                      take_stall(BM_STALL_COMMIT), true);
 }

@@ -895,10 +895,8 @@ static bm_status learned_impl(bm_ctx* ctx, bm_mlp* M, const bm_learned_opts* o, 
         }
         MK(cudaGetLastError());
         // exact set commit of the improving ones, in (delta desc, lo, hi) order
-        const size_t smem = commit_group_smem(n);
-        if (smem + 4096 > ctx->smem_optin) {
-            snprintf(M->err, sizeof M->err, "set commit needs %zu bytes of shared memory for n=%d: n too large",
-                     smem, n);
+        if (!sweep_takes(n, ctx->smem_optin)) {
+            snprintf(M->err, sizeof M->err, "n=%d is too large for a sweep", n);
             return BM_E_INPUT;
         }
         if ((r = launch_set_commit<W16, 2>(ctx, ck + top, nullptr, top, -1, 0, take_stall(BM_STALL_COMMIT)))) {

@@ -52,7 +52,6 @@ template <bool W16>
 __device__ int quad_delta_S(const DevView<W16>& g, const unsigned* __restrict__ adj, int words, const int* M,
                             const int* pm, int q) {
     typedef Ent<W16> EN;
-    const int n = g.n;
     int sg[4], pn[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) { sg[i] = kQuadPerm[q][i]; pn[i] = pm[sg[i]]; }
@@ -155,7 +154,6 @@ template <bool W16>
 __device__ void quad_best(const DevView<W16>& g, const unsigned* __restrict__ adj, int words, const int* M,
                           const int* pm, int& best_d, int& best_q) {
     typedef Ent<W16> EN;
-    const int n = g.n;
     best_d = 0;
     best_q = 0;
     int ie_ij[kQuadMaxInternal], ie_w[kQuadMaxInternal];  // (i << 2 | j), weight

@@ -439,4 +439,10 @@ __host__ __device__ inline size_t commit_group_smem(int n) {
     return (size_t)((n + 15) & ~15) + 6 * (size_t)((n + 8) & ~7);
 }
 
+// Whether a sweep takes n: what a batched instance's commit keeps in a CTA's
+// shared memory fits (n up to 32,615).  k_commit_sets needs less, and the 3-cycle
+// and 4-set rounds, which commit with it too, take every n; for sweeps the bound
+// stands because callers rely on the refusal.
+inline bool sweep_takes(int n, size_t smem_optin) { return commit_group_smem(n) + 4096 <= smem_optin; }
+
 }  // namespace bm

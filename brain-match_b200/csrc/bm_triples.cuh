@@ -80,7 +80,6 @@ template <bool W16>
 __device__ int triple_delta_S(const DevView<W16>& g, const unsigned* __restrict__ adj, int words,
                               int a, int b, int c, int rot) {
     typedef Ent<W16> EN;
-    const int n = g.n;
     const int M[3] = {a, b, c};
     int sig[3];
     if (rot == 0) { sig[0] = b; sig[1] = c; sig[2] = a; }

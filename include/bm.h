@@ -253,22 +253,25 @@ bm_status bm_measure_peaks(int32_t n, double* red_per_s, double* minadd_per_s);
 
 /*
  * Test hook for the timeout paths; no counterpart in the reference.
- * Every wait a kernel makes on another part of the GPU (an mbarrier that the
- * tensor cores or a copy complete, a cluster or grid barrier) is bounded:
- * when it runs out the kernel records an error word, waits (bounded) for its
- * own copies in flight, releases what it holds and returns, and the call
- * reports BM_E_TIMEOUT with the site in bm_last_error.  bm_test_stall(site)
- * makes the next launch at that site take one such wait that nothing
- * completes (CTA 0 skips an arrival, or waits for a barrier phase nothing
- * opens), with a short limit -- no fault, trap or endless loop.  One site at
- * a time, process-wide; 0 clears it.  After BM_E_TIMEOUT a context's matching
+ * Every wait that polls for another part of the GPU (an mbarrier that the
+ * tensor cores or a copy complete, a grid barrier, words exchanged between
+ * CTAs) is bounded: when it runs out the kernel records an error word, waits
+ * (bounded) for its own copies in flight, releases what it holds and returns,
+ * and the call reports BM_E_TIMEOUT with the site in bm_last_error.  The
+ * hardware barriers of a thread block or cluster, whose CTAs run together and
+ * all reach them, are not polled and have no limit.  bm_test_stall(site)
+ * makes the next launch at that site take one polled wait that nothing
+ * completes (a CTA skips an arrival or a word, or waits for a barrier phase
+ * nothing opens), with a short limit -- no fault, trap or endless loop.  One
+ * site at a time, process-wide; 0 clears it.  After BM_E_TIMEOUT a context's matching
  * may be partly committed: set a matching again before the next call.
  */
 #define BM_STALL_HUB_GEMM   1   /* bm_sweep: tensor-core hub GEMM          */
 #define BM_STALL_COMMIT     2   /* bm_sweep, bm_triple_round, bm_quad_round,
                                    bm_learned_sweep: set commit            */
 #define BM_STALL_COMBINE    3   /* bm_sweep: TMA-fed pair combine          */
-#define BM_STALL_GREEDY     4   /* bm_greedy_match: grid barrier           */
+#define BM_STALL_GREEDY     4   /* bm_greedy_match: grid barrier (the call
+                                   takes the grid path at any size)        */
 #define BM_STALL_MLP_GEMM   5   /* bm_mlp_*: tensor-core GEMM              */
 #define BM_STALL_BATCH      6   /* bm_batch_sweeps: persistent sweep grid barrier */
 #define BM_STALL_RANK       7   /* bm_learned_sweep, bm_mlp_rank_pairs: ranking */
