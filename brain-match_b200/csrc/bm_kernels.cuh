@@ -94,7 +94,7 @@ __device__ __forceinline__ int imin(int a, int b) { return a < b ? a : b; }
 // ---------------------------------------------------------------------------
 // Relabel list ids through a map (p for G1 lists, pinv for G2 lists), all lists
 // in one launch: 16 bytes per thread, the lists end to end.  Five launches of
-// 4-byte entries took 48 us at E = 5e6, this one 26 (160 MB).  Thread 0 also
+// 4-byte entries took 48 us at E = 5e6, this one 33 (160 MB).  Thread 0 also
 // clears the rebuild's counters.
 constexpr int kRelabelLists = 5;
 template <bool W16> struct RelabelLists {

@@ -34,8 +34,8 @@ struct GemmOut {
 // CTA (32 CTAs per batch instead of 8 with whole rows), the four K-chunks of a
 // layer all in flight, and the passes that followed the GEMMs -- ReLU' and
 // bias gradient, transposes for the weight gradients -- done in the epilogue
-// from registers (a GEMM 21 -> 10 us; ReLU' 17 us and six transposes of 3.4 us
-// gone; a step of 1,024 rows 178 -> 74 us of kernels).
+// from registers (a GEMM 21 -> 9 us, one of the weight gradients 12; ReLU' 17 us
+// and six transposes of 3.6 us gone; a step of 1,024 rows 178 -> 71 us of kernels).
 constexpr int kMlpStages = 4;
 template <int BN>
 static __global__ void __launch_bounds__(kGemmThreads, 1)
