@@ -84,15 +84,16 @@ __global__ void k_b_relabel(const DevView<W16>* __restrict__ views, const long l
 }
 
 // Matchings of the instances in and out of one staging buffer: p, then pinv, of
-// instance b from 2 (row_base[b] + b).  64 instances took 4 ms per set and get
-// as copies, scores and waits of their own (8 sweeps of the smallest).
+// instance b from 2 (row_base[b] + b).  Instances along x: the other dimensions
+// end at 65,535.  64 instances took 4 ms per set and get as copies, scores and
+// waits of their own (8 sweeps of the smallest).
 template <bool W16>
 __global__ void k_b_maps_in(const DevView<W16>* __restrict__ views, const int* __restrict__ row_base,
                             const int* __restrict__ stage) {
-    const int b = blockIdx.y;
+    const int b = blockIdx.x;
     const DevView<W16>& g = views[b];
     const int* s = stage + 2 * ((size_t)row_base[b] + b);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= g.n; i += gridDim.x * blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i <= g.n; i += gridDim.y * blockDim.x) {
         g.p[i] = s[i];
         g.pinv[i] = s[g.n + 1 + i];
     }
@@ -100,15 +101,15 @@ __global__ void k_b_maps_in(const DevView<W16>* __restrict__ views, const int* _
 template <bool W16>
 __global__ void k_b_maps_out(const DevView<W16>* __restrict__ views, const int* __restrict__ row_base,
                              int* __restrict__ stage) {
-    const int b = blockIdx.y;
+    const int b = blockIdx.x;
     const DevView<W16>& g = views[b];
     int* s = stage + 2 * ((size_t)row_base[b] + b);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= g.n; i += gridDim.x * blockDim.x) s[i] = g.p[i];
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i <= g.n; i += gridDim.y * blockDim.x) s[i] = g.p[i];
 }
 template <bool W16>
 __global__ void k_b_score(const DevView<W16>* __restrict__ views, const long long* __restrict__ e1,
                           unsigned long long* __restrict__ out) {
-    add_score<W16>(views[blockIdx.y], (int)e1[blockIdx.y], out + blockIdx.y);
+    add_score<W16>(views[blockIdx.x], (int)e1[blockIdx.x], out + blockIdx.x, blockIdx.y, gridDim.y);
 }
 
 template <bool W16>
@@ -1051,12 +1052,12 @@ extern "C" bm_status bm_batch_create(bm_batch** out, int32_t count, const int32_
 template <bool W16>
 static bm_status batch_maps_in(bm_batch* B, int k, size_t ints) {
     const DevView<W16>* views = (const DevView<W16>*)B->views;
-    const dim3 grid((B->max_n + 1024) / 1024, k);
+    const dim3 grid(k, (B->max_n + 1024) / 1024);
     BK(cudaMemcpyAsync(B->stage, B->hstage, ints * sizeof(int), cudaMemcpyHostToDevice, B->st));
     BK(cudaMemsetAsync(B->scores, 0, k * sizeof(unsigned long long), B->st));
     k_b_maps_in<W16><<<grid, 256, 0, B->st>>>(views, B->row_base, B->stage);
     BK(cudaGetLastError());
-    k_b_score<W16><<<dim3(16, k), 256, 0, B->st>>>(views, B->e1, B->scores);
+    k_b_score<W16><<<dim3(k, 16), 256, 0, B->st>>>(views, B->e1, B->scores);
     BK(cudaGetLastError());
     BK(cudaMemcpyAsync(B->hscores, B->scores, k * sizeof(unsigned long long), cudaMemcpyDeviceToHost, B->st));
     BK(cudaStreamSynchronize(B->st));
@@ -1099,7 +1100,7 @@ extern "C" bm_status bm_batch_get_mappings(bm_batch* B, int32_t* const* maps) {
     if (B->count > 1)
         for (; k < B->count && B->ctx[k]->mapped && maps[k]; k++) at += 2 * ((size_t)B->ctx[k]->n + 1);
     if (k) {
-        const dim3 grid((B->max_n + 1024) / 1024, k);
+        const dim3 grid(k, (B->max_n + 1024) / 1024);
         if (B->w16) k_b_maps_out<true><<<grid, 256, 0, B->st>>>((const DevView<true>*)B->views, B->row_base, B->stage);
         else k_b_maps_out<false><<<grid, 256, 0, B->st>>>((const DevView<false>*)B->views, B->row_base, B->stage);
         BK(cudaGetLastError());

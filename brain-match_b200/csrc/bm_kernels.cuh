@@ -615,11 +615,12 @@ __device__ __forceinline__ int score_run(int m, int nwarps) {
     return min(kScoreRun, (m / nwarps + 32) & ~31);
 }
 template <bool W16>
-__device__ __forceinline__ void add_score(const DevView<W16>& g, int m, unsigned long long* __restrict__ out) {
+__device__ __forceinline__ void add_score(const DevView<W16>& g, int m, unsigned long long* __restrict__ out, int block,
+                                          int blocks) {
     typedef Ent<W16> EN;
     const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int warp = (block * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (blocks * blockDim.x) >> 5;
     long long s = 0;
     const int run = score_run(m, nwarps);
     for (long long r0 = (long long)warp * run; r0 < m; r0 += (long long)nwarps * run) {
@@ -635,13 +636,15 @@ __device__ __forceinline__ void add_score(const DevView<W16>& g, int m, unsigned
         }
     }
     const int loops = g.offs[g.n];   // G1 self-loops
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < loops; i += gridDim.x * blockDim.x)
+    for (int i = block * blockDim.x + threadIdx.x; i < loops; i += blocks * blockDim.x)
         s += imin(g.selfw[i], g.w2d(g.p[row_of(g.offs, g.n, i)]));
     for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0 && s) atomicAdd(out, (unsigned long long)s);
 }
 template <bool W16>
-__global__ void k_score(DevView<W16> g, int m, unsigned long long* __restrict__ out) { add_score<W16>(g, m, out); }
+__global__ void k_score(DevView<W16> g, int m, unsigned long long* __restrict__ out) {
+    add_score<W16>(g, m, out, blockIdx.x, gridDim.x);
+}
 
 // C[a] += what vertex a's G1 edges and self-loops earn now; one pass over the
 // G1 entries, dealt as in k_score (C zero before).  Most terms of an early
@@ -672,6 +675,5 @@ __global__ void k_contrib(DevView<W16> g, int m, int* __restrict__ C) {
         if (t) atomicAdd(&C[a], t);
     }
 }
-
 
 }  // namespace bm
