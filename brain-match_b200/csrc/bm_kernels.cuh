@@ -625,11 +625,11 @@ __device__ __forceinline__ void add_score(const DevView<W16>& g, int m, unsigned
     const int run = score_run(m, nwarps);
     for (long long r0 = (long long)warp * run; r0 < m; r0 += (long long)nwarps * run) {
         int a = row_of_warp(g.off1o, g.n, (int)r0, lane), end = g.off1o[a + 1];
-        const int r1 = (int)min((long long)m, r0 + run);
+        const int len = (int)min((long long)run, m - r0);   // lists of up to 2^31 - 1 entries
 #pragma unroll
         for (int u = 0; u < kScoreRun / 32; u++) {
+            if (32 * u + lane >= len) continue;
             const int i = (int)r0 + 32 * u + lane;
-            if (i >= r1) continue;
             while (i >= end) end = g.off1o[++a + 1];
             const typename EN::T e = g.ent1o[i];
             s += imin(EN::w(e), g.w2(g.p[a], g.p[EN::id(e)]));
@@ -658,11 +658,11 @@ __global__ void k_contrib(DevView<W16> g, int m, int* __restrict__ C) {
     const int run = score_run(m, nwarps);
     for (long long r0 = (long long)warp * run; r0 < m; r0 += (long long)nwarps * run) {
         int a = row_of_warp(g.off1o, g.n, (int)r0, lane), end = g.off1o[a + 1];
-        const int r1 = (int)min((long long)m, r0 + run);
+        const int len = (int)min((long long)run, m - r0);   // lists of up to 2^31 - 1 entries
 #pragma unroll
         for (int u = 0; u < kScoreRun / 32; u++) {
+            if (32 * u + lane >= len) continue;
             const int i = (int)r0 + 32 * u + lane;
-            if (i >= r1) continue;
             while (i >= end) end = g.off1o[++a + 1];
             const typename EN::T e = g.ent1o[i];
             const int v = EN::id(e), t = imin(EN::w(e), g.w2(g.p[a], g.p[v]));
