@@ -540,15 +540,16 @@ static cudaError_t sort_keys(bm_ctx* ctx, const int* count) {
 // of 18 ms of creation at n = 3,001 and 6 of 130 at n = 8,192 / E = 1e6.)
 template <bool W16>
 static bm_status ensure_order(bm_ctx* ctx) {
-    if (ctx->order) return BM_OK;
+    if (ctx->order_made) return BM_OK;
     const int n = ctx->n;
-    CK(dalloc(ctx, &ctx->order, n * sizeof(int)));
+    if (!ctx->order) CK(dalloc(ctx, &ctx->order, n * sizeof(int)));
     k_row_keys<W16><<<(n + 7) / 8, 256, 0, ctx->st>>>(view<W16>(ctx), ctx->nh ? ctx->is_hub : nullptr,
                                                       (float)ctx->e2 / n, ctx->ckeys, ctx->small + 1);
     CK(cudaGetLastError());
     CK(sort_keys(ctx, ctx->small + 1));
     k_row_order<<<(n + 255) / 256, 256, 0, ctx->st>>>(ctx->ckeys_sorted, n, ctx->order);
     CK(cudaGetLastError());
+    ctx->order_made = true;   // a call that fails before leaves it to the next
     return BM_OK;
 }
 

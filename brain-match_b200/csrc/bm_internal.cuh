@@ -64,6 +64,7 @@ struct bm_ctx {
     unsigned long long* rowbest = nullptr;
     unsigned long long *ckeys = nullptr, *ckeys_sorted = nullptr;
     int* order = nullptr;          // profit rows, heaviest first (made with the first profit matrix)
+    bool order_made = false;
     void* cub_tmp = nullptr;
     size_t cub_bytes = 0;
     int* small = nullptr;          // [0]=row counter [1]=ncand [2]=best delta
